@@ -404,6 +404,9 @@ pg_status pg_test_bounded_wait(int* err_bits, int* left, float* ms);
 /* test support: out2[2k] = the kernels' division-free x[k] / 1.5, out2[2k+1] =
    the IEEE quotient, for n host values.  Uses the GPU. */
 pg_status pg_test_div_1p5(const double* x, long long n, double* out2);
+/* test support: the kernels' reciprocal and reciprocal square root of x[0..n) (positive
+   normal doubles), interleaved in out2[2n]. */
+pg_status pg_test_inv_rsq(const double* x, long long n, double* out2);
 /* test support: one step with host t and dt, the whole cell array (ghosts
    included) after each pass into out[5][zarr][yarr][xarr]: kick1, sweep_x,
    sweep_y, sweep_z, kick2 with the damping.  Blocking. */

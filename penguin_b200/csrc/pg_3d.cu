@@ -241,21 +241,19 @@ __global__ void __launch_bounds__(S3_THREADS, 4)
                     if (v.geomz == 5) w[m] *= radp * v.sinz[sm];
                 }
             }
-            const double cs0 = sqrt(gam * p[2] / r[2]);
-            const double flat = flatten(1.0 / cs0, p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
+            const double cs0 = sound_speed(gam, r[2], p[2]);
+            const double flat = flatten(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
             const int sc_ = min(s, arr - 1);
             const double* wt = (DIR == 0 ? d.wx : (DIR == 1 ? d.wy : v.wz)) + 6 * sc_;
             const double idx = (DIR == 0 ? d.idx_x : (DIR == 1 ? d.idx_y : v.idx_z))[sc_];
-            const double* fa = DIR == 0 ? d.xa : (DIR == 1 ? d.ya : v.za);
             const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], flat);
             const Par P = recon(wt, p[0], p[1], p[2], p[3], p[4], flat);
             const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], flat);
             const Par V = recon(wt, vv[0], vv[1], vv[2], vv[3], vv[4], flat);
             const Par W = recon(wt, w[0], w[1], w[2], w[3], w[4], flat);
-            const double xl = fa[sc_], xr = fa[sc_ + 1];
-            const double sdt = DIR == 0 ? dt : dt / radp;  // set_state receives dt/rad (riemann.cu:111)
-            const Half a = state_at_left_edge(gam, xl, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, W);
-            const Half b = state_at_right_edge(gam, xl, xr, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, W);
+            const double sdt = DIR == 0 ? dt : dt * inv(radp);  // set_state receives dt/rad (riemann.cu:111)
+            const Half a = state_at_left_edge(gam, sdt * idx, cs0, r[2], p[2], u[2], R, P, U, V, W);
+            const Half b = state_at_right_edge(gam, sdt * idx, cs0, r[2], p[2], u[2], R, P, U, V, W);
             st[0 * S3_NST + it] = a.r;
             st[1 * S3_NST + it] = a.p;
             st[2 * S3_NST + it] = a.u;

@@ -182,25 +182,23 @@ __device__ __forceinline__ void edge_states(const Args& a, const Seed& s, int c,
             v[k] = C.u;  // the reference's w slot carries v_r in the azimuthal sweep (w = 0 in 2D)
         }
     }
-    const T cs0 = sqrt(d.gam * p[2] / r[2]);
-    const T flat = flatten<T>(1.0 / cs0, p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
+    const T cs0 = sound_speed(d.gam, r[2], p[2]);
+    const T flat = flatten<T>(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
     const double* wt = ((DIR == 0) ? d.wx : d.wy) + 6 * c;
-    const double* fa = (DIR == 0) ? d.xa : d.ya;
     const double idx = ((DIR == 0) ? d.idx_x : d.idx_y)[c];
     const ParT<T> R = recon<T>(wt, r[0], r[1], r[2], r[3], r[4], flat);
     const ParT<T> P = recon<T>(wt, p[0], p[1], p[2], p[3], p[4], flat);
     const ParT<T> U = recon<T>(wt, u[0], u[1], u[2], u[3], u[4], flat);
     const ParT<T> V = recon<T>(wt, v[0], v[1], v[2], v[3], v[4], flat);
     const ParT<T> Z{T(0.0), T(0.0), T(0.0)};
-    const double xl = fa[c], xr = fa[c + 1];
     const double sdt = (DIR == 0) ? a.dt : a.dt * irad_q;
     // DIR 0: V is r v_phi (the v slot); DIR 1: V is v_r (the w slot), the v slot is w = 0
     if (DIR == 0) {
-        left = state_at_left_edge<T>(d.gam, xl, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, Z);
-        right = state_at_right_edge<T>(d.gam, xl, xr, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, Z);
+        left = state_at_left_edge<T>(d.gam, T(sdt * idx), cs0, r[2], p[2], u[2], R, P, U, V, Z);
+        right = state_at_right_edge<T>(d.gam, T(sdt * idx), cs0, r[2], p[2], u[2], R, P, U, V, Z);
     } else {
-        left = state_at_left_edge<T>(d.gam, xl, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, Z, V);
-        right = state_at_right_edge<T>(d.gam, xl, xr, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, Z, V);
+        left = state_at_left_edge<T>(d.gam, T(sdt * idx), cs0, r[2], p[2], u[2], R, P, U, Z, V);
+        right = state_at_right_edge<T>(d.gam, T(sdt * idx), cs0, r[2], p[2], u[2], R, P, U, Z, V);
     }
 }
 

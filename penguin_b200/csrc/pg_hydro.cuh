@@ -15,33 +15,71 @@
 namespace pg {
 
 template <class T>
+constexpr bool is_double = false;
+template <>
+inline constexpr bool is_double<double> = true;
+
+template <class T>
 struct ParT {
     T sL, a, sR;
 };
 using Par = ParT<double>;
 
+// The smaller / larger of two values by one comparison (no NaN rules; a NaN in
+// the first operand stays).
+template <class T>
+__device__ __forceinline__ T lesser(T a, T b) { return (b < a) ? b : a; }
+template <class T>
+__device__ __forceinline__ T larger(T a, T b) { return (b > a) ? b : a; }
+
+// Reciprocal (of either sign) and reciprocal square root of a normal double to about an
+// ulp: the hardware's approximation (rcp/rsqrt.approx.ftz.f64, which reads and
+// returns the upper 32 bits of a double, so |e| < 2^-19) and one third-order step
+// of Newton's iteration (Householder, "The Numerical Treatment of a Single
+// Nonlinear Equation", 1970): with e = 1 - x y, y (1 + e + e^2) is off by e^3, and
+// with e = 1 - x y^2, y (1 + e/2 + 3 e^2/8) by 5 e^3 / 16.  Three and five
+// FP64 instructions and no branch, where the IEEE quotient and root take about
+// ten each and a slow path: the sweeps are bound by this arithmetic's latency.
+__device__ __forceinline__ double inv(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsq(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+template <class T>
+__device__ __forceinline__ T inv(const T& x) { return 1.0 / x; }
+template <class T>
+__device__ __forceinline__ T rsq(const T& x) { return 1.0 / sqrt(x); }
+
 // src/solver/recon/recon.cu:216-378 (slopes) + src/solver/recon/PPM.cu:64-91 (flattening,
 // monotonicity).  w: {wL0,wL1,wL2, wR0,wR1,wR2} with sL = wL . (a[i-1]-a[i-2], a[i]-a[i-1],
-// a[i+1]-a[i]) and sR = wR . (a[i]-a[i-1], a[i+1]-a[i], a[i+2]-a[i+1]).
+// a[i+1]-a[i]) and sR = wR . (a[i]-a[i-1], a[i+1]-a[i], a[i+2]-a[i+1]).  Each slope takes
+// the size min(|s|, |d|) and the sign of its neighbour difference d; both vanish at an
+// extremum.  The reference's monotonicity test (sR + sL)^2 < 3 (sR + sL) (sL - sR) is, for
+// slopes of one sign, 2 |sR| < |sL|, where it sets sL = 2 sR: the sizes are limited to
+// twice each other.
 template <class T>
 __device__ __forceinline__ ParT<T> recon(const double* __restrict__ w, T am2, T am1, T a0, T ap1, T ap2, T flat) {
     const T d0 = am1 - am2, d1 = a0 - am1, d2 = ap1 - a0, d3 = ap2 - ap1;
-    T sL = w[0] * d0 + w[1] * d1 + w[2] * d2;
-    T sR = w[3] * d1 + w[4] * d2 + w[5] * d3;
-    sL = copysign(fmin(fabs(sL), fabs(d1)), d1);
-    sR = copysign(fmin(fabs(sR), fabs(d2)), d2);
-    if (sR * sL <= 0.0) {
-        sL = 0.0;
-        sR = 0.0;
+    const T sL = w[0] * d0 + w[1] * d1 + w[2] * d2;
+    const T sR = w[3] * d1 + w[4] * d2 + w[5] * d3;
+    T l = lesser(fabs(sL), fabs(d1));
+    T r = lesser(fabs(sR), fabs(d2));
+    // a zero size makes both vanish below; for a derivative it has to be an exact zero here
+    bool zero = signbit(d1) != signbit(d2);
+    if constexpr (!is_double<T>) zero = zero || !(l > 0.0) || !(r > 0.0);
+    if (zero) {
+        l = 0.0;
+        r = 0.0;
     }
-    sR *= (1.0 - flat);
-    sL *= (1.0 - flat);
-    const T t3 = sR + sL;
-    const T t2 = t3 * t3;
-    const T t1 = t3 * 3.0 * (sL - sR);
-    if (t2 < t1) sL = 2.0 * sR;
-    else if (t2 < -t1) sR = 2.0 * sL;
-    return {sL, a0, sR};
+    const T k = 1.0 - flat;
+    return {copysign(lesser(l, 2.0 * r) * k, d1), a0, copysign(lesser(r, 2.0 * l) * k, d2)};
 }
 
 // Averages of the parabola over the fraction x of the cell touching its left /
@@ -49,31 +87,28 @@ __device__ __forceinline__ ParT<T> recon(const double* __restrict__ w, T am2, T 
 // g = 1 - x/1.5 are shared by every field averaged at the same x.
 template <class T>
 struct FracT {
-    T x, h, g;
+    T h, g;
 };
 using Frac = FracT<double>;
 // x / 1.5 correctly rounded without a division: with y = RN(1/1.5) = RN(2/3),
 // q = RN(x y) lies within an ulp of x / 1.5 and the remainder x - 1.5 q is
 // exact in one FMA, so RN(q + (x - 1.5 q) y) is the correctly rounded quotient
 // (Markstein, IBM J. Res. Dev. 34 (1990) 111-119); 2x/3 is never a midpoint of
-// two doubles.  Bit for bit the IEEE quotient the reference computes
-// (src/solver/recon/PPM.cu:100,111), three FP64 instructions.
-template <class T>
-__device__ __forceinline__ T div_1p5(T x) { return x / 1.5; }
-template <>
-__device__ __forceinline__ double div_1p5<double>(double x) {
+// two doubles.  Bit for bit the IEEE quotient x / 1.5.
+__device__ __forceinline__ double div_1p5(double x) {
     constexpr double y = 2.0 / 3.0;
     const double q = x * y;
     const double r = fma(-q, 1.5, x);
     return copysign(fma(r, y, q), x);  // the quotient of a positive divisor keeps x's sign (-0 / 1.5 = -0)
 }
+// of the swept fraction y of the cell at the edge (1 - x / 1.5 in one FMA: within
+// an ulp of 1 of the rounded quotient's)
 template <class T>
-__device__ __forceinline__ FracT<T> frac_left(T x) { return {x, x / 2.0, 1.0 - div_1p5(x)}; }
+__device__ __forceinline__ FracT<T> frac(T y) { return {0.5 * y, 1.0 - y * (2.0 / 3.0)}; }
 template <class T>
-__device__ __forceinline__ FracT<T> frac_right(T x) {
-    const T y = 1.0 - x;
-    return {y, y / 2.0, 1.0 - div_1p5(y)};
-}
+__device__ __forceinline__ FracT<T> frac_left(T x) { return frac(x); }
+template <class T>
+__device__ __forceinline__ FracT<T> frac_right(T x) { return frac<T>(1.0 - x); }
 template <class T>
 __device__ __forceinline__ T aveL(const FracT<T>& f, const ParT<T>& p) {
     const T a6 = 3.0 * (p.sL - p.sR);
@@ -92,27 +127,40 @@ __device__ __forceinline__ T aveR(const FracT<T>& f, const ParT<T>& p) {
 template <class T>
 __device__ __forceinline__ T lim01(T a) { return fmin(fmax(a, T(0.0)), T(1.0)); }  // solve.cu:14
 template <class T>
-__device__ __forceinline__ T exp_lim(T x) { return fmax(1.0 + x, T(1.0e-6)); }  // solve.cu:29
+__device__ __forceinline__ T exp_lim(T x) { return larger(1.0 + x, T(1.0e-6)); }  // solve.cu:29
+
+// sqrt(gam p / r) with one reciprocal root and no division
+template <class T>
+__device__ __forceinline__ T sound_speed(double gam, T r, T p) {
+    const T g = gam * p;
+    return g * rsq(g * r);
+}
+// the product is rounded on its own, so that every pass that forms the CFL rate
+// gets the same bits whatever it is added to
+__device__ __forceinline__ double sound_speed(double gam, double r, double p) {
+    const double g = gam * p;
+    return __dmul_rn(g, rsq(g * r));
+}
 
 // Shock flattening coefficient of the middle cell (src/solver/recon/PPM.cu:7-62).
 // The reference forms the Mach numbers (u0 - up1) / cs and (um1 - u0) / cs only
-// to test their signs; with cs > 0 those are the signs of the differences, so
-// the differences are tested (the quotient would differ only by underflowing a
-// difference below cs 2^-1074 to zero).  inv_cs (1 / cs) is not needed.
+// to test their signs, which are those of the differences.  Its steepness
+// |dp1 / dp2 - 1/2| - 1/4 of either side is (|dp1 - dp2 / 2| - |dp2| / 4) / |dp2|:
+// the numerators decide whether there is a shock and which side is steeper, so
+// one reciprocal is left, on cells that are flattened at all.
 template <class T>
-__device__ __forceinline__ T flatten(T inv_cs, T p0, T pm2, T pm1, T pp1, T pp2, T um1, T u0, T up1) {
-    (void)inv_cs;
+__device__ __forceinline__ T flatten(T p0, T pm2, T pm1, T pp1, T pp2, T um1, T u0, T up1) {
     const T dp1f = pp1 - p0, dp2f = pp2 - pm1;
     const T dp1b = p0 - pm1, dp2b = pp1 - pm2;
-    const T Mf = u0 - up1;
-    const T Mb = um1 - u0;
+    const T wf = fabs(dp2f), wb = fabs(dp2b);
+    const T nf = fabs(dp1f - 0.5 * dp2f) - 0.25 * wf;
+    const T nb = fabs(dp1b - 0.5 * dp2b) - 0.25 * wb;
     T f = 0.0;
-    if ((Mf > 0.0 || Mb > 0.0) && dp2f != 0.0 && dp2b != 0.0) {
-        T ddp = 10.0 * fmax(T(0.0), fabs(dp1f / dp2f - 0.5) - 0.25);
-        f = ddp;
-        ddp = 10.0 * fmax(T(0.0), fabs(dp1b / dp2b - 0.5) - 0.25);
-        f = fmax(f, ddp);
-        f = fmin(T(0.5), f * fmax(fabs(dp1f), fabs(dp1b)) / p0);
+    if ((u0 > up1 || um1 > u0) && wf > 0.0 && wb > 0.0 && (nf > 0.0 || nb > 0.0)) {
+        const bool back = nb * wf > nf * wb;
+        const T big = larger(fabs(dp1f), fabs(dp1b));
+        f = 10.0 * (back ? nb : nf) * big * inv((back ? wb : wf) * p0);
+        f = lesser(T(0.5), f);
     }
     return f;
 }
@@ -124,80 +172,46 @@ struct HalfT {
 using Half = HalfT<double>;
 
 // Interface state on the LEFT edge of a cell = the right state of the face
-// below it (src/solver/riemann/states.cu:151-206).  xl: left face, idx = 1/(xr-xl),
-// sdt: dt/rad, cs0 = sqrt(gam p/r) of the cell averages r0c, p0c, u0c.
+// below it (src/solver/riemann/states.cu:151-206).  sx = dt / (rad (xr - xl)): the
+// swept fraction per unit speed; cs0 = sqrt(gam p/r) of the cell averages r0c, p0c,
+// u0c.  The reference forms the traced positions xl + speed dt and takes xl off
+// again; the swept fraction comes directly from the speed, which only drops
+// that cancellation.  With s = (gam p r)^-1/2 every quotient of the trace is a
+// product: cs = gam p s, 1 / cs = r s, 1 / (r cs) = s.
 template <class T>
-__device__ __forceinline__ HalfT<T> state_at_left_edge(double gam, double xl, double idx, double sdt, T cs0, T r0c,
-                                                       T p0c, T u0c, const ParT<T>& R, const ParT<T>& Pp,
-                                                       const ParT<T>& U, const ParT<T>& V, const ParT<T>& W) {
-    const double hdt = 0.5 * sdt;
-    T tmp = fmin(u0c, T(0.0));
-    tmp = xl - tmp * sdt + cs0 * sdt;
-    FracT<T> q = frac_left(lim01((tmp - xl) * idx));
-    const T rmin = r0c * 1.0e-10, pmin = p0c * 1.0e-10;
-    const T ur = aveL(q, U);
-    const T dis = fmin(ur, T(0.0)) * sdt;
-    tmp = xl - dis;
-    q = frac_left(lim01((tmp - xl) * idx));
-    T r0 = aveL(q, R), p0 = aveL(q, Pp);
+__device__ __forceinline__ HalfT<T> state_at_left_edge(double gam, T sx, T cs0, T r0c, T p0c, T u0c, const ParT<T>& R,
+                                                       const ParT<T>& Pp, const ParT<T>& U, const ParT<T>& V,
+                                                       const ParT<T>& W) {
+    const T one = 1.0, zero = 0.0;
+    FracT<T> q = frac(lesser((cs0 - lesser(u0c, zero)) * sx, one));
+    const T m = lesser(aveL(q, U), zero);
+    q = frac(lesser(-m * sx, one));
+    const T r0 = larger(aveL(q, R), r0c * 1.0e-10), p0 = larger(aveL(q, Pp), p0c * 1.0e-10);
     const T u0 = aveL(q, U);
-    r0 = fmax(r0, rmin);
-    p0 = fmax(p0, pmin);
-    const T ir0 = 1.0 / r0;
-    const T cs = sqrt(gam * p0 * ir0);
-    tmp = xl - dis + cs * sdt;
-    q = frac_left(lim01((tmp - xl) * idx));
-    T u_ = aveL(q, U), p_ = aveL(q, Pp);
-    const T k = 2.0 / (cs * sdt);
-    u_ = (u_ - u0) * k;
-    p_ = (p_ - p0) * k;
-    u_ *= -hdt;
-    p_ *= -hdt;
-    HalfT<T> s;
-    s.r = r0 * exp_lim(u_);
-    s.p = p0 * exp_lim(gam * u_);
-    s.u = u0 + p_ * ir0 + 0.0;
-    s.v = aveL(q, V);
-    s.w = aveL(q, W);
-    return s;
+    const T g = gam * p0;
+    const T s = rsq(g * r0);
+    q = frac(lesser((g * s - m) * sx, one));
+    const T du = (u0 - aveL(q, U)) * (r0 * s), dp = aveL(q, Pp) - p0;
+    return {r0 * exp_lim(du), p0 * exp_lim(gam * du), u0 - dp * s, aveL(q, V), aveL(q, W)};
 }
 
 // Interface state on the RIGHT edge of a cell = the left state of the face
 // above it (src/solver/riemann/states.cu:210-264).
 template <class T>
-__device__ __forceinline__ HalfT<T> state_at_right_edge(double gam, double xl, double xr, double idx, double sdt, T cs0,
-                                                        T r0c, T p0c, T u0c, const ParT<T>& R, const ParT<T>& Pp,
-                                                        const ParT<T>& U, const ParT<T>& V, const ParT<T>& W) {
-    const double hdt = 0.5 * sdt;
-    T tmp = fmax(u0c, T(0.0));
-    tmp = xr - tmp * sdt - cs0 * sdt;
-    FracT<T> q = frac_right(lim01((tmp - xl) * idx));
-    const T rmin = r0c * 1.0e-10, pmin = p0c * 1.0e-10;
-    const T ul = aveR(q, U);
-    const T dis = fmax(ul, T(0.0)) * sdt;
-    tmp = xr - dis;
-    q = frac_right(lim01((tmp - xl) * idx));
-    T r0 = aveR(q, R), p0 = aveR(q, Pp);
+__device__ __forceinline__ HalfT<T> state_at_right_edge(double gam, T sx, T cs0, T r0c, T p0c, T u0c,
+                                                        const ParT<T>& R, const ParT<T>& Pp, const ParT<T>& U,
+                                                        const ParT<T>& V, const ParT<T>& W) {
+    const T one = 1.0, zero = 0.0;
+    FracT<T> q = frac(lesser((cs0 + larger(u0c, zero)) * sx, one));
+    const T m = larger(aveR(q, U), zero);
+    q = frac(lesser(m * sx, one));
+    const T r0 = larger(aveR(q, R), r0c * 1.0e-10), p0 = larger(aveR(q, Pp), p0c * 1.0e-10);
     const T u0 = aveR(q, U);
-    r0 = fmax(r0, rmin);
-    p0 = fmax(p0, pmin);
-    const T ir0 = 1.0 / r0;
-    const T cs = sqrt(gam * p0 * ir0);
-    tmp = xr - dis - cs * sdt;
-    q = frac_right(lim01((tmp - xl) * idx));
-    T u_ = aveR(q, U), p_ = aveR(q, Pp);
-    const T k = 2.0 / (cs * sdt);
-    u_ = (u0 - u_) * k;
-    p_ = (p0 - p_) * k;
-    u_ *= -hdt;
-    p_ *= -hdt;
-    HalfT<T> s;
-    s.r = r0 * exp_lim(u_);
-    s.p = p0 * exp_lim(gam * u_);
-    s.u = u0 + p_ * ir0 + 0.0;
-    s.v = aveR(q, V);
-    s.w = aveR(q, W);
-    return s;
+    const T g = gam * p0;
+    const T s = rsq(g * r0);
+    q = frac(lesser((g * s + m) * sx, one));
+    const T du = (aveR(q, U) - u0) * (r0 * s), dp = p0 - aveR(q, Pp);
+    return {r0 * exp_lim(du), p0 * exp_lim(gam * du), u0 - dp * s, aveR(q, V), aveR(q, W)};
 }
 
 // src/EOS/EOS.cu:4-18 (EOS 0: isothermal, 2: ideal gas; ie: internal_e_flag)
@@ -224,19 +238,17 @@ using Flux = FluxT<double>;
 // candidate is formed.
 template <class T>
 __device__ __forceinline__ FluxT<T> hllc(int eos, int ie, double gam, const HalfT<T>& L, const HalfT<T>& R) {
-    const T cl = sqrt(gam * L.p / L.r);
-    const T cr = sqrt(gam * R.p / R.r);
-    const T c_ = 0.5 * (cr + cl);
-    const T p_ = 0.5 * (R.p + L.p);
-    const T pm = p_ * exp_lim(0.5 * gam * (L.u - R.u) / c_);
-    const T srl = sqrt(L.r), srr = sqrt(R.r);
-    const T is = 1.0 / (srl + srr);
-    const T u_ = (srl * L.u + srr * R.u) * is;
-    const T n2 = 0.5 * srl * srr * (is * is);
-    const T cc = sqrt((cl * cl * srl + cr * cr * srr) * is + n2 * (R.u - L.u) * (R.u - L.u));
+    const T cl = sound_speed(gam, L.r, L.p), cr = sound_speed(gam, R.r, R.p);
+    const T ic = inv(cl + cr);
+    const T pm = 0.5 * (R.p + L.p) * exp_lim(gam * (L.u - R.u) * ic);
+    // Roe's averages weighted with the roots of the densities, through their ratio
+    const T q = R.r * rsq(L.r * R.r), iq = inv(1.0 + q);
+    const T u_ = (L.u + q * R.u) * iq, du = R.u - L.u;
+    const T c2 = (cl * cl + cr * cr * q) * iq + 0.5 * q * (iq * iq) * (du * du);
+    const T cc = c2 * rsq(c2);
     const T sl = u_ - cc, sr = u_ + cc;
-    T sm = (L.r * L.u * cl + R.r * R.u * cr) / (L.r * cl + R.r * cr);
-    sm += (L.p - R.p) / ((L.r + R.r) * (0.5 * (cl + cr)));
+    const T ml = L.r * cl, mr = R.r * cr;
+    const T sm = (ml * L.u + mr * R.u) * inv(ml + mr) + 2.0 * (L.p - R.p) * (inv(L.r + R.r) * ic);
 
     // side of every upwinded quantity: left iff sl >= 0, or sr >= 0 and sm >= 0
     const bool left = (signbit(sl) == 0) || (signbit(sr) == 0 && signbit(sm) == 0);
@@ -248,10 +260,10 @@ __device__ __forceinline__ FluxT<T> hllc(int eos, int ie, double gam, const Half
         F.uprs = (ie == 0) ? S.u * S.p : S.u;
     } else {  // star region on the side of the contact
         const T s_ = left ? sl : sr;
-        const T inv = 1.0 / (s_ - sm);
-        F.r = sm * S.r * (s_ - S.u) * inv;
-        F.pres = (s_ * pm - sm * S.p) * inv;
-        if (ie == 0) F.uprs = sm * (s_ * pm - S.u * S.p) * inv;
+        const T is = inv(s_ - sm);
+        F.r = sm * S.r * (s_ - S.u) * is;
+        F.pres = (s_ * pm - sm * S.p) * is;
+        if (ie == 0) F.uprs = sm * (s_ * pm - S.u * S.p) * is;
         else F.uprs = sm * (s_ * pm - S.u * S.p) / (s_ * pm - sm * S.p);
     }
     F.u = S.u * F.r;
@@ -299,7 +311,9 @@ __device__ __forceinline__ void viscous(const double* __restrict__ X, const doub
 
 // Conservative update with floors (src/solver/sweeps.cu:218-261).  cs2: get_cs2
 // at the cell.  For the isothermal EOS the energy slot is dead (it is
-// overwritten by cs2 r), so it is not formed.
+// overwritten by cs2 r), so it is not formed.  ISO: 2D isothermal, whose zero
+// z-velocity stays as it is.
+template <bool ISO = false>
 __device__ __forceinline__ Cell update_cell(int eos, int ie, double gam, double cs2, Cell Q, const Cell& D,
                                             int* floor_hits) {
     const double r_min = fmax(Q.r * 1.0e-10, SMALLR);
@@ -311,16 +325,18 @@ __device__ __forceinline__ Cell update_cell(int eos, int ie, double gam, double 
     }
     Q.u *= Q.r;
     Q.v *= Q.r;
-    Q.w *= Q.r;
+    if (!ISO) {
+        Q.w *= Q.r;
+        Q.w += D.w;
+        Q.p += D.p;
+    }
     Q.r += D.r;
-    Q.p += D.p;
     Q.u += D.u;
     Q.v += D.v;
-    Q.w += D.w;
-    const double ir = 1.0 / Q.r;
+    const double ir = inv(Q.r);
     Q.u *= ir;
     Q.v *= ir;
-    Q.w *= ir;
+    if (!ISO) Q.w *= ir;
     if (Q.r < r_min) {
         Q.r = r_min;
         Q.p = p_min;

@@ -48,8 +48,12 @@ struct SwCfg {
     static constexpr int YTILE = TL * YCOLS * 5;
     static constexpr int TILE_MAX = ((XTILE > YTILE ? XTILE : YTILE) + 15) / 16 * 16;
     static constexpr bool X_OK = 5 * TL <= 256;                    // a TMA box is at most 256 elements wide
-    static constexpr size_t SMEM = (size_t)(NS * TILE_MAX + 10 * NST + 7 * NFX) * 8 + 8 * NS + 128;
-    static constexpr size_t AD_SMEM = (size_t)(NS * TILE_MAX + 5 * TL * W) * 8 + 8 * NS + 128;
+    // ISO: a 2D isothermal gas carries 4 edge-state fields and 4 fluxes (3 in the
+    // advection) instead of 5 and 7 (5)
+    template <bool ISO>
+    static constexpr size_t smem() { return (size_t)(NS * TILE_MAX + (ISO ? 8 : 10) * NST + (ISO ? 4 : 7) * NFX) * 8 + 8 * NS + 128; }
+    template <bool ISO>
+    static constexpr size_t ad_smem() { return (size_t)(NS * TILE_MAX + (ISO ? 3 : 5) * TL * W) * 8 + 8 * NS + 128; }
 };
 // The variants, in the order of SweepVariant ids (pg_internal.h SWEEP_VARIANTS).
 template <int V> struct SV;
@@ -96,8 +100,7 @@ __device__ __forceinline__ Grav gravity_at(const DiskView& d, double gstar, doub
         g.gz = -0.0;
         if (d.nplanet > 0) {
             const double plm = p.m, plx = p.x;
-            const double Rp = sqrt(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + p.rs * p.rs);
-            const double ir = 1.0 / Rp;
+            const double ir = rsq(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + p.rs * p.rs);
             const double rs_fac = ir * ir * ir;
             g.gx += -plm * (rad - plx * cosfac) * rs_fac - plm * cosfac * iplx2;
             g.gy += -plm * plx * sinfac * rs_fac + plm * sinfac * iplx2;
@@ -156,7 +159,7 @@ template <bool VISC>
 __device__ __forceinline__ Cell kick(const DiskView& d, const Cell& C, double ix, const Grav& g, double vx,
                                      double vy, double mdt, double dt, double* Tu = nullptr, double* Tv = nullptr) {
     Cell T = C;
-    const double ir = VISC ? 1.0 / C.r : 0.0;  // T.r == C.r throughout
+    const double ir = VISC ? inv(C.r) : 0.0;  // T.r == C.r throughout
     double fx = (d.geomx == 1) ? T.v * T.v * ix : 0.0;
     double fy = 0.0;
     const double fz = 0.0;
@@ -216,7 +219,7 @@ __device__ __forceinline__ double signal_rate(const DiskView& d, const Cell& c, 
     // src/timestep/timestep.cu:46-77 (cell widths as reciprocals); with dust the
     // dust speeds also bound dt (:64-74)
     const double rad_cyl = (d.geomy == 3) ? d.radx[i] : 1.0;
-    const double cs = sqrt(d.gam * c.p / c.r);
+    const double cs = sound_speed(d.gam, c.r, c.p);
     double spd = fabs(c.u) + cs;
     if (dc) spd = fmax(fabs(dc->u), spd);
     double tmp = fmax(spd * d.idx_x[i], 0.0);
@@ -233,7 +236,7 @@ __device__ __forceinline__ double signal_rate(const DiskView& d, const Cell& c, 
 __device__ __forceinline__ double signal_rate_at(const DiskView& d, const Cell& c, double radx, double idxx,
                                                  double rot, double idyj, double irad, const DCell* dc = nullptr) {
     const double rad_cyl = (d.geomy == 3) ? radx : 1.0;
-    const double cs = sqrt(d.gam * c.p / c.r);
+    const double cs = sound_speed(d.gam, c.r, c.p);
     double spd = fabs(c.u) + cs;
     if (dc) spd = fmax(fabs(dc->u), spd);
     double tmp = fmax(spd * idxx, 0.0);
@@ -247,19 +250,25 @@ __device__ __forceinline__ double signal_rate_at(const DiskView& d, const Cell& 
 
 // ================================================================ sweeps
 // DIR 0: radial pencils (rows of the array), DIR 1: azimuthal pencils (columns).
-// G: the tile configuration (SwCfg).
-template <int DIR, class G>
+// G: the tile configuration (SwCfg).  ISO: a 2D isothermal gas, which needs neither
+// the energy flux nor the z-velocity (identically zero there): four fields instead
+// of five through the three phases.  The passes are bound by the latency and issue
+// of their FP64 arithmetic, not by memory (0.12 of the copy rate), so what counts is
+// instructions: reciprocals and roots without their IEEE tails (pg_hydro.cuh), and
+// nothing computed that the equation of state does not use.
+template <int DIR, class G, bool ISO>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
     k_sweep(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out, int ntx, int ntiles) {
     constexpr int SW_W = G::W, SW_LEN = G::L, SW_TL = G::TL, SW_P1 = G::P1, SW_P2 = G::P2;
     constexpr int SW_TILE_MAX = G::TILE_MAX, SW_NST = G::NST, SW_NFX = G::NFX, SWY_COLS = G::YCOLS;
     constexpr int SWX_TILE = G::XTILE, SWY_TILE = G::YTILE, NS = G::NS, NT = G::THREADS;
+    constexpr int NH = ISO ? 4 : 5;  // fields of an edge state: r, p, u, then the transverse velocities
     extern __shared__ __align__(128) double smem_raw[];
     double* smem = smem_base128(smem_raw);
     auto stage = [&](int n) { return smem + (n % NS) * SW_TILE_MAX; };
-    double* st = smem + NS * SW_TILE_MAX;  // [10][SW_NST] interface states
-    double* fl = st + 10 * SW_NST;         // [7][SW_NFX] fluxes
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 7 * SW_NFX);
+    double* st = smem + NS * SW_TILE_MAX;  // [2 NH][SW_NST] interface states
+    double* fl = st + 2 * NH * SW_NST;     // [ISO ? 4 : 7][SW_NFX] fluxes
+    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + (ISO ? 4 : 7) * SW_NFX);
     __shared__ int s_inc[SW_W];
     Scalars* sc = d.sc;
     if (sc->done) return;
@@ -267,6 +276,7 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
     const int tid = threadIdx.x;
     const double dt = sc->dt;
     const double gam = d.gam;
+    const int eos = ISO ? 0 : d.eos;
     const uint32_t bytes = (DIR == 0 ? SWX_TILE : SWY_TILE) * 8;
     auto origin = [&](int tile, int& s0, int& q0) {
         const int bx = tile % ntx, by = tile / ntx;
@@ -324,13 +334,14 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
         const int t = 2 + ((DIR == 0) ? it % SW_P1 : it / SW_W);
         const int s = s0 - NPAD + t;
         const int qq = q0 + q;
-        double r[5], p[5], u[5], v[5], w[5];
-        double rad = 1.0, rot = 0.0, irad_q = 1.0;
-        if (DIR == 1) {
+        // sweep order: r, p, u, then for DIR 0 v (angular momentum) and w, for DIR 1 w and v_r
+        double r[5], p[5], u[5], a[5], z[5];
+        double v0 = 0.0, irad_q = 1.0;
+        if (DIR == 1) {  // the azimuthal velocity relative to the disk's rotation
             const int i = min(qq, d.xarr - 1);
-            rad = (d.geomy == 3) ? d.radx[i] : 1.0;
             irad_q = (d.geomy == 3) ? d.irad[i] : 1.0;
-            rot = d.rot[i];
+            v0 = d.rot[i];
+            if (d.geomy == 3) v0 += d.radx[i] * d.frame_omega;
         }
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
@@ -340,44 +351,42 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
             p[k] = c[1];
             if (DIR == 0) {
                 u[k] = c[2];
-                v[k] = c[3];
-                if (d.geomx == 1) v[k] *= d.radx[min(max(s - 2 + k, 0), d.xarr - 1)];
-                w[k] = c[4];
+                a[k] = c[3];
+                if (d.geomx == 1) a[k] *= d.radx[min(max(s - 2 + k, 0), d.xarr - 1)];
+                if (!ISO) z[k] = c[4];
             } else {
-                u[k] = c[3] - rot;
-                if (d.geomy == 3) u[k] -= rad * d.frame_omega;
-                v[k] = c[4];
-                w[k] = c[2];
+                u[k] = c[3] - v0;
+                a[k] = c[2];
+                if (!ISO) z[k] = c[4];
             }
         }
-        const double cs0 = sqrt(gam * p[2] / r[2]);
-        const double flat = flatten(1.0 / cs0, p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
+        const double cs0 = sound_speed(gam, r[2], p[2]);
+        const double flat = flatten(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
         const int sc_ = (DIR == 0) ? min(s, d.xarr - 1) : min(s, d.yarr - 1);
         const double* wt = ((DIR == 0) ? d.wx : d.wy) + 6 * sc_;
-        const double* fa = (DIR == 0) ? d.xa : d.ya;
-        const double idx = ((DIR == 0) ? d.idx_x : d.idx_y)[sc_];
+        const double sx = dt * irad_q * ((DIR == 0) ? d.idx_x : d.idx_y)[sc_];
         const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], flat);
         const Par P = recon(wt, p[0], p[1], p[2], p[3], p[4], flat);
         const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], flat);
-        // in 2D the z-velocity (v here for DIR 1, w for DIR 0) is identically zero, and the
-        // reconstruction of a zero stencil is exactly {+0, a0, +0}: skip it (CTA-uniform)
-        const bool flat2d = d.ndim == 2;
-        const Par V = (DIR == 1 && flat2d) ? Par{0.0, v[2], 0.0} : recon(wt, v[0], v[1], v[2], v[3], v[4], flat);
-        const Par W = (DIR == 0 && flat2d) ? Par{0.0, w[2], 0.0} : recon(wt, w[0], w[1], w[2], w[3], w[4], flat);
-        const double xl = fa[sc_], xr = fa[sc_ + 1];
-        const double sdt = (DIR == 0) ? dt : dt * irad_q;
-        const Half a = state_at_left_edge(gam, xl, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, W);
-        const Half b = state_at_right_edge(gam, xl, xr, idx, sdt, cs0, r[2], p[2], u[2], R, P, U, V, W);
-        st[0 * SW_NST + it] = a.r;
-        st[1 * SW_NST + it] = a.p;
-        st[2 * SW_NST + it] = a.u;
-        st[3 * SW_NST + it] = a.v;
-        st[4 * SW_NST + it] = a.w;
-        st[5 * SW_NST + it] = b.r;
-        st[6 * SW_NST + it] = b.p;
-        st[7 * SW_NST + it] = b.u;
-        st[8 * SW_NST + it] = b.v;
-        st[9 * SW_NST + it] = b.w;
+        const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], flat);
+        // the z-velocity, identically zero in 2D: a zero field's parabola is {0, 0, 0}
+        Par Z{0.0, 0.0, 0.0};
+        if (!ISO && d.ndim != 2) Z = recon(wt, z[0], z[1], z[2], z[3], z[4], flat);
+        else if (!ISO) Z.a = z[2];
+        const Half eL = state_at_left_edge(gam, sx, cs0, r[2], p[2], u[2], R, P, U, A, Z);
+        const Half eR = state_at_right_edge(gam, sx, cs0, r[2], p[2], u[2], R, P, U, A, Z);
+        double* o = st + it;
+        o[0] = eL.r;
+        o[1 * SW_NST] = eL.p;
+        o[2 * SW_NST] = eL.u;
+        o[3 * SW_NST] = eL.v;
+        if (!ISO) o[4 * SW_NST] = eL.w;
+        o += NH * SW_NST;
+        o[0] = eR.r;
+        o[1 * SW_NST] = eR.p;
+        o[2 * SW_NST] = eR.u;
+        o[3 * SW_NST] = eR.v;
+        if (!ISO) o[4 * SW_NST] = eR.w;
     }
     __syncthreads();
 
@@ -385,27 +394,25 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
     for (int it = tid; it < SW_NFX; it += NT) {
         const int q = (DIR == 0) ? it / SW_P2 : it % SW_W;
         const int t = 3 + ((DIR == 0) ? it % SW_P2 : it / SW_W);
-        const int iL = (DIR == 0) ? q * SW_P1 + (t - 3) : (t - 3) * SW_W + q;
-        const int iR = (DIR == 0) ? q * SW_P1 + (t - 2) : (t - 2) * SW_W + q;
-        Half L, R;
-        L.r = st[5 * SW_NST + iL];
-        L.p = st[6 * SW_NST + iL];
-        L.u = st[7 * SW_NST + iL];
-        L.v = st[8 * SW_NST + iL];
-        L.w = st[9 * SW_NST + iL];
-        R.r = st[0 * SW_NST + iR];
-        R.p = st[1 * SW_NST + iR];
-        R.u = st[2 * SW_NST + iR];
-        R.v = st[3 * SW_NST + iR];
-        R.w = st[4 * SW_NST + iR];
-        const Flux F = hllc(d.eos, d.ie, gam, L, R);
-        fl[0 * SW_NFX + it] = F.r;
-        fl[1 * SW_NFX + it] = F.p;
-        fl[2 * SW_NFX + it] = F.u;
-        fl[3 * SW_NFX + it] = F.v;
-        fl[4 * SW_NFX + it] = F.w;
-        fl[5 * SW_NFX + it] = F.pres;
-        fl[6 * SW_NFX + it] = F.uprs;
+        const double* pL = st + NH * SW_NST + ((DIR == 0) ? q * SW_P1 + (t - 3) : (t - 3) * SW_W + q);
+        const double* pR = st + ((DIR == 0) ? q * SW_P1 + (t - 2) : (t - 2) * SW_W + q);
+        Half L{pL[0], pL[SW_NST], pL[2 * SW_NST], pL[3 * SW_NST], 0.0};
+        Half R{pR[0], pR[SW_NST], pR[2 * SW_NST], pR[3 * SW_NST], 0.0};
+        if (!ISO) {
+            L.w = pL[4 * SW_NST];
+            R.w = pR[4 * SW_NST];
+        }
+        const Flux F = hllc(eos, d.ie, gam, L, R);
+        double* o = fl + it;
+        o[0] = F.r;
+        o[1 * SW_NFX] = F.u;
+        o[2 * SW_NFX] = F.v;
+        o[3 * SW_NFX] = F.pres;
+        if (!ISO) {
+            o[4 * SW_NFX] = F.w;
+            o[5 * SW_NFX] = F.p;
+            o[6 * SW_NFX] = F.uprs;
+        }
     }
     __syncthreads();
 
@@ -418,51 +425,49 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
         const bool valid = (DIR == 0) ? (s < NPAD + d.xres && qq < d.ypad + d.yres)
                                       : (s < NPAD + d.yres && qq < NPAD + d.xres);
         if (valid) {
-            const int f0 = (DIR == 0) ? q * SW_P2 + (t - 3) : (t - 3) * SW_W + q;
-            const int f1 = (DIR == 0) ? f0 + 1 : f0 + SW_W;
+            const double* f0 = fl + ((DIR == 0) ? q * SW_P2 + (t - 3) : (t - 3) * SW_W + q);
+            const double* f1 = f0 + ((DIR == 0) ? 1 : SW_W);
             const double g0 = (DIR == 0 && d.geomx == 1) ? d.xa[s] : 1.0;  // eval_gfac (riemann.cu:5-11)
             const double g1 = (DIR == 0 && d.geomx == 1) ? d.xa[s + 1] : 1.0;
-            const double pres0 = fl[5 * SW_NFX + f0], pres1 = fl[5 * SW_NFX + f1];
-            // net_source (src/solver/riemann/riemann.cu:40-87)
-            const double du = 0.5 * (g0 + g1) * (pres0 - pres1);
-            double de = 0.0;
-            if (d.eos == 2) {
-                const double t0 = fl[6 * SW_NFX + f0] * g0, t1 = fl[6 * SW_NFX + f1] * g1;
-                de = (d.ie == 0) ? t0 - t1 : 0.5 * (pres0 + pres1) * (t0 - t1);
+            auto net = [&](int k) { return f0[k * SW_NFX] * g0 - f1[k * SW_NFX] * g1; };
+            const double pres0 = f0[3 * SW_NFX], pres1 = f1[3 * SW_NFX];
+            // net_source (src/solver/riemann/riemann.cu:40-87): along the sweep, and the energy's
+            const double f = (DIR == 0) ? dt * d.ixv[s] : dt * d.iyv[s] * ((d.geomy == 3) ? d.irad[qq] : 1.0);
+            const double Dr = net(0) * f;
+            double Du = (net(1) + 0.5 * (g0 + g1) * (pres0 - pres1)) * f;
+            double Da = net(2) * f;
+            double Dz = 0.0, Dp = 0.0;
+            if (!ISO) {
+                Dz = net(4) * f;
+                double de = 0.0;
+                if (eos == 2) de = (d.ie == 0) ? net(6) : 0.5 * (pres0 + pres1) * net(6);
+                Dp = (net(5) + de) * f;
             }
-            Cell D;
-            D.r = fl[0 * SW_NFX + f0] * g0 - fl[0 * SW_NFX + f1] * g1;
-            D.p = (fl[1 * SW_NFX + f0] * g0 - fl[1 * SW_NFX + f1] * g1) + de;
-            D.u = (fl[2 * SW_NFX + f0] * g0 - fl[2 * SW_NFX + f1] * g1) + du;
-            D.v = fl[3 * SW_NFX + f0] * g0 - fl[3 * SW_NFX + f1] * g1;
-            D.w = fl[4 * SW_NFX + f0] * g0 - fl[4 * SW_NFX + f1] * g1;
             const double* c = (DIR == 0) ? tile + (q * SW_TL + t) * 5 : tile + (t * SWY_COLS + (q + 1)) * 5;
             const Cell C0{c[0], c[1], c[2], c[3], c[4]};
+            Cell D;
+            int i, j;
             if (DIR == 0) {
-                const double f = dt * d.ixv[s];
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (d.geomx == 1) D.v *= d.irad[s];
-                const Cell Q = update_cell(d.eos, d.ie, gam, d.cs2x[s], C0, D, &sc->floor_hits);
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                emit(d, out, s, qq, Q);
+                if (d.geomx == 1) Da *= d.irad[s];
+                D = Cell{Dr, Dp, Du, Da, Dz};
+                i = s;
+                j = qq;
             } else {
-                const double rad = (d.geomy == 3) ? d.radx[qq] : 1.0;
-                const double rot = d.rot[qq];
-                const double f = dt * d.iyv[s] * ((d.geomy == 3) ? d.irad[qq] : 1.0);
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (d.geomy == 3) D.u += (rot + rad * d.frame_omega) * D.r;
-                else D.u += rot * D.r;
-                const Cell E{D.r, D.p, D.w, D.u, D.v};
-                const Cell Q = update_cell(d.eos, d.ie, gam, d.cs2x[qq], C0, E, &sc->floor_hits);
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                int j = s;
+                double v0 = d.rot[qq];
+                if (d.geomy == 3) v0 += d.radx[qq] * d.frame_omega;
+                Du += v0 * Dr;
+                D = Cell{Dr, Dp, Da, Du, Dz};
+                i = qq;
+                j = s;
                 if (d.orbadv) {  // orbital shift T[(j+inc) mod N] = C[j] (orbit.cu:30-46)
                     int js = (s - d.ypad + s_inc[q]) % d.yres;
                     if (js < 0) js += d.yres;
                     j = js + d.ypad;
                 }
-                emit(d, out, qq, j, Q);
             }
+            const Cell Q = update_cell<ISO>(eos, d.ie, gam, d.cs2x[i], C0, D, &sc->floor_hits);
+            if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+            emit(d, out, i, j, Q);
         }
     }
     __syncthreads();  // stage k % NS, the state / flux arrays and s_inc are free again
@@ -470,7 +475,9 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
 }
 
 // ===================================================== residual advection
-template <class G>
+// ISO as in k_sweep: without the pressure (reset from the density after the
+// update) and the z-velocity.
+template <class G, bool ISO>
 __global__ void __launch_bounds__(G::THREADS, G::MINB)
     k_advect(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out, int ntx, int ntiles) {
     constexpr int SW_W = G::W, SW_LEN = G::L, SW_TL = G::TL, SW_TILE_MAX = G::TILE_MAX, SW_NST = G::NST;
@@ -478,8 +485,8 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
     extern __shared__ __align__(128) double smem_raw[];
     double* smem = smem_base128(smem_raw);
     auto stage = [&](int n) { return smem + (n % NS) * SW_TILE_MAX; };
-    double* fl = smem + NS * SW_TILE_MAX;  // [5][SW_TL * SW_W] face fluxes, indexed by face t
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 5 * SW_TL * SW_W);
+    double* fl = smem + NS * SW_TILE_MAX;  // [ISO ? 3 : 5][SW_TL * SW_W] face fluxes, indexed by face t
+    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + (ISO ? 3 : 5) * SW_TL * SW_W);
     Scalars* sc = d.sc;
     if (sc->done) return;
     const int tid = threadIdx.x;
@@ -521,52 +528,26 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
         const int i = min(q0 + q, d.xarr - 1);
         const double speed = d.res[i];
         const double sdt = dt * ((d.geomy == 3) ? d.irad[i] : 1.0);
-        const double idx = d.idx_y[s];
-        double r[5], p[5], u[5], v[5], w[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const double* c = tile + ((t - 2 + k) * SWY_COLS + (q + 1)) * 5;
-            r[k] = c[0]; p[k] = c[1]; u[k] = c[3]; v[k] = c[4]; w[k] = c[2];
-        }
         const double* wt = d.wy + 6 * s;
-        // CTA-uniform: with the isothermal EOS the pressure is reset from the density
-        // after the update, so its flux is never used; in 2D the z-velocity is
-        // identically zero, so its flux is zero
-        const bool need_p = d.eos != 0, need_w = d.ndim != 2;
-        const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], 0.0);
-        const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], 0.0);
-        const Par W = recon(wt, w[0], w[1], w[2], w[3], w[4], 0.0);
-        Par P = R, V = R;
-        if (need_p) P = recon(wt, p[0], p[1], p[2], p[3], p[4], 0.0);
-        if (need_w) V = recon(wt, v[0], v[1], v[2], v[3], v[4], 0.0);
-        const double xl = d.ya[s], xr = d.ya[s + 1];
-        double fr, fp = 0.0, fu, fv = 0.0, fw;
-        int face;
-        if (speed > 0.0) {  // this cell is upwind of its upper face
-            const double x0 = xr - speed * sdt;
-            const Frac q_ = frac_right(lim01((x0 - xl) * idx));
-            fr = aveR(q_, R);
-            if (need_p) fp = aveR(q_, P);
-            fu = aveR(q_, U) * fr;
-            if (need_w) fv = aveR(q_, V) * fr;
-            fw = aveR(q_, W) * fr;
-            face = t + 1;
-        } else {  // ... of its lower face
-            const double x0 = xl - speed * sdt;
-            const Frac q_ = frac_left(lim01((x0 - xl) * idx));
-            fr = aveL(q_, R);
-            if (need_p) fp = aveL(q_, P);
-            fu = aveL(q_, U) * fr;
-            if (need_w) fv = aveL(q_, V) * fr;
-            fw = aveL(q_, W) * fr;
-            face = t;
+        const Frac x = frac(lesser(fabs(speed) * (sdt * d.idx_y[s]), 1.0));
+        const bool up = speed > 0.0;  // this cell is upwind of its upper face, else of its lower one
+        // average of field k of the cells over the swept part
+        const double* c0 = tile + ((t - 2) * SWY_COLS + (q + 1)) * 5;
+        auto ave = [&](int k) {
+            const double* c = c0 + k;
+            const Par A = recon(wt, c[0], c[5 * SWY_COLS], c[10 * SWY_COLS], c[15 * SWY_COLS], c[20 * SWY_COLS], 0.0);
+            return up ? aveR(x, A) : aveL(x, A);
+        };
+        const double fr = ave(0);
+        const double m = fr * speed;
+        double* o = fl + (t + (up ? 1 : 0)) * SW_W + q;
+        o[0] = m;
+        o[1 * NFL] = ave(2) * m;
+        o[2 * NFL] = ave(3) * m;
+        if (!ISO) {
+            o[3 * NFL] = d.ndim != 2 ? ave(4) * m : 0.0;
+            o[4 * NFL] = d.eos != 0 ? ave(1) * speed : 0.0;
         }
-        const int k = face * SW_W + q;
-        fl[0 * NFL + k] = fr * speed;
-        fl[1 * NFL + k] = fp * speed;
-        fl[2 * NFL + k] = fu * speed;
-        fl[3 * NFL + k] = fv * speed;
-        fl[4 * NFL + k] = fw * speed;
     }
     __syncthreads();
 
@@ -577,34 +558,22 @@ __global__ void __launch_bounds__(G::THREADS, G::MINB)
         const int s = s0 - NPAD + t;
         const int i = q0 + q;
         if (s < NPAD + d.yres && i < NPAD + d.xres) {
-            const int k0 = t * SW_W + q, k1 = (t + 1) * SW_W + q;
-            Cell D;
-            D.r = fl[0 * NFL + k0] * 1.0 - fl[0 * NFL + k1] * 1.0;
-            D.p = fl[1 * NFL + k0] * 1.0 - fl[1 * NFL + k1] * 1.0;
-            D.u = fl[2 * NFL + k0] * 1.0 - fl[2 * NFL + k1] * 1.0;
-            D.v = fl[3 * NFL + k0] * 1.0 - fl[3 * NFL + k1] * 1.0;
-            D.w = fl[4 * NFL + k0] * 1.0 - fl[4 * NFL + k1] * 1.0;
+            const double* f0 = fl + t * SW_W + q;
             double f = dt * d.iyv[s];
-            D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-            if (d.geomy > 2) {
-                f = d.irad[i];
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-            }
+            if (d.geomy > 2) f *= d.irad[i];
+            auto net = [&](int k) { return (f0[k * NFL] - f0[k * NFL + SW_W]) * f; };
             const double* c = tile + (t * SWY_COLS + (q + 1)) * 5;
             Cell Q{c[0], c[1], c[2], c[3], c[4]};
-            Q.u *= Q.r;
-            Q.v *= Q.r;
-            Q.w *= Q.r;
-            Q.r += D.r;
-            Q.p += D.p;
-            Q.u += D.w;
-            Q.v += D.u;
-            Q.w += D.v;
-            const double ir = 1.0 / Q.r;
-            Q.u *= ir;
-            Q.v *= ir;
-            Q.w *= ir;
-            if (d.eos == 0) Q.p = d.cs2x[i] * Q.r;
+            const double r = Q.r + net(0);
+            const double ir = inv(r);
+            Q.u = (Q.u * Q.r + net(1)) * ir;
+            Q.v = (Q.v * Q.r + net(2)) * ir;
+            if (!ISO) {
+                Q.w = (Q.w * Q.r + net(3)) * ir;
+                Q.p += net(4);
+            }
+            Q.r = r;
+            if (ISO || d.eos == 0) Q.p = d.cs2x[i] * r;
             if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
             emit(d, out, i, s, Q);
         }
@@ -1189,9 +1158,14 @@ cudaError_t set_kernel_attributes() {
     };
     auto set_v = [&](auto tag) {
         using G = typename decltype(tag)::G;
-        if constexpr (G::X_OK) set((const void*)k_sweep<0, G>, G::SMEM);
-        set((const void*)k_sweep<1, G>, G::SMEM);
-        set((const void*)k_advect<G>, G::AD_SMEM);
+        if constexpr (G::X_OK) {
+            set((const void*)k_sweep<0, G, true>, G::template smem<true>());
+            set((const void*)k_sweep<0, G, false>, G::template smem<false>());
+        }
+        set((const void*)k_sweep<1, G, true>, G::template smem<true>());
+        set((const void*)k_sweep<1, G, false>, G::template smem<false>());
+        set((const void*)k_advect<G, true>, G::template ad_smem<true>());
+        set((const void*)k_advect<G, false>, G::template ad_smem<false>());
     };
     set_v(SV<0>{});
     set_v(SV<1>{});
@@ -1297,16 +1271,16 @@ static unsigned persistent_grid(const void* kernel, int threads, size_t smem, lo
 
 static int kernel_occupancy(const void* kernel, int threads, size_t smem) {
     // occupancy of each kernel, queried once (launches repeat every step)
-    static const void* keys[64] = {nullptr};
-    static int vals[64] = {0};
+    static const void* keys[128] = {nullptr};
+    static int vals[128] = {0};
     int per_sm = 0;
-    for (int n = 0; n < 64 && keys[n]; ++n)
+    for (int n = 0; n < 128 && keys[n]; ++n)
         if (keys[n] == kernel) per_sm = vals[n];
     if (per_sm == 0) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
-        for (int n = 0; n < 64; ++n)
+        for (int n = 0; n < 128; ++n)
             if (!keys[n]) {
                 keys[n] = kernel;
                 vals[n] = per_sm;
@@ -1329,23 +1303,28 @@ void launch_kick1(const DiskView& d, const CellMaps& in, Cell* out, double* vis,
     }
 }
 
-template <int DIR, class G>
+// the 2D isothermal instances of the sweeps and the advection apply
+static bool iso_2d(const DiskView& d) { return d.eos == 0 && d.ndim == 2; }
+
+template <int DIR, class G, bool ISO>
 static void sweep_g(const DiskView& d, const CUtensorMap& m, Cell* out, cudaStream_t s, int cps) {
     if constexpr (DIR == 0 && !G::X_OK) {
         return;  // never chosen: the autotuner skips radial variants whose box does not fit
     } else {
         const int ntx = (int)cdiv(DIR == 0 ? d.xres : d.yres, G::L);
         const int nt = ntx * (int)cdiv(DIR == 0 ? d.yres : d.xres, G::W);
-        const unsigned g = persistent_grid((const void*)k_sweep<DIR, G>, G::THREADS, G::SMEM, nt, cps);
-        k_sweep<DIR, G><<<g, G::THREADS, G::SMEM, s>>>(m, d, out, ntx, nt);
+        constexpr size_t smem = G::template smem<ISO>();
+        const unsigned g = persistent_grid((const void*)k_sweep<DIR, G, ISO>, G::THREADS, smem, nt, cps);
+        k_sweep<DIR, G, ISO><<<g, G::THREADS, smem, s>>>(m, d, out, ntx, nt);
     }
 }
 
-template <class G>
+template <class G, bool ISO>
 static void advect_g(const DiskView& d, const CUtensorMap& m, Cell* out, cudaStream_t s, int cps) {
     const int ntx = (int)cdiv(d.yres, G::L), nt = ntx * (int)cdiv(d.xres, G::W);
-    const unsigned g = persistent_grid((const void*)k_advect<G>, G::THREADS, G::AD_SMEM, nt, cps);
-    k_advect<G><<<g, G::THREADS, G::AD_SMEM, s>>>(m, d, out, ntx, nt);
+    constexpr size_t smem = G::template ad_smem<ISO>();
+    const unsigned g = persistent_grid((const void*)k_advect<G, ISO>, G::THREADS, smem, nt, cps);
+    k_advect<G, ISO><<<g, G::THREADS, smem, s>>>(m, d, out, ntx, nt);
 }
 
 // calls f(SV<v>{}) for the variant id v
@@ -1373,17 +1352,29 @@ static int variant_of(const Tune* t, int k, int dir) {
 
 void launch_sweep_x(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
     const int v = variant_of(t, 0, 0);
-    with_variant(v, [&](auto tag) { sweep_g<0, typename decltype(tag)::G>(d, in.sx[v], out, s, t ? t->cps[1] : 0); });
+    with_variant(v, [&](auto tag) {
+        using G = typename decltype(tag)::G;
+        if (iso_2d(d)) sweep_g<0, G, true>(d, in.sx[v], out, s, t ? t->cps[1] : 0);
+        else sweep_g<0, G, false>(d, in.sx[v], out, s, t ? t->cps[1] : 0);
+    });
 }
 
 void launch_sweep_y(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
     const int v = variant_of(t, 1, 1);
-    with_variant(v, [&](auto tag) { sweep_g<1, typename decltype(tag)::G>(d, in.sy[v], out, s, t ? t->cps[2] : 0); });
+    with_variant(v, [&](auto tag) {
+        using G = typename decltype(tag)::G;
+        if (iso_2d(d)) sweep_g<1, G, true>(d, in.sy[v], out, s, t ? t->cps[2] : 0);
+        else sweep_g<1, G, false>(d, in.sy[v], out, s, t ? t->cps[2] : 0);
+    });
 }
 
 void launch_advect(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
     const int v = variant_of(t, 2, 1);
-    with_variant(v, [&](auto tag) { advect_g<typename decltype(tag)::G>(d, in.sy[v], out, s, t ? t->cps[3] : 0); });
+    with_variant(v, [&](auto tag) {
+        using G = typename decltype(tag)::G;
+        if (iso_2d(d)) advect_g<G, true>(d, in.sy[v], out, s, t ? t->cps[3] : 0);
+        else advect_g<G, false>(d, in.sy[v], out, s, t ? t->cps[3] : 0);
+    });
 }
 
 void launch_kick2(const DiskView& d, const CellMaps& in, const VisMaps& vis, Cell* out, cudaStream_t s,
@@ -1401,7 +1392,7 @@ void launch_kick2(const DiskView& d, const CellMaps& in, const VisMaps& vis, Cel
 
 // CTAs per SM that fit for a pass (0 kick1, 1 sweep_x, 2 sweep_y, 3 advect, 4 kick2) with tile variant v
 int pass_occupancy(const DiskView& d, int pass, int v) {
-    const bool vis = d.visc && d.ndim == 2;
+    const bool vis = d.visc && d.ndim == 2, iso = iso_2d(d);
     int occ = 1;
     switch (pass) {
         case 0: return kernel_occupancy(vis ? (const void*)k_kick1<true> : (const void*)k_kick1<false>, ST_THREADS, K1_SMEM);
@@ -1409,19 +1400,23 @@ int pass_occupancy(const DiskView& d, int pass, int v) {
         case 1:
             with_variant(v, [&](auto tag) {
                 using G = typename decltype(tag)::G;
-                if constexpr (G::X_OK) occ = kernel_occupancy((const void*)k_sweep<0, G>, G::THREADS, G::SMEM);
+                if constexpr (G::X_OK)
+                    occ = iso ? kernel_occupancy((const void*)k_sweep<0, G, true>, G::THREADS, G::template smem<true>())
+                              : kernel_occupancy((const void*)k_sweep<0, G, false>, G::THREADS, G::template smem<false>());
             });
             return occ;
         case 2:
             with_variant(v, [&](auto tag) {
                 using G = typename decltype(tag)::G;
-                occ = kernel_occupancy((const void*)k_sweep<1, G>, G::THREADS, G::SMEM);
+                occ = iso ? kernel_occupancy((const void*)k_sweep<1, G, true>, G::THREADS, G::template smem<true>())
+                          : kernel_occupancy((const void*)k_sweep<1, G, false>, G::THREADS, G::template smem<false>());
             });
             return occ;
         default:
             with_variant(v, [&](auto tag) {
                 using G = typename decltype(tag)::G;
-                occ = kernel_occupancy((const void*)k_advect<G>, G::THREADS, G::AD_SMEM);
+                occ = iso ? kernel_occupancy((const void*)k_advect<G, true>, G::THREADS, G::template ad_smem<true>())
+                          : kernel_occupancy((const void*)k_advect<G, false>, G::THREADS, G::template ad_smem<false>());
             });
             return occ;
     }
@@ -1472,6 +1467,13 @@ __global__ void k_test_div_1p5(const double* x, long long n, double* out) {
         out[2 * k + 1] = __ddiv_rn(a, 1.5);
     }
 }
+// test support: inv and rsq (pg_hydro.cuh)
+__global__ void k_test_inv_rsq(const double* x, long long n, double* out) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
+        out[2 * k] = inv(x[k]);
+        out[2 * k + 1] = rsq(x[k]);
+    }
+}
 }  // namespace pg
 
 extern "C" pg_status pg_test_bounded_wait(int* err_bits, int* left, float* ms) {
@@ -1504,7 +1506,9 @@ extern "C" pg_status pg_test_bounded_wait(int* err_bits, int* left, float* ms) {
     return e == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
 
-extern "C" pg_status pg_test_div_1p5(const double* x, long long n, double* out2) {
+// out2[2n] on the host from a kernel (x, n, out) over x[n]
+static pg_status test_pairs(void (*kernel)(const double*, long long, double*), const double* x, long long n,
+                            double* out2) {
     if (!x || !out2 || n <= 0) return PG_ERR_ARG;
     double *dx = nullptr, *dout = nullptr;
     if (cudaMalloc(&dx, n * sizeof(double)) != cudaSuccess) return PG_ERR_CUDA;
@@ -1514,11 +1518,17 @@ extern "C" pg_status pg_test_div_1p5(const double* x, long long n, double* out2)
     }
     cudaError_t e = cudaMemcpy(dx, x, n * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        pg::k_test_div_1p5<<<592, 256>>>(dx, n, dout);
+        kernel<<<592, 256>>>(dx, n, dout);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(out2, dout, 2 * n * sizeof(double), cudaMemcpyDeviceToHost);
     cudaFree(dx);
     cudaFree(dout);
     return e == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}
+extern "C" pg_status pg_test_div_1p5(const double* x, long long n, double* out2) {
+    return test_pairs(pg::k_test_div_1p5, x, n, out2);
+}
+extern "C" pg_status pg_test_inv_rsq(const double* x, long long n, double* out2) {
+    return test_pairs(pg::k_test_inv_rsq, x, n, out2);
 }
