@@ -15,18 +15,22 @@
 
 namespace pg {
 
-constexpr int DS_LEN = 32, DS_W = 8;
+// Tiles of 32 outputs x 4 pencils: 160 threads and 25 KB of shared memory, so that 6
+// CTAs per SM hide the FP64 latency the passes are bound by.  The w velocity is
+// identically zero (dust runs in 2D) and stays as it is: three fields go through the
+// phases.
+constexpr int DS_LEN = 32, DS_W = DUST_W;
 constexpr int DS_TL = DS_LEN + 2 * NPAD;               // 38
 constexpr int DS_P1 = DS_LEN + 2, DS_P2 = DS_LEN + 1;  // cells with edge states, faces per pencil
-constexpr int DS_THREADS = 288;
+constexpr int DS_THREADS = 160;
+constexpr int DS_MINB = 5;
 constexpr int DS_NST = DS_P1 * DS_W, DS_NFX = DS_P2 * DS_W;
-constexpr int DSY_COLS = DS_W + 2;                     // y tiles start one column early (16-B TMA x)
-constexpr int DSX_TILE = 4 * DS_TL * DS_W;             // 1216 doubles
-constexpr int DSY_TILE = 4 * DS_TL * DSY_COLS;         // 1520 doubles
-constexpr int DS_STAGE = (DSY_TILE + 15) / 16 * 16;    // 128-B aligned stages
-constexpr size_t DS_SMEM = (size_t)(2 * DS_STAGE + 8 * DS_NST + 4 * DS_NFX) * 8 + 16 + 128;
+static_assert(DS_NST <= DS_THREADS, "one cell per thread in each phase");
+constexpr int DS_TILE = 4 * DS_TL * DS_W;              // doubles; a cell is 32 bytes, so any column starts a TMA box
+constexpr int DS_STAGE = (DS_TILE + 15) / 16 * 16;     // 128-B aligned stages
+constexpr size_t DS_SMEM = (size_t)(2 * DS_STAGE + 6 * DS_NST + 3 * DS_NFX) * 8 + 16 + 128;
 constexpr int DA_NF = DS_TL * DS_W;                    // advection faces per tile
-constexpr size_t DA_SMEM = (size_t)(2 * DS_STAGE + 4 * DA_NF) * 8 + 16 + 128;
+constexpr size_t DA_SMEM = (size_t)(2 * DS_STAGE + 3 * DA_NF) * 8 + 16 + 128;
 
 // src/solver/riemann/riemann.cu:5-11
 __device__ __forceinline__ double gfac(int geom, double x) {
@@ -36,24 +40,23 @@ __device__ __forceinline__ double gfac(int geom, double x) {
 }
 
 // ============================================================ dust sweeps
-// DIR 0: radial pencils of rows (fields r, u, r v, w); DIR 1: azimuthal pencils of
-// columns (r, v - orb_rot - r Omega, w, u).
+// DIR 0: radial pencils of rows (fields r, u, r v); DIR 1: azimuthal pencils of
+// columns (r, v - orb_rot - r Omega, u).
 template <int DIR>
-__global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ CUtensorMap tm, const DiskView d,
-                                                      pg_dust* __restrict__ out, int ntx, int ntiles) {
+__global__ void __launch_bounds__(DS_THREADS, DS_MINB)
+    k_dsweep(const __grid_constant__ CUtensorMap tm, const DiskView d, pg_dust* __restrict__ out, int ntx, int ntiles) {
     extern __shared__ __align__(128) double smem_raw[];
     double* smem = smem_base128(smem_raw);
     auto stage = [&](int n) { return smem + (n & 1) * DS_STAGE; };
-    double* st = smem + 2 * DS_STAGE;  // [8][DS_NST]: right state of the left face, left state of the right face
-    double* fl = st + 8 * DS_NST;      // [4][DS_NFX]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 4 * DS_NFX);
+    double* st = smem + 2 * DS_STAGE;  // [6][DS_NST]: right state of the left face, left state of the right face
+    double* fl = st + 6 * DS_NST;      // [3][DS_NFX]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 3 * DS_NFX);
     __shared__ int s_inc[DS_W];
     Scalars* sc = d.sc;
     if (sc->done) return;
     const int tid = threadIdx.x;
     const double dt = sc->dt;
-    const double* fa = (DIR == 0) ? d.xa : d.ya;
-    const int geom = (DIR == 0) ? d.geomx : d.geomy;
+    const double* idx = (DIR == 0) ? d.idx_x : d.idx_y;  // one over a cell's width
     auto origin = [&](int tile, int& s0, int& q0) {
         s0 = NPAD + DS_LEN * (tile % ntx);
         q0 = (DIR == 0 ? d.ypad : NPAD) + DS_W * (tile / ntx);
@@ -61,14 +64,14 @@ __global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ C
     auto issue = [&](int tile, int k) {
         int s0, q0;
         origin(tile, s0, q0);
-        issue_begin(&bar[k & 1], (DIR == 0 ? DSX_TILE : DSY_TILE) * 8);
+        issue_begin(&bar[k & 1], DS_TILE * 8);
         if (DIR == 0) tma_load_2d(stage(k), &tm, 4 * (s0 - NPAD), q0, &bar[k & 1]);
-        else tma_load_2d(stage(k), &tm, 4 * (q0 - 1), s0 - NPAD, &bar[k & 1]);
+        else tma_load_2d(stage(k), &tm, 4 * q0, s0 - NPAD, &bar[k & 1]);
     };
     // tile cell (position along the pencil t, pencil q) -> its 4 doubles
-    auto cellp = [&](const double* T, int t, int q) {
-        return (DIR == 0) ? T + (q * DS_TL + t) * 4 : T + (t * DSY_COLS + (q + 1)) * 4;
-    };
+    auto cellp = [&](const double* T, int t, int q) { return T + ((DIR == 0) ? q * DS_TL + t : t * DS_W + q) * 4; };
+    // dt over the pencil's radius (azimuthal sweeps: dust_flow, dust.cu:120-121)
+    auto pencil_dt = [&](int q) { return dt * ((DIR == 1 && d.geomy == 3) ? d.irad[min(q, d.xarr - 1)] : 1.0); };
     pipe_init(bar);
     if ((int)blockIdx.x >= ntiles) return;
     if (tid == 0) issue(blockIdx.x, 0);
@@ -100,65 +103,45 @@ __global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ C
             const int t = 2 + ((DIR == 0) ? tid % DS_P1 : tid / DS_W);
             const int s = s0 - NPAD + t;
             const int sc_ = (DIR == 0) ? min(s, d.xarr - 1) : min(s, d.yarr - 1);
-            const int i = (DIR == 0) ? 0 : min(q0 + q, d.xarr - 1);
-            double rad = 1.0, rot = 0.0;
+            double v0 = 0.0;
             if (DIR == 1) {
-                rad = (d.geomy == 3) ? d.radx[i] : 1.0;
-                rot = d.rot[i];
+                const int i = min(q0 + q, d.xarr - 1);
+                v0 = d.rot[i];
+                if (d.geomy == 3) v0 += d.radx[i] * d.frame_omega;
             }
-            double r[5], u[5], v[5], w[5];
+            double r[5], u[5], a[5];
 #pragma unroll
             for (int m = 0; m < 5; ++m) {
-                const double* c = cellp(T, t - 2 + m, q);
-                r[m] = c[0];
-                if (DIR == 0) {
-                    u[m] = c[1];
-                    v[m] = c[2];
-                    if (d.geomx == 1) v[m] *= d.radx[min(max(s - 2 + m, 0), d.xarr - 1)];
-                    w[m] = c[3];
-                } else {
-                    u[m] = c[2] - rot;
-                    if (d.geomy == 3) u[m] -= rad * d.frame_omega;
-                    v[m] = c[3];
-                    w[m] = c[1];
-                }
+                // 16-byte loads: 8-byte ones at this 32-byte stride conflict 4 ways
+                const double2* c = reinterpret_cast<const double2*>(cellp(T, t - 2 + m, q));
+                const double2 ru = c[0], vw = c[1];
+                r[m] = ru.x;
+                u[m] = (DIR == 0) ? ru.y : vw.x - v0;
+                a[m] = (DIR == 0) ? vw.x : ru.y;
+                if (DIR == 0 && d.geomx == 1) a[m] *= d.radx[min(max(s - 2 + m, 0), d.xarr - 1)];
             }
             const double* wt = ((DIR == 0) ? d.wx : d.wy) + 6 * sc_;
             const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], 0.0);
             const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], 0.0);
-            const Par V = recon(wt, v[0], v[1], v[2], v[3], v[4], 0.0);
-            const Par W = recon(wt, w[0], w[1], w[2], w[3], w[4], 0.0);
-            const double sdt = (DIR == 0 || geom <= 2) ? dt : dt / rad;  // dust_flow (dust.cu:120-121)
-            const double xl = fa[sc_], xr = fa[sc_ + 1];
+            const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], 0.0);
+            // swept fraction per unit speed: the traced positions of the reference enter
+            // only as fractions of the cell
+            const double sx = pencil_dt(q0 + q) * idx[sc_];
             // left face, from this cell
-            double tmp = xl - fmin(U.a - U.sL, 0.0) * sdt;
-            Frac fq = frac_left(lim01((tmp - xl) / (xr - xl)));
-            const double ur = aveL(fq, U);
-            double u_ = 0.5 * sdt * (ur - u[2]) / (0.5 * (xr - tmp));
-            tmp = xl - fmin(ur, 0.0) * sdt;
-            fq = frac_left(lim01((tmp - xl) / (xr - xl)));
-            const double Srr = aveL(fq, R) * exp_lim(u_);
-            const double Sur = aveL(fq, U) + 0.0;
-            const double Svr = aveL(fq, V), Swr = aveL(fq, W);
-            // right face, from this cell
-            tmp = xr - fmax(U.a + U.sR, 0.0) * sdt;
-            fq = frac_right(lim01((tmp - xl) / (xr - xl)));
-            const double ul = aveR(fq, U);
-            u_ = 0.5 * sdt * (u[2] - ul) / (0.5 * (tmp - xl));
-            tmp = xr - fmax(ul, 0.0) * sdt;
-            fq = frac_right(lim01((tmp - xl) / (xr - xl)));
-            const double Srl = aveR(fq, R) * exp_lim(u_);
-            const double Sul = aveR(fq, U) + 0.0;
-            const double Svl = aveR(fq, V), Swl = aveR(fq, W);
+            double m = lesser(U.a - U.sL, 0.0) * sx;
+            const double ur = aveL(frac(lesser(-m, 1.0)), U);
+            Frac x = frac(lesser(-lesser(ur, 0.0) * sx, 1.0));
             double* o = st + tid;
-            o[0] = Srr;
-            o[DS_NST] = Sur;
-            o[2 * DS_NST] = Svr;
-            o[3 * DS_NST] = Swr;
-            o[4 * DS_NST] = Srl;
-            o[5 * DS_NST] = Sul;
-            o[6 * DS_NST] = Svl;
-            o[7 * DS_NST] = Swl;
+            o[0] = aveL(x, R) * exp_lim(sx * (ur - u[2]) * inv(1.0 + m));
+            o[DS_NST] = aveL(x, U);
+            o[2 * DS_NST] = aveL(x, A);
+            // right face, from this cell
+            m = larger(U.a + U.sR, 0.0) * sx;
+            const double ul = aveR(frac(lesser(m, 1.0)), U);
+            x = frac(lesser(larger(ul, 0.0) * sx, 1.0));
+            o[3 * DS_NST] = aveR(x, R) * exp_lim(sx * (u[2] - ul) * inv(1.0 - m));
+            o[4 * DS_NST] = aveR(x, U);
+            o[5 * DS_NST] = aveR(x, A);
         }
         __syncthreads();
 
@@ -166,20 +149,16 @@ __global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ C
         if (tid < DS_NFX) {
             const int q = (DIR == 0) ? tid / DS_P2 : tid % DS_W;
             const int f = (DIR == 0) ? tid % DS_P2 : tid / DS_W;  // between tile cells 2+f and 3+f
-            const int iL = (DIR == 0) ? q * DS_P1 + f : f * DS_W + q;
-            const int iR = (DIR == 0) ? iL + 1 : iL + DS_W;
-            const int sf = s0 + f;  // face index = index of the right cell
-            const int sfc = (DIR == 0) ? min(sf, d.xarr - 1) : min(sf, d.yarr - 1);
-            double rad = 1.0;
-            if (DIR == 1) rad = (d.geomy == 3) ? d.radx[min(q0 + q, d.xarr - 1)] : 1.0;
-            const double sdt = (DIR == 0 || geom <= 2) ? dt : dt / rad;
+            const double* R = st + ((DIR == 0) ? q * DS_P1 + f + 1 : (f + 1) * DS_W + q);
+            const double* L = st + 3 * DS_NST + ((DIR == 0) ? q * DS_P1 + f : f * DS_W + q);
+            const int sfc = min(s0 + f, (DIR == 0 ? d.xarr : d.yarr) - 1);  // face index = index of the right cell
+            const double sdt = pencil_dt(q0 + q);
             const double rL = cellp(T, 2 + f, q)[0], rR = cellp(T, 3 + f, q)[0];
-            const double Srl = fmin(rL * sdt / (fa[sfc] - fa[sfc - 1]), fmax(st[5 * DS_NST + iL] * st[4 * DS_NST + iL], 0.0));
-            const double Srr = fmax(rR * sdt / (fa[sfc] - fa[sfc + 1]), fmin(st[DS_NST + iR] * st[iR], 0.0));
-            fl[tid] = Srl + Srr;
-            fl[DS_NFX + tid] = Srl * st[5 * DS_NST + iL] + Srr * st[DS_NST + iR];
-            fl[2 * DS_NFX + tid] = Srl * st[6 * DS_NST + iL] + Srr * st[2 * DS_NST + iR];
-            fl[3 * DS_NFX + tid] = Srl * st[7 * DS_NST + iL] + Srr * st[3 * DS_NST + iR];
+            const double ml = lesser(rL * sdt * idx[sfc - 1], larger(L[DS_NST] * L[0], 0.0));
+            const double mr = larger(-rR * sdt * idx[sfc], lesser(R[DS_NST] * R[0], 0.0));
+            fl[tid] = ml + mr;
+            fl[DS_NFX + tid] = ml * L[DS_NST] + mr * R[DS_NST];
+            fl[2 * DS_NFX + tid] = ml * L[2 * DS_NST] + mr * R[2 * DS_NST];
         }
         __syncthreads();
 
@@ -191,35 +170,24 @@ __global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ C
             const bool valid = (DIR == 0) ? (s < NPAD + d.xres && qq < d.ypad + d.yres)
                                           : (s < NPAD + d.yres && qq < NPAD + d.xres);
             if (valid) {
-                const int f0 = (DIR == 0) ? q * DS_P2 + o : o * DS_W + q;
-                const int f1 = (DIR == 0) ? f0 + 1 : f0 + DS_W;
-                const double g0 = gfac(geom, fa[s]), g1 = gfac(geom, fa[s + 1]);
-                DCell D;
-                D.r = fl[f0] * g0 - fl[f1] * g1;
-                D.u = fl[DS_NFX + f0] * g0 - fl[DS_NFX + f1] * g1;
-                D.v = fl[2 * DS_NFX + f0] * g0 - fl[2 * DS_NFX + f1] * g1;
-                D.w = fl[3 * DS_NFX + f0] * g0 - fl[3 * DS_NFX + f1] * g1;
+                const double* f0 = fl + ((DIR == 0) ? q * DS_P2 + o : o * DS_W + q);
+                const double* f1 = f0 + ((DIR == 0) ? 1 : DS_W);
+                const double g0 = (DIR == 0) ? gfac(d.geomx, d.xa[s]) : 1.0;
+                const double g1 = (DIR == 0) ? gfac(d.geomx, d.xa[s + 1]) : 1.0;
+                const double f = (DIR == 0) ? dt * d.ixv[s] : pencil_dt(qq) * d.iyv[s];
+                auto net = [&](int k) { return (f0[k * DS_NFX] * g0 - f1[k * DS_NFX] * g1) * f; };
                 const double* c = cellp(T, NPAD + o, q);
                 const DCell Q{c[0], c[1], c[2], c[3]};
+                const double Dr = net(0);
                 if (DIR == 0) {
-                    const double f = dt / d.xv[s];
-                    D.r *= f; D.u *= f; D.v *= f; D.w *= f;
-                    if (d.geomx == 1) D.v /= d.radx[s];
-                    const DCell N = update_dust(d, Q, D);
+                    const double Da = net(2) * (d.geomx == 1 ? d.irad[s] : 1.0);
+                    const DCell N = update_dust(d, Q, DCell{Dr, net(1), Da, 0.0});
                     if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
                     emit_dust(d, out, s, qq, N);
                 } else {
-                    const double rad = (d.geomy == 3) ? d.radx[qq] : 1.0;
-                    double f = dt / d.yv[s];
-                    D.r *= f; D.u *= f; D.v *= f; D.w *= f;
-                    if (d.geomy > 2) {
-                        f = 1.0 / rad;
-                        D.r *= f; D.u *= f; D.v *= f; D.w *= f;
-                    }
-                    if (d.geomy == 3) D.u += (d.rot[qq] + rad * d.frame_omega) * D.r;
-                    else D.u += d.rot[qq] * D.r;
-                    const DCell E{D.r, D.w, D.u, D.v};
-                    const DCell N = update_dust(d, Q, E);
+                    double v0 = d.rot[qq];
+                    if (d.geomy == 3) v0 += d.radx[qq] * d.frame_omega;
+                    const DCell N = update_dust(d, Q, DCell{Dr, net(2), net(1) + v0 * Dr, 0.0});
                     if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
                     int j = s;
                     if (d.orbadv) {  // TD[(j+inc) mod N] = CD[j] (orbit.cu:30-46)
@@ -237,14 +205,14 @@ __global__ void __launch_bounds__(DS_THREADS) k_dsweep(const __grid_constant__ C
 
 // ===================================================== dust residual advection
 // advection() on Dust (advection.cu:175-233) + advecty (:235-290): the gas's
-// residual speed orb_res, fields (r, v, w, u), update_Dust.
-__global__ void __launch_bounds__(DS_THREADS) k_dadvect(const __grid_constant__ CUtensorMap tm, const DiskView d,
-                                                       pg_dust* __restrict__ out, int ntx, int ntiles) {
+// residual speed orb_res, fields (r, v, u), update_Dust.
+__global__ void __launch_bounds__(DS_THREADS, DS_MINB)
+    k_dadvect(const __grid_constant__ CUtensorMap tm, const DiskView d, pg_dust* __restrict__ out, int ntx, int ntiles) {
     extern __shared__ __align__(128) double smem_raw[];
     double* smem = smem_base128(smem_raw);
     auto stage = [&](int n) { return smem + (n & 1) * DS_STAGE; };
-    double* fl = smem + 2 * DS_STAGE;  // [4][DA_NF] upwind fluxes, indexed by face t
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 4 * DA_NF);
+    double* fl = smem + 2 * DS_STAGE;  // [3][DA_NF] upwind fluxes, indexed by face t
+    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 3 * DA_NF);
     Scalars* sc = d.sc;
     if (sc->done) return;
     const int tid = threadIdx.x;
@@ -256,8 +224,8 @@ __global__ void __launch_bounds__(DS_THREADS) k_dadvect(const __grid_constant__ 
     auto issue = [&](int tile, int k) {
         int s0, q0;
         origin(tile, s0, q0);
-        issue_begin(&bar[k & 1], DSY_TILE * 8);
-        tma_load_2d(stage(k), &tm, 4 * (q0 - 1), s0 - NPAD, &bar[k & 1]);
+        issue_begin(&bar[k & 1], DS_TILE * 8);
+        tma_load_2d(stage(k), &tm, 4 * q0, s0 - NPAD, &bar[k & 1]);
     };
     pipe_init(bar);
     if ((int)blockIdx.x >= ntiles) return;
@@ -277,47 +245,28 @@ __global__ void __launch_bounds__(DS_THREADS) k_dadvect(const __grid_constant__ 
             const int s = min(s0 - NPAD + t, d.yarr - 1);
             const int i = min(q0 + q, d.xarr - 1);
             const double speed = d.res[i];
-            const double rad = (d.geomy == 3) ? d.radx[i] : 1.0;
-            const double sdt = dt / rad;
-            double r[5], u[5], v[5], w[5];
+            const double sdt = dt * ((d.geomy == 3) ? d.irad[i] : 1.0);
+            const double* wt = d.wy + 6 * s;
+            const Frac x = frac(lesser(fabs(speed) * (sdt * d.idx_y[s]), 1.0));
+            const bool up = speed > 0.0;  // this cell is upwind of its upper face, else of its lower one
+            double r[5], u[5], v[5];
 #pragma unroll
             for (int m = 0; m < 5; ++m) {
-                const double* c = T + ((t - 2 + m) * DSY_COLS + (q + 1)) * 4;
-                r[m] = c[0];
-                u[m] = c[2];
-                v[m] = c[3];
-                w[m] = c[1];
+                const double2* c = reinterpret_cast<const double2*>(T + ((t - 2 + m) * DS_W + q) * 4);
+                const double2 ru = c[0];
+                r[m] = ru.x;
+                u[m] = ru.y;
+                v[m] = c[1].x;
             }
-            const double* wt = d.wy + 6 * s;
-            const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], 0.0);
-            const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], 0.0);
-            const Par V = recon(wt, v[0], v[1], v[2], v[3], v[4], 0.0);
-            const Par W = recon(wt, w[0], w[1], w[2], w[3], w[4], 0.0);
-            const double xl = d.ya[s], xr = d.ya[s + 1];
-            double fr, fu, fv, fw;
-            int face;
-            if (speed > 0.0) {
-                const double x0 = xr - speed * sdt;
-                const Frac fq = frac_right(lim01((x0 - xl) / (xr - xl)));
-                fr = aveR(fq, R);
-                fu = aveR(fq, U) * fr;
-                fv = aveR(fq, V) * fr;
-                fw = aveR(fq, W) * fr;
-                face = t + 1;
-            } else {
-                const double x0 = xl - speed * sdt;
-                const Frac fq = frac_left(lim01((x0 - xl) / (xr - xl)));
-                fr = aveL(fq, R);
-                fu = aveL(fq, U) * fr;
-                fv = aveL(fq, V) * fr;
-                fw = aveL(fq, W) * fr;
-                face = t;
-            }
-            const int k = face * DS_W + q;
-            fl[k] = fr * speed;
-            fl[DA_NF + k] = fu * speed;
-            fl[2 * DA_NF + k] = fv * speed;
-            fl[3 * DA_NF + k] = fw * speed;
+            auto ave = [&](const double* a) {
+                const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], 0.0);
+                return up ? aveR(x, A) : aveL(x, A);
+            };
+            const double m = ave(r) * speed;
+            double* o = fl + (t + (up ? 1 : 0)) * DS_W + q;
+            o[0] = m;
+            o[DA_NF] = ave(u) * m;
+            o[2 * DA_NF] = ave(v) * m;
         }
         __syncthreads();
         if (tid < DS_LEN * DS_W) {
@@ -325,21 +274,11 @@ __global__ void __launch_bounds__(DS_THREADS) k_dadvect(const __grid_constant__ 
             const int s = s0 + o, i = q0 + q;
             if (s < NPAD + d.yres && i < NPAD + d.xres) {
                 const int t = NPAD + o;
-                const int k0 = t * DS_W + q, k1 = (t + 1) * DS_W + q;
-                DCell D;
-                D.r = fl[k0] * 1.0 - fl[k1] * 1.0;
-                D.u = fl[DA_NF + k0] * 1.0 - fl[DA_NF + k1] * 1.0;
-                D.v = fl[2 * DA_NF + k0] * 1.0 - fl[2 * DA_NF + k1] * 1.0;
-                D.w = fl[3 * DA_NF + k0] * 1.0 - fl[3 * DA_NF + k1] * 1.0;
-                double f = dt / d.yv[s];
-                D.r *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (d.geomy > 2) {
-                    f = 1.0 / ((d.geomy == 3) ? d.radx[i] : 1.0);
-                    D.r *= f; D.u *= f; D.v *= f; D.w *= f;
-                }
-                const double* c = T + (t * DSY_COLS + (q + 1)) * 4;
-                const DCell Q{c[0], c[1], c[2], c[3]};
-                const DCell N = update_dust(d, Q, DCell{D.r, D.w, D.u, D.v});
+                const double* f0 = fl + t * DS_W + q;
+                const double f = dt * d.iyv[s] * ((d.geomy == 3) ? d.irad[i] : 1.0);
+                auto net = [&](int k) { return (f0[k * DA_NF] - f0[k * DA_NF + DS_W]) * f; };
+                const double* c = T + (t * DS_W + q) * 4;
+                const DCell N = update_dust(d, DCell{c[0], c[1], c[2], c[3]}, DCell{net(0), net(1), net(2), 0.0});
                 if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
                 emit_dust(d, out, i, s, N);
             }

@@ -6,6 +6,7 @@
 #pragma once
 
 #include "pg_common.cuh"
+#include "pg_hydro.cuh"
 
 namespace pg {
 
@@ -53,27 +54,18 @@ __device__ __forceinline__ void emit_dust(const DiskView& d, pg_dust* out, int i
     }
 }
 
-// update_Dust (dust.cu:149-176)
+// update_Dust (dust.cu:149-176); w, zero in 2D, stays
 __device__ __forceinline__ DCell update_dust(const DiskView& d, DCell Q, const DCell& D) {
     const double r_min = fmax(Q.r * 1.0e-10, d.dust_rmin);
-    const double u_old = Q.u, v_old = Q.v, w_old = Q.w;
-    Q.u *= Q.r;
-    Q.v *= Q.r;
-    Q.w *= Q.r;
-    Q.r += D.r;
-    Q.u += D.u;
-    Q.v += D.v;
-    Q.w += D.w;
-    const double ir = 1.0 / Q.r;
-    Q.u *= ir;
-    Q.v *= ir;
-    Q.w *= ir;
-    if (Q.r < r_min) {
+    const double r = Q.r + D.r;
+    if (r < r_min) {
         Q.r = r_min;
-        Q.u = u_old;
-        Q.v = v_old;
-        Q.w = w_old;
+        return Q;
     }
+    const double ir = inv(r);
+    Q.u = (Q.u * Q.r + D.u) * ir;
+    Q.v = (Q.v * Q.r + D.v) * ir;
+    Q.r = r;
     return Q;
 }
 

@@ -391,8 +391,8 @@ static pg_status make_cell_maps(CellMaps& M, const Cell* buf, int xarr, int yarr
 static pg_status make_dust_maps(DustMaps& M, const pg_dust* buf, int xarr, int yarr) {
     if (M.base == buf) return PG_OK;
     pg_status s;
-    if ((s = make_map(&M.sweep_x, buf, 4ull * xarr, yarr, 4 * 38, 8)) != PG_OK) return s;
-    if ((s = make_map(&M.sweep_y, buf, 4ull * xarr, yarr, 4 * 10, 38)) != PG_OK) return s;
+    if ((s = make_map(&M.sweep_x, buf, 4ull * xarr, yarr, 4 * 38, DUST_W)) != PG_OK) return s;
+    if ((s = make_map(&M.sweep_y, buf, 4ull * xarr, yarr, 4 * DUST_W, 38)) != PG_OK) return s;
     M.base = buf;
     return PG_OK;
 }

@@ -39,11 +39,12 @@ struct VisMaps {
     const void* base = nullptr;
     CUtensorMap stencil;   // box {2*34, 10}
 };
+constexpr int DUST_W = 4;  // pencils per tile of the dust passes
 // Tensor maps of one AoS dust buffer (4 doubles per cell).
 struct DustMaps {
     const void* base = nullptr;
-    CUtensorMap sweep_x;   // box {4*38, 8}
-    CUtensorMap sweep_y;   // box {4*10, 38}
+    CUtensorMap sweep_x;   // box {4*38, DUST_W}
+    CUtensorMap sweep_y;   // box {4*DUST_W, 38}
 };
 
 // Pass inputs of one FP64 step, saved for its adjoint (pg_adjoint.cu).
