@@ -675,6 +675,7 @@ struct Engine3 {
     double* tables = nullptr;
     double* stage = nullptr;
     size_t stage_n = 0;
+    HostCopy readback;  // staging of large reads of the state
     Scalars* sc = nullptr;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     int cur = 0;
@@ -1180,8 +1181,7 @@ pg_status pg_disk3_get_state(pg_disk3* dk, double* r, double* p, double* u, doub
     k3_extract<<<1184, 256, 0, E.stream>>>(E.v, E.buf[E.cur], st, st + n, st + 2 * n, st + 3 * n, st + 4 * n);
     PG3_CUDA(cudaGetLastError());
     double* dst[5] = {r, p, u, v, w};
-    for (int f = 0; f < 5; ++f)
-        PG3_CUDA(cudaMemcpyAsync(dst[f], st + f * n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
+    PG3_CUDA(copy_planes_out(E.readback, E.device, st, dst, 5, n, E.stream));
     if (t_out) PG3_CUDA(cudaMemcpyAsync(t_out, &E.sc->t, sizeof(double), cudaMemcpyDeviceToHost, E.stream));
     PG3_CUDA(cudaStreamSynchronize(E.stream));
     return PG_OK;

@@ -460,6 +460,7 @@ struct Engine {
     bool pending = false;
     int cur_base = 0;
     long long steps_base = 0;
+    HostCopy readback;  // staging of large reads of the state
     cudaGraphExec_t graph[2] = {nullptr, nullptr};   // pg_disk_run: one step from buffer k
     cudaGraphExec_t sgraph[2] = {nullptr, nullptr};  // pg_disk_solve: the step after k_set_time, from buffer k
     std::vector<const void*> ghosted;  // buffers whose constant radial ghosts are initialised
@@ -1148,10 +1149,8 @@ pg_status pg_disk_get_state(pg_disk* dk, double* r, double* p, double* u, double
     if (s0 != PG_OK) return s0;
     k_extract<<<1184, 256, 0, E.stream>>>(d, E.buf[E.cur], stage, stage + n, stage + 2 * n, stage + 3 * n);
     PG_CUDA(cudaGetLastError());
-    PG_CUDA(cudaMemcpyAsync(r, stage, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    PG_CUDA(cudaMemcpyAsync(p, stage + n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    PG_CUDA(cudaMemcpyAsync(u, stage + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    if (v) PG_CUDA(cudaMemcpyAsync(v, stage + 3 * n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
+    double* const dst[4] = {r, p, u, v};
+    PG_CUDA(copy_planes_out(E.readback, E.device, stage, dst, v ? 4 : 3, n, E.stream));
     if (t_out) PG_CUDA(cudaMemcpyAsync(t_out, &E.sc->t, sizeof(double), cudaMemcpyDeviceToHost, E.stream));
     PG_CUDA(cudaStreamSynchronize(E.stream));
     return PG_OK;
@@ -1199,9 +1198,8 @@ pg_status pg_disk_get_dust(pg_disk* dk, double* r, double* u, double* v) {
     }
     launch_dust_extract(d, E.dbuf[E.cur], stage, stage + n, stage + 2 * n, E.stream);
     PG_CUDA(cudaGetLastError());
-    PG_CUDA(cudaMemcpyAsync(r, stage, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    PG_CUDA(cudaMemcpyAsync(u, stage + n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
-    PG_CUDA(cudaMemcpyAsync(v, stage + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, E.stream));
+    double* const dst[3] = {r, u, v};
+    PG_CUDA(copy_planes_out(E.readback, E.device, stage, dst, 3, n, E.stream));
     PG_CUDA(cudaStreamSynchronize(E.stream));
     return PG_OK;
 }

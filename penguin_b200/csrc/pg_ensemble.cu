@@ -91,6 +91,7 @@ struct pg_ens {
     Tune32 tune = DEFAULT_TUNE32;  // launch configuration of the passes (pg_ens_autotune)
     double* xfer = nullptr;        // device staging of host exchanges, kept between calls
     size_t xfer_n = 0;
+    HostCopy readback;  // staging of large reads of the state
 
     ~pg_ens() {
         for (auto& g : graph)
@@ -406,10 +407,8 @@ pg_status pg_ens_get_state(pg_ens* e, int k, double* r, double* p, double* u, do
     }
     launch_extract32(e->dV + k, e->cur, st, st + n, st + 2 * n, st + 3 * n, e->stream);
     ENS_CUDA(cudaGetLastError());
-    ENS_CUDA(cudaMemcpyAsync(r, st, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    ENS_CUDA(cudaMemcpyAsync(p, st + n, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    ENS_CUDA(cudaMemcpyAsync(u, st + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    ENS_CUDA(cudaMemcpyAsync(v, st + 3 * n, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+    double* const dst[4] = {r, p, u, v};
+    ENS_CUDA(copy_planes_out(e->readback, e->device, st, dst, 4, n, e->stream));
     if (t_out) ENS_CUDA(cudaMemcpyAsync(t_out, &D.v.d64.sc->t, sizeof(double), cudaMemcpyDeviceToHost, e->stream));
     ENS_CUDA(cudaStreamSynchronize(e->stream));
     return PG_OK;
@@ -580,9 +579,8 @@ pg_status pg_ens_get_dust(pg_ens* e, int k, double* r, double* u, double* v) {
     }
     launch_dextract32(e->dV + k, e->cur, st, st + n, st + 2 * n, e->stream);
     ENS_CUDA(cudaGetLastError());
-    ENS_CUDA(cudaMemcpyAsync(r, st, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    ENS_CUDA(cudaMemcpyAsync(u, st + n, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    ENS_CUDA(cudaMemcpyAsync(v, st + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
+    double* const dst[3] = {r, u, v};
+    ENS_CUDA(copy_planes_out(e->readback, e->device, st, dst, 3, n, e->stream));
     ENS_CUDA(cudaStreamSynchronize(e->stream));
     return PG_OK;
 }

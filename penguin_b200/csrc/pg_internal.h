@@ -101,6 +101,23 @@ double compensated_sum(const double* a, int n);
 int kernels_per_step(const DiskView& d);
 void set_last_error(const char* msg);
 
+// `planes` planes of `count` doubles, back to back in device memory, to host arrays
+// (pg_hostcopy.cu), ordered after s's work; the caller synchronizes s.  The pinned staging
+// (8 MB) is kept with the disk from its first large read on.
+constexpr int COPY_THREADS = 4;
+struct HostCopy {
+    static constexpr size_t SLOT = (size_t)1 << 17;  // doubles
+    double* pinned = nullptr;
+    cudaEvent_t ev[COPY_THREADS][2] = {};
+    HostCopy() = default;
+    HostCopy(const HostCopy&) = delete;
+    HostCopy& operator=(const HostCopy&) = delete;
+    ~HostCopy();
+    double* slot(int w, int k) const { return pinned + (2 * w + k) * SLOT; }
+};
+cudaError_t copy_planes_out(HostCopy& h, int device, const double* src, double* const* dst, int planes, size_t count,
+                            cudaStream_t s);
+
 // tables-only disks and FP32 tensor maps for the FP32 form (pg_engine.cu)
 struct Engine;
 // FP64 disks driven by the adjoint (pg_engine.cu)
