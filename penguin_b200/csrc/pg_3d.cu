@@ -14,13 +14,13 @@
 //                    (src/timestep/timestep.cu:18-97, ndim 3)
 //
 // plus the one-thread clock kernel and the per-row planet angle table of the 2D
-// form.  The sweeps are persistent CTAs that stage each tile (32 outputs along
-// the sweep plus 3 ghosts a side, 4 pencils) with one 3D TMA box copy, two
-// stages in flight, and compute it in three phases (reconstruction and both
-// edge states per cell, HLLC per face, update per cell) with the 2D form's
-// building blocks (pg_hydro.cuh).  Each pass writes the ghost cells the next
-// pass reads (the images the reference's boundx/boundy/boundz copy in place),
-// so no boundary pass runs between stages.
+// form.  Lanes of a warp lie along the radius in every pass.  The radial sweep stages
+// rows with TMA and exchanges edge states and fluxes between lanes by shuffle; the
+// azimuthal and polar sweeps march along their direction with five cells of a column in
+// registers (the 2D form's work layout, pg_kernels.cu, and its building blocks,
+// pg_hydro.cuh).  Each pass writes the ghost cells the next pass reads (the images the
+// reference's boundx/boundy/boundz copy in place), so no boundary pass runs between
+// stages.
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -36,22 +36,16 @@
 
 namespace pg {
 
-// ------------------------------------------------------------ tile shape
-constexpr int S3_W = 4;                       // pencils per tile
-constexpr int S3_L = 32;                      // outputs per pencil
-constexpr int S3_TL = S3_L + 2 * NPAD;        // tile cells along the sweep
-constexpr int S3_P1 = S3_L + 2;               // cells reconstructed per pencil
-constexpr int S3_P2 = S3_L + 1;               // faces per pencil
-constexpr int S3_NST = S3_P1 * S3_W;
-constexpr int S3_NFX = S3_P2 * S3_W;
-constexpr int S3_THREADS = (S3_NST + 31) / 32 * 32;
-constexpr int S3_COLS = S3_W + 2;             // y/z tiles start one column early (16-byte TMA x)
-constexpr int S3_TILE = (S3_TL * S3_COLS * 5 + 15) / 16 * 16;  // doubles, covers the x tile too
-constexpr int S3_NS = 2;
-constexpr size_t S3_SMEM = (size_t)(S3_NS * S3_TILE + 10 * S3_NST + 7 * S3_NFX) * 8 + 8 * S3_NS + 128;
+// ------------------------------------------------------------ work layout
+constexpr int S3_WARPS = 4;                          // warps per CTA, independent of one another
+constexpr int S3_THREADS = 32 * S3_WARPS;
+constexpr int S3_OUT = 30;                           // radial sweep: outputs of a warp's 32 cells
+constexpr int S3_ROWS = RX_TILE_ROWS;                // rows per TMA copy
+constexpr int S3_STAGE = RX_TILE_CELLS * S3_ROWS * 5;  // doubles
 constexpr int K3_THREADS = 256;
-static_assert(S3_W * S3_TL * 5 <= S3_TILE, "the radial tile fits a stage");
-static_assert(5 * S3_TL <= 256 && 5 * S3_COLS <= 256 && S3_TL <= 256, "TMA boxes are at most 256 wide");
+constexpr size_t S3_SMEM = (size_t)S3_WARPS * 2 * S3_STAGE * 8 + S3_WARPS * 16 + 128;
+static_assert(S3_STAGE * 8 % 128 == 0, "128-byte aligned stages");
+static_assert(RX_TILE_CELLS == S3_OUT + 6, "32 lanes and two stencil cells a side");
 
 // Everything a 3D kernel reads: the 2D view's scalars, grid and tables for x
 // and y (and the clock), plus the polar grid and the (x, z) tables.
@@ -145,222 +139,224 @@ __device__ __forceinline__ void emit_z(const View3& v, Cell* out, int i, int j, 
 }
 
 // ================================================================ sweeps
-// DIR 0 radial pencils (tile rows j, one plane k), DIR 1 azimuthal pencils
-// (columns i, one plane k), DIR 2 polar pencils (columns i, one row j).
-// Tile t: a = t % nta along the sweep, b = (t / nta) % ntb across the pencils,
-// c = t / (nta ntb) the plane (DIR 0, 1) or row (DIR 2).
-// 4 CTAs per SM (96 registers; the radial instance spills 12 bytes): 20 warps
-// instead of the 15 its natural 106-110 registers allow, 8-11 % faster
-template <int DIR>
-__global__ void __launch_bounds__(S3_THREADS, 4)
-    k3_sweep(const __grid_constant__ CUtensorMap tm, const View3 v, Cell* __restrict__ out, int nta, int ntb,
-             int ntiles) {
+__device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double down1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+
+// Net flux through a cell's two faces.  The reference stores each flux times its area in
+// shared memory before differencing, so the products are rounded on their own
+// (__dmul_rn: no FMA).
+__device__ __forceinline__ double net3(double f0, double g0, double f1, double g1) {
+    return __dmul_rn(f0, g0) - __dmul_rn(f1, g1);
+}
+// the slots' increments (before the geometric factor) from the fluxes of the two faces
+// (src/solver/riemann/riemann.cu:40-87)
+__device__ __forceinline__ Cell increments(const DiskView& d, const Flux& a, double g0, const Flux& b, double g1) {
+    Cell D;
+    D.r = net3(a.r, g0, b.r, g1);
+    D.u = net3(a.u, g0, b.u, g1) + 0.5 * (g0 + g1) * (a.pres - b.pres);
+    D.v = net3(a.v, g0, b.v, g1);
+    D.w = net3(a.w, g0, b.w, g1);
+    D.p = 0.0;
+    if (d.eos == 2) {
+        double de = net3(a.uprs, g0, b.uprs, g1);
+        if (d.ie != 0) de *= 0.5 * (a.pres + b.pres);
+        D.p = net3(a.p, g0, b.p, g1) + de;
+    }
+    return D;
+}
+
+// Radial sweep (sweeps.cu:263-335) of rows j of one plane k: 4 rows of 36 cells per TMA
+// copy, two copies in flight per warp; lane l holds cell 2 + 30 seg + l.  Compiled for MB
+// CTAs per SM: 3 (168 registers) when warps are few and each runs alone on its scheduler, 4
+// (128 registers, some spilled) when there are rows enough for all: 48x40x36 13.0 / 14.4 us,
+// 128x256x72 166 / 143 us at 3 / 4.
+template <int MB>
+__global__ void __launch_bounds__(S3_THREADS, MB)
+    k3_sweep_x(const __grid_constant__ CUtensorMap tm, const View3 v, Cell* __restrict__ out, int nseg, int len,
+               int nchunk, int nitems) {
     extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    double* st = smem + S3_NS * S3_TILE;  // [10][S3_NST] edge states
-    double* fl = st + 10 * S3_NST;        // [7][S3_NFX] fluxes
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 7 * S3_NFX);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* buf = smem_base128(smem_raw) + (size_t)warp * 2 * S3_STAGE;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_base128(smem_raw) + (size_t)S3_WARPS * 2 * S3_STAGE) + 2 * warp;
     const DiskView& d = v.d;
     Scalars* sc = d.sc;
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncwarp();
+    pdl_enter();
     if (sc->done) return;
-
-    const int tid = threadIdx.x;
-    const double dt = sc->dt;
-    const double gam = d.gam;
-    const int res = DIR == 0 ? d.xres : (DIR == 1 ? d.yres : v.zres);  // cells along the sweep
-    const int qres = DIR == 0 ? d.yres : d.xres;                         // pencils
-    const int arr = DIR == 0 ? d.xarr : (DIR == 1 ? d.yarr : v.zarr);
-    constexpr uint32_t BYTES = (DIR == 0 ? S3_W * S3_TL * 5 : S3_COLS * S3_TL * 5) * 8;
-    auto origin = [&](int tile, int& s0, int& q0, int& c) {
-        const int r = tile / nta;
-        s0 = NPAD + S3_L * (tile % nta);  // first output along the sweep
-        q0 = NPAD + S3_W * (r % ntb);     // first pencil
-        c = NPAD + r / ntb;               // plane k (DIR 0, 1) or row j (DIR 2)
-    };
-    auto issue = [&](int tile, int k) {
-        int s0, q0, c;
-        origin(tile, s0, q0, c);
-        double* dst = smem + (k % S3_NS) * S3_TILE;
-        issue_begin(&bar[k % S3_NS], BYTES);
-        if (DIR == 0) tma_load_3d(dst, &tm, 5 * (s0 - NPAD), q0, c, &bar[k % S3_NS]);
-        else if (DIR == 1) tma_load_3d(dst, &tm, 5 * (q0 - 1), s0 - NPAD, c, &bar[k % S3_NS]);
-        else tma_load_3d(dst, &tm, 5 * (q0 - 1), c, s0 - NPAD, &bar[k % S3_NS]);
-    };
-    pipe_init<S3_NS>(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, ++kt) {
-        const int ahead = (tile + (int)gridDim.x < ntiles) ? 1 : 0;
-        if (tid == 0 && ahead) issue(tile + gridDim.x, kt + 1);
-        int s0, q0, c;
-        origin(tile, s0, q0, c);
-        const double* tl = smem + (kt % S3_NS) * S3_TILE;
-        if (!pipe_wait<S3_NS>(bar, kt, sc)) {
-            pipe_drain<S3_NS>(bar, kt, ahead, sc);
-            return;
+    const double dt = sc->dt, gam = d.gam;
+    int n = 0;  // copies waited for by this warp
+    for (int item = blockIdx.x * S3_WARPS + warp; item < nitems; item += gridDim.x * S3_WARPS) {
+        const int seg = item % nseg, rest = item / nseg;
+        const int k = NPAD + rest / nchunk;
+        const int j0 = NPAD + len * (rest % nchunk), j1 = min(j0 + len, NPAD + d.yres);
+        auto issue = [&](int j, int m) {
+            issue_begin(&bar[m & 1], S3_STAGE * 8);
+            tma_load_3d(buf + (m & 1) * S3_STAGE, &tm, 5 * S3_OUT * seg, j, k, &bar[m & 1]);
+        };
+        if (lane == 0) {
+            issue(j0, n);
+            if (j0 + S3_ROWS < j1) issue(j0 + S3_ROWS, n + 1);
         }
+        const int i = NPAD - 1 + S3_OUT * seg + lane, ic = min(i, d.xarr - 1);
+        const bool output = lane >= 1 && lane <= S3_OUT && i < NPAD + d.xres;
+        double w[6], rad[5];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) w[m] = d.wx[6 * ic + m];
+        // angular momenta r sin(theta) v_phi and r v_theta (sweeps.cu:283-300)
+        const double sz = d.geomx == 2 ? v.sinz[k] : 1.0;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) rad[m] = d.geomx != 0 ? d.radx[min(max(i - 2 + m, 0), d.xarr - 1)] : 1.0;
+        const bool third = d.geomx == 2;
+        const double sx = dt * d.idx_x[ic], f = dt * inv(d.xv[ic]);
+        const double g0 = v.gfx[ic], g1 = v.gfx[ic + 1];
+        const double ir = d.geomx != 0 ? inv(rad[2]) : 1.0, irs = d.geomx != 0 ? inv(rad[2] * sz) : 1.0;
+        const double cs2 = v.cs2[ic + d.xarr * k];
+#pragma unroll 1
+        for (int j = j0; j < j1; j += S3_ROWS, ++n) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&bar[n & 1], (uint32_t)((n >> 1) & 1), sc))) {
+                if (lane == 0 && j + S3_ROWS < j1) mbar_wait(&bar[(n + 1) & 1], (uint32_t)(((n + 1) >> 1) & 1), sc);
+                return;
+            }
+            const double* row = buf + (n & 1) * S3_STAGE + 5 * (lane + 2);
+#pragma unroll 1
+            for (int jj = j; jj < min(j + S3_ROWS, j1); ++jj, row += 5 * RX_TILE_CELLS) {
+                const Cell C0{row[0], row[1], row[2], row[3], row[4]};
+                const double cs0 = sound_speed(gam, C0.r, C0.p);
+                const double flat = flatten(C0.p, row[-9], row[-4], row[6], row[11], row[-3], C0.u, row[7]);
+                auto field = [&](int m) { return recon(w, row[m - 10], row[m - 5], row[m], row[m + 5], row[m + 10], flat); };
+                auto momentum = [&](int m, double g) {
+                    return recon(w, row[m - 10] * (rad[0] * g), row[m - 5] * (rad[1] * g), row[m] * (rad[2] * g),
+                                 row[m + 5] * (rad[3] * g), row[m + 10] * (rad[4] * g), flat);
+                };
+                const Par R = field(0), P = field(1), U = field(2), A = momentum(3, sz);
+                const Par Z = third ? momentum(4, 1.0) : field(4);
+                const Half eL = state_at_left_edge(gam, sx, cs0, C0.r, C0.p, C0.u, R, P, U, A, Z);
+                const Half eR = state_at_right_edge(gam, sx, cs0, C0.r, C0.p, C0.u, R, P, U, A, Z);
+                const Half L{up1(eR.r), up1(eR.p), up1(eR.u), up1(eR.v), up1(eR.w)};
+                const Flux F = hllc(d.eos, d.ie, gam, L, eL);
+                const Flux G{down1(F.r), down1(F.p), down1(F.u), down1(F.v), down1(F.w), down1(F.pres), down1(F.uprs)};
+                Cell D = increments(d, F, g0, G, g1);
+                D.r *= f; D.p *= f; D.u *= f; D.v *= f * irs; D.w *= f;
+                if (third) D.w *= ir;
+                if (output) {
+                    const Cell Q = update_cell(d.eos, d.ie, gam, cs2, C0, D, &sc->floor_hits);
+                    if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                    emit_y(v, out, i, jj, k, Q);
+                }
+            }
+            __syncwarp();  // the copy's reads are done
+            if (lane == 0 && j + 2 * S3_ROWS < j1) issue(j + 2 * S3_ROWS, n + 2);
+        }
+    }
+}
 
-        // ---- P1: reconstruction and both edge states of every cell
-        for (int it = tid; it < S3_NST; it += S3_THREADS) {
-            const int q = DIR == 0 ? it / S3_P1 : it % S3_W;
-            const int t = 2 + (DIR == 0 ? it % S3_P1 : it / S3_W);
-            const int s = s0 - NPAD + t;
-            const int qq = min(q0 + q, d.xarr - 1);
-            // geometry of the pencil: DIR 1 rad_cyl (sweeps.cu:380-386), DIR 2 rad (:486-489)
-            double radp = 1.0;
-            if (DIR == 1 && d.geomy == 4) radp = d.radx[qq] * v.sinz[c];
-            if (DIR == 2 && v.geomz == 5) radp = d.radx[qq];
-            double r[5], p[5], u[5], vv[5], w[5];
+// Azimuthal (DIR 1, sweeps.cu:361-433) and polar (DIR 2, :458-554) sweeps: a lane marches
+// along its column with five cells in registers and the next in flight, like the 2D
+// azimuthal sweep.  Lines of a plane k (DIR 1) or of a row j (DIR 2).  128x256x72, us a
+// sweep, tiles -> runs: radial 250 -> 143, azimuthal 249 -> 132, polar 363 -> 146; FP64 issue
+// and latency bound all three.  At 2 / 3 / 4 CTAs per SM azimuthal 153 / 132 / 163, polar
+// 165 / 146 / 170.
+template <int DIR>
+__global__ void __launch_bounds__(S3_THREADS, 3)
+    k3_march(const Cell* __restrict__ in, const View3 v, Cell* __restrict__ out, int ncol, int len, int nchunk,
+             int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const DiskView& d = v.d;
+    Scalars* sc = d.sc;
+    pdl_enter();
+    if (sc->done) return;
+    const double dt = sc->dt, gam = d.gam;
+    const int res = DIR == 1 ? d.yres : v.zres;
+    const bool sph = DIR == 1 ? d.geomy == 4 : v.geomz == 5;
+    const double* wtab = DIR == 1 ? d.wy : v.wz;
+    const double* idx = DIR == 1 ? d.idx_y : v.idx_z;
+    const double* vol = DIR == 1 ? d.yv : v.zv;
+    const size_t pitch = 5 * (DIR == 1 ? (size_t)d.xarr : (size_t)d.xarr * d.yarr);
+    for (int item = blockIdx.x * S3_WARPS + warp; item < nitems; item += gridDim.x * S3_WARPS) {
+        const int i = NPAD + 32 * (item % ncol) + lane, rest = item / ncol;
+        const int s0 = NPAD + len * (rest % nchunk), s1 = min(s0 + len, NPAD + res);
+        const int line = NPAD + rest / nchunk;  // k (DIR 1) or j (DIR 2)
+        const bool active = i < NPAD + d.xres;
+        const int ic = min(i, NPAD + d.xres - 1);
+        // DIR 1 rad_cyl (sweeps.cu:380-386), DIR 2 rad (:486-489)
+        const double rad = sph ? (DIR == 1 ? d.radx[ic] * v.sinz[line] : d.radx[ic]) : 1.0;
+        const double irad = sph ? inv(rad) : 1.0;
+        const double v0 = DIR == 1 && sph ? rad * d.frame_omega : 0.0;  // the frame's rotation (:388-396)
+        const double sdt = dt * irad;  // set_state receives dt/rad (riemann.cu:111)
+        const double* next = reinterpret_cast<const double*>(
+            in + (DIR == 1 ? at3(v, ic, s0 - NPAD, line) : at3(v, ic, line, s0 - NPAD)));
+        double q[5][5], nx[5];
+#pragma unroll
+        for (int m = 0; m < 5; ++m, next += pitch)
+#pragma unroll
+            for (int c = 0; c < 5; ++c) q[m][c] = next[c];
+        Half pr{};
+        Flux pf{};
+#pragma unroll 1
+        for (int t = s0 - 1; t <= s1; ++t, next += pitch) {
+            if (t < s1) {
+#pragma unroll
+                for (int c = 0; c < 5; ++c) nx[c] = next[c];
+            }
+            const double* w = wtab + 6 * t;
+            // sweep order: DIR 1 v_phi, v_theta, v_r; DIR 2 v_theta, v_r, r sin(theta) v_phi
+            constexpr int cu = DIR == 1 ? 3 : 4, ca = DIR == 1 ? 4 : 2, cz = DIR == 1 ? 2 : 3;
+            double u[5], z[5];
 #pragma unroll
             for (int m = 0; m < 5; ++m) {
-                const double* cp = DIR == 0 ? tl + (q * S3_TL + (t - 2 + m)) * 5 : tl + ((t - 2 + m) * S3_COLS + q + 1) * 5;
-                const int sm = min(max(s - 2 + m, 0), arr - 1);
-                r[m] = cp[0];
-                p[m] = cp[1];
-                if (DIR == 0) {  // angular momenta r sin(theta) v_phi and r v_theta (sweeps.cu:283-300)
-                    u[m] = cp[2];
-                    vv[m] = cp[3];
-                    w[m] = cp[4];
-                    if (d.geomx == 2) {
-                        const double rad = d.radx[sm];
-                        vv[m] *= rad * v.sinz[c];
-                        w[m] *= rad;
-                    } else if (d.geomx == 1) {
-                        vv[m] *= d.radx[sm];
-                    }
-                } else if (DIR == 1) {  // residual of the frame rotation (sweeps.cu:388-396)
-                    u[m] = cp[3];
-                    if (d.geomy == 4) u[m] -= radp * d.frame_omega;
-                    vv[m] = cp[4];
-                    w[m] = cp[2];
-                } else {  // r sin(theta) v_phi of each cell of the pencil (sweeps.cu:491-500)
-                    u[m] = cp[4];
-                    vv[m] = cp[2];
-                    w[m] = cp[3];
-                    if (v.geomz == 5) w[m] *= radp * v.sinz[sm];
+                u[m] = DIR == 1 ? q[m][cu] - v0 : q[m][cu];
+                z[m] = q[m][cz];
+                if (DIR == 2 && sph) z[m] *= rad * v.sinz[t - 2 + m];
+            }
+            const double cs0 = sound_speed(gam, q[2][0], q[2][1]);
+            const double flat = flatten(q[2][1], q[0][1], q[1][1], q[3][1], q[4][1], u[1], u[2], u[3]);
+            const double sx = sdt * idx[t];
+            auto field = [&](int m) { return recon(w, q[0][m], q[1][m], q[2][m], q[3][m], q[4][m], flat); };
+            const Par R = field(0), P = field(1), A = field(ca);
+            const Par U = recon(w, u[0], u[1], u[2], u[3], u[4], flat);
+            const Par Z = recon(w, z[0], z[1], z[2], z[3], z[4], flat);
+            const Half eL = state_at_left_edge(gam, sx, cs0, q[2][0], q[2][1], u[2], R, P, U, A, Z);
+            const Half eR = state_at_right_edge(gam, sx, cs0, q[2][0], q[2][1], u[2], R, P, U, A, Z);
+            Flux F{};
+            if (t >= s0) F = hllc(d.eos, d.ie, gam, pr, eL);
+            if (t > s0) {  // the cell below has both its fluxes
+                const int s = t - 1;
+                const double g0 = DIR == 1 ? 1.0 : v.gfz[s], g1 = DIR == 1 ? 1.0 : v.gfz[s + 1];
+                Cell D = increments(d, pf, g0, F, g1);
+                const double f = sdt * inv(vol[s]);
+                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
+                const Cell C0{q[1][0], q[1][1], q[1][2], q[1][3], q[1][4]};
+                if (DIR == 1) {  // sweeps.cu:403-425 (orb_rot 0)
+                    D = Cell{D.r, D.p, D.w, D.u + v0 * D.r, D.v};
+                } else {  // sweeps.cu:507-532
+                    double Dz = D.w;
+                    if (sph) Dz *= inv(rad * v.sinz[s]);
+                    D = Cell{D.r, D.p, D.v, Dz, D.u};
+                }
+                if (active) {
+                    const int k = DIR == 1 ? line : s;
+                    const Cell Q = update_cell(d.eos, d.ie, gam, v.cs2[i + d.xarr * k], C0, D, &sc->floor_hits);
+                    if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                    if (DIR == 1) emit_z(v, out, i, s, line, Q);
+                    else put3(out, v, i, line, s, Q);
                 }
             }
-            const double cs0 = sound_speed(gam, r[2], p[2]);
-            const double flat = flatten(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
-            const int sc_ = min(s, arr - 1);
-            const double* wt = (DIR == 0 ? d.wx : (DIR == 1 ? d.wy : v.wz)) + 6 * sc_;
-            const double idx = (DIR == 0 ? d.idx_x : (DIR == 1 ? d.idx_y : v.idx_z))[sc_];
-            const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], flat);
-            const Par P = recon(wt, p[0], p[1], p[2], p[3], p[4], flat);
-            const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], flat);
-            const Par V = recon(wt, vv[0], vv[1], vv[2], vv[3], vv[4], flat);
-            const Par W = recon(wt, w[0], w[1], w[2], w[3], w[4], flat);
-            const double sdt = DIR == 0 ? dt : dt * inv(radp);  // set_state receives dt/rad (riemann.cu:111)
-            const Half a = state_at_left_edge(gam, sdt * idx, cs0, r[2], p[2], u[2], R, P, U, V, W);
-            const Half b = state_at_right_edge(gam, sdt * idx, cs0, r[2], p[2], u[2], R, P, U, V, W);
-            st[0 * S3_NST + it] = a.r;
-            st[1 * S3_NST + it] = a.p;
-            st[2 * S3_NST + it] = a.u;
-            st[3 * S3_NST + it] = a.v;
-            st[4 * S3_NST + it] = a.w;
-            st[5 * S3_NST + it] = b.r;
-            st[6 * S3_NST + it] = b.p;
-            st[7 * S3_NST + it] = b.u;
-            st[8 * S3_NST + it] = b.v;
-            st[9 * S3_NST + it] = b.w;
-        }
-        __syncthreads();
-
-        // ---- P2: HLLC flux at every face (left state from cell t-1, right from cell t)
-        for (int it = tid; it < S3_NFX; it += S3_THREADS) {
-            const int q = DIR == 0 ? it / S3_P2 : it % S3_W;
-            const int t = 3 + (DIR == 0 ? it % S3_P2 : it / S3_W);
-            const int iL = DIR == 0 ? q * S3_P1 + (t - 3) : (t - 3) * S3_W + q;
-            const int iR = DIR == 0 ? q * S3_P1 + (t - 2) : (t - 2) * S3_W + q;
-            Half L, R;
-            L.r = st[5 * S3_NST + iL];
-            L.p = st[6 * S3_NST + iL];
-            L.u = st[7 * S3_NST + iL];
-            L.v = st[8 * S3_NST + iL];
-            L.w = st[9 * S3_NST + iL];
-            R.r = st[0 * S3_NST + iR];
-            R.p = st[1 * S3_NST + iR];
-            R.u = st[2 * S3_NST + iR];
-            R.v = st[3 * S3_NST + iR];
-            R.w = st[4 * S3_NST + iR];
-            const Flux F = hllc(d.eos, d.ie, gam, L, R);
-            fl[0 * S3_NFX + it] = F.r;
-            fl[1 * S3_NFX + it] = F.p;
-            fl[2 * S3_NFX + it] = F.u;
-            fl[3 * S3_NFX + it] = F.v;
-            fl[4 * S3_NFX + it] = F.w;
-            fl[5 * S3_NFX + it] = F.pres;
-            fl[6 * S3_NFX + it] = F.uprs;
-        }
-        __syncthreads();
-
-        // ---- P3: flux differences, pressure sources, geometry, conservative update
-        for (int it = tid; it < S3_L * S3_W; it += S3_THREADS) {
-            const int q = DIR == 0 ? it / S3_L : it % S3_W;
-            const int t = 3 + (DIR == 0 ? it % S3_L : it / S3_W);
-            const int s = s0 - NPAD + t;
-            const int qq = q0 + q;
-            if (s >= NPAD + res || qq >= NPAD + qres) continue;
-            const int f0 = DIR == 0 ? q * S3_P2 + (t - 3) : (t - 3) * S3_W + q;
-            const int f1 = DIR == 0 ? f0 + 1 : f0 + S3_W;
-            // net_source (src/solver/riemann/riemann.cu:40-87) with the face areas; the
-            // reference stores each flux times its area in shared memory before
-            // differencing, so the products are rounded on their own (__dmul_rn: no FMA)
-            const double g0 = DIR == 0 ? v.gfx[s] : (DIR == 1 ? 1.0 : v.gfz[s]);
-            const double g1 = DIR == 0 ? v.gfx[s + 1] : (DIR == 1 ? 1.0 : v.gfz[s + 1]);
-            const double pres0 = fl[5 * S3_NFX + f0], pres1 = fl[5 * S3_NFX + f1];
-            const double du = 0.5 * (g0 + g1) * (pres0 - pres1);
-            auto net = [&](int k) { return __dmul_rn(fl[k * S3_NFX + f0], g0) - __dmul_rn(fl[k * S3_NFX + f1], g1); };
-            double de = 0.0;
-            if (d.eos == 2) de = (d.ie == 0) ? net(6) : 0.5 * (pres0 + pres1) * net(6);
-            Cell D;
-            D.r = net(0);
-            D.p = net(1) + de;
-            D.u = net(2) + du;
-            D.v = net(3);
-            D.w = net(4);
-            const double* cp = DIR == 0 ? tl + (q * S3_TL + t) * 5 : tl + (t * S3_COLS + q + 1) * 5;
-            const Cell C0{cp[0], cp[1], cp[2], cp[3], cp[4]};
-            if (DIR == 0) {  // sweeps.cu:306-332
-                const double f = dt / d.xv[s];
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (d.geomx == 2) {
-                    const double rad = d.radx[s];
-                    D.v /= rad * v.sinz[c];
-                    D.w /= rad;
-                } else if (d.geomx == 1) {
-                    D.v /= d.radx[s];
-                }
-                const Cell Q = update_cell(d.eos, d.ie, gam, v.cs2[s + d.xarr * c], C0, D, &sc->floor_hits);
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                emit_y(v, out, s, qq, c, Q);
-            } else if (DIR == 1) {  // sweeps.cu:403-425 (orb_rot 0)
-                const double radp = d.geomy == 4 ? d.radx[qq] * v.sinz[c] : 1.0;
-                const double f = dt / d.yv[s] / radp;
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (d.geomy == 4) D.u += (0.0 + radp * d.frame_omega) * D.r;
-                else D.u += 0.0 * D.r;
-                const Cell E{D.r, D.p, D.w, D.u, D.v};
-                const Cell Q = update_cell(d.eos, d.ie, gam, v.cs2[qq + d.xarr * c], C0, E, &sc->floor_hits);
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                emit_z(v, out, qq, s, c, Q);
-            } else {  // sweeps.cu:507-532
-                const double f = dt / v.zv[s];
-                D.r *= f; D.p *= f; D.u *= f; D.v *= f; D.w *= f;
-                if (v.geomz == 5) {
-                    const double rad = d.radx[qq];
-                    const double g = 1.0 / rad;
-                    D.r *= g; D.p *= g; D.u *= g; D.v *= g; D.w *= g;
-                    D.w /= rad * v.sinz[s];
-                }
-                const Cell E{D.r, D.p, D.v, D.w, D.u};
-                const Cell Q = update_cell(d.eos, d.ie, gam, v.cs2[qq + d.xarr * s], C0, E, &sc->floor_hits);
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                put3(out, v, qq, c, s, Q);
+            pr = eR;
+            pf = F;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                q[0][c] = q[1][c];
+                q[1][c] = q[2][c];
+                q[2][c] = q[3][c];
+                q[3][c] = q[4][c];
+                q[4][c] = nx[c];
             }
         }
-        __syncthreads();  // the stage and the state / flux arrays are free again
     }
 }
 
@@ -371,36 +367,44 @@ __global__ void __launch_bounds__(S3_THREADS, 4)
 struct Grav3 {
     double gx, gy, gz;
 };
-__device__ __forceinline__ Grav3 gravity3(const View3& v, int j, int k, double rad, double pol, const pg_body& pl,
-                                          int which) {
+// the planet's factors of a pass
+struct Planet3 {
+    double m, x, ix2, irs, irs3;
+};
+__device__ __forceinline__ Planet3 planet3(const pg_body& p) {
+    const double irs = 1.0 / p.rs;
+    return Planet3{p.m, p.x, 1.0 / p.x / p.x, irs, irs * irs * irs};
+}
+__device__ __forceinline__ Grav3 gravity3(const View3& v, int j, int k, double rad, double irad, double pol,
+                                          const Planet3& pl, int which) {
     const DiskView& d = v.d;
     Grav3 g{0.0, 0.0, 0.0};
     if (d.geomx != 2) return g;
-    g.gx = -1.0 / rad / rad;
+    g.gx = -irad * irad;
     if (d.nplanet > 0) {
         const double sinfac = d.trig[4 * j + 2 * which], cosfac = d.trig[4 * j + 2 * which + 1];
         const double sinpol = v.sinpol[k], cospol = v.cospol[k];
         const double plm = pl.m, plx = pl.x;
-        const double Rp = sqrt(rad * rad + plx * plx - 2.0 * plx * rad * cosfac * sinpol);
-        const double rs_fac = fmax(4.0 - 3.0 * Rp / pl.rs, 1.0) / fmax(pl.rs * pl.rs * pl.rs, Rp * Rp * Rp);
-        const double fx = -plm * (rad - plx * cosfac * sinpol) * rs_fac - plm * sinpol * cosfac / plx / plx;
-        const double fy = -plm * plx * sinfac * rs_fac + plm * sinpol * sinfac / plx / plx;
-        const double fz = plm * plx * cosfac * cospol * rs_fac - plm * cospol * cosfac / (sinpol * plx * plx);
-        g.gx += fx;
-        g.gy += fy;
-        g.gz += fz;
+        const double R2 = rad * rad + plx * plx - 2.0 * plx * rad * cosfac * sinpol;
+        const double ir = rsq(R2);
+        // max(4 - 3 Rp / rs, 1) / max(rs^3, Rp^3)
+        const double rs_fac = fmax(4.0 - 3.0 * (R2 * ir) * pl.irs, 1.0) * fmin(pl.irs3, ir * ir * ir);
+        g.gx += -plm * (rad - plx * cosfac * sinpol) * rs_fac - plm * sinpol * cosfac * pl.ix2;
+        g.gy += -plm * plx * sinfac * rs_fac + plm * sinpol * sinfac * pl.ix2;
+        g.gz += plm * plx * cosfac * cospol * rs_fac - plm * cospol * cosfac * inv(sinpol) * pl.ix2;
     }
     if (pol < v.zmin) g.gz *= -1.0;
     return g;
 }
-__device__ __forceinline__ void fict3(const View3& v, int k, double rad, double pol, const Cell& T, double& fx,
+__device__ __forceinline__ void fict3(const View3& v, double irad, double itan, double pol, const Cell& T, double& fx,
                                       double& fy, double& fz) {
     fx = 0.0;
     fy = 0.0;
     fz = 0.0;
     if (v.d.geomx == 2) {
-        fx = T.v * T.v / rad + T.w * T.w / rad;
-        fz = T.v * T.v / rad / v.tanz[k];
+        const double c = T.v * T.v * irad;
+        fx = c + T.w * T.w * irad;
+        fz = c * itan;
         if (pol < v.zmin) fz *= -1.0;
     }
 }
@@ -413,77 +417,78 @@ __device__ __forceinline__ double rate3(const View3& v, const Cell& c, int i, in
         rad = d.radx[i];
         rad_cyl = rad * v.sinz[k];
     }
-    const double cs = sqrt(d.gam * c.p / c.r);
+    const double cs = sound_speed(d.gam, c.r, c.p);
     double spd = fabs(c.u) + cs;
-    double tmp = fmax(spd / fabs(d.xa[i + 1] - d.xa[i]), 0.0);
+    double tmp = fmax(spd * d.idx_x[i], 0.0);
     spd = fabs(c.v - rad_cyl * d.frame_omega - 0.0) + cs;
-    tmp = fmax(spd / (fabs(d.ya[j + 1] - d.ya[j]) * rad_cyl), tmp);
+    tmp = fmax(spd * d.idx_y[j] * inv(rad_cyl), tmp);
     spd = fabs(c.w) + cs;
-    tmp = fmax(spd / (fabs(v.za[k + 1] - v.za[k]) * rad), tmp);
+    tmp = fmax(spd * v.idx_z[k] * inv(rad), tmp);
     return tmp;
 }
 
 // PASS 1: first half-kick with the bodies of the previous step; PASS 2: the
 // predictor / corrector half-kick with the bodies at t + dt, then wave damping
-// and the signal rate of the result.  One thread per interior cell.
-// 4 CTAs of 256 threads per SM (64 registers; kick2 spills ~40 bytes): the
-// passes wait on loads, and 32 warps hide them better than 16-24 (20-23 % faster)
+// and the signal rate of the result.  A warp takes rows (j, k) and its lanes the cells of
+// a row: the row's factors are found once per row, not divided out of a cell's index.
 template <int PASS>
 __global__ void __launch_bounds__(K3_THREADS, 4) k3_kick(const View3 v, const Cell* __restrict__ in, Cell* __restrict__ out) {
     const DiskView& d = v.d;
     Scalars* sc = d.sc;
+    pdl_enter();
     if (sc->done) return;
     const double dt = sc->dt, hdt = 0.5 * dt;
-    const pg_body pl = PASS == 1 ? sc->planet_cur : sc->planet_next;
-    const long long n = (long long)d.xres * d.yres * v.zres;
+    const Planet3 pl = planet3(PASS == 1 ? sc->planet_cur : sc->planet_next);
+    const int rows = d.yres * v.zres, lane = threadIdx.x & 31;
+    const bool sph = d.geomx == 2;
     double vmax = 0.0;
-    for (long long m = (long long)blockIdx.x * blockDim.x + threadIdx.x; m < n; m += (long long)gridDim.x * blockDim.x) {
-        const int i = NPAD + (int)(m % d.xres);
-        const long long rest = m / d.xres;
-        const int j = NPAD + (int)(rest % d.yres);
-        const int k = NPAD + (int)(rest / d.yres);
-        const Cell C = get3(in, v, i, j, k);
-        const double rad = d.radx[i], pol = v.zc[k];
-        const Grav3 g = gravity3(v, j, k, rad, pol, pl, PASS - 1);
-        double fx, fy, fz;
-        fict3(v, k, rad, pol, C, fx, fy, fz);
-        if (PASS == 2) {  // the predictor over mdt = dt/2 (sweeps.cu:658-675)
-            Cell T = C;
-            T.u = C.u + fx * hdt + g.gx * hdt;
-            T.v = C.v + fy * hdt + g.gy * hdt;
-            T.w = C.w + fz * hdt + g.gz * hdt;
-            fict3(v, k, rad, pol, T, fx, fy, fz);
-        }
-        Cell Q;
-        Q.u = C.u + fx * hdt + g.gx * hdt;
-        Q.v = C.v + fy * hdt + g.gy * hdt;
-        Q.w = C.w + fz * hdt + g.gz * hdt;
-        Q.r = C.r;
-        Q.p = C.p;
-        if (PASS == 1) {
-            emit_x(v, out, i, j, k, Q);
-            continue;
-        }
-        if (d.kill) {  // relax towards init_C (killwave.cu:48-100)
-            const double* kt = d.killx + 4 * i;
-            const double* I = v.initc + 5 * ((size_t)i + (size_t)d.xarr * k);
+    for (int row = (blockIdx.x * K3_THREADS + threadIdx.x) >> 5; row < rows; row += gridDim.x * (K3_THREADS / 32)) {
+        const int j = NPAD + row % d.yres, k = NPAD + row / d.yres;
+        const double pol = v.zc[k], itan = sph ? inv(v.tanz[k]) : 0.0;
+        for (int i = NPAD + lane; i < NPAD + d.xres; i += 32) {
+            const Cell C = get3(in, v, i, j, k);
+            const double rad = d.radx[i], irad = sph ? inv(rad) : 0.0;
+            const Grav3 g = gravity3(v, j, k, rad, irad, pol, pl, PASS - 1);
+            double fx, fy, fz;
+            fict3(v, irad, itan, pol, C, fx, fy, fz);
+            if (PASS == 2) {  // the predictor over mdt = dt/2 (sweeps.cu:658-675)
+                Cell T = C;
+                T.u = C.u + fx * hdt + g.gx * hdt;
+                T.v = C.v + fy * hdt + g.gy * hdt;
+                T.w = C.w + fz * hdt + g.gz * hdt;
+                fict3(v, irad, itan, pol, T, fx, fy, fz);
+            }
+            Cell Q;
+            Q.u = C.u + fx * hdt + g.gx * hdt;
+            Q.v = C.v + fy * hdt + g.gy * hdt;
+            Q.w = C.w + fz * hdt + g.gz * hdt;
+            Q.r = C.r;
+            Q.p = C.p;
+            if (PASS == 1) {
+                emit_x(v, out, i, j, k, Q);
+                continue;
+            }
+            if (d.kill) {  // relax towards init_C (killwave.cu:48-100)
+                const double* kt = d.killx + 4 * i;
+                const double* I = v.initc + 5 * ((size_t)i + (size_t)d.xarr * k);
 #pragma unroll
-            for (int side = 0; side < 2; ++side) {
-                const double tau = kt[2 * side + 1];
-                if (tau > 0.0) {
-                    double f = kt[2 * side];
-                    f *= dt / tau;
-                    Q.r += f * (I[0] - Q.r);
-                    Q.p += f * (I[1] - Q.p);
-                    Q.u += f * (I[2] - Q.u);
-                    Q.v += f * (I[3] - Q.v);
-                    Q.w += f * (I[4] - Q.w);
+                for (int side = 0; side < 2; ++side) {
+                    const double tau = kt[2 * side + 1];
+                    if (tau > 0.0) {
+                        double f = kt[2 * side];
+                        f *= dt / tau;
+                        Q.r += f * (I[0] - Q.r);
+                        Q.p += f * (I[1] - Q.p);
+                        Q.u += f * (I[2] - Q.u);
+                        Q.v += f * (I[3] - Q.v);
+                        Q.w += f * (I[4] - Q.w);
+                    }
                 }
             }
+            if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+            put3(out, v, i, j, k, Q);
+            vmax = fmax(vmax, rate3(v, Q, i, j, k));
         }
-        if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-        put3(out, v, i, j, k, Q);
-        vmax = fmax(vmax, rate3(v, Q, i, j, k));
     }
     if (PASS == 2) block_max_to<K3_THREADS>(&sc->vmax_bits, vmax);
 }
@@ -668,7 +673,7 @@ struct Engine3 {
     View3 v{};
     Cell* buf[2] = {nullptr, nullptr};
     bool own_buffers = true;  // false: the caller's Grid buffers (pg_grid_*)
-    CUtensorMap maps[2][3];  // per buffer: radial, azimuthal, polar boxes
+    CUtensorMap maps[2];  // per buffer: the radial sweep's box
     const void* map_base[2] = {nullptr, nullptr};
     std::vector<const void*> ghosted;  // caller buffers whose bound-0 ghosts hold the device init_C
     std::vector<double> hxa, hya, hza; // host faces of each axis (ghosts included), for snapshots
@@ -683,9 +688,11 @@ struct Engine3 {
     long long steps_base = 0;
     bool pending = false;
     bool fresh = true;
+    // of each sweep: CTAs, warps across the radius, rows of a run, runs per line, runs
+    bool dense = false;  // the radial sweep's instance
     unsigned grid_sweep[3] = {0, 0, 0};
+    int across[3], len[3], chunks[3], items[3];
     unsigned grid_kick = 0;
-    int nta[3], ntb[3], ntiles[3];
 };
 
 static pg_status fail3(pg_status s, const char* fmt, ...) {
@@ -744,11 +751,18 @@ static pg_status make_maps(Engine3& E, int b) {
     const DiskView& d = E.v.d;
     const uint64_t d0 = 5ull * d.xarr, d1 = d.yarr, d2 = E.v.zarr;
     pg_status s;
-    if ((s = make_map3_f64(&E.maps[b][0], E.buf[b], d0, d1, d2, 5 * S3_TL, S3_W, 1)) != PG_OK) return s;
-    if ((s = make_map3_f64(&E.maps[b][1], E.buf[b], d0, d1, d2, 5 * S3_COLS, S3_TL, 1)) != PG_OK) return s;
-    if ((s = make_map3_f64(&E.maps[b][2], E.buf[b], d0, d1, d2, 5 * S3_COLS, 1, S3_TL)) != PG_OK) return s;
+    if ((s = make_map3_f64(&E.maps[b], E.buf[b], d0, d1, d2, 5 * RX_TILE_CELLS, S3_ROWS, 1)) != PG_OK) return s;
     E.map_base[b] = E.buf[b];
     return PG_OK;
+}
+
+// one sweep from buffer b to the other
+static void enqueue_sweep(Engine3& E, int dir, int b) {
+    Cell* out = E.buf[1 - b];
+    const int a = E.across[dir], l = E.len[dir], c = E.chunks[dir], n = E.items[dir];
+    if (dir == 0) launch_step(E.dense ? k3_sweep_x<4> : k3_sweep_x<3>, E.grid_sweep[0], S3_THREADS, S3_SMEM, E.stream, E.maps[b], E.v, out, a, l, c, n);
+    else if (dir == 1) launch_step(k3_march<1>, E.grid_sweep[1], S3_THREADS, 0, E.stream, E.buf[b], E.v, out, a, l, c, n);
+    else launch_step(k3_march<2>, E.grid_sweep[2], S3_THREADS, 0, E.stream, E.buf[b], E.v, out, a, l, c, n);
 }
 
 // the five passes of one step from buffer c (newest state ends in 1 - c)
@@ -757,11 +771,11 @@ static void enqueue_passes(Engine3& E, int c) {
     cudaStream_t s = E.stream;
     Cell* A = E.buf[c];
     Cell* B = E.buf[1 - c];
-    k3_kick<1><<<E.grid_kick, K3_THREADS, 0, s>>>(v, A, B);
-    k3_sweep<0><<<E.grid_sweep[0], S3_THREADS, S3_SMEM, s>>>(E.maps[1 - c][0], v, A, E.nta[0], E.ntb[0], E.ntiles[0]);
-    k3_sweep<1><<<E.grid_sweep[1], S3_THREADS, S3_SMEM, s>>>(E.maps[c][1], v, B, E.nta[1], E.ntb[1], E.ntiles[1]);
-    k3_sweep<2><<<E.grid_sweep[2], S3_THREADS, S3_SMEM, s>>>(E.maps[1 - c][2], v, A, E.nta[2], E.ntb[2], E.ntiles[2]);
-    k3_kick<2><<<E.grid_kick, K3_THREADS, 0, s>>>(v, A, B);
+    launch_step(k3_kick<1>, E.grid_kick, K3_THREADS, 0, s, v, A, B);
+    enqueue_sweep(E, 0, 1 - c);
+    enqueue_sweep(E, 1, c);
+    enqueue_sweep(E, 2, 1 - c);
+    launch_step(k3_kick<2>, E.grid_kick, K3_THREADS, 0, s, v, A, B);
 }
 
 static pg_status resolve3(Engine3& E) {
@@ -962,20 +976,25 @@ static pg_status create3(const pg_params* P, int device, cudaStream_t stream, En
         return bad(fail3(PG_ERR_CUDA, "table kernel failed"));
     for (int b = 0; own && b < 2; ++b)
         if ((s = make_maps(*E, b)) != PG_OK) return bad(s);
-    cudaFuncSetAttribute(k3_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
-    cudaFuncSetAttribute(k3_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
-    cudaFuncSetAttribute(k3_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
-    const int res[3] = {Q.xres, Q.yres, Q.zres};
+    // rows enough for eight a warp at 4 CTAs per SM
+    E->dense = (long long)((Q.xres + S3_OUT - 1) / S3_OUT) * Q.yres * Q.zres >= 8ll * 4 * S3_WARPS * 148;
+    const void* sweep_x = E->dense ? (const void*)k3_sweep_x<4> : (const void*)k3_sweep_x<3>;
+    cudaFuncSetAttribute(sweep_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
+    cudaFuncSetAttribute(sweep_x, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    const int along[3] = {Q.yres, Q.yres, Q.zres};  // rows a run is cut from
+    const int lines[3] = {Q.zres, Q.zres, Q.yres};
     for (int a = 0; a < 3; ++a) {
-        E->nta[a] = (res[a] + S3_L - 1) / S3_L;
-        E->ntb[a] = ((a == 0 ? Q.yres : Q.xres) + S3_W - 1) / S3_W;
-        E->ntiles[a] = E->nta[a] * E->ntb[a] * (a == 2 ? Q.yres : Q.zres);
+        E->across[a] = (Q.xres + (a == 0 ? S3_OUT : 32) - 1) / (a == 0 ? S3_OUT : 32);
+        const void* kernel = a == 0 ? sweep_x : (a == 1 ? (const void*)k3_march<1> : (const void*)k3_march<2>);
+        const size_t smem = a == 0 ? S3_SMEM : 0;
+        const long long resident = S3_WARPS * (long long)occupancy_grid(kernel, S3_THREADS, smem, 1ll << 40);
+        E->len[a] = run_length((long long)E->across[a] * lines[a], along[a], resident, a == 0 ? 1.5 : 3.5);
+        E->chunks[a] = (along[a] + E->len[a] - 1) / E->len[a];
+        E->items[a] = E->across[a] * E->chunks[a] * lines[a];
+        E->grid_sweep[a] = occupancy_grid(kernel, S3_THREADS, smem, (E->items[a] + S3_WARPS - 1) / S3_WARPS);
     }
-    E->grid_sweep[0] = occupancy_grid((const void*)k3_sweep<0>, S3_THREADS, S3_SMEM, E->ntiles[0]);
-    E->grid_sweep[1] = occupancy_grid((const void*)k3_sweep<1>, S3_THREADS, S3_SMEM, E->ntiles[1]);
-    E->grid_sweep[2] = occupancy_grid((const void*)k3_sweep<2>, S3_THREADS, S3_SMEM, E->ntiles[2]);
-    const long long ncin = (long long)Q.xres * Q.yres * Q.zres;
-    E->grid_kick = occupancy_grid((const void*)k3_kick<2>, K3_THREADS, 0, (ncin + K3_THREADS - 1) / K3_THREADS);
+    E->grid_kick = occupancy_grid((const void*)k3_kick<2>, K3_THREADS, 0,
+                                  ((long long)Q.yres * Q.zres + K3_THREADS / 32 - 1) / (K3_THREADS / 32));
     *out = E;
     return PG_OK;
 }
@@ -1295,14 +1314,11 @@ pg_status pg_disk3_pass_times(pg_disk3* dk, int nsteps, double* ms6) {
         cudaEventRecord(ev[1], E.stream);
         k3_kick<1><<<E.grid_kick, K3_THREADS, 0, E.stream>>>(v, A, B);
         cudaEventRecord(ev[2], E.stream);
-        k3_sweep<0><<<E.grid_sweep[0], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[1 - c][0], v, A, E.nta[0], E.ntb[0],
-                                                                          E.ntiles[0]);
+        enqueue_sweep(E, 0, 1 - c);
         cudaEventRecord(ev[3], E.stream);
-        k3_sweep<1><<<E.grid_sweep[1], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[c][1], v, B, E.nta[1], E.ntb[1],
-                                                                          E.ntiles[1]);
+        enqueue_sweep(E, 1, c);
         cudaEventRecord(ev[4], E.stream);
-        k3_sweep<2><<<E.grid_sweep[2], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[1 - c][2], v, A, E.nta[2], E.ntb[2],
-                                                                          E.ntiles[2]);
+        enqueue_sweep(E, 2, 1 - c);
         cudaEventRecord(ev[5], E.stream);
         k3_kick<2><<<E.grid_kick, K3_THREADS, 0, E.stream>>>(v, A, B);
         cudaEventRecord(ev[6], E.stream);
@@ -1381,14 +1397,11 @@ pg_status pg_disk3_stages(pg_disk3* dk, double t, double dt, pg_cell* out) {
     };
     k3_kick<1><<<E.grid_kick, K3_THREADS, 0, E.stream>>>(v, A, B);
     PG3_CUDA(grab(B, 0));
-    k3_sweep<0><<<E.grid_sweep[0], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[1 - c][0], v, A, E.nta[0], E.ntb[0],
-                                                                      E.ntiles[0]);
+    enqueue_sweep(E, 0, 1 - c);
     PG3_CUDA(grab(A, 1));
-    k3_sweep<1><<<E.grid_sweep[1], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[c][1], v, B, E.nta[1], E.ntb[1],
-                                                                      E.ntiles[1]);
+    enqueue_sweep(E, 1, c);
     PG3_CUDA(grab(B, 2));
-    k3_sweep<2><<<E.grid_sweep[2], S3_THREADS, S3_SMEM, E.stream>>>(E.maps[1 - c][2], v, A, E.nta[2], E.ntb[2],
-                                                                      E.ntiles[2]);
+    enqueue_sweep(E, 2, 1 - c);
     PG3_CUDA(grab(A, 3));
     k3_kick<2><<<E.grid_kick, K3_THREADS, 0, E.stream>>>(v, A, B);
     PG3_CUDA(grab(B, 4));

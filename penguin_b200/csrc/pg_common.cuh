@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
+
 #include "penguin_b200.h"
 
 namespace pg {
@@ -145,6 +147,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, Scalar
         }
     return true;
 }
+// Programmatic dependent launch: a kernel of a step is set up while the one before it drains
+// (launch_step below) and waits here until that one has completed and its writes are visible.
+// Every access to memory that an earlier kernel writes comes after this call.  The launch is
+// triggered by the end of the predecessor's blocks: triggered at their start, waiting blocks
+// held the SMs' slots, and the 126x389 disk's step took 48 us instead of 42 alone, 26 instead
+// of 20 with two others beside it (45 and 21 without dependent launches).
+__device__ __forceinline__ void pdl_enter() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Dynamic shared memory rounded up to 128 B (TMA destinations); kernels request 128 B extra.
 __device__ __forceinline__ double* smem_base128(double* p) {
     const uintptr_t a = reinterpret_cast<uintptr_t>(p);
@@ -278,5 +288,25 @@ __device__ __forceinline__ void pipe_drain(uint64_t* bar, int k, int issued_ahea
         for (int m = 1; m <= issued_ahead && m < NS; ++m)
             mbar_wait(&bar[(k + m) % NS], (uint32_t)(((k + m) / NS) & 1), sc);
 }
+
+#ifdef __CUDACC__
+// Launch of a kernel that begins with pdl_enter(): it may start before its predecessor in
+// the stream has finished.  Between the short kernels of a small grid the plain launch's
+// drain and ramp are as long as the kernels.
+template <class... P, class... A>
+inline cudaError_t launch_step(void (*kernel)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, A&&... a) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(a)...);
+}
+#endif
 
 }  // namespace pg

@@ -23,6 +23,29 @@ constexpr SweepVariant SWEEP_VARIANTS[NSWEEP_VARIANTS] = {
 // the radial box holds 5 (L + 6) doubles in one row, at most 256 TMA elements
 inline bool sweep_variant_x_ok(int v) { return 5 * (SWEEP_VARIANTS[v].len + 2 * NPAD) <= 256; }
 
+// Time of `warps` runs of `rows` rows each (the extra rows at a run's ends included) in units
+// of a row's time on a full GPU, where `resident` warps fit at once: whole waves of runs when
+// there are more, and with fewer a row that is quicker for the idle issue slots, down to its
+// latency.  The weights are those of the azimuthal sweeps measured from 126x389 to 1024x3072.
+inline double run_cost(long long warps, long long resident, double rows) {
+    if (warps <= resident) return rows * (0.55 + 0.45 * (double)warps / (double)resident);
+    return rows * (double)((warps + resident - 1) / resident);
+}
+// The run length of least run_cost for `lines` warps across and `rows` rows of each line
+inline int run_length(long long lines, int rows, long long resident, double extra) {
+    int best = 2;
+    double least = 1e300;
+    for (int len = 2; len <= 64; len += (len < 16 ? 1 : 4)) {
+        const double cost = run_cost(lines * ((rows + len - 1) / len), resident, len + extra);
+        if (cost < least) {
+            least = cost;
+            best = len;
+        }
+    }
+    return best;
+}
+constexpr int RX_TILE_CELLS = 36, RX_TILE_ROWS = 4;  // the radial sweep's TMA box
+
 // Tensor maps of one AoS cell buffer, one per tile shape.
 struct CellMaps {
     const void* base = nullptr;

@@ -1,0 +1,48 @@
+"""Reading a state back: small reads, reads cut into chunks for several threads (from 8 MB on,
+with a last chunk of any size) and reads into page-locked arrays.  Needs a B200."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from penguin_b200 import initial as I
+from penguin_b200 import params as P
+from penguin_b200._lib import check, lib
+from penguin_b200.disk import Disk
+from penguin_b200.disk3 import Disk3
+
+pytestmark = pytest.mark.gpu
+
+
+def _ptr(a):
+    return a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))
+
+
+# 2^18 cells are the 8 MB of four planes; 2^15 doubles a chunk
+@pytest.mark.parametrize("size", [(510, 514), (512, 512), (514, 513), (1030, 777)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_get_state_returns_what_was_set(size):
+    p = P.reference_disk(*size)
+    st = I.disk_state(p, seed=3)
+    d = Disk(p)
+    d.set_state(0.0, st)
+    for _ in range(2):  # the second read finds the slots made by the first
+        g = d.get_state()
+        for k in ("r", "u", "v"):
+            assert np.array_equal(g[k], st[k]), k
+    locked = [torch.empty(p.yres, p.xres, dtype=torch.float64).pin_memory().numpy() for _ in range(4)]
+    check(lib().pg_disk_get_state(d._h, *(_ptr(a) for a in locked), None))
+    for a, k in zip(locked, ("r", "p", "u", "v")):
+        assert np.array_equal(a, g[k]), k
+    d.close()
+
+
+def test_get_state_3d_returns_what_was_set():
+    p = P.cartesian_box(66, 61, 63)
+    st = I.box_state(p, seed=3)
+    d = Disk3(p)
+    d.set_state(0.0, st)
+    g = d.get_state()
+    for k in "rpuvw":
+        assert np.array_equal(g[k], st[k]), k
+    d.close()
