@@ -33,7 +33,6 @@ pg_status ens_fail(pg_status s, const std::string& m) {
         if (e_ != cudaSuccess) return ens_fail(PG_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-inline int cdivi(int a, int b) { return (a + b - 1) / b; }
 
 constexpr int kPasses = 5;       // kick1, radial sweep, azimuthal sweep, advection, kick2
 constexpr int kTotalsBlocks = 296;
@@ -65,7 +64,6 @@ struct EDisk {
     float* trig = nullptr;
     double* cs64 = nullptr;
     float* dbuf = nullptr;   // dust_flag: two buffers of NPL residual planes
-    float* dflux = nullptr;  // dust face fluxes
     bool fresh = true;
     View32 v{};
 };
@@ -78,17 +76,12 @@ struct pg_ens {
     bool own_stream = false;
     std::vector<EDisk> disks;
     View32* dV = nullptr;
-    int* dFirst = nullptr;
-    int4* dTiles = nullptr;             // per tile of each kind: {disk, origin along the fast index, along the slow}
-    CUtensorMap* dMaps = nullptr;
+    Runs32 runs{};                      // the passes' runs (build_runs32)
     double* dPart = nullptr;
-    int ntiles[3] = {0, 0, 0};
-    int* dDoff = nullptr;               // [3][n + 1] running counts of dust faces and cells
-    long long dcount[3] = {0, 0, 0};    // radial faces, azimuthal faces, cells of all dust disks
-    int maxn = 0;
+    int ndust = 0;                      // members with dust
     int cur = 0;
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    Tune32 tune = DEFAULT_TUNE32;  // launch configuration of the passes (pg_ens_autotune)
+    Tune32 tune{};  // launch configuration of the passes (pg_ens_autotune)
     double* xfer = nullptr;        // device staging of host exchanges, kept between calls
     size_t xfer_n = 0;
     HostCopy readback;  // staging of large reads of the state
@@ -103,15 +96,11 @@ struct pg_ens {
             cudaFree(D.trig);
             cudaFree(D.cs64);
             cudaFree(D.dbuf);
-            cudaFree(D.dflux);
             if (D.E) engine_destroy(D.E);
         }
         cudaFree(dV);
-        cudaFree(dFirst);
-        cudaFree(dTiles);
-        cudaFree(dMaps);
+        cudaFree(runs.d);
         cudaFree(dPart);
-        cudaFree(dDoff);
         cudaFree(xfer);
         if (own_stream && stream) cudaStreamDestroy(stream);
     }
@@ -125,13 +114,12 @@ namespace {
 // request waits for the stream before replacing the buffer.
 pg_status xfer_buffer(pg_ens* e, size_t count, double** out);
 
-// Kernels of one step reading buffer `in`: clocks, planet tables, five passes.
+// Kernels of one step reading buffer `in`: clocks and planet tables, five passes.
 pg_status enqueue_step(pg_ens* e, int in) {
     launch_time32(e->dV, e->n, e->stream);
-    launch_trig32(e->dV, e->n, e->maxn, e->stream);
     for (int p = 0; p < kPasses; ++p) {
-        launch_pass32(p, e->dV, e->dTiles, e->n, e->ntiles, in ^ (p & 1), e->stream, &e->tune);
-        launch_dust_pass32(p, e->dV, e->dDoff, e->n, e->dcount, in ^ (p & 1), e->stream);
+        launch_pass32(p, e->dV, e->runs, in ^ (p & 1), e->stream, e->tune);
+        if (e->ndust) launch_dust_pass32(p, e->dV, e->runs, in ^ (p & 1), e->stream);
     }
     ENS_CUDA(cudaGetLastError());
     return PG_OK;
@@ -199,10 +187,6 @@ pg_status pg_ens_create(const pg_params* P, int n, int device, void* stream, pg_
     pg_status s = pg_ens_check_params(P, n);
     if (s != PG_OK) return s;
     ENS_CUDA(cudaSetDevice(device));
-    static std::once_flag attrs;
-    static cudaError_t attr_err = cudaSuccess;
-    std::call_once(attrs, [] { attr_err = set_attributes32(); });
-    ENS_CUDA(attr_err);
     pg_ens* e = new pg_ens();
     auto bail = [&](pg_status st) {
         delete e;
@@ -217,16 +201,11 @@ pg_status pg_ens_create(const pg_params* P, int n, int device, void* stream, pg_
         e->own_stream = true;
     }
     e->disks.resize(n);
-    std::vector<int> first(3 * (n + 1), 0);
     cudaError_t ce;
-    if ((ce = cudaMalloc(&e->dMaps, sizeof(CUtensorMap) * 7 * (size_t)n)) != cudaSuccess ||
-        (ce = cudaMalloc(&e->dV, sizeof(View32) * (size_t)n)) != cudaSuccess ||
-        (ce = cudaMalloc(&e->dFirst, sizeof(int) * first.size())) != cudaSuccess ||
+    if ((ce = cudaMalloc(&e->dV, sizeof(View32) * (size_t)n)) != cudaSuccess ||
         (ce = cudaMalloc(&e->dPart, sizeof(double) * 2 * kTotalsBlocks)) != cudaSuccess)
         return bail(ens_fail(PG_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(ce)));
-    std::vector<CUtensorMap> maps(7 * (size_t)n);
     std::vector<View32> hv(n);
-    std::vector<int> doff(3 * (n + 1), 0);
     for (int k = 0; k < n; ++k) {
         EDisk& D = e->disks[k];
         if ((s = table_engine_create(&P[k], device, e->stream, &D.E)) != PG_OK) return bail(s);
@@ -243,9 +222,6 @@ pg_status pg_ens_create(const pg_params* P, int n, int device, void* stream, pg_
         v.orbadv = d.orbadv;
         v.kill = d.kill;
         v.nplanet = d.nplanet;
-        v.ntx[0] = cdivi(d.xres, 32);
-        v.ntx[1] = cdivi(d.yres, 32);
-        v.ntx[2] = cdivi(d.xres, 32);
         v.gam = (float)d.gam;
         const size_t plane = (size_t)v.pitch * v.yarr;
         const size_t ntab = (size_t)X_NSLOT * v.xn + (size_t)Y_NSLOT * v.yn;
@@ -267,68 +243,33 @@ pg_status pg_ens_create(const pg_params* P, int n, int device, void* stream, pg_
         v.trig = D.trig;
         v.cs64 = D.cs64;
         v.d64 = d;
-        v.maps = e->dMaps + 7 * (size_t)k;
-        CUtensorMap* m = &maps[7 * (size_t)k];
-        for (int b = 0; b < 2; ++b) {
-            if ((s = make_map3_f32(&m[3 * b + 0], v.buf[b], v.pitch, v.yarr, NPL, 40, 8, NPL)) != PG_OK ||
-                (s = make_map3_f32(&m[3 * b + 1], v.buf[b], v.pitch, v.yarr, NPL, 12, 38, NPL)) != PG_OK ||
-                (s = make_map3_f32(&m[3 * b + 2], v.buf[b], v.pitch, v.yarr, NPL, 36, 10, NPL)) != PG_OK)
-                return bail(s);
-        }
-        if ((s = make_map3_f32(&m[6], v.vis, v.pitch, v.yarr, 2, 36, 10, 2)) != PG_OK) return bail(s);
-        long long nd3[3] = {0, 0, 0};
         if (P[k].dust_flag) {
             // init_CD everywhere: zero residuals
-            const size_t nf = (size_t)(v.xres + 1) * (v.yres + 1);
-            if ((ce = cudaMalloc(&D.dbuf, sizeof(float) * 2 * NPL * plane)) != cudaSuccess ||
-                (ce = cudaMalloc(&D.dflux, sizeof(float) * 3 * nf)) != cudaSuccess)
+            if ((ce = cudaMalloc(&D.dbuf, sizeof(float) * 2 * NPL * plane)) != cudaSuccess)
                 return bail(ens_fail(PG_ERR_CUDA, std::string("cudaMalloc: ") + cudaGetErrorString(ce)));
             cudaMemsetAsync(D.dbuf, 0, sizeof(float) * 2 * NPL * plane, e->stream);
-            cudaMemsetAsync(D.dflux, 0, sizeof(float) * 3 * nf, e->stream);
             v.dbuf[0] = D.dbuf;
             v.dbuf[1] = D.dbuf + NPL * plane;
-            v.dflux = D.dflux;
             v.dust = 1;
             v.st_h = (float)(P[k].stokes * P[k].sc_h);
             v.dust_rmin = (float)(P[k].d_g_ratio * SMALLR);
-            nd3[0] = (long long)(v.xres + 1) * v.yres;
-            nd3[1] = (long long)v.xres * (v.yres + 1);
-            nd3[2] = (long long)v.xres * v.yres;
-        }
-        for (int r = 0; r < 3; ++r) {
-            doff[r * (n + 1) + k + 1] = doff[r * (n + 1) + k] + (int)nd3[r];
-            e->dcount[r] += nd3[r];
+            ++e->ndust;
         }
         launch_init_tables32(v, D.tab, D.tab + (size_t)X_NSLOT * v.xn, D.cs64, e->stream);
-        first[0 * (n + 1) + k + 1] = first[0 * (n + 1) + k] + v.ntx[0] * cdivi(d.yres, 8);
-        first[1 * (n + 1) + k + 1] = first[1 * (n + 1) + k] + v.ntx[1] * cdivi(d.xres, 8);
-        first[2 * (n + 1) + k + 1] = first[2 * (n + 1) + k] + v.ntx[2] * cdivi(d.yres, 8);
-        e->maxn = std::max(e->maxn, std::max(v.xn, v.yn));
         hv[k] = v;
     }
-    for (int p = 0; p < 3; ++p) e->ntiles[p] = first[p * (n + 1) + n];
-    // tile table: a tile's disk and origin (32 cells along the fast index x 8
-    // along the slow), so the passes need no search over the disks' offsets
-    std::vector<int4> tiles;
-    tiles.reserve((size_t)e->ntiles[0] + e->ntiles[1] + e->ntiles[2]);
-    for (int p = 0; p < 3; ++p)
-        for (int k = 0; k < n; ++k) {
-            const int ntx = hv[k].ntx[p];
-            for (int loc = 0; loc < first[p * (n + 1) + k + 1] - first[p * (n + 1) + k]; ++loc)
-                tiles.push_back(make_int4(k, NPAD + 32 * (loc % ntx), NPAD + 8 * (loc / ntx), 0));
-        }
-    if ((ce = cudaMalloc(&e->dTiles, sizeof(int4) * tiles.size())) != cudaSuccess ||
-        (ce = cudaMemcpyAsync(e->dTiles, tiles.data(), sizeof(int4) * tiles.size(), cudaMemcpyHostToDevice,
-                              e->stream)) != cudaSuccess ||
-        (ce = cudaMalloc(&e->dDoff, sizeof(int) * doff.size())) != cudaSuccess ||
-        (ce = cudaMemcpyAsync(e->dDoff, doff.data(), sizeof(int) * doff.size(), cudaMemcpyHostToDevice, e->stream)) !=
+    std::vector<int> xs(n), ys(n);
+    for (int k = 0; k < n; ++k) {
+        xs[k] = hv[k].xres;
+        ys[k] = hv[k].yres;
+    }
+    std::vector<int4> runs;
+    build_runs32(xs.data(), ys.data(), n, &runs, &e->runs);
+    if ((ce = cudaMalloc(&e->runs.d, sizeof(int4) * runs.size())) != cudaSuccess ||
+        (ce = cudaMemcpyAsync(e->runs.d, runs.data(), sizeof(int4) * runs.size(), cudaMemcpyHostToDevice, e->stream)) !=
             cudaSuccess ||
-        (ce = cudaMemcpyAsync(e->dMaps, maps.data(), sizeof(CUtensorMap) * maps.size(), cudaMemcpyHostToDevice,
-                              e->stream)) != cudaSuccess ||
         (ce = cudaMemcpyAsync(e->dV, hv.data(), sizeof(View32) * hv.size(), cudaMemcpyHostToDevice, e->stream)) !=
             cudaSuccess ||
-        (ce = cudaMemcpyAsync(e->dFirst, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice,
-                              e->stream)) != cudaSuccess ||
         (ce = cudaStreamSynchronize(e->stream)) != cudaSuccess || (ce = cudaGetLastError()) != cudaSuccess)
         return bail(ens_fail(PG_ERR_CUDA, std::string("ensemble set-up: ") + cudaGetErrorString(ce)));
     *out = e;
@@ -537,7 +478,7 @@ pg_status pg_ens_torque(pg_ens* e, int k, double* torque) {
     return PG_OK;
 }
 
-int pg_ens_kernels_per_step(const pg_ens* e) { return e ? 2 + kPasses + (e->dcount[2] > 0 ? 6 : 0) : 0; }
+int pg_ens_kernels_per_step(const pg_ens* e) { return e ? 1 + kPasses + (e->ndust > 0 ? 3 : 0) : 0; }
 
 // dust_flag members: the interior dust (absolute r, v_r, v_phi) of the newest state
 pg_status pg_ens_set_dust(pg_ens* e, int k, const double* r, const double* u, const double* v) {
@@ -597,11 +538,10 @@ pg_status pg_ens_profile(pg_ens* e, int nsteps, double end_time, float* ms, int 
         const int c0 = e->cur;
         ENS_CUDA(cudaEventRecord(ev[0], e->stream));
         launch_time32(e->dV, e->n, e->stream);
-        launch_trig32(e->dV, e->n, e->maxn, e->stream);
         for (int p = 0; p < kPasses; ++p) {
             ENS_CUDA(cudaEventRecord(ev[1 + p], e->stream));
-            launch_pass32(p, e->dV, e->dTiles, e->n, e->ntiles, c0 ^ (p & 1), e->stream, &e->tune);
-            launch_dust_pass32(p, e->dV, e->dDoff, e->n, e->dcount, c0 ^ (p & 1), e->stream);
+            launch_pass32(p, e->dV, e->runs, c0 ^ (p & 1), e->stream, e->tune);
+            if (e->ndust) launch_dust_pass32(p, e->dV, e->runs, c0 ^ (p & 1), e->stream);
         }
         ENS_CUDA(cudaEventRecord(ev[6], e->stream));
         ENS_CUDA(cudaGetLastError());
@@ -617,12 +557,12 @@ pg_status pg_ens_profile(pg_ens* e, int nsteps, double end_time, float* ms, int 
     return PG_OK;
 }
 
-// For each pass and each compiled occupancy variant, every CTAs-per-SM cap up to
-// what the variant allows: the mean time of `reps` launches on the current
+// For each pass and each of its two lists of runs, every CTAs-per-SM cap up to
+// what the kernel allows: the mean time of `reps` launches on the current
 // state (read from the current buffer, written to the other, which the next
 // step overwrites), and the fastest is kept.  The disks' device scalars (the
 // signal-rate maximum the timed kick2 launches raise, floor counters) are saved
-// before and restored after.  Results do not depend on the choice: tiles are
+// before and restored after.  Results do not depend on the choice: runs are
 // independent and the CFL rate is a maximum.
 pg_status pg_ens_autotune(pg_ens* e, int reps, int* out10) {
     if (!e || reps < 1) return ens_fail(PG_ERR_ARG, "bad argument");
@@ -639,15 +579,15 @@ pg_status pg_ens_autotune(pg_ens* e, int reps, int* out10) {
         float best = -1.0f;
         int bv = e->tune.v[p], bc = e->tune.cps[p];
         for (int v = 0; v < 2; ++v) {
-            const int occ = pass_occupancy32(p, v);
+            const int occ = pass_occupancy32(p);
             for (int cap = 1; cap <= occ; ++cap) {
                 Tune32 t = e->tune;
                 t.v[p] = v;
                 t.cps[p] = (cap == occ) ? 0 : cap;
-                launch_pass32(p, e->dV, e->dTiles, e->n, e->ntiles, e->cur, e->stream, &t);  // warm-up
+                launch_pass32(p, e->dV, e->runs, e->cur, e->stream, t);  // warm-up
                 ENS_CUDA(cudaEventRecord(a, e->stream));
                 for (int r = 0; r < reps; ++r)
-                    launch_pass32(p, e->dV, e->dTiles, e->n, e->ntiles, e->cur, e->stream, &t);
+                    launch_pass32(p, e->dV, e->runs, e->cur, e->stream, t);
                 ENS_CUDA(cudaEventRecord(b, e->stream));
                 ENS_CUDA(cudaEventSynchronize(b));
                 ENS_CUDA(cudaGetLastError());

@@ -3,16 +3,14 @@
 // The same five fused passes as the FP64 kernels (kick1 C->T, radial sweep T->C,
 // azimuthal sweep + orbital shift C->T, residual advection T->C, kick2 +
 // damping + CFL rate C->T), on FP32 residual planes.  Every pass is ONE
-// persistent launch over the concatenated tile lists of all disks in the
-// ensemble: a CTA walks tiles blockIdx.x, blockIdx.x + gridDim.x, ... and finds
-// each tile's disk by binary search over per-disk tile offsets, so disks of
-// uneven size share the GPU without one launch per disk.  Tiles arrive through
-// 3D TMA copies (x, y, plane) whose tensor maps live in device memory, one set
-// per disk, double-buffered as in the FP64 kernels.
+// persistent launch over the concatenated runs of all disks in the ensemble (a run: some
+// rows of 32 neighbouring radii of one disk), so disks of uneven size share the
+// GPU without one launch per disk.
 //
-// A disk whose clock reached end_time has its tiles copied through unchanged, so
+// A disk whose clock reached end_time has its runs copied through unchanged, so
 // the two state buffers of all disks stay in step.
 #include <cstdio>
+#include <vector>
 
 #include "pg_common.cuh"
 #include "pg_f32.cuh"
@@ -22,42 +20,23 @@
 namespace pg {
 namespace f32 {
 
-constexpr int T_LEN = 32, T_W = 8;           // outputs along / across the sweep per tile
-constexpr int P1N = (T_LEN + 2) * T_W;       // 272 reconstructed cells
-constexpr int P2N = (T_LEN + 1) * T_W;       // 264 faces
-constexpr int SWT = 288;                     // sweep threads
-constexpr int XB_W = 40, XB_H = 8, XPL = XB_W * XB_H, XS = XPL * NPL;                  // radial tile: 960 floats
-constexpr int YB_W = 12, YB_H = 38, YPL = YB_W * YB_H, YS = (YPL * NPL + 31) / 32 * 32;  // azimuthal: 1376
-constexpr int SB_W = 36, SB_H = 10, SPL = SB_W * SB_H, SS = (SPL * NPL + 31) / 32 * 32;  // stencil: 1088
-constexpr int VS = (SPL * 2 + 31) / 32 * 32;                                            // stress: 736
-constexpr int STT = 256;                     // stencil threads (32 x 8 cells)
-constexpr int NSX = 13, NSY = 8;             // floats kept per reconstructed cell
-constexpr int NFA = (T_LEN + 6) * T_W;       // advection faces per tile
-constexpr size_t SX_SMEM = (size_t)(2 * XS + NSX * P1N + 4 * P2N) * 4 + 16 + 128;
-constexpr size_t SY_SMEM = (size_t)(2 * YS + NSY * P1N + 4 * P2N) * 4 + 16 + 128;
-constexpr size_t AD_SMEM = (size_t)(2 * YS + 3 * NFA) * 4 + 16 + 128;
-constexpr size_t K1_SMEM = (size_t)(2 * SS) * 4 + 16 + 128;
-constexpr size_t K2_SMEM = (size_t)(3 * SS + 2 * VS) * 4 + 16 + 128;
-static_assert(XS % 32 == 0 && YS % 32 == 0 && SS % 32 == 0 && VS % 32 == 0, "128-B aligned TMA stages");
-static_assert((2 * XS + NSX * P1N + 4 * P2N) % 2 == 0 && (2 * YS + NSY * P1N + 4 * P2N) % 2 == 0 &&
-                  (2 * YS + 3 * NFA) % 2 == 0 && (3 * SS + 2 * VS) % 2 == 0,
-              "8-B aligned barriers");
+// A pass's work is cut into runs: a warp takes the rows j0 .. j1-1 of its 32
+// neighbouring radii one after the other (int4 {disk, first lane's radius, j0, j1}, a
+// table built with the ensemble).  Lanes along the radius make every access to a plane
+// a coalesced row segment and every per-radius factor a register for the whole run;
+// what a cell needs of its neighbours comes by shuffle or stays from the row before.
+// No shared memory and no barrier: tiles whose phases met at __syncthreads spent half
+// their instructions on table loads, tile addresses and the exchange, and waited on
+// barriers and L1 for most of the rest (55 % of issue slots at 1024x3072).  There, us a
+// pass, tiles -> runs: kick1 75 -> 53, sweep_x 148 -> 78, sweep_y 135 -> 70, advection
+// 81 -> 39, kick2 140 -> 84; what bounds them is instruction issue.  All are compiled for 5
+// CTAs of 4 warps per SM; at 3 / 4 / 6 / 7 kick1 takes 80 / 85 / 67 / 74, sweep_x
+// 102 / 101 / 84 / 88, sweep_y 74 / 74 / 78 / 83, kick2 98 / 103 / 120 / 126, and the
+// advection at 4 / 6 / 7 39 / 43 / 43.
+constexpr int MW = 4, MT = 32 * MW;  // warps of a CTA, independent of one another
 
-__device__ __forceinline__ float* smem_base128f(float* p) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    return reinterpret_cast<float*>((a + 127) & ~uintptr_t(127));
-}
-
-// disk owning global tile `tile`: the largest k with first[k] <= tile
-__device__ __forceinline__ int find_disk(const int* __restrict__ first, int nd, int tile) {
-    int lo = 0, hi = nd - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (first[mid] <= tile) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
+__device__ __forceinline__ float up1(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ float down1(float v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
 // Planar multi-value tables: value m of slot group `slot` at index i.
 template <int N>
@@ -89,71 +68,121 @@ __device__ __forceinline__ void emit32(const View32& w, float* out, int i, int j
     }
 }
 
+// What the marching passes read of the disk's descriptor in every row, in registers: the
+// descriptor lies in global memory, and the rows' stores would make each use of it a load.
+struct Disk32 {
+    int pitch, yres, yn;
+    size_t pl;
+    const float* ty;
+    float* out;
+    __device__ __forceinline__ Disk32(const View32& w, int in)
+        : pitch(w.pitch), yres(w.yres), yn(w.yn), pl(w.plane()), ty(w.ty), out(w.buf[in ^ 1]) {}
+    __device__ __forceinline__ float y(int slot, int j) const { return ty[slot * yn + j]; }
+    template <int N>
+    __device__ __forceinline__ void ys(int slot, int j, float* o) const {
+#pragma unroll
+        for (int m = 0; m < N; ++m) o[m] = ty[(slot + m) * yn + j];
+    }
+    // the new residuals of interior cell (i, j) and their periodic image (emit32)
+    __device__ __forceinline__ void emit(int i, int j, float a, float b, float c) const {
+        float* o = out + ((size_t)j * pitch + i);
+        o[0] = a;
+        o[pl] = b;
+        o[2 * pl] = c;
+        if (j < 2 * NPAD || j >= yres) {
+            o += (long long)(j < 2 * NPAD ? yres : -yres) * pitch;
+            o[0] = a;
+            o[pl] = b;
+            o[2 * pl] = c;
+        }
+    }
+};
+
+// What the half-kicks need of a lane's radius.
+struct Kick32 {
+    float sbg, abg, v2r, ir, rad, dr;  // dr: r - x_p
+    float nu, nul, nur, vb[7], X[5];   // viscosity here and at the neighbours, stencil factors
+    float m, xp, rs2, ip2;             // the planet
+    const float* trig;                 // per-row table of its angles, null without a planet
+};
+__device__ __forceinline__ Kick32 kick_tables(const View32& w, int i, int which) {
+    Kick32 c;
+    c.sbg = w.x(X_SBG)[i];
+    c.abg = w.x(X_ABG)[i];
+    c.v2r = w.x(X_V2R)[i];
+    c.ir = w.x(X_IRAD)[i];
+    c.rad = w.x(X_RAD)[i];
+    c.dr = w.tcol()[2 * i + which];
+    const float* s = w.tscal() + 4 * which;
+    c.m = s[0];
+    c.xp = s[1];
+    c.rs2 = s[2];
+    c.ip2 = s[3];
+    c.trig = w.nplanet ? w.trig + 3 * which : nullptr;
+    c.nu = c.nul = c.nur = 0.0f;
+    if (w.visc) {
+        const float* nu = w.x(X_NU);
+        c.nu = nu[i];
+        c.nul = nu[max(i - 1, 0)];
+        c.nur = nu[min(i + 1, w.xarr - 1)];
+        xload<7>(w, X_VBG, i, c.vb);
+        xload<5>(w, X_VISX, i, c.X);
+    }
+    return c;
+}
+
 // Star + planet gravity (forces.cu:182-327) without the star term, which is in
 // X_ABG.  |r - r_p|^2 = (r - x_p)^2 + 2 r x_p (1 - cos) + rs^2 has no cancellation.
-// which: 0 = planet of the first half-kick, 1 = planet at t + dt.
-__device__ __forceinline__ void gravity32(const View32& w, int i, int j, int which, float& gx, float& gy) {
+__device__ __forceinline__ void gravity32(const Kick32& c, int j, float& gx, float& gy) {
     gx = 0.0f;
     gy = 0.0f;
-    if (w.nplanet == 0) return;
-    const float* tr = w.trow(j) + 3 * which;
-    const float* s = w.tscal() + 4 * which;
-    const float m = s[0], xp = s[1], rs2 = s[2], ip2 = s[3];
-    const float dr = w.tcol()[2 * i + which];
-    const float rad = w.x(X_RAD)[i];
-    const float R2 = dr * dr + 2.0f * rad * xp * tr[2] + rs2;
-    const float ir = rsqrtf(R2);
+    if (!c.trig) return;
+    const float* tr = c.trig + TRIG_ROW * j;
+    const float R2 = c.dr * c.dr + 2.0f * c.rad * c.xp * tr[2] + c.rs2;
+    const float ir = rsq32(R2);
     const float rf = ir * ir * ir;
-    gx = -m * (dr + xp * tr[2]) * rf - m * tr[1] * ip2;
-    gy = -m * xp * tr[0] * rf + m * tr[0] * ip2;
+    gx = -c.m * (c.dr + c.xp * tr[2]) * rf - c.m * tr[1] * c.ip2;
+    gy = -c.m * c.xp * tr[0] * rf + c.m * tr[0] * c.ip2;
 }
 
 // Half-kick of the residual velocities (sweeps.cu:597-711 with geomx 1):
 // v^2/r - 1/r^2 = X_ABG + (2 v0/r + dv/r) dv.  mdt != 0 re-evaluates the
 // curvature term at the mdt-predicted velocity (sweeps.cu:663-687).
-__device__ __forceinline__ void kick32(const View32& w, int i, float dS, float& du, float& dv, float vx, float vy,
-                                       float gx, float gy, float mdt, float dt, bool visc) {
-    const float iS = visc ? 1.0f / (w.x(X_SBG)[i] + dS) : 0.0f;
-    const float abg = w.x(X_ABG)[i], v2r = w.x(X_V2R)[i], ir = w.x(X_IRAD)[i];
-    float fx = abg + (v2r + dv * ir) * dv + vx * iS;
+__device__ __forceinline__ void kick32(const Kick32& c, float dS, float& du, float& dv, float vx, float vy, float gx,
+                                       float gy, float mdt, float dt, bool visc) {
+    const float iS = visc ? rcp32(c.sbg + dS) : 0.0f;
+    float fx = c.abg + (c.v2r + dv * c.ir) * dv + vx * iS;
     const float fy = vy * iS;
     if (mdt != 0.0f) {
         const float dvT = dv + fy * mdt + gy * mdt;
-        fx = abg + (v2r + dvT * ir) * dvT + vx * iS;
+        fx = c.abg + (c.v2r + dvT * c.ir) * dvT + vx * iS;
     }
     du = du + fx * dt + gx * dt;
     dv = dv + fy * dt + gy * dt;
 }
 
-// Viscous force density at stencil-tile cell (x, y) of planes {dS, du, dv} with
-// row length SB_W: residual part plus background part (viscosity.cu:84-194).
-__device__ __forceinline__ void stress32(const View32& w, const float* tile, int x, int y, int i, int j, float& vx,
-                                         float& vy) {
-    const float* nu = w.x(X_NU);
-    float vb[7], X[5], Y[4];
-    xload<7>(w, X_VBG, i, vb);
-    xload<5>(w, X_VISX, i, X);
-    yload<4>(w, Y_VISY, j, Y);
-    const float* S = tile;
-    const float* U = tile + SPL;
-    const float* V = tile + 2 * SPL;
-    const int c = y * SB_W + x;
-    const float n1 = nu[i];
-    const float nr1 = (w.x(X_SBG)[i] + S[c]) * n1;
-    const float dndx = (vb[6] + S[c + 1] * nu[i + 1] - S[c - 1] * nu[i - 1]) * X[0];
-    const float dndy = (S[c + SB_W] - S[c - SB_W]) * n1 * Y[0] * X[4];
-    float u[9], v[9];
-#pragma unroll
-    for (int n = 0; n < 9; ++n) {
-        const int dx = (n % 3) - 1;
-        const int dy = (n < 3) ? 0 : (n < 6 ? -1 : 1);
-        u[n] = U[c + dy * SB_W + dx];
-        v[n] = V[c + dy * SB_W + dx];
-    }
+// One row's residuals at the lane's radius, the velocities at its neighbours' too.
+struct Row32 {
+    float S, u[3], v[3];
+};
+__device__ __forceinline__ Row32 row32(float S, float u, float v) {
+    return Row32{S, {up1(u), u, down1(u)}, {up1(v), v, down1(v)}};
+}
+// Viscous force density of the middle of three rows: residual part plus background
+// part (viscosity.cu:84-194).
+__device__ __forceinline__ void stress32(const Disk32& D, const Kick32& c, int j, const Row32& lo, const Row32& mid,
+                                         const Row32& hi, float& vx, float& vy) {
+    float Y[4];
+    D.ys<4>(Y_VISY, j, Y);
+    const float nr1 = (c.sbg + mid.S) * c.nu;
+    const float dndx = (c.vb[6] + down1(mid.S) * c.nur - up1(mid.S) * c.nul) * c.X[0];
+    const float dndy = (hi.S - lo.S) * c.nu * Y[0] * c.X[4];
+    const float u[9] = {mid.u[0], mid.u[1], mid.u[2], lo.u[0], lo.u[1], lo.u[2], hi.u[0], hi.u[1], hi.u[2]};
+    const float v[9] = {mid.v[0], mid.v[1], mid.v[2], lo.v[0], lo.v[1], lo.v[2], hi.v[0], hi.v[1], hi.v[2]};
     float fx, fy;
-    viscous32(X, Y, u, v, nr1, dndx, dndy, fx, fy);
-    vx = fx + vb[0] * nr1 + vb[1] * dndx + vb[2] * dndy;
-    vy = fy + vb[3] * nr1 + vb[4] * dndx + vb[5] * dndy;
+    viscous32(c.X, Y, u, v, nr1, dndx, dndy, fx, fy);
+    vx = fx + c.vb[0] * nr1 + c.vb[1] * dndx + c.vb[2] * dndy;
+    vy = fy + c.vb[3] * nr1 + c.vb[4] * dndx + c.vb[5] * dndy;
 }
 
 // CFL signal rate (timestep.cu:46-77) in FP64 from the residuals.
@@ -182,9 +211,11 @@ __device__ __forceinline__ double drate64(const View32& w, int i, int j, float d
 // limiter (src/solver/dust/dust.cu:6-147) and updated by update_Dust
 // (dust.cu:149-176) in residual form, e.g. v_new - v = (D(Sigma v) - v D Sigma) /
 // Sigma_new with the transported field taken relative to a neighbouring cell.
-// Each sweep is two launches over all dust disks: one thread per face (the two
-// edge states it needs and the limited fluxes into a scratch array), then one
-// thread per cell.  The dust planes carry no ghost images: rows wrap, and the
+// Each sweep is one launch over the dusty disks' runs, laid out like the gas's: edge states,
+// limited face fluxes and the update of a cell stay in registers, neighbours by shuffle or
+// from the row before.  (As one launch per face and one per cell through a scratch array of
+// fluxes, every face formed both its cells' states again: 65 us a sweep at 682x2046, three
+// times the gas's.)  The dust planes carry no ghost images: rows wrap, and the
 // radial ghosts of boundary 0 hold init_CD, i.e. zero residuals.
 struct DR {
     float S, u, v;  // residuals
@@ -210,308 +241,287 @@ __device__ __forceinline__ float exp_limf(float x) { return fmaxf(1.0f + x, 1.0e
 struct DEdge {
     float S, u, t;  // density and normal velocity (absolute), transported field relative to the cell
 };
+// One edge state of a dust cell (dust.cu:6-103; SIDE 0 left, 1 right) from its parabolas;
+// sx = sdt / dx, uc the cell's normal velocity, Sc its density.
+template <int SIDE>
+__device__ __forceinline__ DEdge dust_edge(float sx, float Sc, float uc, const Par32& R, const Par32& U,
+                                           const Par32& T) {
+    auto away = [](float u) { return SIDE == 0 ? fmaxf(-u, 0.0f) : fmaxf(u, 0.0f); };
+    auto ave = [](const Frac32& q, const Par32& p) { return SIDE == 0 ? aveL32(q, p) : aveR32(q, p); };
+    const float d = away(SIDE == 0 ? uc - U.sL : uc + U.sR) * sx;  // swept fraction
+    const float ud = ave(frac32(fminf(d, 1.0f)), U);
+    const Frac32 q = frac32(fminf(away(uc + ud) * sx, 1.0f));
+    const float c = sx * (SIDE == 0 ? ud : -ud) / (1.0f - d);  // the cell's compression
+    return DEdge{(Sc + ave(q, R)) * exp_limf(c), uc + ave(q, U), ave(q, T)};
+}
+struct DFlux {
+    float r, u, t;  // mass, normal momentum, transported field relative to the face's lower cell
+};
+// dust_flow's limited upwind flux (dust.cu:120-147) between lower cell a and upper cell b:
+// no more than the cells hold (Sa sxa, Sb sxb); jump: the transported field from a to b
+__device__ __forceinline__ DFlux dust_flux(float Sa, float sxa, const DEdge& a, float Sb, float sxb, const DEdge& b,
+                                           float jump) {
+    const float Fl = fminf(Sa * sxa, fmaxf(a.u * a.S, 0.0f));
+    const float Fr = fmaxf(-Sb * sxb, fminf(b.u * b.S, 0.0f));
+    return DFlux{Fl + Fr, Fl * a.u + Fr * b.u, Fl * a.t + Fr * (jump + b.t)};
+}
+// update_Dust (dust.cu:149-176) in residual form: DS and the increments Dn = D(Sigma u_n) -
+// u_n D Sigma and Dt of the residuals n and t; true where the density fell to its floor
+__device__ __forceinline__ void update_dust32(const View32& w, Scalars* sc, float sbg, float DS, float Dn, float Dt,
+                                              float& S, float& n, float& t) {
+    const float Sc = sbg + S, Sn = Sc + DS;
+    const float rmin = fmaxf(Sc * 1.0e-10f, w.dust_rmin);
+    if (Sn < rmin) {
+        S = rmin - sbg;
+    } else {
+        const float iS = rcp32(Sn);
+        S += DS;
+        n += Dn * iS;
+        t += Dt * iS;
+    }
+    if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+}
 
-// Both edge states of dust cell c of a pencil (dust.cu:6-103): DIR 0 radial
-// (row q; normal v_r, transported r v_phi), DIR 1 azimuthal (column q; normal
-// v_phi - orb_rot - r Omega, transported v_r).  Also the cell's averages.
-template <int DIR>
-__device__ __forceinline__ void dust_edges(const View32& w, const float* b, int c, int q, float dtf, DEdge& L,
-                                           DEdge& R, float& Sc, float& tc) {
-    float aS[5], aU[5], aT[5];
-    const DR C = (DIR == 0) ? dload(w, b, c, q) : dload(w, b, q, c);
-    float idx, sdt, uc;
-    const float* wt;
-    float wts[6];
-    if (DIR == 0) {
-        float db[12];
+// radial dust sweep: normal v_r, transported r v_phi
+__global__ void __launch_bounds__(MT, 5) k32d_sweep_x(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                     int nruns, int in) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
+        if (!w.dust) continue;
+        Scalars* sc = w.d64.sc;
+        const bool done = sc->done != 0;
+        const float dtf = (float)sc->dt;
+        const size_t pl = w.plane(), pitch = w.pitch;
+        const int i = run.y + lane, c = min(i, w.xarr - 3);
+        const bool output = lane >= 1 && lane <= 30 && i < NPAD + w.xres;
+        const float* src = w.dbuf[in] + (size_t)run.z * pitch + c;
+        float* dst = w.dbuf[in ^ 1] + (size_t)run.z * pitch + c;
+        if (done) {
+            for (int j = run.z; j < run.w; ++j, src += pitch, dst += pitch)
+                if (output) {
+                    dst[0] = src[0];
+                    dst[pl] = src[pl];
+                    dst[2 * pl] = src[2 * pl];
+                }
+            continue;
+        }
+        float db[12], wt[6], rad[5];
         xload<12>(w, X_DDBG, c, db);
-        const float* rad = w.x(X_RAD);
+        xload<6>(w, X_WX, c, wt);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) rad[m] = w.x(X_RAD)[c - 2 + m];
+        const float sbg = w.x(X_DSBG)[c], ubg = w.x(X_DUBG)[c], sx = dtf * w.x(X_IDX)[c];
+        const float g0 = w.x(X_XA)[c], g1 = w.x(X_XA)[c + 1], f = dtf * w.x(X_IXV)[c], irad = w.x(X_IRAD)[c];
+#pragma unroll 1
+        for (int j = run.z; j < run.w; ++j, src += pitch, dst += pitch) {
+            float aS[5], aU[5], aT[5];
+            const float S0 = src[0], u0 = src[pl], v0 = src[2 * pl];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+                if (m == 2) {
+                    aS[m] = aU[m] = aT[m] = 0.0f;
+                    continue;
+                }
+                const int kk = m < 2 ? m : m - 1;
+                aS[m] = db[kk] + (src[m - 2] - S0);
+                aU[m] = db[4 + kk] + (src[pl + m - 2] - u0);
+                aT[m] = db[8 + kk] + (rad[m] * src[2 * pl + m - 2] - rad[2] * v0);
+            }
+            const Par32 R = recon32(wt, aS[0], aS[1], aS[3], aS[4], 0.0f);
+            const Par32 U = recon32(wt, aU[0], aU[1], aU[3], aU[4], 0.0f);
+            const Par32 T = recon32(wt, aT[0], aT[1], aT[3], aT[4], 0.0f);
+            const float Sc = sbg + S0, uc = ubg + u0;
+            const DEdge b = dust_edge<0>(sx, Sc, uc, R, U, T), e = dust_edge<1>(sx, Sc, uc, R, U, T);
+            const float jump = up1(aT[3]);  // from the lower cell
+            const DEdge a{up1(e.S), up1(e.u), up1(e.t)};
+            const DFlux F = dust_flux(up1(Sc), up1(sx), a, Sc, sx, b, jump);
+            const DFlux G{down1(F.r), down1(F.u), down1(F.t)};
+            const float DS = (F.r * g0 - G.r * g1) * f;
+            const float Dn = (g0 * (F.u - F.r * uc) - g1 * (G.u - G.r * uc)) * f;
+            const float Dt = (g0 * (F.t - F.r * jump) - g1 * G.t) * f * irad;
+            if (output) {
+                float S = S0, u = u0, v = v0;
+                update_dust32(w, sc, sbg, DS, Dn, Dt, S, u, v);
+                dst[0] = S;
+                dst[pl] = u;
+                dst[2 * pl] = v;
+            }
+        }
+    }
+}
+
+// Five rows of a dust column in registers and the next in flight; rows wrap.
+struct DColumn {
+    float S[5], u[5], v[5], nS, nu, nv;
+    const float* p;  // row `row` of the column
+    int row, end;
+    size_t pl, pitch, wrap;
+    __device__ __forceinline__ DColumn(const View32& w, int in, int c, int first) {
+        pl = w.plane();
+        pitch = w.pitch;
+        wrap = pitch * w.yres;
+        end = NPAD + w.yres;
+        row = first < NPAD ? first + w.yres : first;
+        p = w.dbuf[in] + (size_t)row * pitch + c;
 #pragma unroll
         for (int m = 0; m < 5; ++m) {
-            if (m == 2) {
-                aS[m] = aU[m] = aT[m] = 0.0f;
-                continue;
-            }
-            const int kk = m < 2 ? m : m - 1;
-            const DR N = dload(w, b, c - 2 + m, q);
-            aS[m] = db[kk] + (N.S - C.S);
-            aU[m] = db[4 + kk] + (N.u - C.u);
-            aT[m] = db[8 + kk] + (rad[c - 2 + m] * N.v - rad[c] * C.v);
+            S[m] = p[0];
+            u[m] = p[pl];
+            v[m] = p[2 * pl];
+            next();
         }
-        xload<6>(w, X_WX, c, wts);
-        wt = wts;
-        idx = w.x(X_IDX)[c];
-        sdt = dtf;
-        Sc = w.x(X_DSBG)[c] + C.S;
-        uc = w.x(X_DUBG)[c] + C.u;
-        tc = C.v;  // only differences of r v_phi are used
-    } else {
+        fetch();
+    }
+    __device__ __forceinline__ void next() {
+        p += pitch;
+        if (++row == end) {
+            row = NPAD;
+            p -= wrap;
+        }
+    }
+    __device__ __forceinline__ void fetch() {
+        nS = p[0];
+        nu = p[pl];
+        nv = p[2 * pl];
+        next();
+    }
+    __device__ __forceinline__ void shift() {
 #pragma unroll
-        for (int m = 0; m < 5; ++m) {
-            if (m == 2) {
-                aS[m] = aU[m] = aT[m] = 0.0f;
-                continue;
-            }
-            const DR N = dload(w, b, q, c - 2 + m);
-            aS[m] = N.S - C.S;
-            aU[m] = N.v - C.v;
-            aT[m] = N.u - C.u;
+        for (int m = 0; m < 4; ++m) {
+            S[m] = S[m + 1];
+            u[m] = u[m + 1];
+            v[m] = v[m + 1];
         }
-        const int cw = wrap32(w, c);
-        yload<6>(w, Y_WY, cw, wts);
-        wt = wts;
-        idx = w.y(Y_IDY)[cw];
-        sdt = dtf * w.x(X_IRAD)[q];
-        Sc = w.x(X_DSBG)[q] + C.S;
-        uc = w.x(X_DEPS)[q] + C.v;
-        tc = C.u;
+        S[4] = nS;
+        u[4] = nu;
+        v[4] = nv;
     }
-    const Par32 Rp = recon32(wt, aS[0], aS[1], aS[3], aS[4], 0.0f);
-    const Par32 Up = recon32(wt, aU[0], aU[1], aU[3], aU[4], 0.0f);
-    const Par32 Tp = recon32(wt, aT[0], aT[1], aT[3], aT[4], 0.0f);
-    const float dx = 1.0f / idx;
-    {  // left edge: the right state of the face below
-        const float ue = uc - Up.sL;
-        const Frac32 q1 = frac32(lim01f(-fminf(ue, 0.0f) * sdt * idx));
-        const float urd = aveL32(q1, Up);
-        const float u_ = sdt * urd / (dx + fminf(ue, 0.0f) * sdt);
-        const float ur = uc + urd;
-        const Frac32 q2 = frac32(lim01f(-fminf(ur, 0.0f) * sdt * idx));
-        L.S = (Sc + aveL32(q2, Rp)) * exp_limf(u_);
-        L.u = uc + aveL32(q2, Up);
-        L.t = aveL32(q2, Tp);
-    }
-    {  // right edge: the left state of the face above
-        const float ue = uc + Up.sR;
-        const Frac32 q1 = frac32(lim01f(fmaxf(ue, 0.0f) * sdt * idx));
-        const float uld = aveR32(q1, Up);
-        const float u_ = -sdt * uld / (dx - fmaxf(ue, 0.0f) * sdt);
-        const float ul = uc + uld;
-        const Frac32 q2 = frac32(lim01f(fmaxf(ul, 0.0f) * sdt * idx));
-        R.S = (Sc + aveR32(q2, Rp)) * exp_limf(u_);
-        R.u = uc + aveR32(q2, Up);
-        R.t = aveR32(q2, Tp);
-    }
-}
+};
 
-// dust offsets: [3][nd + 1] running counts of radial faces, azimuthal faces, cells
-__device__ __forceinline__ bool dust_unit(const int* doff, int nd, int row, long long g, int& k, int& loc) {
-    const int* o = doff + row * (nd + 1);
-    if (g >= o[nd]) return false;
-    k = find_disk(o, nd, (int)g);
-    loc = (int)(g - o[k]);
-    return true;
-}
-
-// face fluxes of the dust sweeps: DIR 0 radial, DIR 1 azimuthal
-template <int DIR>
-__global__ void __launch_bounds__(256) k32d_faces(const View32* __restrict__ V, const int* __restrict__ doff, int nd,
-                                                 int in) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int k, loc;
-    if (!dust_unit(doff, nd, DIR, g, k, loc)) return;
-    const View32& w = V[k];
-    if (w.d64.sc->done) return;
-    const float dtf = (float)w.d64.sc->dt;
-    const float* b = w.dbuf[in];
-    int f, q;
-    if (DIR == 0) {
-        f = NPAD + loc % (w.xres + 1);
-        q = NPAD + loc / (w.xres + 1);
-    } else {
-        q = NPAD + loc % w.xres;
-        f = NPAD + loc / w.xres;
-    }
-    DEdge La, Ra, Lb, Rb;
-    float Sa, ta, Sb, tb;
-    dust_edges<DIR>(w, b, f - 1, q, dtf, La, Ra, Sa, ta);
-    dust_edges<DIR>(w, b, f, q, dtf, Lb, Rb, Sb, tb);
-    float ia, ib, sdt;
-    if (DIR == 0) {
-        ia = w.x(X_IDX)[f - 1];
-        ib = w.x(X_IDX)[f];
-        sdt = dtf;
-    } else {
-        ia = w.y(Y_IDY)[wrap32(w, f - 1)];
-        ib = w.y(Y_IDY)[wrap32(w, f)];
-        sdt = dtf * w.x(X_IRAD)[q];
-    }
-    // dust_flow's limiter (dust.cu:120-147)
-    const float Fl = fminf(Sa * sdt * ia, fmaxf(Ra.u * Ra.S, 0.0f));
-    const float Fr = fmaxf(-Sb * sdt * ib, fminf(Lb.u * Lb.S, 0.0f));
-    // the jump of the transported field from cell a to cell b
-    float jab;
-    if (DIR == 0) jab = w.x(X_DDBG + 10)[f - 1] + (w.x(X_RAD)[f] * tb - w.x(X_RAD)[f - 1] * ta);
-    else jab = tb - ta;
-    const size_t fp = (size_t)(w.xres + 1) * (w.yres + 1);
-    const size_t m = (DIR == 0) ? (size_t)(q - NPAD) * (w.xres + 1) + (f - NPAD)
-                                : (size_t)(f - NPAD) * (w.xres + 1) + (q - NPAD);
-    w.dflux[m] = Fl + Fr;
-    w.dflux[fp + m] = Fl * Ra.u + Fr * Lb.u;
-    w.dflux[2 * fp + m] = Fl * Ra.t + Fr * (jab + Lb.t);  // relative to cell a
-}
-
-// update_Dust of one cell from its two faces; DIR 1 writes at the orbital-shifted row
-template <int DIR>
-__global__ void __launch_bounds__(256) k32d_update(const View32* __restrict__ V, const int* __restrict__ doff, int nd,
-                                                  int in) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int k, loc;
-    if (!dust_unit(doff, nd, 2, g, k, loc)) return;
-    const View32& w = V[k];
-    Scalars* sc = w.d64.sc;
-    const int i = NPAD + loc % w.xres, j = NPAD + loc / w.xres;
-    const float* b = w.dbuf[in];
-    DR Q = dload(w, b, i, j);
-    int jo = j;
-    if (!sc->done) {
+// azimuthal dust sweep (normal v_phi - orb_rot - r Omega, transported v_r) writing each cell
+// at the gas's shifted row of its radius (orbit.cu:30-46)
+__global__ void __launch_bounds__(MT, 5) k32d_sweep_y(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                     int nruns, int in) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
+        if (!w.dust) continue;
+        Scalars* sc = w.d64.sc;
+        const bool done = sc->done != 0;
         const float dtf = (float)sc->dt;
-        const size_t fp = (size_t)(w.xres + 1) * (w.yres + 1);
-        size_t m0, m1;
-        float f, g0 = 1.0f, g1 = 1.0f;
-        if (DIR == 0) {
-            m0 = (size_t)(j - NPAD) * (w.xres + 1) + (i - NPAD);
-            m1 = m0 + 1;
-            g0 = w.x(X_XA)[i];
-            g1 = w.x(X_XA)[i + 1];
-            f = dtf * w.x(X_IXV)[i];
-        } else {
-            m0 = (size_t)(j - NPAD) * (w.xres + 1) + (i - NPAD);
-            m1 = m0 + (w.xres + 1);
-            f = dtf * w.y(Y_IYV)[j] * w.x(X_IRAD)[i];
+        const Disk32 D(w, in);
+        const int i = run.y + lane, c = min(i, NPAD + w.xres - 1);
+        const bool active = i < NPAD + w.xres;
+        float* dst = w.dbuf[in ^ 1];
+        if (done) {
+            for (int j = run.z; j < run.w; ++j)
+                if (active) dstore(w, dst, i, j, dload(w, w.dbuf[in], i, j));
+            continue;
         }
-        const float F0 = w.dflux[m0], F1 = w.dflux[m1];
-        const float U0 = w.dflux[fp + m0], U1 = w.dflux[fp + m1];
-        const float T0 = w.dflux[2 * fp + m0], T1 = w.dflux[2 * fp + m1];
-        float un, jm;  // normal velocity of the cell; jump of the transported field from the cell below
-        if (DIR == 0) {
-            un = w.x(X_DUBG)[i] + Q.u;
-            const DR P = dload(w, b, i - 1, j);
-            jm = -(w.x(X_DDBG + 9)[i] + (w.x(X_RAD)[i - 1] * P.v - w.x(X_RAD)[i] * Q.v));
-        } else {
-            un = w.x(X_DEPS)[i] + Q.v;
-            const DR P = dload(w, b, i, j - 1);
-            jm = Q.u - P.u;
+        int js = run.z - NPAD;
+        if (w.orbadv) {
+            js = (js + w.d64.inc[c]) % D.yres;
+            if (js < 0) js += D.yres;
         }
-        const float DS = (F0 * g0 - F1 * g1) * f;
-        const float Dn = (g0 * (U0 - F0 * un) - g1 * (U1 - F1 * un)) * f;  // D(Sigma u_n) - u_n D Sigma
-        const float Dt = (g0 * (T0 - F0 * jm) - g1 * T1) * f;              // D(Sigma t) - t D Sigma
-        const float Sc = w.x(X_DSBG)[i] + Q.S;
-        const float Sn = Sc + DS;
-        const float rmin = fmaxf(Sc * 1.0e-10f, w.dust_rmin);
-        if (Sn < rmin) {
-            Q.S = rmin - w.x(X_DSBG)[i];
-        } else {
-            const float iS = 1.0f / Sn;
-            Q.S += DS;
-            if (DIR == 0) {
-                Q.u += Dn * iS;
-                Q.v += Dt * w.x(X_IRAD)[i] * iS;
-            } else {
-                Q.v += Dn * iS;
-                Q.u += Dt * iS;
+        const float sbg = w.x(X_DSBG)[c], ubg = w.x(X_DEPS)[c], sdt = dtf * w.x(X_IRAD)[c];
+        DColumn q(w, in, c, run.z - NPAD);
+        DEdge pe{};  // the right edge of the cell below, its density and swept fraction
+        float pS = 0.0f, psx = 0.0f;
+        DFlux pf{};
+#pragma unroll 1
+        for (int t = run.z - 1; t <= run.w; ++t) {
+            const int tw = t < NPAD ? t + D.yres : (t >= NPAD + D.yres ? t - D.yres : t);
+            float wt[6];
+            D.ys<6>(Y_WY, tw, wt);
+            const float sx = sdt * D.y(Y_IDY, tw);
+            const Par32 R = recon32(wt, q.S[0] - q.S[2], q.S[1] - q.S[2], q.S[3] - q.S[2], q.S[4] - q.S[2], 0.0f);
+            const Par32 U = recon32(wt, q.v[0] - q.v[2], q.v[1] - q.v[2], q.v[3] - q.v[2], q.v[4] - q.v[2], 0.0f);
+            const Par32 T = recon32(wt, q.u[0] - q.u[2], q.u[1] - q.u[2], q.u[3] - q.u[2], q.u[4] - q.u[2], 0.0f);
+            const float Sc = sbg + q.S[2], uc = ubg + q.v[2];
+            const DEdge b = dust_edge<0>(sx, Sc, uc, R, U, T), e = dust_edge<1>(sx, Sc, uc, R, U, T);
+            const DFlux F = dust_flux(pS, psx, pe, Sc, sx, b, q.u[2] - q.u[1]);
+            if (t > run.z) {  // the cell below has both its fluxes
+                float S = q.S[1], u = q.u[1], v = q.v[1];
+                const float f = sdt * D.y(Y_IYV, t - 1), un = ubg + v;
+                const float DS = (pf.r - F.r) * f;
+                const float Dn = ((pf.u - pf.r * un) - (F.u - F.r * un)) * f;
+                const float Dt = ((pf.t - pf.r * (q.u[1] - q.u[0])) - F.t) * f;
+                if (active) {
+                    update_dust32(w, sc, sbg, DS, Dn, Dt, S, v, u);
+                    dstore(w, dst, i, js + NPAD, DR{S, u, v});
+                }
+                if (++js == D.yres) js = 0;
             }
-        }
-        if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-        if (DIR == 1 && w.orbadv) {  // the gas's shift of this radius (orbit.cu:30-46)
-            int js = (j - NPAD + w.d64.inc[i]) % w.yres;
-            if (js < 0) js += w.yres;
-            jo = js + NPAD;
+            pe = e;
+            pS = Sc;
+            psx = sx;
+            pf = F;
+            q.shift();
+            q.fetch();
         }
     }
-    dstore(w, w.dbuf[in ^ 1], i, jo, Q);
 }
 
-// residual advection of the dust by orb_res (advection.cu:175-357): the face
-// flux from the upwind cell
-__global__ void __launch_bounds__(256) k32d_adv_faces(const View32* __restrict__ V, const int* __restrict__ doff,
-                                                     int nd, int in) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int k, loc;
-    if (!dust_unit(doff, nd, 1, g, k, loc)) return;
-    const View32& w = V[k];
-    if (w.d64.sc->done) return;
-    const float dtf = (float)w.d64.sc->dt;
-    const float* b = w.dbuf[in];
-    const int q = NPAD + loc % w.xres, f = NPAD + loc / w.xres;
-    const float speed = (float)w.d64.res[q];
-    const int c = speed > 0.0f ? f - 1 : f;  // the upwind cell
-    float aS[5], aV[5], aU[5];
-    const DR C = dload(w, b, q, c);
-#pragma unroll
-    for (int m = 0; m < 5; ++m) {
-        const DR N = dload(w, b, q, c - 2 + m);
-        aS[m] = N.S - C.S;
-        aV[m] = N.v - C.v;
-        aU[m] = N.u - C.u;
-    }
-    const int cw = wrap32(w, c);
-    float wt[6];
-    yload<6>(w, Y_WY, cw, wt);
-    const Par32 Rp = recon32(wt, aS[0], aS[1], aS[3], aS[4], 0.0f);
-    const Par32 Vp = recon32(wt, aV[0], aV[1], aV[3], aV[4], 0.0f);
-    const Par32 Up = recon32(wt, aU[0], aU[1], aU[3], aU[4], 0.0f);
-    const float sdt = dtf * w.x(X_IRAD)[q], idx = w.y(Y_IDY)[cw];
-    const float Sc = w.x(X_DSBG)[q] + C.S;
-    float fr, fv, fu;
-    if (speed > 0.0f) {
-        const Frac32 fq = frac32(lim01f(speed * sdt * idx));
-        fr = Sc + aveR32(fq, Rp);
-        fv = aveR32(fq, Vp);
-        fu = aveR32(fq, Up);
-    } else {
-        const Frac32 fq = frac32(lim01f(-speed * sdt * idx));
-        fr = Sc + aveL32(fq, Rp);
-        fv = aveL32(fq, Vp);
-        fu = aveL32(fq, Up);
-    }
-    if (c == f) {  // relative to the face's lower cell f - 1
-        const DR P = dload(w, b, q, f - 1);
-        fv += C.v - P.v;
-        fu += C.u - P.u;
-    }
-    const float F = fr * speed;
-    const size_t fp = (size_t)(w.xres + 1) * (w.yres + 1);
-    const size_t m = (size_t)(f - NPAD) * (w.xres + 1) + (q - NPAD);
-    w.dflux[m] = F;
-    w.dflux[fp + m] = F * fv;
-    w.dflux[2 * fp + m] = F * fu;
-}
-
-__global__ void __launch_bounds__(256) k32d_adv_update(const View32* __restrict__ V, const int* __restrict__ doff,
-                                                      int nd, int in) {
-    const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    int k, loc;
-    if (!dust_unit(doff, nd, 2, g, k, loc)) return;
-    const View32& w = V[k];
-    Scalars* sc = w.d64.sc;
-    const int i = NPAD + loc % w.xres, j = NPAD + loc / w.xres;
-    const float* b = w.dbuf[in];
-    DR Q = dload(w, b, i, j);
-    if (!sc->done) {
+// residual advection of the dust by orb_res (advection.cu:175-357)
+__global__ void __launch_bounds__(MT, 6) k32d_advect(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                    int nruns, int in) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
+        if (!w.dust) continue;
+        Scalars* sc = w.d64.sc;
+        const bool done = sc->done != 0;
         const float dtf = (float)sc->dt;
-        const size_t fp = (size_t)(w.xres + 1) * (w.yres + 1);
-        const size_t m0 = (size_t)(j - NPAD) * (w.xres + 1) + (i - NPAD), m1 = m0 + (w.xres + 1);
-        const float f = dtf * w.y(Y_IYV)[j] * w.x(X_IRAD)[i];
-        const DR P = dload(w, b, i, j - 1);
-        const float F0 = w.dflux[m0], F1 = w.dflux[m1];
-        const float DS = (F0 - F1) * f;
-        const float Dv = ((w.dflux[fp + m0] - F0 * (Q.v - P.v)) - w.dflux[fp + m1]) * f;
-        const float Du = ((w.dflux[2 * fp + m0] - F0 * (Q.u - P.u)) - w.dflux[2 * fp + m1]) * f;
-        const float Sc = w.x(X_DSBG)[i] + Q.S;
-        const float Sn = Sc + DS;
-        const float rmin = fmaxf(Sc * 1.0e-10f, w.dust_rmin);
-        if (Sn < rmin) {
-            Q.S = rmin - w.x(X_DSBG)[i];
-        } else {
-            const float iS = 1.0f / Sn;
-            Q.S += DS;
-            Q.v += Dv * iS;
-            Q.u += Du * iS;
+        const Disk32 D(w, in);
+        const int i = run.y + lane, c = min(i, NPAD + w.xres - 1);
+        const bool active = i < NPAD + w.xres;
+        float* dst = w.dbuf[in ^ 1];
+        if (done) {
+            for (int j = run.z; j < run.w; ++j)
+                if (active) dstore(w, dst, i, j, dload(w, w.dbuf[in], i, j));
+            continue;
         }
-        if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+        const float speed = (float)w.d64.res[c], sbg = w.x(X_DSBG)[c], sdt = dtf * w.x(X_IRAD)[c];
+        const float swept = fabsf(speed) * sdt;
+        const bool up = speed > 0.0f;
+        DColumn q(w, in, c, run.z - NPAD);
+        float pr = 0.0f, pv = 0.0f, pu = 0.0f;  // the row before: mass flux and the carried v and u
+#pragma unroll 1
+        for (int t = run.z - 1; t <= run.w; ++t) {
+            const int tw = t < NPAD ? t + D.yres : (t >= NPAD + D.yres ? t - D.yres : t);
+            float wt[6];
+            D.ys<6>(Y_WY, tw, wt);
+            const Par32 R = recon32(wt, q.S[0] - q.S[2], q.S[1] - q.S[2], q.S[3] - q.S[2], q.S[4] - q.S[2], 0.0f);
+            const Par32 N = recon32(wt, q.v[0] - q.v[2], q.v[1] - q.v[2], q.v[3] - q.v[2], q.v[4] - q.v[2], 0.0f);
+            const Par32 T = recon32(wt, q.u[0] - q.u[2], q.u[1] - q.u[2], q.u[3] - q.u[2], q.u[4] - q.u[2], 0.0f);
+            const Frac32 x = frac32(fminf(swept * D.y(Y_IDY, tw), 1.0f));
+            const float F = ((sbg + q.S[2]) + (up ? aveR32(x, R) : aveL32(x, R))) * speed;
+            // carried v and u, relative to the cell's own
+            const float fv = up ? aveR32(x, N) : aveL32(x, N), fu = up ? aveR32(x, T) : aveL32(x, T);
+            const int j = up ? t : t - 1;
+            if (active && j >= run.z && j < run.w) {
+                float S = up ? q.S[2] : q.S[1], u = up ? q.u[2] : q.u[1], v = up ? q.v[2] : q.v[1];
+                const float f = sdt * D.y(Y_IYV, j);
+                const float jv = q.v[2] - q.v[1], ju = q.u[2] - q.u[1];  // from the row below to this one
+                const float Dv = (up ? pr * (pv - jv) - F * fv : pr * pv - F * (fv + jv)) * f;
+                const float Du = (up ? pr * (pu - ju) - F * fu : pr * pu - F * (fu + ju)) * f;
+                update_dust32(w, sc, sbg, (pr - F) * f, Dv, Du, S, v, u);
+                dstore(w, dst, i, j, DR{S, u, v});
+            }
+            pr = F;
+            pv = fv;
+            pu = fu;
+            q.shift();
+            q.fetch();
+        }
     }
-    dstore(w, w.dbuf[in ^ 1], i, j, Q);
 }
 
 // Drag of the dust towards the gas in a half-kick (sweeps.cu:626-707, the
@@ -540,702 +550,539 @@ __device__ __forceinline__ void dust_drag32(const View32& w, int i, float Sg, fl
 }
 
 // ============================================================ radial sweep
-// Each pass is compiled for two occupancies (MB: the CTAs per SM its register
-// budget must allow); the ensemble's autotuner picks one per pass.
-template <int MB>
-__global__ void __launch_bounds__(SWT, MB) k32_sweep_x(const View32* __restrict__ V, const int4* __restrict__ tiles,
-                                                   int nd, int ntiles, int in) {
-    extern __shared__ __align__(128) float fsm_raw[];
-    float* sm = smem_base128f(fsm_raw);
-    auto stage = [&](int n) { return sm + (n & 1) * XS; };
-    float* st = sm + 2 * XS;      // [NSX][P1N]
-    float* fl = st + NSX * P1N;   // [4][P2N]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 4 * P2N);
-    const int tid = threadIdx.x;
-    auto locate = [&](int tile, int& k, int& s0, int& q0) {  // the tile's disk and origin (pg_ens tile table)
-        const int4 t = tiles[tile];
-        k = t.x;
-        s0 = t.y;
-        q0 = t.z;
-    };
-    auto issue = [&](int tile, int kt) {
-        int k, s0, q0;
-        locate(tile, k, s0, q0);
-        issue_begin(&bar[kt & 1], XS * 4);
-        tma_load_3d(stage(kt), V[k].maps + 3 * in + 0, s0 - NPAD, q0, 0, &bar[kt & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int k, s0, q0;
-        locate(tile_id, k, s0, q0);
-        const View32& w = V[k];
+// Lanes 1..30 of a run update; lane l's left face takes its left state from lane l - 1, its right flux
+// from lane l + 1.
+__global__ void __launch_bounds__(MT, 5) k32_sweep_x(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                  int nruns, int in) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_enter();
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
         Scalars* sc = w.d64.sc;
-        const float* T = stage(kt);
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
         const bool done = sc->done != 0;
-        const float dtf = (float)sc->dt;
-        const float gam = w.gam;
-        if (!done) {
-            // ---- P1: deviations, reconstruction, both edge states of every cell
-            if (tid < P1N) {
-                const int q = tid / (T_LEN + 2), t = 2 + tid % (T_LEN + 2);
-                const int s = s0 - NPAD + t;
-                const int sc_ = min(s, w.xarr - 1);
-                const float* r0 = T + q * XB_W + (t - 2);
-                float dS[5], du[5], dv[5];
-#pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    dS[m] = r0[m];
-                    du[m] = r0[XPL + m];
-                    dv[m] = r0[2 * XPL + m];
-                }
-                float db[16];
-                xload<16>(w, X_DBG, sc_, db);
-                const float* cs2t = w.x(X_CS2);
-                const float* radt = w.x(X_RAD);
-                const float cs2c = cs2t[sc_], radc = radt[sc_];
-                float aS[5], aP[5], aU[5], aL[5];
-#pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    if (m == 2) {
-                        aS[m] = aP[m] = aU[m] = aL[m] = 0.0f;
-                        continue;
-                    }
-                    const int kk = m < 2 ? m : m - 1;
-                    const int sk = min(max(s - 2 + m, 0), w.xarr - 1);
-                    aS[m] = (dS[m] - dS[2]) + db[kk];
-                    aP[m] = (cs2t[sk] * dS[m] - cs2c * dS[2]) + db[4 + kk];
-                    aU[m] = (du[m] - du[2]) + db[8 + kk];
-                    aL[m] = (radt[sk] * dv[m] - radc * dv[2]) + db[12 + kk];
-                }
-                const float Sc = w.x(X_SBG)[sc_] + dS[2];
-                const float pc = w.x(X_PBG)[sc_] + cs2c * dS[2];
-                const float uc = w.x(X_UBG)[sc_] + du[2];
-                const float cs0 = sqrtf(gam * pc / Sc);
-                const float flat = flatten32(1.0f / cs0, pc, aP[0], aP[1], aP[3], aP[4], aU[1], aU[3]);
-                float wt[6];
-                xload<6>(w, X_WX, sc_, wt);
-                const Par32 R = recon32(wt, aS[0], aS[1], aS[3], aS[4], flat);
-                const Par32 P = recon32(wt, aP[0], aP[1], aP[3], aP[4], flat);
-                const Par32 U = recon32(wt, aU[0], aU[1], aU[3], aU[4], flat);
-                const Par32 L = recon32(wt, aL[0], aL[1], aL[3], aL[4], flat);
-                const float idx = w.x(X_IDX)[sc_];
-                const HS a = left_edge32(gam, idx, dtf, cs0, Sc, pc, uc, R, P, U, L);
-                const HS b = right_edge32(gam, idx, dtf, cs0, Sc, pc, uc, R, P, U, L);
-                float* o = st + tid;
-                o[0] = a.rd;
-                o[P1N] = a.pd;
-                o[2 * P1N] = a.u;
-                o[3 * P1N] = a.v;
-                o[4 * P1N] = b.rd;
-                o[5 * P1N] = b.pd;
-                o[6 * P1N] = b.u;
-                o[7 * P1N] = b.v;
-                o[8 * P1N] = aS[3];  // jumps to the right neighbour
-                o[9 * P1N] = aP[3];
-                o[10 * P1N] = aL[3];
-                o[11 * P1N] = Sc;
-                o[12 * P1N] = pc;
-            }
-            __syncthreads();
-            // ---- P2: HLLC at every face, referenced to the face's left cell
-            if (tid < P2N) {
-                const int q = tid / (T_LEN + 1), f = tid % (T_LEN + 1);
-                const int iL = q * (T_LEN + 2) + f, iR = iL + 1;
-                HS L, R;
-                L.rd = st[4 * P1N + iL];
-                L.pd = st[5 * P1N + iL];
-                L.u = st[6 * P1N + iL];
-                L.v = st[7 * P1N + iL];
-                R.rd = st[iR] + st[8 * P1N + iL];
-                R.pd = st[P1N + iR] + st[9 * P1N + iL];
-                R.u = st[2 * P1N + iR];
-                R.v = st[3 * P1N + iR] + st[10 * P1N + iL];
-                const FX F = hllc32(gam, st[11 * P1N + iL], st[12 * P1N + iL], L, R);
-                fl[tid] = F.r;
-                fl[P2N + tid] = F.u;
-                fl[2 * P2N + tid] = F.v;
-                fl[3 * P2N + tid] = F.pd;
-            }
-            __syncthreads();
+        const float dtf = (float)sc->dt, gam = w.gam;
+        const int i = run.y + lane, c = min(i, w.xarr - 3);  // c: the stencil stays in the row
+        const bool output = lane >= 1 && lane <= 30 && i < NPAD + w.xres;
+        const float* src = w.buf[in] + (size_t)run.z * w.pitch + c;
+        const Disk32 D(w, in);
+        if (done) {
+            for (int j = run.z; j < run.w; ++j, src += D.pitch)
+                if (output) D.emit(i, j, src[0], src[D.pl], src[2 * D.pl]);
+            continue;
         }
-        // ---- P3: residual update (sweeps.cu:218-261, 300-335)
-        if (tid < T_LEN * T_W) {
-            const int q = tid / T_LEN, o = tid % T_LEN;
-            const int s = s0 + o, j = q0 + q;
-            if (s < NPAD + w.xres && j < NPAD + w.yres) {
-                const float* c = T + q * XB_W + NPAD + o;
-                const float dS0 = c[0], du0 = c[XPL], dv0 = c[2 * XPL];
-                float dSn = dS0, dun = du0, dvn = dv0;
-                if (!done) {
-                    const int iC = q * (T_LEN + 2) + 1 + o;
-                    const int f0 = q * (T_LEN + 1) + o, f1 = f0 + 1;
-                    const float g0 = w.x(X_XA)[s], g1 = w.x(X_XA)[s + 1];
-                    const float f = dtf * w.x(X_IXV)[s];
-                    const float Fr0 = fl[f0], Fr1 = fl[f1];
-                    const float Dr = (Fr0 * g0 - Fr1 * g1) * f;
-                    // pres0 - pres1 = (p[s-1] - p[s]) + (pd0 - pd1)
-                    const float dpres = (fl[3 * P2N + f0] - fl[3 * P2N + f1]) - st[9 * P1N + iC - 1];
-                    const float Du = ((fl[P2N + f0] * g0 - fl[P2N + f1] * g1) + 0.5f * (g0 + g1) * dpres) * f;
-                    // D(Sigma v) - v D(Sigma) with l = r v: faces referenced to cells s-1 and s
-                    const float Dv = (g0 * Fr0 * (fl[2 * P2N + f0] - st[10 * P1N + iC - 1]) - g1 * Fr1 * fl[2 * P2N + f1]) *
-                                     f * w.x(X_IRAD)[s];
-                    const float Sc = st[11 * P1N + iC];
-                    const float uc = w.x(X_UBG)[s] + du0;
-                    const float Sn = Sc + Dr;
-                    const float rmin = fmaxf(Sc * 1.0e-10f, 1.0e-10f);
-                    if (Sn < rmin) {
-                        dSn = rmin - w.x(X_SBG)[s];
-                        atomicAdd(&sc->floor_hits, 1);
-                    } else {
-                        const float iS = 1.0f / Sn;
-                        dSn = dS0 + Dr;
-                        dun = du0 + (Du - uc * Dr) * iS;
-                        dvn = dv0 + Dv * iS;
-                    }
-                    if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+        float db[16], wt[6], cs2[5], rad[5];
+        xload<16>(w, X_DBG, c, db);
+        xload<6>(w, X_WX, c, wt);
+#pragma unroll
+        for (int m = 0; m < 5; ++m) {
+            cs2[m] = w.x(X_CS2)[c - 2 + m];
+            rad[m] = w.x(X_RAD)[c - 2 + m];
+        }
+        const float sbg = w.x(X_SBG)[c], pbg = w.x(X_PBG)[c], ubg = w.x(X_UBG)[c], sx = dtf * w.x(X_IDX)[c];
+        const float g0 = w.x(X_XA)[c], g1 = w.x(X_XA)[c + 1], f = dtf * w.x(X_IXV)[c], irad = w.x(X_IRAD)[c];
+#pragma unroll 1
+        for (int j = run.z; j < run.w; ++j, src += D.pitch) {
+            float dS[5], du[5], dv[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+                dS[m] = src[m - 2];
+                du[m] = src[D.pl + m - 2];
+                dv[m] = src[2 * D.pl + m - 2];
+            }
+            float aS[5], aP[5], aU[5], aL[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+                if (m == 2) {
+                    aS[m] = aP[m] = aU[m] = aL[m] = 0.0f;
+                    continue;
                 }
-                emit32(w, w.buf[in ^ 1], s, j, dSn, dun, dvn);
+                const int kk = m < 2 ? m : m - 1;
+                aS[m] = (dS[m] - dS[2]) + db[kk];
+                aP[m] = (cs2[m] * dS[m] - cs2[2] * dS[2]) + db[4 + kk];
+                aU[m] = (du[m] - du[2]) + db[8 + kk];
+                aL[m] = (rad[m] * dv[m] - rad[2] * dv[2]) + db[12 + kk];
+            }
+            const float Sc = sbg + dS[2];
+            const float pc = pbg + cs2[2] * dS[2];
+            const float uc = ubg + du[2];
+            const float cs0 = gam * pc * rsq32(gam * pc * Sc);
+            const float flat = flatten32(pc, aP[0], aP[1], aP[3], aP[4], aU[1], aU[3]);
+            const Par32 R = recon32(wt, aS[0], aS[1], aS[3], aS[4], flat);
+            const Par32 P = recon32(wt, aP[0], aP[1], aP[3], aP[4], flat);
+            const Par32 U = recon32(wt, aU[0], aU[1], aU[3], aU[4], flat);
+            const Par32 A = recon32(wt, aL[0], aL[1], aL[3], aL[4], flat);
+            const HS a = edge32<0>(gam, sx, cs0, Sc, pc, uc, R, P, U, A);
+            const HS b = edge32<1>(gam, sx, cs0, Sc, pc, uc, R, P, U, A);
+            // HLLC at the left face, referenced to its left cell (jumps from there to this cell)
+            const float jS = up1(aS[3]), jP = up1(aP[3]), jL = up1(aL[3]);
+            const HS L{up1(b.rd), up1(b.pd), up1(b.u), up1(b.v)};
+            const HS Rr{a.rd + jS, a.pd + jP, a.u, a.v + jL};
+            const FX F = hllc32(gam, up1(Sc), up1(pc), L, Rr);
+            // residual update (sweeps.cu:218-261, 300-335)
+            const float Fr1 = down1(F.r);
+            const float Dr = (F.r * g0 - Fr1 * g1) * f;
+            // pres0 - pres1 = (p[s-1] - p[s]) + (pd0 - pd1)
+            const float dpres = (F.pd - down1(F.pd)) - jP;
+            const float Du = ((F.u * g0 - down1(F.u) * g1) + 0.5f * (g0 + g1) * dpres) * f;
+            // D(Sigma v) - v D(Sigma) with l = r v: faces referenced to cells s-1 and s
+            const float Dv = (g0 * F.r * (F.v - jL) - g1 * Fr1 * down1(F.v)) * f * irad;
+            if (output) {
+                float dSn = dS[2], dun = du[2], dvn = dv[2];
+                const float Sn = Sc + Dr;
+                const float rmin = fmaxf(Sc * 1.0e-10f, 1.0e-10f);
+                if (Sn < rmin) {
+                    dSn = rmin - sbg;
+                    atomicAdd(&sc->floor_hits, 1);
+                } else {
+                    const float iS = rcp32(Sn);
+                    dSn += Dr;
+                    dun += (Du - uc * Dr) * iS;
+                    dvn += Dv * iS;
+                }
+                if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                D.emit(i, j, dSn, dun, dvn);
             }
         }
-        __syncthreads();
     }
 }
 
 // ========================================= azimuthal sweep + orbital shift
-template <int MB>
-__global__ void __launch_bounds__(SWT, MB) k32_sweep_y(const View32* __restrict__ V, const int4* __restrict__ tiles,
-                                                   int nd, int ntiles, int in) {
-    extern __shared__ __align__(128) float fsm_raw[];
-    float* sm = smem_base128f(fsm_raw);
-    auto stage = [&](int n) { return sm + (n & 1) * YS; };
-    float* st = sm + 2 * YS;      // [NSY][P1N]
-    float* fl = st + NSY * P1N;   // [4][P2N]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 4 * P2N);
-    __shared__ int s_inc[T_W];
-    const int tid = threadIdx.x;
-    auto locate = [&](int tile, int& k, int& s0, int& q0) {  // the tile's disk and origin (pg_ens tile table)
-        const int4 t = tiles[tile];
-        k = t.x;
-        s0 = t.y;
-        q0 = t.z;
-    };
-    auto issue = [&](int tile, int kt) {
-        int k, s0, q0;
-        locate(tile, k, s0, q0);
-        issue_begin(&bar[kt & 1], YPL * NPL * 4);
-        tma_load_3d(stage(kt), V[k].maps + 3 * in + 1, q0 - NPAD, s0 - NPAD, 0, &bar[kt & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int k, s0, q0;
-        locate(tile_id, k, s0, q0);
-        const View32& w = V[k];
+// A lane marches along its column: five rows of it in registers, the next in flight.
+__global__ void __launch_bounds__(MT, 5) k32_sweep_y(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                  int nruns, int in) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_enter();
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
         Scalars* sc = w.d64.sc;
-        const float* T = stage(kt);
         const bool done = sc->done != 0;
         const double dt = sc->dt;
-        const float dtf = (float)dt;
-        const float gam = w.gam;
-        if (tid < T_W) {
+        const float dtf = (float)dt, gam = w.gam;
+        const int i = run.y + lane, c = min(i, NPAD + w.xres - 1);
+        const bool active = i < NPAD + w.xres;
+        const Disk32 D(w, in);
+        if (done) {
+            const float* src = w.buf[in] + (size_t)run.z * w.pitch + c;
+            for (int j = run.z; j < run.w; ++j, src += D.pitch)
+                if (active) D.emit(i, j, src[0], src[D.pl], src[2 * D.pl]);
+            continue;
+        }
+        int js = run.z - NPAD;  // row the first output goes to (orbit.cu:30-46)
+        if (w.orbadv) {
             // set_orbital_advection (src/orbit/orbit.cu:74-99) in FP64 for this column
-            const int i = q0 + tid;
-            int shift = 0;
-            if (!done && w.orbadv && i < NPAD + w.xres) {
-                const DiskView& d = w.d64;
-                const double dy = d.dy0 * d.radx[i];
-                const double rot = d.rot[i];
-                shift = __double2int_rd(rot * dt / dy + 0.5);
-                double speed = shift * dy / dt;
-                speed = rot - speed;
-                if (s0 == NPAD) {
-                    d.res[i] = speed;
-                    d.inc[i] = shift;
-                }
+            const DiskView& d = w.d64;
+            const double dy = d.dy0 * d.radx[c];
+            const double rot = d.rot[c];
+            const int shift = __double2int_rd(rot * dt / dy + 0.5);
+            double speed = shift * dy / dt;
+            speed = rot - speed;
+            if (run.z == NPAD && active) {
+                d.res[i] = speed;
+                d.inc[i] = shift;
             }
-            s_inc[tid] = shift;
+            js = (js + shift) % w.yres;
+            if (js < 0) js += w.yres;
         }
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
-        if (!done) {
-            // ---- P1: background-relative deviations along the column
-            if (tid < P1N) {
-                const int q = tid % T_W, t = 2 + tid / T_W;
-                const int i = min(q0 + q, w.xarr - 1);
-                const int jc = min(s0 - NPAD + t, w.yarr - 1);
-                const float* col = T + (q + NPAD) + (t - 2) * YB_W;
-                float dS[5], du[5], dv[5];
+        const float cs2 = w.x(X_CS2)[c], cs0 = w.x(X_CS0)[c], eps = w.x(X_EPS)[c], sbg = w.x(X_SBG)[c];
+        const float pbg = w.x(X_PBG)[c], irad = w.x(X_IRAD)[c], sdt = dtf * irad;
+        const float* next = w.buf[in] + (size_t)(run.z - NPAD) * w.pitch + c;
+        float dS[5], du[5], dv[5], nS = 0.0f, nu = 0.0f, nv = 0.0f;
 #pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    dS[m] = col[m * YB_W];
-                    du[m] = col[YPL + m * YB_W];
-                    dv[m] = col[2 * YPL + m * YB_W];
-                }
-                float aS[5], aN[5], aT[5];
-#pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    aS[m] = dS[m] - dS[2];
-                    aN[m] = dv[m] - dv[2];
-                    aT[m] = du[m] - du[2];
-                }
-                const float cs2 = w.x(X_CS2)[i];
-                const float Sc = w.x(X_SBG)[i] + dS[2];
-                const float pc = cs2 * Sc;
-                const float cs0 = w.x(X_CS0)[i];
-                const float un = dv[2] + w.x(X_EPS)[i];
-                // p = cs2 Sigma along the column: pressure ratios are density ratios
-                const float flat = flatten32(1.0f / cs0, Sc, aS[0], aS[1], aS[3], aS[4], aN[1], aN[3]);
-                float wt[6];
-                yload<6>(w, Y_WY, jc, wt);
-                const Par32 R = recon32(wt, aS[0], aS[1], aS[3], aS[4], flat);
-                const Par32 N = recon32(wt, aN[0], aN[1], aN[3], aN[4], flat);
-                const Par32 Tt = recon32(wt, aT[0], aT[1], aT[3], aT[4], flat);
-                const Par32 P{cs2 * R.sL, cs2 * R.sR};
-                const float sdt = dtf * w.x(X_IRAD)[i];
-                const float idy = w.y(Y_IDY)[jc];
-                HS a = left_edge32(gam, idy, sdt, cs0, Sc, pc, un, R, P, N, Tt);
-                HS b = right_edge32(gam, idy, sdt, cs0, Sc, pc, un, R, P, N, Tt);
-                a.rd += dS[2];
-                a.pd += cs2 * dS[2];
-                a.v += du[2];
-                b.rd += dS[2];
-                b.pd += cs2 * dS[2];
-                b.v += du[2];
-                float* o = st + tid;
-                o[0] = a.rd;
-                o[P1N] = a.pd;
-                o[2 * P1N] = a.u;
-                o[3 * P1N] = a.v;
-                o[4 * P1N] = b.rd;
-                o[5 * P1N] = b.pd;
-                o[6 * P1N] = b.u;
-                o[7 * P1N] = b.v;
-            }
-            __syncthreads();
-            // ---- P2: HLLC referenced to the background (constant along the column)
-            if (tid < P2N) {
-                const int q = tid % T_W, f = tid / T_W;
-                const int i = min(q0 + q, w.xarr - 1);
-                const int iL = f * T_W + q, iR = iL + T_W;
-                HS L, R;
-                L.rd = st[4 * P1N + iL];
-                L.pd = st[5 * P1N + iL];
-                L.u = st[6 * P1N + iL];
-                L.v = st[7 * P1N + iL];
-                R.rd = st[iR];
-                R.pd = st[P1N + iR];
-                R.u = st[2 * P1N + iR];
-                R.v = st[3 * P1N + iR];
-                const FX F = hllc32(gam, w.x(X_SBG)[i], w.x(X_PBG)[i], L, R);
-                fl[tid] = F.r;
-                fl[P2N + tid] = F.u;
-                fl[2 * P2N + tid] = F.v;
-                fl[3 * P2N + tid] = F.pd;
-            }
-            __syncthreads();
+        for (int m = 0; m < 5; ++m, next += D.pitch) {
+            dS[m] = next[0];
+            du[m] = next[D.pl];
+            dv[m] = next[2 * D.pl];
         }
-        // ---- P3: residual update (sweeps.cu:361-433) and the orbital shift (orbit.cu:30-46)
-        if (tid < T_LEN * T_W) {
-            const int q = tid % T_W, o = tid / T_W;
-            const int j = s0 + o, i = q0 + q;
-            if (j < NPAD + w.yres && i < NPAD + w.xres) {
-                const float* c = T + (NPAD + o) * YB_W + NPAD + q;
-                const float dS0 = c[0], du0 = c[YPL], dv0 = c[2 * YPL];
-                float dSn = dS0, dun = du0, dvn = dv0;
-                int jo = j;
-                if (!done) {
-                    const int f0 = o * T_W + q, f1 = f0 + T_W;
-                    const float f = dtf * w.y(Y_IYV)[j] * w.x(X_IRAD)[i];
-                    const float Fr0 = fl[f0], Fr1 = fl[f1];
-                    const float Dr = (Fr0 - Fr1) * f;
-                    const float Dn = ((fl[P2N + f0] - fl[P2N + f1]) + (fl[3 * P2N + f0] - fl[3 * P2N + f1])) * f;
-                    const float Dt = (Fr0 * (fl[2 * P2N + f0] - du0) - Fr1 * (fl[2 * P2N + f1] - du0)) * f;
-                    const float Sc = w.x(X_SBG)[i] + dS0;
-                    const float Sn = Sc + Dr;
-                    const float un = dv0 + w.x(X_EPS)[i];
-                    const float rmin = fmaxf(Sc * 1.0e-10f, 1.0e-10f);
+        HS pb{};   // the right edge of the cell below
+        FX pf{};   // the flux at the face below it
+#pragma unroll 1
+        for (int t = run.z - 1; t <= run.w; ++t, next += D.pitch) {
+            if (t < run.w) {
+                nS = next[0];
+                nu = next[D.pl];
+                nv = next[2 * D.pl];
+            }
+            float aS[5], aN[5], aT[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) {
+                aS[m] = dS[m] - dS[2];
+                aN[m] = dv[m] - dv[2];
+                aT[m] = du[m] - du[2];
+            }
+            const float Sc = sbg + dS[2];
+            const float pc = cs2 * Sc;
+            const float un = dv[2] + eps;
+            // p = cs2 Sigma along the column: pressure ratios are density ratios
+            const float flat = flatten32(Sc, aS[0], aS[1], aS[3], aS[4], aN[1], aN[3]);
+            float wt[6];
+            D.ys<6>(Y_WY, t, wt);
+            const Par32 R = recon32(wt, aS[0], aS[1], aS[3], aS[4], flat);
+            const Par32 N = recon32(wt, aN[0], aN[1], aN[3], aN[4], flat);
+            const Par32 Tt = recon32(wt, aT[0], aT[1], aT[3], aT[4], flat);
+            const Par32 P{cs2 * R.sL, cs2 * R.sR};
+            const float sx = sdt * D.y(Y_IDY, t);
+            HS a = edge32<0>(gam, sx, cs0, Sc, pc, un, R, P, N, Tt);
+            HS b = edge32<1>(gam, sx, cs0, Sc, pc, un, R, P, N, Tt);
+            // relative to the background, which is constant along the column
+            a.rd += dS[2];
+            a.pd += cs2 * dS[2];
+            a.v += du[2];
+            b.rd += dS[2];
+            b.pd += cs2 * dS[2];
+            b.v += du[2];
+            FX F{};
+            if (t >= run.z) F = hllc32(gam, sbg, pbg, pb, a);
+            if (t > run.z) {  // the cell below has both its fluxes
+                const int j = t - 1;
+                const float dS0 = dS[1], du0 = du[1], dv0 = dv[1];
+                const float f = dtf * D.y(Y_IYV, j) * irad;
+                const float Dr = (pf.r - F.r) * f;
+                const float Dn = ((pf.u - F.u) + (pf.pd - F.pd)) * f;
+                const float Dt = (pf.r * (pf.v - du0) - F.r * (F.v - du0)) * f;
+                if (active) {
+                    float dSn = dS0, dun = du0, dvn = dv0;
+                    const float S0 = sbg + dS0;
+                    const float Sn = S0 + Dr;
+                    const float rmin = fmaxf(S0 * 1.0e-10f, 1.0e-10f);
                     if (Sn < rmin) {
-                        dSn = rmin - w.x(X_SBG)[i];
+                        dSn = rmin - sbg;
                         atomicAdd(&sc->floor_hits, 1);
                     } else {
-                        const float iS = 1.0f / Sn;
+                        const float iS = rcp32(Sn);
                         dSn = dS0 + Dr;
-                        dvn = dv0 + (Dn - un * Dr) * iS;
+                        dvn = dv0 + (Dn - (dv0 + eps) * Dr) * iS;
                         dun = du0 + Dt * iS;
                     }
                     if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                    if (w.orbadv) {
-                        int js = (j - NPAD + s_inc[q]) % w.yres;
-                        if (js < 0) js += w.yres;
-                        jo = js + NPAD;
-                    }
+                    D.emit(i, js + NPAD, dSn, dun, dvn);
                 }
-                emit32(w, w.buf[in ^ 1], i, jo, dSn, dun, dvn);
+                if (++js == D.yres) js = 0;
             }
+            pb = b;
+            pf = F;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                dS[m] = dS[m + 1];
+                du[m] = du[m + 1];
+                dv[m] = dv[m + 1];
+            }
+            dS[4] = nS;
+            du[4] = nu;
+            dv[4] = nv;
         }
-        __syncthreads();
     }
 }
 
 // ===================================================== residual advection
-template <int MB>
-__global__ void __launch_bounds__(SWT, MB) k32_advect(const View32* __restrict__ V, const int4* __restrict__ tiles,
-                                                  int nd, int ntiles, int in) {
-    extern __shared__ __align__(128) float fsm_raw[];
-    float* sm = smem_base128f(fsm_raw);
-    auto stage = [&](int n) { return sm + (n & 1) * YS; };
-    float* fl = sm + 2 * YS;  // [3][NFA]: mass flux, then the upwind carriers of v and u
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 3 * NFA);
-    const int tid = threadIdx.x;
-    auto locate = [&](int tile, int& k, int& s0, int& q0) {  // the tile's disk and origin (pg_ens tile table)
-        const int4 t = tiles[tile];
-        k = t.x;
-        s0 = t.y;
-        q0 = t.z;
-    };
-    auto issue = [&](int tile, int kt) {
-        int k, s0, q0;
-        locate(tile, k, s0, q0);
-        issue_begin(&bar[kt & 1], YPL * NPL * 4);
-        tma_load_3d(stage(kt), V[k].maps + 3 * in + 1, q0 - NPAD, s0 - NPAD, 0, &bar[kt & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int k, s0, q0;
-        locate(tile_id, k, s0, q0);
-        const View32& w = V[k];
+// advection.cu:20-170.  The residual speed of a column has one sign: every cell feeds
+// the same one of its two faces, and with this row's flux and the last one's the update
+// of this row (upwards) or the last (downwards) is complete.
+__global__ void __launch_bounds__(MT, 5) k32_advect(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                 int nruns, int in) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_enter();
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
         Scalars* sc = w.d64.sc;
-        const float* T = stage(kt);
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
         const bool done = sc->done != 0;
         const double dt = sc->dt;
         const float dtf = (float)dt;
-        if (!done) {
-            // ---- P1: upwind PPM average over the swept fraction (advection.cu:20-67)
-            if (tid < P1N) {
-                const int q = tid % T_W, t = 2 + tid / T_W;
-                const int i = min(q0 + q, w.xarr - 1);
-                const int jc = min(s0 - NPAD + t, w.yarr - 1);
-                const DiskView& d = w.d64;
-                const double speed = d.res[i];
-                // the swept fraction in FP64: |res| dt / (r dphi)
-                const float yf = (float)fmin(fmax(fabs(speed) * (dt * d.irad[i]) * d.idx_y[jc], 0.0), 1.0);
-                const float* col = T + (q + NPAD) + (t - 2) * YB_W;
-                float dS[5], du[5], dv[5];
+        const int i = run.y + lane, c = min(i, NPAD + w.xres - 1);
+        const bool active = i < NPAD + w.xres;
+        const Disk32 D(w, in);
+        if (done) {
+            const float* src = w.buf[in] + (size_t)run.z * w.pitch + c;
+            for (int j = run.z; j < run.w; ++j, src += D.pitch)
+                if (active) D.emit(i, j, src[0], src[D.pl], src[2 * D.pl]);
+            continue;
+        }
+        const DiskView& d = w.d64;
+        const double speed = d.res[c];
+        const double* idy = d.idx_y;
+        const double sx = fabs(speed) * (dt * d.irad[c]);
+        const bool up = speed > 0.0;
+        const float spf = (float)speed, sbg = w.x(X_SBG)[c], irad = w.x(X_IRAD)[c];
+        const float* next = w.buf[in] + (size_t)(run.z - NPAD) * w.pitch + c;
+        float dS[5], du[5], dv[5], nS = 0.0f, nu = 0.0f, nv = 0.0f;
 #pragma unroll
-                for (int m = 0; m < 5; ++m) {
-                    dS[m] = col[m * YB_W];
-                    du[m] = col[YPL + m * YB_W];
-                    dv[m] = col[2 * YPL + m * YB_W];
-                }
-                float wt[6];
-                yload<6>(w, Y_WY, jc, wt);
-                const Par32 R = recon32(wt, dS[0] - dS[2], dS[1] - dS[2], dS[3] - dS[2], dS[4] - dS[2], 0.0f);
-                const Par32 N = recon32(wt, dv[0] - dv[2], dv[1] - dv[2], dv[3] - dv[2], dv[4] - dv[2], 0.0f);
-                const Par32 Tt = recon32(wt, du[0] - du[2], du[1] - du[2], du[3] - du[2], du[4] - du[2], 0.0f);
-                const Frac32 qf = frac32(yf);
-                float fr, fn, ft;
-                int face;
-                if (speed > 0.0) {
-                    fr = aveR32(qf, R);
-                    fn = aveR32(qf, N);
-                    ft = aveR32(qf, Tt);
-                    face = t + 1;
-                } else {
-                    fr = aveL32(qf, R);
-                    fn = aveL32(qf, N);
-                    ft = aveL32(qf, Tt);
-                    face = t;
-                }
-                const float Sc = w.x(X_SBG)[i] + dS[2];
-                const int m = face * T_W + q;
-                fl[m] = (Sc + fr) * (float)speed;
-                fl[NFA + m] = dv[2] + fn;
-                fl[2 * NFA + m] = du[2] + ft;
-            }
-            __syncthreads();
+        for (int m = 0; m < 5; ++m, next += D.pitch) {
+            dS[m] = next[0];
+            du[m] = next[D.pl];
+            dv[m] = next[2 * D.pl];
         }
-        // ---- P2: flux difference and update_Cell_advect (advection.cu:88-105, 153-170)
-        if (tid < T_LEN * T_W) {
-            const int q = tid % T_W, o = tid / T_W;
-            const int s = s0 + o, i = q0 + q;
-            if (s < NPAD + w.yres && i < NPAD + w.xres) {
-                const float* c = T + (NPAD + o) * YB_W + NPAD + q;
-                const float dS0 = c[0], du0 = c[YPL], dv0 = c[2 * YPL];
-                float dSn = dS0, dun = du0, dvn = dv0;
-                if (!done) {
-                    const int k0 = (NPAD + o) * T_W + q, k1 = k0 + T_W;
-                    const float f = dtf * w.y(Y_IYV)[s] * w.x(X_IRAD)[i];
-                    const float F0 = fl[k0], F1 = fl[k1];
-                    const float Dr = (F0 - F1) * f;
-                    const float Sn = (w.x(X_SBG)[i] + dS0) + Dr;
-                    const float iS = 1.0f / Sn;
-                    dSn = dS0 + Dr;
-                    dvn = dv0 + (F0 * (fl[NFA + k0] - dv0) - F1 * (fl[NFA + k1] - dv0)) * f * iS;
-                    dun = du0 + (F0 * (fl[2 * NFA + k0] - du0) - F1 * (fl[2 * NFA + k1] - du0)) * f * iS;
-                    if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                }
-                emit32(w, w.buf[in ^ 1], i, s, dSn, dun, dvn);
+        float pr = 0.0f, pn = 0.0f, pt = 0.0f;  // the row before: mass flux and the carried v and u
+#pragma unroll 1
+        for (int t = run.z - 1; t <= run.w; ++t, next += D.pitch) {
+            if (t < run.w) {
+                nS = next[0];
+                nu = next[D.pl];
+                nv = next[2 * D.pl];
             }
+            // the swept fraction in FP64: |res| dt / (r dphi)
+            const Frac32 qf = frac32((float)fmin(sx * idy[t], 1.0));
+            float wt[6];
+            D.ys<6>(Y_WY, t, wt);
+            const Par32 R = recon32(wt, dS[0] - dS[2], dS[1] - dS[2], dS[3] - dS[2], dS[4] - dS[2], 0.0f);
+            const Par32 N = recon32(wt, dv[0] - dv[2], dv[1] - dv[2], dv[3] - dv[2], dv[4] - dv[2], 0.0f);
+            const Par32 Tt = recon32(wt, du[0] - du[2], du[1] - du[2], du[3] - du[2], du[4] - du[2], 0.0f);
+            const float fr = ((sbg + dS[2]) + (up ? aveR32(qf, R) : aveL32(qf, R))) * spf;
+            const float fn = dv[2] + (up ? aveR32(qf, N) : aveL32(qf, N));
+            const float ft = du[2] + (up ? aveR32(qf, Tt) : aveL32(qf, Tt));
+            const int j = up ? t : t - 1;
+            if (active && j >= run.z && j < run.w) {
+                const float dS0 = up ? dS[2] : dS[1], du0 = up ? du[2] : du[1], dv0 = up ? dv[2] : dv[1];
+                const float f = dtf * D.y(Y_IYV, j) * irad;
+                const float Dr = (pr - fr) * f;
+                const float Sn = (sbg + dS0) + Dr;
+                const float iS = rcp32(Sn);
+                if (!(Sn > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                D.emit(i, j, dS0 + Dr, du0 + (pr * (pt - du0) - fr * (ft - du0)) * f * iS,
+                       dv0 + (pr * (pn - dv0) - fr * (fn - dv0)) * f * iS);
+            }
+            pr = fr;
+            pn = fn;
+            pt = ft;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                dS[m] = dS[m + 1];
+                du[m] = du[m + 1];
+                dv[m] = dv[m + 1];
+            }
+            dS[4] = nS;
+            du[4] = nu;
+            dv[4] = nv;
         }
-        __syncthreads();
     }
 }
 
 // ====================================================== kick 1 (+ stress)
-template <int MB>
-__global__ void __launch_bounds__(STT, MB) k32_kick1(const View32* __restrict__ V, const int4* __restrict__ tiles, int nd,
-                                                 int ntiles, int in) {
-    extern __shared__ __align__(128) float fsm_raw[];
-    float* sm = smem_base128f(fsm_raw);
-    auto stage = [&](int n) { return sm + (n & 1) * SS; };
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * SS);
-    const int tid = threadIdx.x;
-    auto locate = [&](int tile, int& k, int& i0, int& j0) {  // the tile's disk and origin (pg_ens tile table)
-        const int4 t = tiles[tile];
-        k = t.x;
-        i0 = t.y;
-        j0 = t.z;
-    };
-    auto issue = [&](int tile, int kt) {
-        int k, i0, j0;
-        locate(tile, k, i0, j0);
-        issue_begin(&bar[kt & 1], SPL * NPL * 4);
-        tma_load_3d(stage(kt), V[k].maps + 3 * in + 2, i0 - NPAD, j0 - 1, 0, &bar[kt & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int k, i0, j0;
-        locate(tile_id, k, i0, j0);
-        const View32& w = V[k];
+// Lanes 1..30 of a run have an output; the stress stencil's rows stay in registers.
+__global__ void __launch_bounds__(MT, 5) k32_kick1(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                int nruns, int in) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_enter();
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
         Scalars* sc = w.d64.sc;
-        const float* T = stage(kt);
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
-        const bool done = sc->done != 0;
+        const bool done = sc->done != 0, visc = w.visc != 0;
         const float hdt = (float)(0.5 * sc->dt);
-        const int hx = tid % T_LEN, hy = tid / T_LEN;
-        const int i = i0 + hx, j = j0 + hy;
-        if (i < NPAD + w.xres && j < NPAD + w.yres) {
-            const int x = hx + NPAD, y = hy + 1;
-            const int c = y * SB_W + x;
-            const float dS0 = T[c];
-            float du = T[SPL + c], dv = T[2 * SPL + c];
-            const float gu = du, gv = dv;  // the gas cell the dust drag relaxes to
-            DR D{0.0f, 0.0f, 0.0f};
-            if (w.dust) D = dload(w, w.dbuf[in], i, j);
-            if (!done) {
-                float vx = 0.0f, vy = 0.0f;
-                if (w.visc) {
-                    stress32(w, T, x, y, i, j, vx, vy);
-                    // kept for the predictor of kick2, with the periodic image
-                    const size_t pl = w.plane();
-                    size_t m = (size_t)j * w.pitch + i;
-                    w.vis[m] = vx;
-                    w.vis[pl + m] = vy;
-                    int jimg = -1;
-                    if (j < 2 * NPAD) jimg = j + w.yres;
-                    else if (j >= w.yres) jimg = j - w.yres;
-                    if (jimg >= 0) {
-                        m = (size_t)jimg * w.pitch + i;
-                        w.vis[m] = vx;
-                        w.vis[pl + m] = vy;
-                    }
+        const int i = run.y + lane, c = min(i, w.xarr - 1);
+        const bool output = lane >= 1 && lane <= 30 && i < NPAD + w.xres;
+        const Disk32 D(w, in);
+        const float* next = w.buf[in] + (size_t)run.z * w.pitch + c;
+        if (done) {
+            for (int j = run.z; j < run.w; ++j, next += D.pitch)
+                if (output) {
+                    D.emit(i, j, next[0], next[D.pl], next[2 * D.pl]);
+                    if (w.dust) dstore(w, w.dbuf[in ^ 1], i, j, dload(w, w.dbuf[in], i, j));
                 }
-                float gx, gy;
-                gravity32(w, i, j, 0, gx, gy);
-                kick32(w, i, dS0, du, dv, vx, vy, gx, gy, 0.0f, hdt, w.visc != 0);
-                if (w.dust) dust_drag32(w, i, w.x(X_SBG)[i] + dS0, gu, gv, 0.0f, 0.0f, gx, gy, 0.0f, hdt, D);
-            }
-            emit32(w, w.buf[in ^ 1], i, j, dS0, du, dv);
-            if (w.dust) dstore(w, w.dbuf[in ^ 1], i, j, D);
+            continue;
         }
-        __syncthreads();
+        const Kick32 K = kick_tables(w, c, 0);
+        const bool dusty = w.dust != 0;
+        float* vis = w.vis + ((size_t)run.z * D.pitch + c);
+        const float* const last = next + (size_t)(run.w - run.z) * D.pitch;
+        next -= D.pitch;
+        Row32 lo{}, mid = row32(next[0], next[D.pl], next[2 * D.pl]);
+        next += D.pitch;
+        Row32 hi = row32(next[0], next[D.pl], next[2 * D.pl]);
+        next += D.pitch;
+        float nS = next[0], nu = next[D.pl], nv = next[2 * D.pl];  // a row ahead of the stencil
+#pragma unroll 1
+        for (int j = run.z; j < run.w; ++j, vis += D.pitch) {
+            lo = mid;
+            mid = hi;
+            hi = row32(nS, nu, nv);
+            if (next < last) {
+                next += D.pitch;
+                nS = next[0];
+                nu = next[D.pl];
+                nv = next[2 * D.pl];
+            }
+            float vx = 0.0f, vy = 0.0f;
+            if (visc) stress32(D, K, j, lo, mid, hi, vx, vy);
+            if (!output) continue;
+            if (visc) {  // kept for the predictor of kick2, with the periodic image
+                vis[0] = vx;
+                vis[D.pl] = vy;
+                if (j < 2 * NPAD || j >= D.yres) {
+                    float* s = vis + (long long)(j < 2 * NPAD ? D.yres : -D.yres) * D.pitch;
+                    s[0] = vx;
+                    s[D.pl] = vy;
+                }
+            }
+            float gx, gy, du = mid.u[1], dv = mid.v[1];
+            gravity32(K, j, gx, gy);
+            kick32(K, mid.S, du, dv, vx, vy, gx, gy, 0.0f, hdt, visc);
+            D.emit(i, j, mid.S, du, dv);
+            if (dusty) {
+                DR q = dload(w, w.dbuf[in], i, j);
+                dust_drag32(w, i, K.sbg + mid.S, mid.u[1], mid.v[1], 0.0f, 0.0f, gx, gy, 0.0f, hdt, q);
+                dstore(w, w.dbuf[in ^ 1], i, j, q);
+            }
+        }
     }
 }
 
 // ============================================ kick 2 + damping + CFL speed
-template <int MB>
-__global__ void __launch_bounds__(STT, MB) k32_kick2(const View32* __restrict__ V, const int4* __restrict__ tiles, int nd,
-                                                 int ntiles, int in) {
-    extern __shared__ __align__(128) float fsm_raw[];
-    float* sm = smem_base128f(fsm_raw);
-    auto stage = [&](int n) { return sm + (n & 1) * SS; };
-    auto vstage = [&](int n) { return sm + 2 * SS + (n & 1) * VS; };
-    float* tp = sm + 2 * SS + 2 * VS;  // predicted state with 1 halo, same layout as a stage
-    uint64_t* bar = reinterpret_cast<uint64_t*>(tp + SS);
-    const int tid = threadIdx.x;
-    auto locate = [&](int tile, int& k, int& i0, int& j0) {  // the tile's disk and origin (pg_ens tile table)
-        const int4 t = tiles[tile];
-        k = t.x;
-        i0 = t.y;
-        j0 = t.z;
-    };
-    auto issue = [&](int tile, int kt) {
-        int k, i0, j0;
-        locate(tile, k, i0, j0);
-        const View32& w = V[k];
-        issue_begin(&bar[kt & 1], (SPL * NPL + (w.visc ? SPL * 2 : 0)) * 4);
-        tma_load_3d(stage(kt), w.maps + 3 * in + 2, i0 - NPAD, j0 - 1, 0, &bar[kt & 1]);
-        if (w.visc) tma_load_3d(vstage(kt), w.maps + 6, i0 - NPAD, j0 - 1, 0, &bar[kt & 1]);
-    };
-    pipe_init(bar);
-    double vmax = 0.0;
-    int vk = -1;  // disk whose signal rate vmax holds
-    if ((int)blockIdx.x < ntiles) {
-        if (tid == 0) issue(blockIdx.x, 0);
-        int kt = 0;
-        for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-            if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-            int k, i0, j0;
-            locate(tile_id, k, i0, j0);
-            const View32& w = V[k];
-            Scalars* sc = w.d64.sc;
-            if (k != vk) {  // uniform over the CTA: flush the previous disk's maximum
-                if (vk >= 0) block_max_to<STT>(&V[vk].d64.sc->vmax_bits, vmax);
-                vmax = 0.0;
-                vk = k;
-            }
-            const float* T = stage(kt);
-            const float* TV = vstage(kt);
-            if (!pipe_wait(bar, kt, sc)) {
-                pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-                return;
-            }
-            const bool done = sc->done != 0;
-            const double dt = sc->dt;
-            const float dtf = (float)dt, hdt = (float)(0.5 * dt);
-            const bool visc = w.visc != 0;
-            if (!done && visc) {
-                // predictor (sweeps.cu:713-729, mdt = dt = dt/2) with the stress of kick1, on
-                // the tile and its halo; outside the radial range the ghosts keep init_C (zero
-                // residuals) as boundx2 does for boundary 0 (boundary.cu:722-820)
-                for (int it = tid; it < (T_LEN + 2) * SB_H; it += STT) {
-                    const int hx = it % (T_LEN + 2), hy = it / (T_LEN + 2);
-                    const int x = hx + NPAD - 1, y = hy;
-                    const int i = i0 - 1 + hx, j = j0 - 1 + hy;
-                    const int c = y * SB_W + x;
-                    float dS = T[c], du = T[SPL + c], dv = T[2 * SPL + c];
-                    if (i >= NPAD && i < NPAD + w.xres && j < w.yarr) {
-                        float gx, gy;
-                        gravity32(w, i, j, 1, gx, gy);
-                        kick32(w, i, dS, du, dv, TV[c], TV[SPL + c], gx, gy, hdt, hdt, true);
-                    }
-                    tp[c] = dS;
-                    tp[SPL + c] = du;
-                    tp[2 * SPL + c] = dv;
+// A row is predicted (sweeps.cu:713-729, mdt = dt = dt/2) with the stress of kick1 when
+// it enters; outside the radial range the ghosts keep init_C (zero residuals) as boundx2
+// does for boundary 0 (boundary.cu:722-820).
+__global__ void __launch_bounds__(MT, 5) k32_kick2(const View32* __restrict__ V, const int4* __restrict__ runs,
+                                                int nruns, int in) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_enter();
+    for (int it = blockIdx.x * MW + warp; it < nruns; it += gridDim.x * MW) {
+        const int4 run = runs[it];
+        const View32& w = V[run.x];
+        Scalars* sc = w.d64.sc;
+        const bool done = sc->done != 0, visc = w.visc != 0;
+        const double dt = sc->dt;
+        const float dtf = (float)dt, hdt = (float)(0.5 * dt);
+        const int i = run.y + lane, c = min(i, w.xarr - 1);
+        const bool inside = i >= NPAD && i < NPAD + w.xres;
+        const bool output = inside && lane >= 1 && lane <= 30;
+        const Disk32 D(w, in);
+        const float* next = w.buf[in] + (size_t)run.z * w.pitch + c;
+        if (done) {
+            for (int j = run.z; j < run.w; ++j, next += D.pitch)
+                if (output) {
+                    D.emit(i, j, next[0], next[D.pl], next[2 * D.pl]);
+                    if (w.dust) dstore(w, w.dbuf[in ^ 1], i, j, dload(w, w.dbuf[in], i, j));
                 }
-                __syncthreads();
-            }
-            const int hx = tid % T_LEN, hy = tid / T_LEN;
-            const int i = i0 + hx, j = j0 + hy;
-            if (i < NPAD + w.xres && j < NPAD + w.yres) {
-                const int x = hx + NPAD, y = hy + 1;
-                const int c = y * SB_W + x;
-                float dS = T[c], du = T[SPL + c], dv = T[2 * SPL + c];
-                DR D{0.0f, 0.0f, 0.0f};
-                if (w.dust) D = dload(w, w.dbuf[in], i, j);
-                if (!done) {
-                    float vx = 0.0f, vy = 0.0f;
-                    if (visc) stress32(w, tp, x, y, i, j, vx, vy);
-                    float gx, gy;
-                    gravity32(w, i, j, 1, gx, gy);
-                    if (w.dust) {
-                        // the gas velocity predicted over mdt (sweeps.cu:679-687), towards which
-                        // the dust's corrector relaxes
-                        const float iS = visc ? 1.0f / (w.x(X_SBG)[i] + dS) : 0.0f;
-                        const float ir = w.x(X_IRAD)[i];
-                        const float fx0 = w.x(X_ABG)[i] + (w.x(X_V2R)[i] + dv * ir) * dv + vx * iS;
-                        const float tu = du + fx0 * hdt + gx * hdt, tv = dv + vy * iS * hdt + gy * hdt;
-                        dust_drag32(w, i, w.x(X_SBG)[i] + dS, du, dv, tu, tv, gx, gy, hdt, hdt, D);
-                        vmax = fmax(vmax, drate64(w, i, j, D.u, D.v));
-                    }
-                    kick32(w, i, dS, du, dv, vx, vy, gx, gy, hdt, hdt, visc);
-                    if (w.kill) {
-                        // killwave (killwave.cu:48-100): relax towards init_C, i.e. residuals towards 0
-                        float kw[4];
-                        xload<4>(w, X_KILL, i, kw);
-#pragma unroll
-                        for (int side = 0; side < 2; ++side) {
-                            const float itau = kw[2 * side + 1];
-                            if (itau > 0.0f) {
-                                const float f = kw[2 * side] * (dtf * itau);
-                                dS -= f * dS;
-                                du -= f * du;
-                                dv -= f * dv;
-                            }
-                        }
-                    }
-                    if (!(w.x(X_SBG)[i] + dS > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                    vmax = fmax(vmax, rate64(w, i, j, du, dv));
-                }
-                emit32(w, w.buf[in ^ 1], i, j, dS, du, dv);
-                if (w.dust) dstore(w, w.dbuf[in ^ 1], i, j, D);
-            }
-            __syncthreads();
+            continue;
         }
+        const Kick32 K = kick_tables(w, c, 1);
+        const DiskView& d = w.d64;
+        // the CFL rate (timestep.cu:46-77) in FP64 from the residuals
+        const double ubg = d.initx[5 * c + 2], vbg = d.initx[5 * c + 3] - d.radx[c] * d.frame_omega - d.rot[c];
+        const double cs = w.cs64[c], idx = d.idx_x[c], irad = d.irad[c];
+        float kw[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (w.kill) xload<4>(w, X_KILL, c, kw);
+        const double* idy = d.idx_y;
+        const bool dusty = w.dust != 0, damped = kw[1] > 0.0f || kw[3] > 0.0f;
+        double vmax = 0.0;
+        int jn = run.z - 1;  // the next row to enter the stencil
+        next -= D.pitch;
+        const float* const last = next + (size_t)(run.w - run.z + 1) * D.pitch;
+        const float* nvis = w.vis + ((size_t)jn * D.pitch + c);
+        float u = 0.0f, v = 0.0f, gx = 0.0f, gy = 0.0f;      // the middle row before the kick, its gravity
+        float un = 0.0f, vn = 0.0f, gxn = 0.0f, gyn = 0.0f;  // ... of the row that entered last
+        float nS, nu, nv, nx = 0.0f, ny = 0.0f;              // the row after it and its stress, in flight
+        auto fetch = [&]() {
+            nS = next[0];
+            nu = next[D.pl];
+            nv = next[2 * D.pl];
+            if (visc) {
+                nx = nvis[0];
+                ny = nvis[D.pl];
+            }
+        };
+        Row32 lo{}, mid{}, hi{};
+        auto enter = [&]() {
+            const float S = nS, fx = nx, fy = ny;
+            un = nu;
+            vn = nv;
+            if (next < last) {
+                next += D.pitch;
+                nvis += D.pitch;
+                fetch();
+            }
+            gravity32(K, jn, gxn, gyn);
+            float pu = un, pv = vn;
+            if (visc) {
+                if (inside) kick32(K, S, pu, pv, fx, fy, gxn, gyn, hdt, hdt, true);
+                hi = row32(S, pu, pv);
+            } else {
+                hi.S = S;
+            }
+            ++jn;
+        };
+        fetch();
+#pragma unroll 1
+        for (int j = run.z - 2; j < run.w; ++j) {  // two rows enter before the first output
+            lo = mid;
+            mid = hi;
+            u = un;
+            v = vn;
+            gx = gxn;
+            gy = gyn;
+            enter();
+            if (j < run.z) continue;
+            float vx = 0.0f, vy = 0.0f;
+            if (visc) stress32(D, K, j, lo, mid, hi, vx, vy);
+            if (!output) continue;
+            float dS = mid.S, du = u, dv = v;
+            if (dusty) {
+                // the gas velocity predicted over mdt (sweeps.cu:679-687), towards which
+                // the dust's corrector relaxes
+                DR q = dload(w, w.dbuf[in], i, j);
+                const float iS = visc ? rcp32(K.sbg + dS) : 0.0f;
+                const float fx0 = K.abg + (K.v2r + dv * K.ir) * dv + vx * iS;
+                const float tu = du + fx0 * hdt + gx * hdt, tv = dv + vy * iS * hdt + gy * hdt;
+                dust_drag32(w, i, K.sbg + dS, du, dv, tu, tv, gx, gy, hdt, hdt, q);
+                vmax = fmax(vmax, drate64(w, i, j, q.u, q.v));
+                dstore(w, w.dbuf[in ^ 1], i, j, q);
+            }
+            kick32(K, dS, du, dv, vx, vy, gx, gy, hdt, hdt, visc);
+            if (damped) {
+                // killwave (killwave.cu:48-100): relax towards init_C, i.e. residuals towards 0
+#pragma unroll
+                for (int side = 0; side < 2; ++side) {
+                    const float itau = kw[2 * side + 1];
+                    if (itau > 0.0f) {
+                        const float f = kw[2 * side] * (dtf * itau);
+                        dS -= f * dS;
+                        du -= f * du;
+                        dv -= f * dv;
+                    }
+                }
+            }
+            if (!(K.sbg + dS > 0.0f)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+            const double a = (fabs(ubg + (double)du) + cs) * idx;
+            const double b = (fabs(vbg + (double)dv) + cs) * (idy[j] * irad);
+            vmax = fmax(vmax, fmax(a, b));
+            D.emit(i, j, dS, du, dv);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+        if (lane == 0) atomic_max_pos(&sc->vmax_bits, vmax);
     }
-    if (vk >= 0) block_max_to<STT>(&V[vk].d64.sc->vmax_bits, vmax);
 }
 
 // ================================================================ misc
-// One thread per disk: dt, clock and planet of the step.
-__global__ void k32_time(const View32* __restrict__ V, int nd) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < nd) advance_clock(V[k].d64);
-}
-
-// Per disk (blockIdx.y): the step's planet table (see TRIG_ROW).
-__global__ void k32_trig(const View32* __restrict__ V) {
-    const View32& w = V[blockIdx.y];
+// One block per disk: its first thread sets dt, clock and planet of the step, then all fill
+// its planet table (see TRIG_ROW).
+__global__ void __launch_bounds__(1024) k32_time(const View32* __restrict__ V) {
+    pdl_enter();
+    const View32& w = V[blockIdx.x];
+    if (threadIdx.x == 0) advance_clock(w.d64);
+    __syncthreads();
     const Scalars* sc = w.d64.sc;
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const pg_body& a = sc->planet_cur;
     const pg_body& b = sc->planet_next;
-    if (k < w.yarr) {
+    const double ya = a.y + 0.0 * a.vy, yb = b.y + 0.0 * b.vy;
+    for (int k = threadIdx.x; k < w.yarr; k += blockDim.x) {
         float* t = w.trig + (size_t)TRIG_ROW * k;
 #pragma unroll
         for (int which = 0; which < 2; ++which) {
-            const pg_body& p = which ? b : a;
             double s, c;
-            sincos(0.5 * (w.d64.ycj[k] - (p.y + 0.0 * p.vy)), &s, &c);
+            sincos(0.5 * (w.d64.ycj[k] - (which ? yb : ya)), &s, &c);
             t[3 * which] = (float)(2.0 * s * c);
             t[3 * which + 1] = (float)(1.0 - 2.0 * s * s);
             t[3 * which + 2] = (float)(2.0 * s * s);
         }
     }
-    if (k < w.xarr) {
+    for (int k = threadIdx.x; k < w.xarr; k += blockDim.x) {
         float* c = w.trig + (size_t)TRIG_ROW * w.yn + 2 * k;
         c[0] = (float)(w.d64.radx[k] - a.x);
         c[1] = (float)(w.d64.radx[k] - b.x);
     }
-    if (k == 0) {
+    if (threadIdx.x == 0) {
         float* s = w.trig + (size_t)TRIG_ROW * w.yn + 2 * (size_t)w.xn;
         s[0] = (float)a.m;
         s[1] = (float)a.x;
@@ -1485,7 +1332,7 @@ __global__ void k32_init_tables(const View32 w, float* tx, float* ty, double* cs
 // ============================================================== launchers
 static inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
-static unsigned persistent_grid(const void* kernel, int threads, size_t smem, long long ntiles, int cap = 0) {
+static int sm_count32() {
     static int nsm = 0;
     if (nsm == 0) {
         int dev = 0;
@@ -1493,6 +1340,11 @@ static unsigned persistent_grid(const void* kernel, int threads, size_t smem, lo
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         if (nsm <= 0) nsm = 148;
     }
+    return nsm;
+}
+
+static unsigned persistent_grid(const void* kernel, int threads, size_t smem, long long ntiles, int cap = 0) {
+    const int nsm = sm_count32();
     static const void* keys[16] = {nullptr};
     static int vals[16] = {0};
     int per_sm = 0;
@@ -1515,104 +1367,80 @@ static unsigned persistent_grid(const void* kernel, int threads, size_t smem, lo
     return (unsigned)(g < 1 ? 1 : g);
 }
 
-// The two compiled occupancies of each pass (kick1, sweep x, sweep y, advect,
-// kick2): variant 0 is the one the register count allows by itself, variant 1
-// one CTA per SM more (fewer registers, possibly spills).
-constexpr int MB32[5][2] = {{4, 5}, {3, 4}, {4, 5}, {5, 6}, {4, 5}};
-
-template <int P, int V>
-static const void* pass_kernel() {
-    constexpr int MB = MB32[P][V];
-    if constexpr (P == 0) return (const void*)k32_kick1<MB>;
-    else if constexpr (P == 1) return (const void*)k32_sweep_x<MB>;
-    else if constexpr (P == 2) return (const void*)k32_sweep_y<MB>;
-    else if constexpr (P == 3) return (const void*)k32_advect<MB>;
-    else return (const void*)k32_kick2<MB>;
+static const void* pass_kernel(int pass) {
+    static const void* const k[5] = {(const void*)k32_kick1, (const void*)k32_sweep_x, (const void*)k32_sweep_y,
+                                     (const void*)k32_advect, (const void*)k32_kick2};
+    return k[pass];
 }
-static const void* pass_kernel(int pass, int v) {
-    static const void* const k[5][2] = {{pass_kernel<0, 0>(), pass_kernel<0, 1>()},
-                                        {pass_kernel<1, 0>(), pass_kernel<1, 1>()},
-                                        {pass_kernel<2, 0>(), pass_kernel<2, 1>()},
-                                        {pass_kernel<3, 0>(), pass_kernel<3, 1>()},
-                                        {pass_kernel<4, 0>(), pass_kernel<4, 1>()}};
-    return k[pass][v ? 1 : 0];
-}
-static const int PASS_THREADS[5] = {STT, SWT, SWT, SWT, STT};
-static const size_t PASS_SMEM[5] = {K1_SMEM, SX_SMEM, SY_SMEM, AD_SMEM, K2_SMEM};
 
-int pass_occupancy32(int pass, int variant) {
+int pass_occupancy32(int pass) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel(pass, variant), PASS_THREADS[pass],
-                                                      PASS_SMEM[pass]) != cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pass_kernel(pass), MT, 0) != cudaSuccess)
         return 1;
     return per_sm < 1 ? 1 : per_sm;
 }
 
-cudaError_t set_attributes32() {
-    cudaError_t e = cudaSuccess;
-    auto set = [&](const void* f, size_t bytes) {
-        cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (r != cudaSuccess) e = r;
-        r = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        if (r != cudaSuccess) e = r;
-    };
-    for (int p = 0; p < 5; ++p)
-        for (int v = 0; v < 2; ++v) set(pass_kernel(p, v), PASS_SMEM[p]);
-    return e;
+// The runs of the three kinds (radial sweep; azimuthal sweep and advection; kicks) over
+// disks of these sizes, as int4 {disk, first lane's radius, first row, last row + 1}.
+// Long runs waste little on the rows that only feed the stencils at their ends and on the
+// tables they load, short ones give the warps that hide latency: per kind the length with
+// the least run_cost (pg_internal.h) at 20 resident warps an SM.  1024x3072, us a pass at
+// 4 / 16 / 24 / 48 / 96 rows: radial sweep 92 / 90 / 90 / 90 / 128, azimuthal
+// 120 / 103 / 101 / 105 / 155, kick2 131 / 120 / 116 / 111 / 194.
+// Variant 1 is half as long, for the autotuner to try.
+void build_runs32(const int* xres, const int* yres, int nd, std::vector<int4>* runs, Runs32* R) {
+    runs->clear();
+    const int resident = 20 * sm_count32();
+    for (int kind = 0; kind < 3; ++kind) {
+        const int out = kind == 1 ? 32 : 30, first = kind == 1 ? NPAD : NPAD - 1;
+        int len = 2;
+        double best = 1e300;
+        for (int l = 2; l <= 64; l += (l < 16 ? 1 : 4)) {
+            long long warps = 0;
+            for (int k = 0; k < nd; ++k) warps += (long long)((xres[k] + out - 1) / out) * ((yres[k] + l - 1) / l);
+            const double cost = run_cost(warps, resident, l + (kind == 0 ? 1.5 : 3.5));
+            if (cost < best) {
+                best = cost;
+                len = l;
+            }
+        }
+        for (int v = 0; v < 2; ++v) {
+            const int l = len >> v;
+            R->first[v][kind] = (int)runs->size();
+            for (int k = 0; k < nd; ++k)
+                for (int j = 0; j < yres[k]; j += l)
+                    for (int i = 0; i < xres[k]; i += out)
+                        runs->push_back(make_int4(k, first + i, NPAD + j, NPAD + (j + l < yres[k] ? j + l : yres[k])));
+            R->count[v][kind] = (int)runs->size() - R->first[v][kind];
+        }
+    }
 }
 
-void launch_time32(const View32* V, int nd, cudaStream_t s) { k32_time<<<cdiv(nd, 64), 64, 0, s>>>(V, nd); }
-void launch_trig32(const View32* V, int nd, int maxn, cudaStream_t s) {
-    k32_trig<<<dim3(cdiv(maxn, 128), nd), 128, 0, s>>>(V);
-}
-template <int P, int V>
-static void launch_variant(const View32* V_, const int4* first, int nd, int nt, int in, int cap, cudaStream_t s) {
-    constexpr int MB = MB32[P][V];
-    const unsigned g = persistent_grid(pass_kernel<P, V>(), PASS_THREADS[P], PASS_SMEM[P], nt, cap);
-    if constexpr (P == 0) k32_kick1<MB><<<g, STT, K1_SMEM, s>>>(V_, first, nd, nt, in);
-    else if constexpr (P == 1) k32_sweep_x<MB><<<g, SWT, SX_SMEM, s>>>(V_, first, nd, nt, in);
-    else if constexpr (P == 2) k32_sweep_y<MB><<<g, SWT, SY_SMEM, s>>>(V_, first, nd, nt, in);
-    else if constexpr (P == 3) k32_advect<MB><<<g, SWT, AD_SMEM, s>>>(V_, first, nd, nt, in);
-    else k32_kick2<MB><<<g, STT, K2_SMEM, s>>>(V_, first, nd, nt, in);
-}
-template <int P>
-static void launch_p(const View32* V, const int4* first, int nd, int nt, int in, const Tune32* t, cudaStream_t s) {
-    const int v = t ? t->v[P] : DEFAULT_TUNE32.v[P];
-    const int cap = t ? t->cps[P] : 0;
-    if (v) launch_variant<P, 1>(V, first, nd, nt, in, cap, s);
-    else launch_variant<P, 0>(V, first, nd, nt, in, cap, s);
-}
-// tiles: the ensemble's tile table, radial-sweep tiles, then azimuthal, then stencil
-void launch_pass32(int pass, const View32* V, const int4* tiles, int nd, const int* ntiles, int in, cudaStream_t s,
-                   const Tune32* t) {
-    const int4* tx = tiles;
-    const int4* ty = tiles + ntiles[0];
-    const int4* ts = tiles + ntiles[0] + ntiles[1];
+void launch_time32(const View32* V, int nd, cudaStream_t s) { launch_step(k32_time, nd, 1024, 0, s, V); }
+void launch_pass32(int pass, const View32* V, const Runs32& R, int in, cudaStream_t s, const Tune32& t) {
+    static constexpr int KIND[5] = {2, 0, 1, 1, 2};
+    const int v = t.v[pass], kind = KIND[pass], n = R.count[v][kind];
+    const int4* runs = R.d + R.first[v][kind];
+    const unsigned g = persistent_grid(pass_kernel(pass), MT, 0, cdiv(n, MW), t.cps[pass]);
     switch (pass) {
-        case 0: launch_p<0>(V, ts, nd, ntiles[2], in, t, s); break;
-        case 1: launch_p<1>(V, tx, nd, ntiles[0], in, t, s); break;
-        case 2: launch_p<2>(V, ty, nd, ntiles[1], in, t, s); break;
-        case 3: launch_p<3>(V, ty, nd, ntiles[1], in, t, s); break;
-        default: launch_p<4>(V, ts, nd, ntiles[2], in, t, s); break;
+        case 0: launch_step(k32_kick1, g, MT, 0, s, V, runs, n, in); break;
+        case 1: launch_step(k32_sweep_x, g, MT, 0, s, V, runs, n, in); break;
+        case 2: launch_step(k32_sweep_y, g, MT, 0, s, V, runs, n, in); break;
+        case 3: launch_step(k32_advect, g, MT, 0, s, V, runs, n, in); break;
+        default: launch_step(k32_kick2, g, MT, 0, s, V, runs, n, in); break;
     }
 }
 void launch_cfl32(const View32* Vk, int b, cudaStream_t s) { k32_cfl<<<592, 256, 0, s>>>(Vk, b); }
-// the dust part of pass 1 (radial sweep), 2 (azimuthal sweep), 3 (advection);
-// counts: radial faces, azimuthal faces, cells of all dust disks
-void launch_dust_pass32(int pass, const View32* V, const int* doff, int nd, const long long* counts, int in,
-                        cudaStream_t s) {
-    auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
-    if (counts[2] == 0) return;
-    if (pass == 1) {
-        k32d_faces<0><<<grid(counts[0]), 256, 0, s>>>(V, doff, nd, in);
-        k32d_update<0><<<grid(counts[2]), 256, 0, s>>>(V, doff, nd, in);
-    } else if (pass == 2) {
-        k32d_faces<1><<<grid(counts[1]), 256, 0, s>>>(V, doff, nd, in);
-        k32d_update<1><<<grid(counts[2]), 256, 0, s>>>(V, doff, nd, in);
-    } else if (pass == 3) {
-        k32d_adv_faces<<<grid(counts[1]), 256, 0, s>>>(V, doff, nd, in);
-        k32d_adv_update<<<grid(counts[2]), 256, 0, s>>>(V, doff, nd, in);
-    }
+// the dust part of pass 1 (radial sweep), 2 (azimuthal sweep), 3 (advection), on the gas's runs
+void launch_dust_pass32(int pass, const View32* V, const Runs32& R, int in, cudaStream_t s) {
+    auto go = [&](auto kernel, int kind) {
+        const int n = R.count[0][kind];
+        launch_step(kernel, persistent_grid((const void*)kernel, MT, 0, cdiv(n, MW)), MT, 0, s, V,
+                    R.d + R.first[0][kind], n, in);
+    };
+    if (pass == 1) go(k32d_sweep_x, 0);
+    else if (pass == 2) go(k32d_sweep_y, 1);
+    else if (pass == 3) go(k32d_advect, 1);
 }
 void launch_dfill32(const View32* Vk, int b, const double* r, const double* u, const double* v, cudaStream_t s) {
     k32_dfill<<<592, 256, 0, s>>>(Vk, b, r, u, v);

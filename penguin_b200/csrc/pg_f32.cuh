@@ -80,21 +80,17 @@ constexpr int TRIG_ROW = 6;
 struct View32 {
     int xres, yres, xarr, yarr, pitch, xn, yn;
     int visc, orbadv, kill, nplanet, pad0;
-    int ntx[3];  // tiles along the fast index: 0 radial sweep, 1 azimuthal sweep / advection, 2 stencil
-    int pad1;
     float gam, pad2;
     float* buf[2];            // two state buffers, NPL planes of pitch * yarr floats each
     float* vis;               // viscous force density of kick1 (2 planes)
-    const CUtensorMap* maps;  // buf0 {X, Y, S}, buf1 {X, Y, S}, vis
     const float* tx;
     const float* ty;
     float* trig;
     const double* cs64;       // sqrt(gam cs2) per radius, FP64 (CFL rate)
     DiskView d64;             // FP64 grid, tables, orbital-advection arrays, scalars
     // dust_flag: residual planes {dSigma_d, dv_r,d, dv_phi,d} against init_CD, no ghost
-    // images (radial ghosts: zero residuals; rows wrap), and face-flux scratch
+    // images (radial ghosts: zero residuals; rows wrap)
     float* dbuf[2];
-    float* dflux;             // 3 planes of (xres + 1) * (yres + 1) faces
     int dust;
     float st_h;               // Stokes number times h/r: t_s = st_h / (c_s Sigma) (dust.cu:1-4)
     float dust_rmin;          // D_G_ratio * smallr
@@ -112,27 +108,34 @@ struct Par32 {
     float sL, sR;  // parabola of one cell relative to its average
 };
 
+// The hardware's reciprocal (1 ulp) and reciprocal square root (2^-22.9) of a normal
+// number, one instruction each: the full-range division and square root they replace are
+// no closer (2 ulp and 2^-23 after a division) and five to ten instructions.
+__device__ __forceinline__ float rcp32(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsq32(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// of a product of two floored states, which may leave the normal range
+__device__ __forceinline__ float rsq32_floor(float x) { return rsq32(fmaxf(x, 1.0e-37f)); }
+
 // recon.cu:216-378 + PPM.cu:64-91 with the centre value subtracted: am2..ap2 are
-// the neighbours' differences from the centre.
+// the neighbours' differences from the centre.  Sizes and signs as in recon (pg_hydro.cuh).
 __device__ __forceinline__ Par32 recon32(const float* __restrict__ w, float am2, float am1, float ap1, float ap2,
                                          float flat) {
     const float d0 = am1 - am2, d1 = -am1, d2 = ap1, d3 = ap2 - ap1;
-    float sL = w[0] * d0 + w[1] * d1 + w[2] * d2;
-    float sR = w[3] * d1 + w[4] * d2 + w[5] * d3;
-    sL = copysignf(fminf(fabsf(sL), fabsf(d1)), d1);
-    sR = copysignf(fminf(fabsf(sR), fabsf(d2)), d2);
-    if (sR * sL <= 0.0f) {
-        sL = 0.0f;
-        sR = 0.0f;
-    }
-    sR *= (1.0f - flat);
-    sL *= (1.0f - flat);
-    const float t3 = sR + sL;
-    const float t2 = t3 * t3;
-    const float t1 = t3 * 3.0f * (sL - sR);
-    if (t2 < t1) sL = 2.0f * sR;
-    else if (t2 < -t1) sR = 2.0f * sL;
-    return {sL, sR};
+    const float sL = w[0] * d0 + w[1] * d1 + w[2] * d2;
+    const float sR = w[3] * d1 + w[4] * d2 + w[5] * d3;
+    float l = fminf(fabsf(sL), fabsf(d1));
+    float r = fminf(fabsf(sR), fabsf(d2));
+    if (signbit(d1) != signbit(d2)) l = r = 0.0f;
+    const float k = 1.0f - flat;
+    return {copysignf(fminf(l, 2.0f * r) * k, d1), copysignf(fminf(r, 2.0f * l) * k, d2)};
 }
 
 struct Frac32 {
@@ -151,18 +154,21 @@ __device__ __forceinline__ float aveR32(const Frac32& f, const Par32& p) {
 
 // PPM.cu:7-62 on deviations: pm2..pp2 are p differences from the centre, p0 its
 // absolute value; um1/up1 the velocity differences.
-__device__ __forceinline__ float flatten32(float inv_cs, float p0, float pm2, float pm1, float pp1, float pp2,
-                                           float um1, float up1) {
+__device__ __forceinline__ float flatten32(float p0, float pm2, float pm1, float pp1, float pp2, float um1,
+                                           float up1) {
     const float dp1f = pp1, dp2f = pp2 - pm1;
     const float dp1b = -pm1, dp2b = pp1 - pm2;
-    (void)inv_cs;  // the signs of the Mach numbers are those of the velocity differences (flatten, pg_hydro.cuh)
-    const float Mf = -up1;
-    const float Mb = um1;
+    // the signs of the Mach numbers are those of the velocity differences; the steeper side
+    // by its numerator |dp1 - dp2 / 2| - |dp2| / 4 (flatten, pg_hydro.cuh)
+    const float wf = fabsf(dp2f), wb = fabsf(dp2b);
+    const float nf = fabsf(dp1f - 0.5f * dp2f) - 0.25f * wf;
+    const float nb = fabsf(dp1b - 0.5f * dp2b) - 0.25f * wb;
     float f = 0.0f;
-    if ((Mf > 0.0f || Mb > 0.0f) && dp2f != 0.0f && dp2b != 0.0f) {
-        f = 10.0f * fmaxf(0.0f, fabsf(dp1f / dp2f - 0.5f) - 0.25f);
-        f = fmaxf(f, 10.0f * fmaxf(0.0f, fabsf(dp1b / dp2b - 0.5f) - 0.25f));
-        f = fminf(0.5f, f * fmaxf(fabsf(dp1f), fabsf(dp1b)) / p0);
+    if ((up1 < 0.0f || um1 > 0.0f) && wf > 0.0f && wb > 0.0f && (nf > 0.0f || nb > 0.0f)) {
+        const bool back = nb * wf > nf * wb;
+        // two reciprocals: the product of a tiny jump and the pressure may leave the normal range
+        f = 10.0f * ((back ? nb : nf) * rcp32(back ? wb : wf)) * (fmaxf(fabsf(dp1f), fabsf(dp1b)) * rcp32(p0));
+        f = fminf(0.5f, f);
     }
     return f;
 }
@@ -173,18 +179,21 @@ struct HS {
     float v;       // transported field (deviation from a reference value)
 };
 
-// states.cu:151-206 (left edge of a cell) in deviation form.  rc, pc, uc: the
-// cell's absolute average density, pressure, normal velocity; R, P, U, V its
-// parabolas relative to the averages.  The result's rd, pd, v are relative to
-// the cell's averages.  The factor -hdt * 2/(cs sdt) of the reference is -1/cs.
-__device__ __forceinline__ HS left_edge32(float gam, float idx, float sdt, float cs0, float rc, float pc, float uc,
-                                          const Par32& R, const Par32& P, const Par32& U, const Par32& V) {
-    Frac32 q = frac32(lim01f((cs0 - fminf(uc, 0.0f)) * sdt * idx));
-    const float ur = uc + aveL32(q, U);
-    const float dis = fminf(ur, 0.0f) * sdt;
-    q = frac32(lim01f(-dis * idx));
-    float r0d = aveL32(q, R), p0d = aveL32(q, P);
-    const float u0d = aveL32(q, U);
+// states.cu:151-206 (left edge of a cell, SIDE 0) and 210-264 (right edge, SIDE 1) in
+// deviation form.  rc, pc, uc: the cell's absolute average density, pressure, normal
+// velocity; R, P, U, V its parabolas relative to the averages.  The result's rd, pd, v are
+// relative to the cell's averages.  sx = sdt / dx: the swept fraction per unit speed;
+// s = (gam p r)^-1/2 makes every quotient of the trace a product (pg_hydro.cuh).
+template <int SIDE>
+__device__ __forceinline__ HS edge32(float gam, float sx, float cs0, float rc, float pc, float uc, const Par32& R,
+                                     const Par32& P, const Par32& U, const Par32& V) {
+    auto away = [](float u) { return SIDE == 0 ? fmaxf(-u, 0.0f) : fmaxf(u, 0.0f); };  // speed towards the edge
+    auto ave = [](const Frac32& q, const Par32& p) { return SIDE == 0 ? aveL32(q, p) : aveR32(q, p); };
+    Frac32 q = frac32(fminf((cs0 + away(uc)) * sx, 1.0f));
+    const float m = away(uc + ave(q, U));
+    q = frac32(fminf(m * sx, 1.0f));
+    float r0d = ave(q, R), p0d = ave(q, P);
+    const float u0d = ave(q, U);
     float r0 = rc + r0d, p0 = pc + p0d;
     const float rmin = rc * 1.0e-10f, pmin = pc * 1.0e-10f;
     if (r0 < rmin) {
@@ -195,53 +204,18 @@ __device__ __forceinline__ HS left_edge32(float gam, float idx, float sdt, float
         p0 = pmin;
         p0d = pmin - pc;
     }
-    const float ir0 = 1.0f / r0;
-    const float cs = sqrtf(gam * p0 * ir0);
-    const float ics = 1.0f / cs;
-    q = frac32(lim01f((cs * sdt - dis) * idx));
-    const float u_ = (u0d - aveL32(q, U)) * ics;
-    const float p_ = (p0d - aveL32(q, P)) * ics;
-    HS s;
-    s.rd = (1.0f + u_ > 1.0e-6f) ? r0d + r0 * u_ : r0 * 1.0e-6f - rc;
+    const float g = gam * p0;
+    const float s = rsq32_floor(g * r0);
+    q = frac32(fminf((g * s + m) * sx, 1.0f));
+    const float eu = ave(q, U) - u0d, ep = ave(q, P) - p0d;
+    const float u_ = (SIDE == 0 ? -eu : eu) * (r0 * s);
+    HS h;
+    h.rd = (1.0f + u_ > 1.0e-6f) ? r0d + r0 * u_ : r0 * 1.0e-6f - rc;
     const float gu = gam * u_;
-    s.pd = (1.0f + gu > 1.0e-6f) ? p0d + p0 * gu : p0 * 1.0e-6f - pc;
-    s.u = uc + u0d + p_ * ir0;
-    s.v = aveL32(q, V);
-    return s;
-}
-
-// states.cu:210-264 (right edge of a cell) in deviation form.
-__device__ __forceinline__ HS right_edge32(float gam, float idx, float sdt, float cs0, float rc, float pc, float uc,
-                                           const Par32& R, const Par32& P, const Par32& U, const Par32& V) {
-    Frac32 q = frac32(lim01f((cs0 + fmaxf(uc, 0.0f)) * sdt * idx));
-    const float ul = uc + aveR32(q, U);
-    const float dis = fmaxf(ul, 0.0f) * sdt;
-    q = frac32(lim01f(dis * idx));
-    float r0d = aveR32(q, R), p0d = aveR32(q, P);
-    const float u0d = aveR32(q, U);
-    float r0 = rc + r0d, p0 = pc + p0d;
-    const float rmin = rc * 1.0e-10f, pmin = pc * 1.0e-10f;
-    if (r0 < rmin) {
-        r0 = rmin;
-        r0d = rmin - rc;
-    }
-    if (p0 < pmin) {
-        p0 = pmin;
-        p0d = pmin - pc;
-    }
-    const float ir0 = 1.0f / r0;
-    const float cs = sqrtf(gam * p0 * ir0);
-    const float ics = 1.0f / cs;
-    q = frac32(lim01f((dis + cs * sdt) * idx));
-    const float u_ = (aveR32(q, U) - u0d) * ics;
-    const float p_ = (aveR32(q, P) - p0d) * ics;
-    HS s;
-    s.rd = (1.0f + u_ > 1.0e-6f) ? r0d + r0 * u_ : r0 * 1.0e-6f - rc;
-    const float gu = gam * u_;
-    s.pd = (1.0f + gu > 1.0e-6f) ? p0d + p0 * gu : p0 * 1.0e-6f - pc;
-    s.u = uc + u0d + p_ * ir0;
-    s.v = aveR32(q, V);
-    return s;
+    h.pd = (1.0f + gu > 1.0e-6f) ? p0d + p0 * gu : p0 * 1.0e-6f - pc;
+    h.u = uc + u0d + (SIDE == 0 ? -ep : ep) * s;
+    h.v = ave(q, V);
+    return h;
 }
 
 struct FX {
@@ -257,22 +231,22 @@ struct FX {
 __device__ __forceinline__ FX hllc32(float gam, float rref, float pref, const HS& L, const HS& R) {
     const float Lr = rref + L.rd, Rr = rref + R.rd;
     const float Lp = pref + L.pd, Rp = pref + R.pd;
-    const float cl = sqrtf(gam * Lp / Lr);
-    const float cr = sqrtf(gam * Rp / Rr);
-    const float c_ = 0.5f * (cr + cl);
+    const float gl = gam * Lp, gr = gam * Rp;
+    const float cl = gl * rsq32_floor(gl * Lr), cr = gr * rsq32_floor(gr * Rr);
+    const float ic = rcp32(cl + cr);
     const float pbd = 0.5f * (R.pd + L.pd);
     const float pb = pref + pbd;
-    const float x = 0.5f * gam * (L.u - R.u) / c_;
+    const float x = gam * (L.u - R.u) * ic;
     const float pmd = (1.0f + x > 1.0e-6f) ? pbd + pb * x : pb * 1.0e-6f - pref;
-    const float srl = sqrtf(Lr), srr = sqrtf(Rr);
-    const float is = 1.0f / (srl + srr);
-    const float u_ = (srl * L.u + srr * R.u) * is;
-    const float n2 = 0.5f * srl * srr * (is * is);
+    // Roe's averages through the ratio of the roots of the densities
+    const float q = Rr * rsq32_floor(Lr * Rr), iq = rcp32(1.0f + q);
+    const float u_ = (L.u + q * R.u) * iq;
     const float du = R.u - L.u;
-    const float cc = sqrtf((cl * cl * srl + cr * cr * srr) * is + n2 * du * du);
+    const float c2 = (cl * cl + cr * cr * q) * iq + 0.5f * q * (iq * iq) * (du * du);
+    const float cc = c2 * rsq32(c2);
     const float sl = u_ - cc, sr = u_ + cc;
-    float sm = (Lr * L.u * cl + Rr * R.u * cr) / (Lr * cl + Rr * cr);
-    sm += (L.pd - R.pd) / ((Lr + Rr) * (0.5f * (cl + cr)));
+    const float ml = Lr * cl, mr = Rr * cr;
+    const float sm = (ml * L.u + mr * R.u) * rcp32(ml + mr) + 2.0f * (L.pd - R.pd) * (rcp32(Lr + Rr) * ic);
     const bool left = (signbit(sl) == 0) || (signbit(sr) == 0 && signbit(sm) == 0);
     const HS& S = left ? L : R;
     const float Sr = left ? Lr : Rr;
@@ -282,7 +256,7 @@ __device__ __forceinline__ FX hllc32(float gam, float rref, float pref, const HS
         F.pd = S.pd;
     } else {
         const float s_ = left ? sl : sr;
-        const float inv = 1.0f / (s_ - sm);
+        const float inv = rcp32(s_ - sm);
         F.r = sm * Sr * (s_ - S.u) * inv;
         F.pd = (s_ * pmd - sm * S.pd) * inv;
     }

@@ -4,6 +4,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "pg_common.cuh"
 
 namespace pg {
@@ -179,22 +181,24 @@ namespace f32 {
 struct View32;
 // FP32-form launchers (pg_f32.cu); pass 0 kick1, 1 radial sweep, 2 azimuthal sweep,
 // 3 advection, 4 kick2, reading buffer `in` and writing the other one
-cudaError_t set_attributes32();
 void launch_time32(const View32* V, int nd, cudaStream_t s);
-void launch_trig32(const View32* V, int nd, int maxn, cudaStream_t s);
 // Launch configuration of the five FP32 passes (kick1, sweep x, sweep y, advect,
-// kick2): the compiled occupancy variant (0 or 1) and a CTAs-per-SM cap (0 = none).
+// kick2): which of the two lists of runs (0 or 1) and a CTAs-per-SM cap (0 = none).
 struct Tune32 {
     int v[5];
     int cps[5];
 };
-constexpr Tune32 DEFAULT_TUNE32{{0, 1, 0, 0, 1}, {0, 0, 0, 0, 0}};
-void launch_pass32(int pass, const View32* V, const int4* tiles, int nd, const int* ntiles, int in, cudaStream_t s,
-                   const Tune32* t = nullptr);
-int pass_occupancy32(int pass, int variant);
+// The runs of an ensemble's passes in device memory: per list (0 or 1) and kind (radial
+// sweep; azimuthal sweep and advection; kicks) the first and how many.
+struct Runs32 {
+    int4* d;
+    int first[2][3], count[2][3];
+};
+void launch_pass32(int pass, const View32* V, const Runs32& R, int in, cudaStream_t s, const Tune32& t);
+void build_runs32(const int* xres, const int* yres, int nd, std::vector<int4>* runs, Runs32* R);
+int pass_occupancy32(int pass);
 void launch_cfl32(const View32* Vk, int b, cudaStream_t s);
-void launch_dust_pass32(int pass, const View32* V, const int* doff, int nd, const long long* counts, int in,
-                        cudaStream_t s);
+void launch_dust_pass32(int pass, const View32* V, const Runs32& R, int in, cudaStream_t s);
 void launch_dfill32(const View32* Vk, int b, const double* r, const double* u, const double* v, cudaStream_t s);
 void launch_dextract32(const View32* Vk, int b, double* r, double* u, double* v, cudaStream_t s);
 void launch_fill32(const View32* Vk, int b, const double* r, const double* u, const double* v, cudaStream_t s);
