@@ -15,22 +15,15 @@
 
 namespace pg {
 
-// Tiles of 32 outputs x 4 pencils: 160 threads and 25 KB of shared memory, so that 6
-// CTAs per SM hide the FP64 latency the passes are bound by.  The w velocity is
-// identically zero (dust runs in 2D) and stays as it is: three fields go through the
-// phases.
-constexpr int DS_LEN = 32, DS_W = DUST_W;
-constexpr int DS_TL = DS_LEN + 2 * NPAD;               // 38
-constexpr int DS_P1 = DS_LEN + 2, DS_P2 = DS_LEN + 1;  // cells with edge states, faces per pencil
-constexpr int DS_THREADS = 160;
-constexpr int DS_MINB = 5;
-constexpr int DS_NST = DS_P1 * DS_W, DS_NFX = DS_P2 * DS_W;
-static_assert(DS_NST <= DS_THREADS, "one cell per thread in each phase");
-constexpr int DS_TILE = 4 * DS_TL * DS_W;              // doubles; a cell is 32 bytes, so any column starts a TMA box
-constexpr int DS_STAGE = (DS_TILE + 15) / 16 * 16;     // 128-B aligned stages
-constexpr size_t DS_SMEM = (size_t)(2 * DS_STAGE + 6 * DS_NST + 3 * DS_NFX) * 8 + 16 + 128;
-constexpr int DA_NF = DS_TL * DS_W;                    // advection faces per tile
-constexpr size_t DA_SMEM = (size_t)(2 * DS_STAGE + 3 * DA_NF) * 8 + 16 + 128;
+// Lanes of a warp lie along the radius and the warp takes a run of rows one after the
+// other, as in the gas's passes (pg_kernels.cu): neighbours come by shuffle (radial sweep)
+// or stay in registers from the row before (azimuthal passes), no barrier and no shared
+// memory.  Bound by FP64 issue and latency; with tiles of 32 x 4 cells whose phases met at
+// barriers the sweeps and the advection of gas and dust took 133 us at 384x1024, with these
+// 112.  The w velocity is identically zero (dust runs in 2D) and stays as it is.
+constexpr int DS_WARPS = 4;  // warps per CTA, independent of one another
+constexpr int DS_THREADS = 32 * DS_WARPS;
+constexpr int DS_OUT = 30;   // radial sweep: outputs of a warp's 32 cells
 
 // src/solver/riemann/riemann.cu:5-11
 __device__ __forceinline__ double gfac(int geom, double x) {
@@ -39,251 +32,215 @@ __device__ __forceinline__ double gfac(int geom, double x) {
     return 1.0;
 }
 
-// ============================================================ dust sweeps
-// DIR 0: radial pencils of rows (fields r, u, r v); DIR 1: azimuthal pencils of
-// columns (r, v - orb_rot - r Omega, u).
-template <int DIR>
-__global__ void __launch_bounds__(DS_THREADS, DS_MINB)
-    k_dsweep(const __grid_constant__ CUtensorMap tm, const DiskView d, pg_dust* __restrict__ out, int ntx, int ntiles) {
-    extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n & 1) * DS_STAGE; };
-    double* st = smem + 2 * DS_STAGE;  // [6][DS_NST]: right state of the left face, left state of the right face
-    double* fl = st + 6 * DS_NST;      // [3][DS_NFX]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 3 * DS_NFX);
-    __shared__ int s_inc[DS_W];
-    Scalars* sc = d.sc;
-    if (sc->done) return;
-    const int tid = threadIdx.x;
-    const double dt = sc->dt;
-    const double* idx = (DIR == 0) ? d.idx_x : d.idx_y;  // one over a cell's width
-    auto origin = [&](int tile, int& s0, int& q0) {
-        s0 = NPAD + DS_LEN * (tile % ntx);
-        q0 = (DIR == 0 ? d.ypad : NPAD) + DS_W * (tile / ntx);
-    };
-    auto issue = [&](int tile, int k) {
-        int s0, q0;
-        origin(tile, s0, q0);
-        issue_begin(&bar[k & 1], DS_TILE * 8);
-        if (DIR == 0) tma_load_2d(stage(k), &tm, 4 * (s0 - NPAD), q0, &bar[k & 1]);
-        else tma_load_2d(stage(k), &tm, 4 * q0, s0 - NPAD, &bar[k & 1]);
-    };
-    // tile cell (position along the pencil t, pencil q) -> its 4 doubles
-    auto cellp = [&](const double* T, int t, int q) { return T + ((DIR == 0) ? q * DS_TL + t : t * DS_W + q) * 4; };
-    // dt over the pencil's radius (azimuthal sweeps: dust_flow, dust.cu:120-121)
-    auto pencil_dt = [&](int q) { return dt * ((DIR == 1 && d.geomy == 3) ? d.irad[min(q, d.xarr - 1)] : 1.0); };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int s0, q0;
-        origin(tile_id, s0, q0);
-        const double* T = stage(kt);
-        if (DIR == 1 && tid < DS_W) {
-            // the gas's set_orbital_advection (orbit.cu:74-99): the same shift for the dust
-            const int i = q0 + tid;
-            int shift = 0;
-            if (d.orbadv && i < NPAD + d.xres) {
-                const double dy = d.dy0 * d.radx[i];
-                shift = __double2int_rd(d.rot[i] * dt / dy + 0.5);
-            }
-            s_inc[tid] = shift;
-        }
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
+// A cell's states at one of its faces (dust_flux, dust.cu:6-103): mass density times the
+// compression factor, normal and transported velocity.  SIDE 0: its left face, 1: its right.
+struct DEdge {
+    double r, u, a;
+};
+template <int SIDE>
+__device__ __forceinline__ DEdge dust_edge(double sx, double uc, const Par& R, const Par& U, const Par& A) {
+    auto ave = [](const Frac& f, const Par& p) { return SIDE == 0 ? aveL(f, p) : aveR(f, p); };
+    // sx: swept fraction per unit speed; the traced positions of the reference enter only
+    // as fractions of the cell
+    const double m = (SIDE == 0 ? lesser(U.a - U.sL, 0.0) : larger(U.a + U.sR, 0.0)) * sx;
+    const double un = ave(frac(lesser(SIDE == 0 ? -m : m, 1.0)), U);
+    const Frac x = frac(lesser((SIDE == 0 ? -lesser(un, 0.0) : larger(un, 0.0)) * sx, 1.0));
+    const double e = (SIDE == 0) ? exp_lim(sx * (un - uc) * inv(1.0 + m)) : exp_lim(sx * (uc - un) * inv(1.0 - m));
+    return DEdge{ave(x, R) * e, ave(x, U), ave(x, A)};
+}
+struct DFlux {
+    double r, u, a;
+};
+// limited mass flux and the upwind transport at a face between the cells of densities rL, rR
+__device__ __forceinline__ DFlux dust_flux(double rL, double sxL, const DEdge& L, double rR, double sxR, const DEdge& R) {
+    const double ml = lesser(rL * sxL, larger(L.u * L.r, 0.0));
+    const double mr = larger(-rR * sxR, lesser(R.u * R.r, 0.0));
+    return DFlux{ml + mr, ml * L.u + mr * R.u, ml * L.a + mr * R.a};
+}
+__device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double down1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+// r, v_r, v_phi of a cell
+__device__ __forceinline__ void load3(const pg_dust* c, double& r, double& u, double& v) {
+    const double2* q = reinterpret_cast<const double2*>(c);
+    const double2 ru = q[0];
+    r = ru.x;
+    u = ru.y;
+    v = q[1].x;
+}
 
-        // ---- P1: per cell, the state at its left face (seen from the right) and at
-        // its right face (seen from the left), dust_flux (dust.cu:6-103)
-        if (tid < DS_NST) {
-            const int q = (DIR == 0) ? tid / DS_P1 : tid % DS_W;
-            const int t = 2 + ((DIR == 0) ? tid % DS_P1 : tid / DS_W);
-            const int s = s0 - NPAD + t;
-            const int sc_ = (DIR == 0) ? min(s, d.xarr - 1) : min(s, d.yarr - 1);
-            double v0 = 0.0;
-            if (DIR == 1) {
-                const int i = min(q0 + q, d.xarr - 1);
-                v0 = d.rot[i];
-                if (d.geomy == 3) v0 += d.radx[i] * d.frame_omega;
-            }
+// ============================================================ dust sweeps
+// Radial (fields r, u, r v): lane l holds cell 2 + 30 seg + l, lanes 1..30 update.
+__global__ void __launch_bounds__(DS_THREADS, 5)
+    k_dsweep_x(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int nseg, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Scalars* sc = d.sc;
+    pdl_enter();
+    if (sc->done) return;
+    const double dt = sc->dt;
+    for (int item = blockIdx.x * DS_WARPS + warp; item < nitems; item += gridDim.x * DS_WARPS) {
+        const int i = NPAD - 1 + DS_OUT * (item % nseg) + lane;
+        const int c = min(i, d.xarr - 3);  // the stencil stays in the row
+        const bool output = lane >= 1 && lane <= DS_OUT && i < NPAD + d.xres;
+        const int j0 = d.ypad + len * (item / nseg), j1 = min(j0 + len, d.ypad + d.yres);
+        double w[6], rad[5];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) w[m] = d.wx[6 * c + m];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) rad[m] = (d.geomx == 1) ? d.radx[c - 2 + m] : 1.0;
+        const double sx = dt * d.idx_x[c], f = dt * d.ixv[c], irad = (d.geomx == 1) ? d.irad[c] : 1.0;
+        const double g0 = gfac(d.geomx, d.xa[c]), g1 = gfac(d.geomx, d.xa[c + 1]), sxl = up1(sx);
+        const pg_dust* src = in + c + (size_t)d.xarr * j0;
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j, src += d.xarr) {
             double r[5], u[5], a[5];
 #pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                // 16-byte loads: 8-byte ones at this 32-byte stride conflict 4 ways
-                const double2* c = reinterpret_cast<const double2*>(cellp(T, t - 2 + m, q));
-                const double2 ru = c[0], vw = c[1];
-                r[m] = ru.x;
-                u[m] = (DIR == 0) ? ru.y : vw.x - v0;
-                a[m] = (DIR == 0) ? vw.x : ru.y;
-                if (DIR == 0 && d.geomx == 1) a[m] *= d.radx[min(max(s - 2 + m, 0), d.xarr - 1)];
+            for (int m = 0; m < 5; ++m) load3(src + m - 2, r[m], u[m], a[m]);
+            const double v = a[2];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) a[m] *= rad[m];
+            const Par R = recon(w, r[0], r[1], r[2], r[3], r[4], 0.0);
+            const Par U = recon(w, u[0], u[1], u[2], u[3], u[4], 0.0);
+            const Par A = recon(w, a[0], a[1], a[2], a[3], a[4], 0.0);
+            const DEdge b = dust_edge<0>(sx, u[2], R, U, A), e = dust_edge<1>(sx, u[2], R, U, A);
+            const DFlux F = dust_flux(up1(r[2]), sxl, DEdge{up1(e.r), up1(e.u), up1(e.a)}, r[2], sx, b);
+            const double Dr = (F.r * g0 - down1(F.r) * g1) * f;
+            const double Du = (F.u * g0 - down1(F.u) * g1) * f;
+            const double Da = (F.a * g0 - down1(F.a) * g1) * f * irad;
+            if (output) {
+                const DCell N = update_dust(d, DCell{r[2], u[2], v, 0.0}, DCell{Dr, Du, Da, 0.0});
+                if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                emit_dust(d, out, i, j, N);
             }
-            const double* wt = ((DIR == 0) ? d.wx : d.wy) + 6 * sc_;
-            const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], 0.0);
-            const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], 0.0);
-            const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], 0.0);
-            // swept fraction per unit speed: the traced positions of the reference enter
-            // only as fractions of the cell
-            const double sx = pencil_dt(q0 + q) * idx[sc_];
-            // left face, from this cell
-            double m = lesser(U.a - U.sL, 0.0) * sx;
-            const double ur = aveL(frac(lesser(-m, 1.0)), U);
-            Frac x = frac(lesser(-lesser(ur, 0.0) * sx, 1.0));
-            double* o = st + tid;
-            o[0] = aveL(x, R) * exp_lim(sx * (ur - u[2]) * inv(1.0 + m));
-            o[DS_NST] = aveL(x, U);
-            o[2 * DS_NST] = aveL(x, A);
-            // right face, from this cell
-            m = larger(U.a + U.sR, 0.0) * sx;
-            const double ul = aveR(frac(lesser(m, 1.0)), U);
-            x = frac(lesser(larger(ul, 0.0) * sx, 1.0));
-            o[3 * DS_NST] = aveR(x, R) * exp_lim(sx * (u[2] - ul) * inv(1.0 - m));
-            o[4 * DS_NST] = aveR(x, U);
-            o[5 * DS_NST] = aveR(x, A);
         }
-        __syncthreads();
+    }
+}
 
-        // ---- P2: limited mass flux and the upwind transport at every face
-        if (tid < DS_NFX) {
-            const int q = (DIR == 0) ? tid / DS_P2 : tid % DS_W;
-            const int f = (DIR == 0) ? tid % DS_P2 : tid / DS_W;  // between tile cells 2+f and 3+f
-            const double* R = st + ((DIR == 0) ? q * DS_P1 + f + 1 : (f + 1) * DS_W + q);
-            const double* L = st + 3 * DS_NST + ((DIR == 0) ? q * DS_P1 + f : f * DS_W + q);
-            const int sfc = min(s0 + f, (DIR == 0 ? d.xarr : d.yarr) - 1);  // face index = index of the right cell
-            const double sdt = pencil_dt(q0 + q);
-            const double rL = cellp(T, 2 + f, q)[0], rR = cellp(T, 3 + f, q)[0];
-            const double ml = lesser(rL * sdt * idx[sfc - 1], larger(L[DS_NST] * L[0], 0.0));
-            const double mr = larger(-rR * sdt * idx[sfc], lesser(R[DS_NST] * R[0], 0.0));
-            fl[tid] = ml + mr;
-            fl[DS_NFX + tid] = ml * L[DS_NST] + mr * R[DS_NST];
-            fl[2 * DS_NFX + tid] = ml * L[2 * DS_NST] + mr * R[2 * DS_NST];
+// the five rows of a lane's column that a marching pass holds, and the next one in flight
+struct DColumn {
+    double r[5], u[5], v[5], nr = 0.0, nu = 0.0, nv = 0.0;
+    const pg_dust* next;
+    int pitch;
+    __device__ __forceinline__ DColumn(const pg_dust* first, int pitch_) : next(first), pitch(pitch_) {
+#pragma unroll
+        for (int m = 0; m < 5; ++m, next += pitch) load3(next, r[m], u[m], v[m]);
+    }
+    __device__ __forceinline__ void fetch() {
+        load3(next, nr, nu, nv);
+        next += pitch;
+    }
+    __device__ __forceinline__ void shift() {
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            r[m] = r[m + 1];
+            u[m] = u[m + 1];
+            v[m] = v[m + 1];
         }
-        __syncthreads();
+        r[4] = nr;
+        u[4] = nu;
+        v[4] = nv;
+    }
+};
 
-        // ---- P3: flux differences and update_Dust (dust.cu:149-235, 256-326)
-        if (tid < DS_LEN * DS_W) {
-            const int q = (DIR == 0) ? tid / DS_LEN : tid % DS_W;
-            const int o = (DIR == 0) ? tid % DS_LEN : tid / DS_W;
-            const int s = s0 + o, qq = q0 + q;
-            const bool valid = (DIR == 0) ? (s < NPAD + d.xres && qq < d.ypad + d.yres)
-                                          : (s < NPAD + d.yres && qq < NPAD + d.xres);
-            if (valid) {
-                const double* f0 = fl + ((DIR == 0) ? q * DS_P2 + o : o * DS_W + q);
-                const double* f1 = f0 + ((DIR == 0) ? 1 : DS_W);
-                const double g0 = (DIR == 0) ? gfac(d.geomx, d.xa[s]) : 1.0;
-                const double g1 = (DIR == 0) ? gfac(d.geomx, d.xa[s + 1]) : 1.0;
-                const double f = (DIR == 0) ? dt * d.ixv[s] : pencil_dt(qq) * d.iyv[s];
-                auto net = [&](int k) { return (f0[k * DS_NFX] * g0 - f1[k * DS_NFX] * g1) * f; };
-                const double* c = cellp(T, NPAD + o, q);
-                const DCell Q{c[0], c[1], c[2], c[3]};
-                const double Dr = net(0);
-                if (DIR == 0) {
-                    const double Da = net(2) * (d.geomx == 1 ? d.irad[s] : 1.0);
-                    const DCell N = update_dust(d, Q, DCell{Dr, net(1), Da, 0.0});
+// Azimuthal (fields r, v - orb_rot - r Omega, u) and the orbital shift.
+__global__ void __launch_bounds__(DS_THREADS, 5)
+    k_dsweep_y(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int ncol, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Scalars* sc = d.sc;
+    pdl_enter();
+    if (sc->done) return;
+    const double dt = sc->dt;
+    for (int item = blockIdx.x * DS_WARPS + warp; item < nitems; item += gridDim.x * DS_WARPS) {
+        const int i = NPAD + 32 * (item % ncol) + lane;
+        const bool active = i < NPAD + d.xres;
+        const int c = min(i, NPAD + d.xres - 1);
+        const int s0 = NPAD + len * (item / ncol), s1 = min(s0 + len, NPAD + d.yres);
+        double v0 = d.rot[c];
+        if (d.geomy == 3) v0 += d.radx[c] * d.frame_omega;
+        const double sdt = dt * ((d.geomy == 3) ? d.irad[c] : 1.0);
+        int shift = 0;
+        if (d.orbadv) {  // the gas's set_orbital_advection (orbit.cu:74-99): the same shift for the dust
+            const double dy = d.dy0 * d.radx[c];
+            shift = __double2int_rd(d.rot[c] * dt / dy + 0.5);
+        }
+        int js = (s0 - d.ypad + shift) % d.yres;  // TD[(j+inc) mod N] = CD[j] (orbit.cu:30-46)
+        if (js < 0) js += d.yres;
+        DColumn q(in + c + (size_t)d.xarr * (s0 - NPAD), d.xarr);
+        DEdge pe{};  // the right edge of the cell below, its swept fraction per unit speed
+        double psx = 0.0;
+        DFlux pf{};  // the flux at the face below it
+#pragma unroll 1
+        for (int t = s0 - 1; t <= s1; ++t) {
+            if (t < s1) q.fetch();
+            double u[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) u[m] = q.v[m] - v0;
+            const double* w = d.wy + 6 * t;
+            const double sx = sdt * d.idx_y[t];
+            const Par R = recon(w, q.r[0], q.r[1], q.r[2], q.r[3], q.r[4], 0.0);
+            const Par U = recon(w, u[0], u[1], u[2], u[3], u[4], 0.0);
+            const Par A = recon(w, q.u[0], q.u[1], q.u[2], q.u[3], q.u[4], 0.0);
+            const DEdge b = dust_edge<0>(sx, u[2], R, U, A), e = dust_edge<1>(sx, u[2], R, U, A);
+            const DFlux F = dust_flux(q.r[1], psx, pe, q.r[2], sx, b);
+            if (t > s0) {  // the cell below has both its fluxes
+                const double f = sdt * d.iyv[t - 1], Dr = (pf.r - F.r) * f;
+                if (active) {
+                    const DCell N = update_dust(d, DCell{q.r[1], q.u[1], q.v[1], 0.0},
+                                                DCell{Dr, (pf.a - F.a) * f, (pf.u - F.u) * f + v0 * Dr, 0.0});
                     if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                    emit_dust(d, out, s, qq, N);
-                } else {
-                    double v0 = d.rot[qq];
-                    if (d.geomy == 3) v0 += d.radx[qq] * d.frame_omega;
-                    const DCell N = update_dust(d, Q, DCell{Dr, net(2), net(1) + v0 * Dr, 0.0});
-                    if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                    int j = s;
-                    if (d.orbadv) {  // TD[(j+inc) mod N] = CD[j] (orbit.cu:30-46)
-                        int js = (s - d.ypad + s_inc[q]) % d.yres;
-                        if (js < 0) js += d.yres;
-                        j = js + d.ypad;
-                    }
-                    emit_dust(d, out, qq, j, N);
+                    emit_dust(d, out, i, js + d.ypad, N);
                 }
+                if (++js == d.yres) js = 0;
             }
+            pe = e;
+            psx = sx;
+            pf = F;
+            q.shift();
         }
-        __syncthreads();
     }
 }
 
 // ===================================================== dust residual advection
-// advection() on Dust (advection.cu:175-233) + advecty (:235-290): the gas's
-// residual speed orb_res, fields (r, v, u), update_Dust.
-__global__ void __launch_bounds__(DS_THREADS, DS_MINB)
-    k_dadvect(const __grid_constant__ CUtensorMap tm, const DiskView d, pg_dust* __restrict__ out, int ntx, int ntiles) {
-    extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n & 1) * DS_STAGE; };
-    double* fl = smem + 2 * DS_STAGE;  // [3][DA_NF] upwind fluxes, indexed by face t
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + 3 * DA_NF);
+// advection() on Dust (advection.cu:175-233) + advecty (:235-290): the gas's residual speed
+// orb_res, fields (r, v, u), update_Dust.  The speed of a column has one sign: every row
+// feeds the same one of its two faces.
+__global__ void __launch_bounds__(DS_THREADS, 5)
+    k_dadvect(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int ncol, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
+    pdl_enter();
     if (sc->done) return;
-    const int tid = threadIdx.x;
     const double dt = sc->dt;
-    auto origin = [&](int tile, int& s0, int& q0) {
-        s0 = NPAD + DS_LEN * (tile % ntx);
-        q0 = NPAD + DS_W * (tile / ntx);
-    };
-    auto issue = [&](int tile, int k) {
-        int s0, q0;
-        origin(tile, s0, q0);
-        issue_begin(&bar[k & 1], DS_TILE * 8);
-        tma_load_2d(stage(k), &tm, 4 * q0, s0 - NPAD, &bar[k & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int s0, q0;
-        origin(tile_id, s0, q0);
-        const double* T = stage(kt);
-        if (!pipe_wait(bar, kt, sc)) {
-            pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-            return;
-        }
-        if (tid < DS_NST) {
-            const int q = tid % DS_W, t = 2 + tid / DS_W;
-            const int s = min(s0 - NPAD + t, d.yarr - 1);
-            const int i = min(q0 + q, d.xarr - 1);
-            const double speed = d.res[i];
-            const double sdt = dt * ((d.geomy == 3) ? d.irad[i] : 1.0);
-            const double* wt = d.wy + 6 * s;
-            const Frac x = frac(lesser(fabs(speed) * (sdt * d.idx_y[s]), 1.0));
-            const bool up = speed > 0.0;  // this cell is upwind of its upper face, else of its lower one
-            double r[5], u[5], v[5];
-#pragma unroll
-            for (int m = 0; m < 5; ++m) {
-                const double2* c = reinterpret_cast<const double2*>(T + ((t - 2 + m) * DS_W + q) * 4);
-                const double2 ru = c[0];
-                r[m] = ru.x;
-                u[m] = ru.y;
-                v[m] = c[1].x;
-            }
+    for (int item = blockIdx.x * DS_WARPS + warp; item < nitems; item += gridDim.x * DS_WARPS) {
+        const int i = NPAD + 32 * (item % ncol) + lane;
+        const bool active = i < NPAD + d.xres;
+        const int c = min(i, NPAD + d.xres - 1);
+        const int s0 = NPAD + len * (item / ncol), s1 = min(s0 + len, NPAD + d.yres);
+        const double speed = d.res[c], sdt = dt * ((d.geomy == 3) ? d.irad[c] : 1.0), sx = fabs(speed) * sdt;
+        const bool up = speed > 0.0;  // a row is upwind of its upper face, else of its lower one
+        DColumn q(in + c + (size_t)d.xarr * (s0 - NPAD), d.xarr);
+        DFlux pf{};  // the flux that the row below fed
+#pragma unroll 1
+        for (int t = s0 - 1; t <= s1; ++t) {
+            if (t < s1) q.fetch();
+            const double* w = d.wy + 6 * t;
+            const Frac x = frac(lesser(sx * d.idx_y[t], 1.0));
             auto ave = [&](const double* a) {
-                const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], 0.0);
+                const Par A = recon(w, a[0], a[1], a[2], a[3], a[4], 0.0);
                 return up ? aveR(x, A) : aveL(x, A);
             };
-            const double m = ave(r) * speed;
-            double* o = fl + (t + (up ? 1 : 0)) * DS_W + q;
-            o[0] = m;
-            o[DA_NF] = ave(u) * m;
-            o[2 * DA_NF] = ave(v) * m;
-        }
-        __syncthreads();
-        if (tid < DS_LEN * DS_W) {
-            const int q = tid % DS_W, o = tid / DS_W;
-            const int s = s0 + o, i = q0 + q;
-            if (s < NPAD + d.yres && i < NPAD + d.xres) {
-                const int t = NPAD + o;
-                const double* f0 = fl + t * DS_W + q;
-                const double f = dt * d.iyv[s] * ((d.geomy == 3) ? d.irad[i] : 1.0);
-                auto net = [&](int k) { return (f0[k * DA_NF] - f0[k * DA_NF + DS_W]) * f; };
-                const double* c = T + (t * DS_W + q) * 4;
-                const DCell N = update_dust(d, DCell{c[0], c[1], c[2], c[3]}, DCell{net(0), net(1), net(2), 0.0});
+            const double m = ave(q.r) * speed;
+            const DFlux F{m, ave(q.u) * m, ave(q.v) * m};
+            const int j = up ? t : t - 1;  // the row that has both its fluxes now
+            if (active && j >= s0 && j < s1) {
+                const double f = sdt * d.iyv[j];
+                const DCell Q{up ? q.r[2] : q.r[1], up ? q.u[2] : q.u[1], up ? q.v[2] : q.v[1], 0.0};
+                const DCell N = update_dust(d, Q, DCell{(pf.r - F.r) * f, (pf.u - F.u) * f, (pf.a - F.a) * f, 0.0});
                 if (!(N.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                emit_dust(d, out, i, s, N);
+                emit_dust(d, out, i, j, N);
             }
+            pf = F;
+            q.shift();
         }
-        __syncthreads();
     }
 }
 
@@ -345,45 +302,32 @@ __global__ void k_dust_extract(const DiskView d, const pg_dust* buf, double* r, 
 // ============================================================== launchers
 static inline unsigned dcdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
-static unsigned dust_grid(const void* kernel, size_t smem, long long ntiles) {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
+// one marching pass: runs of `lines` warps across the radius, of the length of least run_cost
+template <class K>
+static void march_dust(K kernel, const DiskView& d, int lines, double extra, const pg_dust* in, pg_dust* out,
+                       cudaStream_t s) {
+    static int nsm = 0, per_sm = 0;  // of this kernel
+    if (per_sm == 0) {
+        int dev = 0, n = 0, k = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 148;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        nsm = n > 0 ? n : 148;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, DS_THREADS, 0) != cudaSuccess || k < 1) k = 1;
+        per_sm = k;
     }
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, DS_THREADS, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    long long g = (long long)per_sm * nsm;
-    if (g > ntiles) g = ntiles;
-    return (unsigned)(g < 1 ? 1 : g);
+    const int len = run_length(lines, d.yres, (long long)DS_WARPS * nsm * per_sm, extra);
+    const int items = lines * (int)dcdiv(d.yres, len);
+    const unsigned most = (unsigned)(nsm * per_sm), all = dcdiv(items, DS_WARPS);
+    launch_step(kernel, all < most ? all : most, DS_THREADS, 0, s, in, d, out, lines, len, items);
 }
-
-cudaError_t set_dust_attributes() {
-    cudaError_t e = cudaSuccess;
-    auto set = [&](const void* f, size_t bytes) {
-        cudaError_t r = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (r != cudaSuccess) e = r;
-    };
-    set((const void*)k_dsweep<0>, DS_SMEM);
-    set((const void*)k_dsweep<1>, DS_SMEM);
-    set((const void*)k_dadvect, DA_SMEM);
-    return e;
+void launch_dsweep_x(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
+    march_dust(k_dsweep_x, d, (int)dcdiv(d.xres, DS_OUT), 1.5, in, out, s);
 }
-
-void launch_dsweep_x(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s) {
-    const int ntx = (int)dcdiv(d.xres, DS_LEN), nt = ntx * (int)dcdiv(d.yres, DS_W);
-    k_dsweep<0><<<dust_grid((const void*)k_dsweep<0>, DS_SMEM, nt), DS_THREADS, DS_SMEM, s>>>(in.sweep_x, d, out, ntx, nt);
+void launch_dsweep_y(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
+    march_dust(k_dsweep_y, d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
 }
-void launch_dsweep_y(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s) {
-    const int ntx = (int)dcdiv(d.yres, DS_LEN), nt = ntx * (int)dcdiv(d.xres, DS_W);
-    k_dsweep<1><<<dust_grid((const void*)k_dsweep<1>, DS_SMEM, nt), DS_THREADS, DS_SMEM, s>>>(in.sweep_y, d, out, ntx, nt);
-}
-void launch_dadvect(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s) {
-    const int ntx = (int)dcdiv(d.yres, DS_LEN), nt = ntx * (int)dcdiv(d.xres, DS_W);
-    k_dadvect<<<dust_grid((const void*)k_dadvect, DA_SMEM, nt), DS_THREADS, DA_SMEM, s>>>(in.sweep_y, d, out, ntx, nt);
+void launch_dadvect(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
+    march_dust(k_dadvect, d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
 }
 void launch_dust_init(const DiskView& d, pg_dust* buf, cudaStream_t s) { k_dust_init<<<592, 256, 0, s>>>(d, buf); }
 void launch_dust_xghosts(const DiskView& d, pg_dust* buf, cudaStream_t s) {

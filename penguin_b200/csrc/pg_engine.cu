@@ -388,15 +388,6 @@ static pg_status make_cell_maps(CellMaps& M, const Cell* buf, int xarr, int yarr
     return PG_OK;
 }
 
-static pg_status make_dust_maps(DustMaps& M, const pg_dust* buf, int xarr, int yarr) {
-    if (M.base == buf) return PG_OK;
-    pg_status s;
-    if ((s = make_map(&M.sweep_x, buf, 4ull * xarr, yarr, 4 * 38, DUST_W)) != PG_OK) return s;
-    if ((s = make_map(&M.sweep_y, buf, 4ull * xarr, yarr, 4 * DUST_W, 38)) != PG_OK) return s;
-    M.base = buf;
-    return PG_OK;
-}
-
 static pg_status make_vis_maps(VisMaps& M, const double* vis, int xarr, int yarr) {
     if (M.base == vis) return PG_OK;
     pg_status s;
@@ -468,7 +459,6 @@ struct Engine {
     pg_body* grid_planet = nullptr;    // drop-in mode: the caller's planets array
     double* part = nullptr;            // per-block partial sums of diagnostics
     pg_dust* dbuf[2] = {nullptr, nullptr};  // dust_flag: the dust of buf[k] is dbuf[k]
-    DustMaps dmaps[2];
     Tune tune;                               // launch configuration (pg_disk_autotune)
     Cell* ave = nullptr;                     // time average (pg_disk_set_average)
     double* snap = nullptr;                  // pinned staging of snapshots
@@ -709,7 +699,8 @@ static pg_status enqueue_stages(Engine& E, const StepRecord* rec = nullptr) {
     const bool dust = d.dust != 0;
     if (dust)
         for (int k = 0; k < 2; ++k)
-            if ((s = make_dust_maps(E.dmaps[k], E.dbuf[k], d.xarr, d.yarr)) != PG_OK) return s;
+            if (reinterpret_cast<uintptr_t>(E.dbuf[k]) % 16 != 0)
+                return fail(PG_ERR_CONFIG, "the dust buffers must be 16-byte aligned");
     save(0);
     launch_kick1(d, maps(c), E.buf[1 - c], E.vis, E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
                  &E.tune);
@@ -718,12 +709,12 @@ static pg_status enqueue_stages(Engine& E, const StepRecord* rec = nullptr) {
     c = 1 - c;
     save(1);
     launch_sweep_x(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
-    if (dust) launch_dsweep_x(d, E.dmaps[c], D[1 - c], E.stream);
+    if (dust) launch_dsweep_x(d, D[c], D[1 - c], E.stream);
     c = 1 - c;
     if (d.ndim > 1) {
         save(2);
         launch_sweep_y(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
-        if (dust) launch_dsweep_y(d, E.dmaps[c], D[1 - c], E.stream);
+        if (dust) launch_dsweep_y(d, D[c], D[1 - c], E.stream);
         if (rec) {
             cudaMemcpyAsync(rec->res, E.res, d.xarr * sizeof(double), cudaMemcpyDeviceToDevice, E.stream);
             cudaMemcpyAsync(rec->inc, E.inc, d.xarr * sizeof(int), cudaMemcpyDeviceToDevice, E.stream);
@@ -733,7 +724,7 @@ static pg_status enqueue_stages(Engine& E, const StepRecord* rec = nullptr) {
     if (d.ndim > 1 && d.orbadv) {
         save(3);
         launch_advect(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
-        if (dust) launch_dadvect(d, E.dmaps[c], D[1 - c], E.stream);
+        if (dust) launch_dadvect(d, D[c], D[1 - c], E.stream);
         c = 1 - c;
     }
     save(4);
@@ -752,7 +743,6 @@ static pg_status engine_create(const pg_params* P, int device, void* stream, Eng
     static bool attrs = false;
     if (!attrs) {
         PG_CUDA(set_kernel_attributes());
-        PG_CUDA(set_dust_attributes());
         attrs = true;
     }
     Engine* E = new Engine();
@@ -1711,7 +1701,8 @@ pg_status pg_disk_profile(pg_disk* dk, int nsteps, double end_time, float* ms, i
     const bool dust = d.dust != 0;
     if (dust)
         for (int k = 0; k < 2; ++k)
-            if ((s = make_dust_maps(E.dmaps[k], E.dbuf[k], d.xarr, d.yarr)) != PG_OK) return s;
+            if (reinterpret_cast<uintptr_t>(E.dbuf[k]) % 16 != 0)
+                return fail(PG_ERR_CONFIG, "the dust buffers must be 16-byte aligned");
     cudaEvent_t ev[7];
     for (auto& x : ev) PG_CUDA(cudaEventCreate(&x));
     for (int step = 0; step < nsteps; ++step) {
@@ -1724,18 +1715,18 @@ pg_status pg_disk_profile(pg_disk* dk, int nsteps, double end_time, float* ms, i
         c = 1 - c;
         PG_CUDA(cudaEventRecord(ev[2], E.stream));
         launch_sweep_x(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
-        if (dust) launch_dsweep_x(d, E.dmaps[c], D[1 - c], E.stream);
+        if (dust) launch_dsweep_x(d, D[c], D[1 - c], E.stream);
         c = 1 - c;
         PG_CUDA(cudaEventRecord(ev[3], E.stream));
         if (d.ndim > 1) {
             launch_sweep_y(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
-            if (dust) launch_dsweep_y(d, E.dmaps[c], D[1 - c], E.stream);
+            if (dust) launch_dsweep_y(d, D[c], D[1 - c], E.stream);
             c = 1 - c;
         }
         PG_CUDA(cudaEventRecord(ev[4], E.stream));
         if (d.ndim > 1 && d.orbadv) {
             launch_advect(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
-            if (dust) launch_dadvect(d, E.dmaps[c], D[1 - c], E.stream);
+            if (dust) launch_dadvect(d, D[c], D[1 - c], E.stream);
             c = 1 - c;
         }
         PG_CUDA(cudaEventRecord(ev[5], E.stream));

@@ -64,14 +64,6 @@ struct VisMaps {
     const void* base = nullptr;
     CUtensorMap stencil;   // box {2*34, 10}
 };
-constexpr int DUST_W = 4;  // pencils per tile of the dust passes
-// Tensor maps of one AoS dust buffer (4 doubles per cell).
-struct DustMaps {
-    const void* base = nullptr;
-    CUtensorMap sweep_x;   // box {4*38, DUST_W}
-    CUtensorMap sweep_y;   // box {4*DUST_W, 38}
-};
-
 // Pass inputs of one FP64 step, saved for its adjoint (pg_adjoint.cu).
 struct StepRecord {
     Cell* stage[5];     // inputs of kick1, sweep_x, sweep_y, advect, kick2 (xarr*yarr AoS each)
@@ -165,10 +157,9 @@ pg_status make_map3_f32(CUtensorMap* m, const float* base, uint64_t pitch, uint6
 cudaError_t set_kernel_attributes();
 
 // dust passes (pg_dust.cu)
-cudaError_t set_dust_attributes();
-void launch_dsweep_x(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s);
-void launch_dsweep_y(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s);
-void launch_dadvect(const DiskView& d, const DustMaps& in, pg_dust* out, cudaStream_t s);
+void launch_dsweep_x(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s);
+void launch_dsweep_y(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s);
+void launch_dadvect(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s);
 void launch_dust_init(const DiskView& d, pg_dust* buf, cudaStream_t s);
 void launch_dust_xghosts(const DiskView& d, pg_dust* buf, cudaStream_t s);
 void launch_dust_images(const DiskView& d, pg_dust* buf, cudaStream_t s);
