@@ -170,18 +170,18 @@ pg_status pg_disk_get_state(pg_disk* d, double* r, double* p, double* u, double*
 /* Autotuner: times every launch configuration of each pass of the step on the
    disk's current state over `reps` launches and keeps the fastest; the state is
    unchanged and results stay bit for bit the same.  The sweeps and the
-   residual advection choose a tile variant (pg_sweep_variant: pencils per
-   tile, outputs per pencil, cells per thread, TMA stages in flight), every pass
-   its CTAs per SM.  It replaces the reference's fixed tiling
+   residual advection choose a variant (pg_sweep_variant: the rows a warp takes),
+   every pass its CTAs per SM.  It replaces the reference's fixed tiling
    (include/parameters.h:81-97, x_xdiv / x_ydiv / y_xdiv / y_ydiv).  choice (may
    be NULL, 8 ints): the variants of sweep_x, sweep_y, advect, then the CTAs per
    SM of kick1, sweep_x, sweep_y, advect, kick2 (0: all that fit).
    pg_disk_set_tuning applies a choice found earlier. */
 pg_status pg_disk_autotune(pg_disk* d, int reps, int* choice);
 pg_status pg_disk_set_tuning(pg_disk* d, const int* choice);
-/* Tile variant v of the FP64 sweeps and advection (0 .. 9), 6 ints: pencils
-   per tile, outputs per pencil, cells per thread, TMA stages, threads per CTA,
-   CTAs per SM its registers are compiled for.  PG_ERR_ARG past the last. */
+/* Variant v of the FP64 sweeps and advection (0 .. 9), 6 ints: neighbouring
+   radii a warp holds, rows it takes one after the other (0: by the grid's size),
+   the same per thread, copies in flight, threads per CTA, CTAs per SM its
+   registers are compiled for.  PG_ERR_ARG past the last. */
 pg_status pg_sweep_variant(int v, int* out6);
 /* test support: the per-index 4th-order slope weights the kernels apply in
    direction dir (0 radial, 1 azimuthal) of the grid P builds, 6 per index
@@ -293,8 +293,8 @@ int pg_ens_kernels_per_step(const pg_ens* e);
    1 kick1, 2 sweep_x, 3 sweep_y, 4 advect, 5 kick2). */
 pg_status pg_ens_profile(pg_ens* e, int nsteps, double end_time, float* ms, int nslot);
 /* Launch-configuration autotuner of the five FP32 passes: for each pass the
-   compiled occupancy variant (0/1) and CTAs-per-SM cap (0 = none) with the
-   shortest time on the current state, `reps` launches per candidate.  The
+   list of runs (0: the default lengths, 1: half as long) and CTAs-per-SM cap
+   (0 = none) with the shortest time on the current state, `reps` launches per candidate.  The
    state is not changed and results are bit for bit the same under any choice.
    out10 (optional): variants of kick1, sweep x, sweep y, advect, kick2, then
    their caps. */

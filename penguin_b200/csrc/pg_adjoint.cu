@@ -2080,6 +2080,9 @@ static pg_status adj_make_disk(pg_adj* a) {
     // rounding apart.  The adjoint transposes the sweep with one face at the
     // seam, so its passes read weights whose ghost rows are their images'.
     const DiskView& d = engine_view(a->E);
+    // the records' constant radial ghosts; everything else in them is written by the passes
+    for (int left = 2 * 5 * a->every, at = 0; left > 0; left -= 32768, at += 32768)
+        launch_init_xghosts(d, a->stages + (size_t)at * a->ncell(), a->stream, left < 32768 ? left : 32768);
     std::vector<double> wy(6 * (size_t)d.yarr);
     if (!a->wy_seam && (s = adj_alloc(a, &a->wy_seam, wy.size() * sizeof(double))) != PG_OK) return s;
     ADJ_CUDA(cudaMemcpyAsync(wy.data(), d.wy, wy.size() * sizeof(double), cudaMemcpyDeviceToHost, a->stream));
@@ -2335,9 +2338,12 @@ pg_status pg_adj_backward(pg_adj* a, const double* grad_out, double* grad_sigma0
     cudaStream_t st_engine = engine_set_stream(a->E, a->fstream);
     auto recompute = [&](int seg, int bank) -> pg_status {
         const int n0 = seg * a->every, n1 = std::min(n0 + a->every, N);
-        pg_status r = engine_restore(a->E, a->ckpt + (size_t)seg * a->ncell(), a->ckpt_sc + seg);
+        pg_status r = engine_restore(a->E, a->ckpt + (size_t)seg * a->ncell(), a->ckpt_sc + seg,
+                                     record_slot(a, 0, bank).stage[0]);
         for (int n = n0; n < n1 && r == PG_OK; ++n) {
-            const StepRecord rec = record_slot(a, n - n0, bank);
+            StepRecord rec = record_slot(a, n - n0, bank);
+            rec.entered = true;
+            if (n + 1 < n1) rec.next = record_slot(a, n + 1 - n0, bank).stage[0];
             r = engine_step(a->E, a->ts[n], a->dts[n], &rec);
         }
         if (r != PG_OK) return r;

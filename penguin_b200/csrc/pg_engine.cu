@@ -373,26 +373,8 @@ pg_status make_map3_f64(CUtensorMap* m, const void* base, uint64_t d0, uint64_t 
 static pg_status make_cell_maps(CellMaps& M, const Cell* buf, int xarr, int yarr) {
     if (M.base == buf) return PG_OK;
     pg_status s;
-    if ((s = make_map(&M.stencil, buf, 5ull * xarr, yarr, 5 * 34, 10)) != PG_OK) return s;
-    for (int v = 0; v < NSWEEP_VARIANTS; ++v) {
-        const SweepVariant& g = SWEEP_VARIANTS[v];
-        const uint32_t tl = (uint32_t)(g.len + 2 * NPAD);
-        if (sweep_variant_x_ok(v)) {
-            if ((s = make_map(&M.sx[v], buf, 5ull * xarr, yarr, 5 * tl, (uint32_t)g.w)) != PG_OK) return s;
-        } else {
-            memset(&M.sx[v], 0, sizeof(CUtensorMap));
-        }
-        if ((s = make_map(&M.sy[v], buf, 5ull * xarr, yarr, 5 * (uint32_t)(g.w + 2), tl)) != PG_OK) return s;
-    }
+    if ((s = make_map(&M.sx, buf, 5ull * xarr, yarr, 5 * RX_TILE_CELLS, RX_TILE_ROWS)) != PG_OK) return s;
     M.base = buf;
-    return PG_OK;
-}
-
-static pg_status make_vis_maps(VisMaps& M, const double* vis, int xarr, int yarr) {
-    if (M.base == vis) return PG_OK;
-    pg_status s;
-    if ((s = make_map(&M.stencil, vis, 2ull * xarr, yarr, 2 * 34, 10)) != PG_OK) return s;
-    M.base = vis;
     return PG_OK;
 }
 
@@ -443,7 +425,6 @@ struct Engine {
     double* grid = nullptr;  // xa | xv | ya | yv (owned mode)
     double* tab = nullptr;   // weights and per-index tables
     CellMaps maps[2];
-    VisMaps vmap;
     int cur = 0;
     bool fresh = true;       // no step taken since the state was set
     // device-loop bookkeeping: steps past end_time are no-ops on the device, so the
@@ -669,9 +650,6 @@ static pg_status resolve_cur(Engine& E) {
     return PG_OK;
 }
 
-// Kernels of one step after the time kernel; in = E.cur.  With rec, the input
-// of every pass, kick1's stress and the orbital-advection arrays are copied
-// out for the adjoint.
 // the captured steps hold the view, the tensor maps and the launch configuration
 static void drop_graphs(Engine& E) {
     for (auto* gs : {E.graph, E.sgraph})
@@ -682,18 +660,15 @@ static void drop_graphs(Engine& E) {
             }
 }
 
-static pg_status enqueue_stages(Engine& E, const StepRecord* rec = nullptr) {
+// Kernels of one step after the time kernel; in = E.cur.
+static pg_status enqueue_stages(Engine& E) {
     const DiskView& d = E.view;
     pg_status s;
     int c = E.cur;
-    const size_t ncell = (size_t)d.xarr * d.yarr;
-    auto save = [&](int k) {
-        if (rec) cudaMemcpyAsync(rec->stage[k], E.buf[c], ncell * sizeof(Cell), cudaMemcpyDeviceToDevice, E.stream);
-    };
-    auto maps = [&](int k) -> const CellMaps& { return E.maps[k]; };
     for (int k = 0; k < 2; ++k)
         if ((s = make_cell_maps(E.maps[k], E.buf[k], d.xarr, d.yarr)) != PG_OK) return s;
-    if (d.visc && (s = make_vis_maps(E.vmap, E.vis, d.xarr, d.yarr)) != PG_OK) return s;
+    if (d.visc && reinterpret_cast<uintptr_t>(E.vis) % 16 != 0)
+        return fail(PG_ERR_CONFIG, "the viscous force buffer must be 16-byte aligned");
     // dust (dust_flag) takes as many passes as the gas, so dbuf[k] pairs with buf[k]
     pg_dust* const* D = E.dbuf;
     const bool dust = d.dust != 0;
@@ -701,37 +676,48 @@ static pg_status enqueue_stages(Engine& E, const StepRecord* rec = nullptr) {
         for (int k = 0; k < 2; ++k)
             if (reinterpret_cast<uintptr_t>(E.dbuf[k]) % 16 != 0)
                 return fail(PG_ERR_CONFIG, "the dust buffers must be 16-byte aligned");
-    save(0);
-    launch_kick1(d, maps(c), E.buf[1 - c], E.vis, E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
+    launch_kick1(d, E.buf[c], E.buf[1 - c], E.vis, E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
                  &E.tune);
-    if (rec && d.visc)
-        cudaMemcpyAsync(rec->vis, E.vis, 2 * ncell * sizeof(double), cudaMemcpyDeviceToDevice, E.stream);
     c = 1 - c;
-    save(1);
-    launch_sweep_x(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
+    launch_sweep_x(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
     if (dust) launch_dsweep_x(d, D[c], D[1 - c], E.stream);
     c = 1 - c;
     if (d.ndim > 1) {
-        save(2);
-        launch_sweep_y(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
+        launch_sweep_y(d, E.buf[c], E.buf[1 - c], E.stream, &E.tune);
         if (dust) launch_dsweep_y(d, D[c], D[1 - c], E.stream);
-        if (rec) {
-            cudaMemcpyAsync(rec->res, E.res, d.xarr * sizeof(double), cudaMemcpyDeviceToDevice, E.stream);
-            cudaMemcpyAsync(rec->inc, E.inc, d.xarr * sizeof(int), cudaMemcpyDeviceToDevice, E.stream);
-        }
         c = 1 - c;
     }
     if (d.ndim > 1 && d.orbadv) {
-        save(3);
-        launch_advect(d, maps(c), E.buf[1 - c], E.stream, &E.tune);
+        launch_advect(d, E.buf[c], E.buf[1 - c], E.stream, &E.tune);
         if (dust) launch_dadvect(d, D[c], D[1 - c], E.stream);
         c = 1 - c;
     }
-    save(4);
-    launch_kick2(d, maps(c), E.vmap, E.buf[1 - c], E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
+    launch_kick2(d, E.buf[c], E.vis, E.buf[1 - c], E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
                  &E.tune);
     c = 1 - c;
     E.cur = c;
+    PG_CUDA(cudaGetLastError());
+    return PG_OK;
+}
+
+// The same step for the adjoint (2D gas): every pass reads and writes the record's
+// buffers in place, so that the pass inputs, kick1's stress and the orbital-advection
+// arrays are recorded without a copy.  The last pass leaves the newest state in
+// rec.next, or in the disk's own buffer.
+static pg_status enqueue_recorded(Engine& E, const StepRecord& rec) {
+    DiskView d = E.view;
+    d.res = rec.res;
+    d.inc = rec.inc;
+    CellMaps m;
+    pg_status s = make_cell_maps(m, rec.stage[1], d.xarr, d.yarr);
+    if (s != PG_OK) return s;
+    Cell* swept = rec.stage[d.orbadv ? 3 : 4];
+    launch_kick1(d, rec.stage[0], rec.stage[1], rec.vis, E.stream, nullptr, nullptr, &E.tune);
+    launch_sweep_x(d, m, rec.stage[2], E.stream, &E.tune);
+    launch_sweep_y(d, rec.stage[2], swept, E.stream, &E.tune);
+    if (d.orbadv) launch_advect(d, swept, rec.stage[4], E.stream, &E.tune);
+    launch_kick2(d, rec.stage[4], rec.vis, rec.next ? rec.next : E.buf[0], E.stream, nullptr, nullptr, &E.tune);
+    E.cur = 0;
     PG_CUDA(cudaGetLastError());
     return PG_OK;
 }
@@ -790,24 +776,6 @@ pg_status table_engine_create(const pg_params* P, int device, cudaStream_t s, En
 void engine_destroy(Engine* E) { delete E; }
 const DiskView& engine_view(const Engine* E) { return E->view; }
 void engine_init_planet(Engine* E, double t) { launch_init_planet(E->view, E->P, t, E->stream); }
-
-// 3D FP32 tensor map over `planes` planes of rows x pitch floats.
-pg_status make_map3_f32(CUtensorMap* m, const float* base, uint64_t pitch, uint64_t rows, uint64_t planes,
-                        uint32_t bx, uint32_t by, uint32_t bz) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(PG_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-    if (reinterpret_cast<uintptr_t>(base) % 16 != 0 || (pitch * 4) % 16 != 0)
-        return fail(PG_ERR_CONFIG, "FP32 planes must have 16-byte aligned rows");
-    cuuint64_t dims[3] = {pitch, rows, planes};
-    cuuint64_t strides[2] = {pitch * 4, pitch * rows * 4};
-    cuuint32_t box[3] = {bx, by, bz};
-    cuuint32_t es[3] = {1, 1, 1};
-    CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, es,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(PG_ERR_CUDA, "cuTensorMapEncodeTiled (3D FP32) failed (%d)", (int)r);
-    return PG_OK;
-}
 
 __global__ void k_fill(const DiskView d, Cell* buf, const double* r, const double* p, const double* u,
                        const double* v) {
@@ -1044,15 +1012,22 @@ pg_status engine_set_state_device(Engine* E, double t, const double* r, const do
     return set_state_device(*E, t, r, p, u, v);
 }
 
-// One step of main.cu's loop with a given dt (pg_disk_solve), optionally recording.
+// One step of main.cu's loop with a given dt (pg_disk_solve), optionally recording:
+// from the disk's newest state, or from rec->stage[0] where it is already there.
 pg_status engine_step(Engine* E, double t, double dt, const StepRecord* rec) {
     pg_status s0 = resolve_cur(*E);
     if (s0 != PG_OK) return s0;
-    launch_set_time(E->view, t, dt, E->stream);
-    if (rec) PG_CUDA(cudaMemcpyAsync(rec->planets, &E->sc->planet_cur, 2 * sizeof(pg_body), cudaMemcpyDeviceToDevice,
-                                     E->stream));
     E->fresh = false;
-    return enqueue_stages(*E, rec);
+    if (!rec) {
+        launch_set_time(E->view, t, dt, E->stream);
+        return enqueue_stages(*E);
+    }
+    if (!rec->entered) {
+        const size_t n = (size_t)E->view.xarr * E->view.yarr;
+        PG_CUDA(cudaMemcpyAsync(rec->stage[0], E->buf[E->cur], n * sizeof(Cell), cudaMemcpyDeviceToDevice, E->stream));
+    }
+    launch_set_time(E->view, t, dt, E->stream, rec->planets);
+    return enqueue_recorded(*E, *rec);
 }
 
 // The newest state (all cells, ghosts included) and the device scalars (clock, planets).
@@ -1071,11 +1046,11 @@ cudaStream_t engine_set_stream(Engine* E, cudaStream_t s) {
     return old;
 }
 
-pg_status engine_restore(Engine* E, const Cell* cells, const Scalars* sc) {
+pg_status engine_restore(Engine* E, const Cell* cells, const Scalars* sc, Cell* into) {
     const size_t n = (size_t)E->view.xarr * E->view.yarr;
     E->cur = 0;
     E->pending = false;
-    PG_CUDA(cudaMemcpyAsync(E->buf[0], cells, n * sizeof(Cell), cudaMemcpyDeviceToDevice, E->stream));
+    PG_CUDA(cudaMemcpyAsync(into ? into : E->buf[0], cells, n * sizeof(Cell), cudaMemcpyDeviceToDevice, E->stream));
     PG_CUDA(cudaMemcpyAsync(E->sc, sc, sizeof(Scalars), cudaMemcpyDeviceToDevice, E->stream));
     E->fresh = false;
     return PG_OK;
@@ -1092,15 +1067,14 @@ pg_status engine_run_pass(Engine* E, int pass, const Cell* in, Cell* out, const 
     PG_CUDA(cudaMemcpyAsync(E->buf[0], in, n * sizeof(Cell), cudaMemcpyDeviceToDevice, E->stream));
     for (int k = 0; k < 2; ++k)
         if ((s = make_cell_maps(E->maps[k], E->buf[k], d.xarr, d.yarr)) != PG_OK) return s;
-    if (d.visc && (s = make_vis_maps(E->vmap, E->vis, d.xarr, d.yarr)) != PG_OK) return s;
     if (pass == 4 && d.visc && vis_in)
         PG_CUDA(cudaMemcpyAsync(E->vis, vis_in, 2 * n * sizeof(double), cudaMemcpyDeviceToDevice, E->stream));
     switch (pass) {
-        case 0: launch_kick1(d, E->maps[0], E->buf[1], E->vis, E->stream, nullptr, nullptr, &E->tune); break;
+        case 0: launch_kick1(d, E->buf[0], E->buf[1], E->vis, E->stream, nullptr, nullptr, &E->tune); break;
         case 1: launch_sweep_x(d, E->maps[0], E->buf[1], E->stream, &E->tune); break;
-        case 2: launch_sweep_y(d, E->maps[0], E->buf[1], E->stream, &E->tune); break;
-        case 3: launch_advect(d, E->maps[0], E->buf[1], E->stream, &E->tune); break;
-        default: launch_kick2(d, E->maps[0], E->vmap, E->buf[1], E->stream, nullptr, nullptr, &E->tune); break;
+        case 2: launch_sweep_y(d, E->buf[0], E->buf[1], E->stream, &E->tune); break;
+        case 3: launch_advect(d, E->buf[0], E->buf[1], E->stream, &E->tune); break;
+        default: launch_kick2(d, E->buf[0], E->vis, E->buf[1], E->stream, nullptr, nullptr, &E->tune); break;
     }
     PG_CUDA(cudaGetLastError());
     PG_CUDA(cudaMemcpyAsync(out, E->buf[1], n * sizeof(Cell), cudaMemcpyDeviceToDevice, E->stream));
@@ -1226,16 +1200,15 @@ pg_status pg_disk_solve(pg_disk* dk, double t, double dt) {
     PG_CUDA(cudaSetDevice(E.device));
     pg_status s0 = resolve_cur(E);
     if (s0 != PG_OK) return s0;
-    // this step's t and dt go in as launch arguments of k_set_time; the rest of the
-    // step (planet angles, five passes) is one captured graph per starting buffer,
-    // one launch instead of six behind the host's dt read-back
-    launch_set_time_only(E.view, t, dt, E.stream);
+    // this step's t and dt go in as launch arguments of k_set_time; the five passes are one
+    // captured graph per starting buffer, one launch instead of five behind the host's dt
+    // read-back
+    launch_set_time(E.view, t, dt, E.stream);
     PG_CUDA(cudaGetLastError());
     const int c0 = E.cur;
     if (!E.sgraph[c0]) {
         cudaGraph_t g;
         PG_CUDA(cudaStreamBeginCapture(E.stream, cudaStreamCaptureModeThreadLocal));
-        launch_planet_trig(E.view, E.stream);
         pg_status s = enqueue_stages(E);
         cudaError_t ce = cudaStreamEndCapture(E.stream, &g);
         E.cur = c0;
@@ -1413,8 +1386,7 @@ pg_status pg_disk_torque(pg_disk* dk, double* torque) {
 int pg_kernels_per_step(const pg_disk* dk) { return dk ? kernels_per_step(dk->E->view) : 0; }
 
 // Autotuner: for every pass, times each launch configuration (for the sweeps
-// and the advection each tile variant of SWEEP_VARIANTS: pencils per tile,
-// outputs per pencil, cells per thread, TMA stages; for every pass the CTAs per
+// and the advection each run length of SWEEP_LENGTHS; for every pass the CTAs per
 // SM from 1 to what fits) on the disk's current state with CUDA events over
 // `reps` launches and keeps the fastest.  The state, clock and planet are
 // restored afterwards; the per-cell arithmetic does not depend on the
@@ -1443,17 +1415,16 @@ pg_status pg_disk_autotune(pg_disk* dk, int reps, int* choice) {
     launch_set_time(d, h.t, dt, E.stream);
     for (int k = 0; k < 2; ++k)
         if ((s = make_cell_maps(E.maps[k], E.buf[k], d.xarr, d.yarr)) != PG_OK) return s;
-    if (d.visc && (s = make_vis_maps(E.vmap, E.vis, d.xarr, d.yarr)) != PG_OK) return s;
     cudaEvent_t e0, e1;
     PG_CUDA(cudaEventCreate(&e0));
     PG_CUDA(cudaEventCreate(&e1));
     auto launch = [&](int p, const Tune& t) {
         switch (p) {
-            case 0: launch_kick1(d, E.maps[c], E.buf[1 - c], E.vis, E.stream, nullptr, nullptr, &t); break;
+            case 0: launch_kick1(d, E.buf[c], E.buf[1 - c], E.vis, E.stream, nullptr, nullptr, &t); break;
             case 1: launch_sweep_x(d, E.maps[c], E.buf[1 - c], E.stream, &t); break;
-            case 2: launch_sweep_y(d, E.maps[c], E.buf[1 - c], E.stream, &t); break;
-            case 3: launch_advect(d, E.maps[c], E.buf[1 - c], E.stream, &t); break;
-            default: launch_kick2(d, E.maps[c], E.vmap, E.buf[1 - c], E.stream, nullptr, nullptr, &t); break;
+            case 2: launch_sweep_y(d, E.buf[c], E.buf[1 - c], E.stream, &t); break;
+            case 3: launch_advect(d, E.buf[c], E.buf[1 - c], E.stream, &t); break;
+            default: launch_kick2(d, E.buf[c], E.vis, E.buf[1 - c], E.stream, nullptr, nullptr, &t); break;
         }
     };
     Tune best = E.tune;
@@ -1462,8 +1433,7 @@ pg_status pg_disk_autotune(pg_disk* dk, int reps, int* choice) {
         float best_ms = 1.0e30f;
         const int nv = (p >= 1 && p <= 3) ? NSWEEP_VARIANTS : 1;
         for (int v = 0; v < nv; ++v) {
-            if (p == 1 && !sweep_variant_x_ok(v)) continue;
-            const int occ = pass_occupancy(d, p, v);
+            const int occ = pass_occupancy(d, p);
             for (int cps = 1; cps <= occ; ++cps) {
                 Tune t = best;
                 if (p >= 1 && p <= 3) t.v[p - 1] = v;
@@ -1487,6 +1457,8 @@ pg_status pg_disk_autotune(pg_disk* dk, int reps, int* choice) {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    for (int& v : best.v)
+        if (v < 0) v = 0;  // a pass this disk does not run
     E.tune = best;
     drop_graphs(E);
     PG_CUDA(cudaMemcpyAsync(E.buf[c], saved, n * sizeof(Cell), cudaMemcpyDeviceToDevice, E.stream));
@@ -1649,12 +1621,11 @@ pg_status pg_recon_weights(const pg_params* P, int dir, double* w) {
 
 pg_status pg_sweep_variant(int v, int* out6) {
     if (v < 0 || v >= NSWEEP_VARIANTS || !out6) return fail(PG_ERR_ARG, "no such tile variant");
-    const SweepVariant& g = SWEEP_VARIANTS[v];
-    out6[0] = g.w;
-    out6[1] = g.len;
-    out6[2] = g.cpt;
-    out6[3] = g.stages;
-    sweep_variant_launch(v, &out6[4], &out6[5]);
+    out6[0] = 32;                 // neighbouring radii of a warp
+    out6[1] = SWEEP_LENGTHS[v];   // rows it takes (0: by the grid's size)
+    out6[2] = SWEEP_LENGTHS[v];   // ... one after the other in each thread
+    out6[3] = 2;
+    sweep_launch_shape(&out6[4], &out6[5]);
     return PG_OK;
 }
 
@@ -1662,7 +1633,7 @@ pg_status pg_disk_set_tuning(pg_disk* dk, const int* choice) {
     if (!dk || !choice) return fail(PG_ERR_ARG, "bad argument");
     Tune t;
     for (int k = 0; k < 3; ++k) {
-        if (choice[k] < 0 || choice[k] >= NSWEEP_VARIANTS || (k == 0 && !sweep_variant_x_ok(choice[k])))
+        if (choice[k] < 0 || choice[k] >= NSWEEP_VARIANTS)
             return fail(PG_ERR_ARG, "no such tile variant for this pass");
         t.v[k] = choice[k];
     }
@@ -1696,7 +1667,6 @@ pg_status pg_disk_profile(pg_disk* dk, int nsteps, double end_time, float* ms, i
     pg_status s;
     for (int k = 0; k < 2; ++k)
         if ((s = make_cell_maps(E.maps[k], E.buf[k], d.xarr, d.yarr)) != PG_OK) return s;
-    if (d.visc && (s = make_vis_maps(E.vmap, E.vis, d.xarr, d.yarr)) != PG_OK) return s;
     pg_dust* const* D = E.dbuf;
     const bool dust = d.dust != 0;
     if (dust)
@@ -1710,7 +1680,7 @@ pg_status pg_disk_profile(pg_disk* dk, int nsteps, double end_time, float* ms, i
         PG_CUDA(cudaEventRecord(ev[0], E.stream));
         launch_time_step(d, E.stream);
         PG_CUDA(cudaEventRecord(ev[1], E.stream));
-        launch_kick1(d, E.maps[c], E.buf[1 - c], E.vis, E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
+        launch_kick1(d, E.buf[c], E.buf[1 - c], E.vis, E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
                      &E.tune);
         c = 1 - c;
         PG_CUDA(cudaEventRecord(ev[2], E.stream));
@@ -1719,18 +1689,18 @@ pg_status pg_disk_profile(pg_disk* dk, int nsteps, double end_time, float* ms, i
         c = 1 - c;
         PG_CUDA(cudaEventRecord(ev[3], E.stream));
         if (d.ndim > 1) {
-            launch_sweep_y(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
+            launch_sweep_y(d, E.buf[c], E.buf[1 - c], E.stream, &E.tune);
             if (dust) launch_dsweep_y(d, D[c], D[1 - c], E.stream);
             c = 1 - c;
         }
         PG_CUDA(cudaEventRecord(ev[4], E.stream));
         if (d.ndim > 1 && d.orbadv) {
-            launch_advect(d, E.maps[c], E.buf[1 - c], E.stream, &E.tune);
+            launch_advect(d, E.buf[c], E.buf[1 - c], E.stream, &E.tune);
             if (dust) launch_dadvect(d, D[c], D[1 - c], E.stream);
             c = 1 - c;
         }
         PG_CUDA(cudaEventRecord(ev[5], E.stream));
-        launch_kick2(d, E.maps[c], E.vmap, E.buf[1 - c], E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
+        launch_kick2(d, E.buf[c], E.vis, E.buf[1 - c], E.stream, dust ? D[c] : nullptr, dust ? D[1 - c] : nullptr,
                      &E.tune);
         c = 1 - c;
         PG_CUDA(cudaEventRecord(ev[6], E.stream));

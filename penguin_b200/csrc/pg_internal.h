@@ -10,21 +10,10 @@
 
 namespace pg {
 
-// Tile variants of the FP64 sweeps and residual advection, the autotuner's knobs
-// (pg_disk_autotune): pencils per tile W, outputs per pencil L, cells per thread
-// in each phase, TMA stages in flight, and CTAs per SM the registers are
-// compiled for (0: as many as ~96 registers a thread allow; more caps the
-// registers and may spill).  pg_kernels.cu instantiates each (SV<v>).
-struct SweepVariant {
-    int w, len, cpt, stages, minb;
-};
+// Rows a warp of the FP64 sweeps and the residual advection takes one after the other
+// (pg_kernels.cu): the autotuner's variants.  0: run_length picks by the grid's size.
 constexpr int NSWEEP_VARIANTS = 10;
-constexpr SweepVariant SWEEP_VARIANTS[NSWEEP_VARIANTS] = {
-    {8, 32, 1, 2, 0}, {4, 32, 1, 2, 0}, {16, 16, 1, 2, 0}, {8, 16, 1, 2, 0}, {8, 32, 2, 2, 0},
-    {8, 32, 1, 3, 0}, {4, 32, 1, 3, 0}, {4, 64, 1, 2, 0}, {4, 32, 1, 2, 5}, {8, 32, 1, 2, 3}};
-// the radial box holds 5 (L + 6) doubles in one row, at most 256 TMA elements
-inline bool sweep_variant_x_ok(int v) { return 5 * (SWEEP_VARIANTS[v].len + 2 * NPAD) <= 256; }
-
+constexpr int SWEEP_LENGTHS[NSWEEP_VARIANTS] = {0, 4, 6, 8, 12, 16, 24, 48, 64, 96};
 // Time of `warps` runs of `rows` rows each (the extra rows at a run's ends included) in units
 // of a row's time on a full GPU, where `resident` warps fit at once: whole waves of runs when
 // there are more, and with fewer a row that is quicker for the idle issue slots, down to its
@@ -48,25 +37,23 @@ inline int run_length(long long lines, int rows, long long resident, double extr
 }
 constexpr int RX_TILE_CELLS = 36, RX_TILE_ROWS = 4;  // the radial sweep's TMA box
 
-// Tensor maps of one AoS cell buffer, one per tile shape.
+// Tensor map of one AoS cell buffer.
 struct CellMaps {
     const void* base = nullptr;
-    CUtensorMap stencil;                   // box {5*34, 10}: 32x8 cells + 1 halo
-    CUtensorMap sx[NSWEEP_VARIANTS];       // box {5*(L+6), W}: x-pencils (variants whose box fits)
-    CUtensorMap sy[NSWEEP_VARIANTS];       // box {5*(W+2), L+6}: y-pencils, one extra column each side
+    CUtensorMap sx;                        // box {5*36, 4}: the radial sweep
 };
 // Launch configuration of the FP64 passes (pg_disk_autotune).
 struct Tune {
-    int v[3] = {0, 0, 0};          // tile variant of sweep_x, sweep_y, advect (SWEEP_VARIANTS)
+    int v[3] = {0, 0, 0};          // variant of sweep_x, sweep_y, advect (SWEEP_LENGTHS)
     int cps[5] = {0, 0, 0, 0, 0};  // CTAs per SM: kick1, sweep_x, sweep_y, advect, kick2 (0: all that fit)
 };
-struct VisMaps {
-    const void* base = nullptr;
-    CUtensorMap stencil;   // box {2*34, 10}
-};
+
 // Pass inputs of one FP64 step, saved for its adjoint (pg_adjoint.cu).
 struct StepRecord {
-    Cell* stage[5];     // inputs of kick1, sweep_x, sweep_y, advect, kick2 (xarr*yarr AoS each)
+    Cell* stage[5];     // inputs of kick1, sweep_x, sweep_y, advect, kick2 (xarr*yarr AoS each; bound-0
+                        // radial ghosts already in place)
+    Cell* next;         // where kick2 leaves the new state: the next step's stage[0], or null (the disk's buffer)
+    bool entered;       // stage[0] holds the step's input already
     double* vis;        // kick1's viscous force density (2 per cell, xarr*yarr)
     pg_body* planets;   // planet of the first half-kick, planet at t + dt
     double* res;        // orbital-advection residual speed per radius (xarr)
@@ -92,23 +79,21 @@ void grid3_release();
 
 // launch helpers (pg_kernels.cu)
 void launch_init_tables(const DiskView& d, const pg_params& P, double* tab_base, cudaStream_t s);
-void launch_init_xghosts(const DiskView& d, Cell* buf, cudaStream_t s);
+void launch_init_xghosts(const DiskView& d, Cell* buf, cudaStream_t s, int nbuf = 1);
 void launch_bound(const DiskView& d, Cell* buf, cudaStream_t s);
 void launch_cfl(const DiskView& d, const Cell* buf, cudaStream_t s, const pg_dust* dbuf = nullptr);
-void launch_set_time(const DiskView& d, double t, double dt, cudaStream_t s);  // the two below
-void launch_set_time_only(const DiskView& d, double t, double dt, cudaStream_t s);
-void launch_planet_trig(const DiskView& d, cudaStream_t s);
+void launch_set_time(const DiskView& d, double t, double dt, cudaStream_t s, pg_body* planets = nullptr);
 void launch_time_step(const DiskView& d, cudaStream_t s);
 void launch_run_begin(Scalars* sc, double end_time, bool fresh, cudaStream_t s);
-void launch_kick1(const DiskView& d, const CellMaps& in, Cell* out, double* vis, cudaStream_t s,
+void launch_kick1(const DiskView& d, const Cell* in, Cell* out, double* vis, cudaStream_t s,
                   const pg_dust* din = nullptr, pg_dust* dout = nullptr, const Tune* t = nullptr);
 void launch_sweep_x(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t = nullptr);
-void launch_sweep_y(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t = nullptr);
-void launch_advect(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t = nullptr);
-void launch_kick2(const DiskView& d, const CellMaps& in, const VisMaps& vis, Cell* out, cudaStream_t s,
+void launch_sweep_y(const DiskView& d, const Cell* in, Cell* out, cudaStream_t s, const Tune* t = nullptr);
+void launch_advect(const DiskView& d, const Cell* in, Cell* out, cudaStream_t s, const Tune* t = nullptr);
+void launch_kick2(const DiskView& d, const Cell* in, const double* vis, Cell* out, cudaStream_t s,
                   const pg_dust* din = nullptr, pg_dust* dout = nullptr, const Tune* t = nullptr);
-int pass_occupancy(const DiskView& d, int pass, int v);
-void sweep_variant_launch(int v, int* threads, int* minb);
+int pass_occupancy(const DiskView& d, int pass);
+void sweep_launch_shape(int* threads, int* minb);
 // the ghost rows of the periodic azimuth take the weights of the rows they image
 void periodic_seam_weights(double* wy, int ypad, int yres);
 void launch_init_planet(const DiskView& d, const pg_params& P, double t, cudaStream_t s);
@@ -120,10 +105,10 @@ void set_last_error(const char* msg);
 
 // `planes` planes of `count` doubles, back to back in device memory, to host arrays
 // (pg_hostcopy.cu), ordered after s's work; the caller synchronizes s.  The pinned staging
-// (8 MB) is kept with the disk from its first large read on.
+// (2 MB) is kept with the disk from its first large read on.
 constexpr int COPY_THREADS = 4;
 struct HostCopy {
-    static constexpr size_t SLOT = (size_t)1 << 17;  // doubles
+    static constexpr size_t SLOT = (size_t)1 << 15;  // doubles
     double* pinned = nullptr;
     cudaEvent_t ev[COPY_THREADS][2] = {};
     HostCopy() = default;
@@ -143,7 +128,7 @@ pg_status engine_set_state_device(Engine* E, double t, const double* r, const do
                                   const double* v);
 pg_status engine_step(Engine* E, double t, double dt, const StepRecord* rec);
 pg_status engine_save(Engine* E, Cell* cells, Scalars* sc);
-pg_status engine_restore(Engine* E, const Cell* cells, const Scalars* sc);
+pg_status engine_restore(Engine* E, const Cell* cells, const Scalars* sc, Cell* into = nullptr);
 // the stream the engine launches on; returns the previous one
 cudaStream_t engine_set_stream(Engine* E, cudaStream_t s);
 pg_status engine_extract_device(Engine* E, double* r, double* p, double* u, double* v);
@@ -152,8 +137,6 @@ pg_status table_engine_create(const pg_params* P, int device, cudaStream_t s, En
 void engine_destroy(Engine* E);
 const DiskView& engine_view(const Engine* E);
 void engine_init_planet(Engine* E, double t);
-pg_status make_map3_f32(CUtensorMap* m, const float* base, uint64_t pitch, uint64_t rows, uint64_t planes,
-                        uint32_t bx, uint32_t by, uint32_t bz);
 cudaError_t set_kernel_attributes();
 
 // dust passes (pg_dust.cu)

@@ -12,9 +12,8 @@
 //                    (src/killwave/killwave.cu:17-103) and the CFL signal speed
 //                    for the next step (src/timestep/timestep.cu:18-97)
 //
-// plus a one-thread time kernel (dt, planet).  Every pass reads its tile with a
-// TMA bulk tensor copy into shared memory and writes each cell together with its
-// ghost images, so no separate boundary pass is needed between stages.
+// plus a one-block clock kernel (dt, planet and its table).  Every pass writes each cell
+// together with its ghost images, so no separate boundary pass is needed between stages.
 #include <cstdio>
 
 #include "pg_common.cuh"
@@ -25,64 +24,29 @@
 
 namespace pg {
 
-// ---------------------------------------------------------------- tiles
-// Sweep and advection tiles: L outputs along the sweep times W pencils per CTA,
-// each thread taking CPT cells (or faces, or outputs) of a phase, with NS TMA
-// stages in flight (SwCfg).  The autotuner (pg_disk_autotune) picks one of the
-// variants listed in SWEEP_VARIANTS per pass; the per-cell arithmetic does not
-// depend on the choice.
-template <int W_, int L_, int CPT_, int NS_, int MINB_ = 0>
-struct SwCfg {
-    static constexpr int W = W_, L = L_, CPT = CPT_, NS = NS_;
-    static constexpr int TL = L + 2 * NPAD;                       // tile cells along the sweep
-    static constexpr int P1 = L + 2;                               // cells reconstructed per pencil
-    static constexpr int P2 = L + 1;                               // faces per pencil
-    static constexpr int NST = P1 * W;                             // reconstructed cells
-    static constexpr int NFX = P2 * W;                             // faces
-    static constexpr int NOUT = L * W;                             // outputs
-    static constexpr int THREADS = ((NST + CPT - 1) / CPT + 31) / 32 * 32;
-    // CTAs per SM the registers allow at ~96 registers a thread, unless given
-    static constexpr int MINB = MINB_ > 0 ? MINB_ : (65536 / (THREADS * 96) > 0 ? 65536 / (THREADS * 96) : 1);
-    static constexpr int YCOLS = W + 2;                            // y tiles start one column early (16-B TMA x)
-    static constexpr int XTILE = W * TL * 5;                       // doubles
-    static constexpr int YTILE = TL * YCOLS * 5;
-    static constexpr int TILE_MAX = ((XTILE > YTILE ? XTILE : YTILE) + 15) / 16 * 16;
-    static constexpr bool X_OK = 5 * TL <= 256;                    // a TMA box is at most 256 elements wide
-    // ISO: a 2D isothermal gas carries 4 edge-state fields and 4 fluxes (3 in the
-    // advection) instead of 5 and 7 (5)
-    template <bool ISO>
-    static constexpr size_t smem() { return (size_t)(NS * TILE_MAX + (ISO ? 8 : 10) * NST + (ISO ? 4 : 7) * NFX) * 8 + 8 * NS + 128; }
-    template <bool ISO>
-    static constexpr size_t ad_smem() { return (size_t)(NS * TILE_MAX + (ISO ? 3 : 5) * TL * W) * 8 + 8 * NS + 128; }
-};
-// The variants, in the order of SweepVariant ids (pg_internal.h SWEEP_VARIANTS).
-template <int V> struct SV;
-template <> struct SV<0> { using G = SwCfg<8, 32, 1, 2>; };   // default
-template <> struct SV<1> { using G = SwCfg<4, 32, 1, 2>; };
-template <> struct SV<2> { using G = SwCfg<16, 16, 1, 2>; };
-template <> struct SV<3> { using G = SwCfg<8, 16, 1, 2>; };
-template <> struct SV<4> { using G = SwCfg<8, 32, 2, 2>; };
-template <> struct SV<5> { using G = SwCfg<8, 32, 1, 3>; };
-template <> struct SV<6> { using G = SwCfg<4, 32, 1, 3>; };
-template <> struct SV<7> { using G = SwCfg<4, 64, 1, 2>; };   // azimuthal passes only (x box too wide)
-template <> struct SV<8> { using G = SwCfg<4, 32, 1, 2, 5>; };  // registers capped for 5 CTAs per SM
-template <> struct SV<9> { using G = SwCfg<8, 32, 1, 2, 3>; };  // registers capped for 3 CTAs per SM
-static_assert(NSWEEP_VARIANTS == 10, "SV<> and SWEEP_VARIANTS list the same variants");
+// ------------------------------------------------- the sweeps' work layout
+// Lanes of a warp lie along the radius, which is contiguous in memory, in every
+// pass, and a warp takes `len` rows of its 30 or 32 radii one after the other.  No
+// barrier separates the phases of a cell: what a cell needs of its neighbours comes
+// by shuffle (radial sweep) or stays in registers from the row before (azimuthal
+// passes).  Tiles of 32 x 8 cells whose phases met at __syncthreads and exchanged
+// states and fluxes through shared memory spent 900-1000 instructions a cell, 350 of
+// them FP64, and a quarter of their time at the barriers; the sweeps spend 720-770 now.
+// What is left to bound them is FP64 issue and latency: about half of the FP64 rate, a
+// third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1 108 -> 88, sweep_x 298 -> 123,
+// sweep_y 328 -> 123, advection 154 -> 72, kick2 177 -> 160.
+// Each kernel is compiled for the CTAs per SM that were fastest there: sweep_x at 3 / 4 / 5
+// 123 / 129 / 151, sweep_y 123 / 139 / 246, advection at 4 / 5 / 6 72 / 72 / 115 (adiabatic
+// 512x1536: 26 / 32 / 43), kick1 at 3 / 4 / 5 106 / 88 / 104, kick2 at 2 / 3 / 4 201 / 160 / 182.
+constexpr int SW_WARPS = 4;                       // warps per CTA, independent of one another
+constexpr int RX_OUT = 30;                        // radial sweep: outputs of a warp's 32 cells
+constexpr int RX_ROWS = RX_TILE_ROWS;             // rows per TMA copy
+constexpr int RX_STAGE = RX_TILE_CELLS * RX_ROWS * 5;  // doubles
+static_assert(RX_TILE_CELLS == RX_OUT + 6, "32 lanes and two stencil cells a side");
+static_assert(RX_STAGE * 8 % 128 == 0, "128-byte aligned stages");
+constexpr size_t RX_SMEM = (size_t)SW_WARPS * 2 * RX_STAGE * 8 + SW_WARPS * 16 + 128;
 
-constexpr int ST_TX = 32, ST_TY = 8;        // stencil kernels: 32 x 8 outputs
-constexpr int ST_HX = ST_TX + 2, ST_HY = ST_TY + 2;
-constexpr int ST_THREADS = ST_TX * ST_TY;
-constexpr int ST_TILE_N = ST_HX * ST_HY * 5;          // doubles in one cell tile
-constexpr int ST_TILE = (ST_TILE_N + 15) / 16 * 16;     // rounded so every TMA target is 128-B aligned
-constexpr int ST_VIS_N = ST_HX * ST_HY * 2;
-constexpr int ST_VIS = (ST_VIS_N + 15) / 16 * 16;
-constexpr size_t K1_SMEM = (size_t)2 * ST_TILE * 8 + 16 + 128;
-constexpr int ST_GRAV = (ST_HX * ST_HY * 3 + 15) / 16 * 16;  // kick2: gravity of the predictor, per tile cell
-// kick2: the tile's per-radius (34) and per-row (10) tables, staged once per tile
-enum KRad { KR_RAD, KR_IRAD, KR_GSTAR, KR_NU, KR_IDX, KR_ROT, KR_VX, KR_KILL = KR_VX + 5, KR_N = KR_KILL + 4 };
-enum KRow { KY_SIN, KY_COS, KY_IDY, KY_VY, KY_N = KY_VY + 4 };
-constexpr int ST_TAB = (KR_N * ST_HX + KY_N * ST_HY + 15) / 16 * 16;
-constexpr size_t K5_SMEM = (size_t)(3 * ST_TILE + 2 * ST_VIS + ST_GRAV + ST_TAB) * 8 + 16 + 128;
+constexpr int KK_OUT = 30;                        // half-kicks: outputs of a warp's 32 cells
 
 // --------------------------------------------------------- source terms
 struct Grav {
@@ -189,20 +153,6 @@ __device__ __forceinline__ Cell kick(const DiskView& d, const Cell& C, double ix
     return o;
 }
 
-// Gathers the 3x3 stencil around tile cell (hx, hy) of a [ST_HY][ST_HX][5] tile.
-__device__ __forceinline__ void gather9(const double* tile, int hx, int hy, const double nu[3], double* u,
-                                        double* v, double* nr) {
-#pragma unroll
-    for (int n = 0; n < 9; ++n) {
-        const int dx = (n % 3) - 1;
-        const int dy = (n < 3) ? 0 : (n < 6 ? -1 : 1);
-        const double* c = tile + ((hy + dy) * ST_HX + (hx + dx)) * 5;
-        nr[n] = c[0] * nu[n % 3];
-        u[n] = c[2];
-        v[n] = c[3];
-    }
-}
-
 // add_grid (src/output/output.cu:250-275): A += C (0.5 dt) / T on the interior
 __device__ __forceinline__ void accumulate_average(const DiskView& d, int i, int j, const Cell& C, double hdt) {
     const double fac = hdt / d.ave_T;
@@ -231,634 +181,587 @@ __device__ __forceinline__ double signal_rate(const DiskView& d, const Cell& c, 
     return tmp;
 }
 
-// signal_rate with the cell's table entries passed in (kick2's staged tables):
-// the same expressions
-__device__ __forceinline__ double signal_rate_at(const DiskView& d, const Cell& c, double radx, double idxx,
-                                                 double rot, double idyj, double irad, const DCell* dc = nullptr) {
-    const double rad_cyl = (d.geomy == 3) ? radx : 1.0;
-    const double cs = sound_speed(d.gam, c.r, c.p);
-    double spd = fabs(c.u) + cs;
-    if (dc) spd = fmax(fabs(dc->u), spd);
-    double tmp = fmax(spd * idxx, 0.0);
-    if (d.ndim > 1) {
-        spd = fabs(c.v - rad_cyl * d.frame_omega - rot) + cs;
-        if (dc) spd = fmax(fabs(dc->v - rad_cyl * d.frame_omega - rot), spd);
-        tmp = fmax(spd * (idyj * ((d.geomy == 3) ? irad : 1.0)), tmp);
+// What a marching pass writes: cell (i, j) at `o` and its periodic azimuthal image; a cell
+// with radial images (bound 1 and 2, a lane at the edge) takes emit's general way.
+struct Emitter {
+    int lo, hi;        // rows below lo have an image yres rows up, rows from hi on yres rows down
+    long long image;   // doubles between a row and its image
+    bool edge;
+    __device__ __forceinline__ Emitter(const DiskView& d, int i) {
+        lo = d.ndim > 1 ? 2 * NPAD : 0;
+        hi = d.ndim > 1 ? d.yres : 0x7fffffff;
+        image = 5ll * d.xarr * d.yres;
+        const int nx = d.xres + NPAD;
+        edge = (d.bound_lft != 0 && i < 2 * NPAD) || (d.bound_rgh != 0 && i >= nx - NPAD);
     }
-    return tmp;
+    __device__ __forceinline__ void put(double* o, const Cell& c) const {
+        o[0] = c.r;
+        o[1] = c.p;
+        o[2] = c.u;
+        o[3] = c.v;
+        o[4] = c.w;
+    }
+    __device__ __forceinline__ void operator()(const DiskView& d, Cell* out, double* o, int i, int j, const Cell& c) const {
+        put(o, c);
+        if (j < lo || j >= hi) put(o + (j < lo ? image : -image), c);
+        if (edge) emit(d, out, i, j, c);
+    }
+};
+__device__ __forceinline__ double* cell_at(const DiskView& d, Cell* out, int i, int j) {
+    return reinterpret_cast<double*>(out + ((size_t)i + (size_t)d.xarr * j));
 }
 
 // ================================================================ sweeps
-// DIR 0: radial pencils (rows of the array), DIR 1: azimuthal pencils (columns).
-// G: the tile configuration (SwCfg).  ISO: a 2D isothermal gas, which needs neither
-// the energy flux nor the z-velocity (identically zero there): four fields instead
-// of five through the three phases.  The passes are bound by the latency and issue
-// of their FP64 arithmetic, not by memory (0.12 of the copy rate), so what counts is
-// instructions: reciprocals and roots without their IEEE tails (pg_hydro.cuh), and
-// nothing computed that the equation of state does not use.
-template <int DIR, class G, bool ISO>
-__global__ void __launch_bounds__(G::THREADS, G::MINB)
-    k_sweep(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out, int ntx, int ntiles) {
-    constexpr int SW_W = G::W, SW_LEN = G::L, SW_TL = G::TL, SW_P1 = G::P1, SW_P2 = G::P2;
-    constexpr int SW_TILE_MAX = G::TILE_MAX, SW_NST = G::NST, SW_NFX = G::NFX, SWY_COLS = G::YCOLS;
-    constexpr int SWX_TILE = G::XTILE, SWY_TILE = G::YTILE, NS = G::NS, NT = G::THREADS;
-    constexpr int NH = ISO ? 4 : 5;  // fields of an edge state: r, p, u, then the transverse velocities
+// ISO: a 2D isothermal gas, which needs neither the energy flux nor the z-velocity
+// (identically zero in 2D): nothing is computed that the equation of state does not use.
+// The passes are bound by the latency and issue of their FP64 arithmetic (0.12 of the
+// copy rate), so what counts is instructions: reciprocals and roots without their
+// IEEE tails (pg_hydro.cuh).
+
+// A warp's bounded wait for its own tile (mbar_wait: on a time-out the error word is set)
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, Scalars* sc) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, sc));
+}
+__device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double down1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+
+// Radial sweep (src/solver/sweeps.cu:263-335).  A warp stages 4 rows of 36 cells per
+// TMA copy, two copies in flight; lane l holds cell 2 + 30 seg + l: it reconstructs it,
+// takes its left face's left state from the lane below and its right face's flux from
+// the lane above, and lanes 1..30 update.
+template <bool ISO>
+__global__ void __launch_bounds__(32 * SW_WARPS, 3)
+    k_sweep_x(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out, int nseg, int len,
+              int nitems) {
     extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n % NS) * SW_TILE_MAX; };
-    double* st = smem + NS * SW_TILE_MAX;  // [2 NH][SW_NST] interface states
-    double* fl = st + 2 * NH * SW_NST;     // [ISO ? 4 : 7][SW_NFX] fluxes
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + (ISO ? 4 : 7) * SW_NFX);
-    __shared__ int s_inc[SW_W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* buf = smem_base128(smem_raw) + (size_t)warp * 2 * RX_STAGE;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smem_base128(smem_raw) + (size_t)SW_WARPS * 2 * RX_STAGE) + 2 * warp;
     Scalars* sc = d.sc;
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncwarp();
+    pdl_enter();
     if (sc->done) return;
-
-    const int tid = threadIdx.x;
-    const double dt = sc->dt;
-    const double gam = d.gam;
+    const double dt = sc->dt, gam = d.gam;
     const int eos = ISO ? 0 : d.eos;
-    const uint32_t bytes = (DIR == 0 ? SWX_TILE : SWY_TILE) * 8;
-    auto origin = [&](int tile, int& s0, int& q0) {
-        const int bx = tile % ntx, by = tile / ntx;
-        s0 = NPAD + SW_LEN * bx;                     // first output along the sweep
-        q0 = (DIR == 0 ? d.ypad : NPAD) + SW_W * by;  // first pencil
-    };
-    auto issue = [&](int tile, int k) {
-        int s0, q0;
-        origin(tile, s0, q0);
-        issue_begin(&bar[k % NS], bytes);
-        if (DIR == 0) issue_box(stage(k), &tm, 5 * (s0 - NPAD), q0, &bar[k % NS]);
-        else issue_box(stage(k), &tm, 5 * (q0 - 1), s0 - NPAD, &bar[k % NS]);
-    };
-    pipe_init<NS>(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0)
-        for (int m = 0; m < NS - 1; ++m)
-            if ((int)blockIdx.x + m * (int)gridDim.x < ntiles) issue(blockIdx.x + m * gridDim.x, m);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-    // tiles issued beyond this one (the one NS - 1 ahead is issued now)
-    int ahead = 0;
-    while (ahead < NS - 1 && tile_id + (ahead + 1) * (int)gridDim.x < ntiles) ++ahead;
-    if (tid == 0 && ahead == NS - 1) issue(tile_id + (NS - 1) * gridDim.x, kt + NS - 1);
-    int s0, q0;
-    origin(tile_id, s0, q0);
-    double* tile = stage(kt);
+    const int jend = d.ypad + d.yres;
+    int k = 0;  // copies waited for by this warp
+    for (int item = blockIdx.x * SW_WARPS + warp; item < nitems; item += gridDim.x * SW_WARPS) {
+        const int seg = item % nseg, j0 = d.ypad + len * (item / nseg), j1 = min(j0 + len, jend);
+        auto issue = [&](int j, int n) {  // rows j .. j + 3 into copy n
+            issue_begin(&bar[n & 1], RX_STAGE * 8);
+            issue_box(buf + (n & 1) * RX_STAGE, &tm, 5 * RX_OUT * seg, j, &bar[n & 1]);
+        };
+        if (lane == 0) {
+            issue(j0, k);
+            if (j0 + RX_ROWS < j1) issue(j0 + RX_ROWS, k + 1);
+        }
+        const int i = NPAD - 1 + RX_OUT * seg + lane, ic = min(i, d.xarr - 1);
+        const bool output = lane >= 1 && lane <= RX_OUT && i < NPAD + d.xres;
+        const Emitter emit_to(d, i);
+        double* o = cell_at(d, out, ic, j0);
+        double w[6], rad[5];
+#pragma unroll
+        for (int m = 0; m < 6; ++m) w[m] = d.wx[6 * ic + m];
+#pragma unroll
+        for (int m = 0; m < 5; ++m) rad[m] = d.geomx == 1 ? d.radx[min(max(i - 2 + m, 0), d.xarr - 1)] : 1.0;
+        const double sx = dt * d.idx_x[ic];
+        const double f = dt * d.ixv[ic];
+        const double irad = d.geomx == 1 ? d.irad[ic] : 1.0;
+        const double cs2 = d.cs2x[ic];
+        const double g0 = d.geomx == 1 ? d.xa[ic] : 1.0, g1 = d.geomx == 1 ? d.xa[ic + 1] : 1.0;  // riemann.cu:5-11
+        for (int j = j0; j < j1; j += RX_ROWS, ++k) {
+            if (!warp_wait(&bar[k & 1], (uint32_t)((k >> 1) & 1), sc)) {
+                if (lane == 0 && j + RX_ROWS < j1) mbar_wait(&bar[(k + 1) & 1], (uint32_t)(((k + 1) >> 1) & 1), sc);
+                return;
+            }
+            const double* row = buf + (k & 1) * RX_STAGE + 5 * (lane + 2);
+#pragma unroll 1
+            for (int jj = j; jj < min(j + RX_ROWS, j1); ++jj, row += 5 * RX_TILE_CELLS) {
+                auto field = [&](int m, double flat) {
+                    return recon(w, row[m - 10], row[m - 5], row[m], row[m + 5], row[m + 10], flat);
+                };
+                const Cell C0{row[0], row[1], row[2], row[3], row[4]};
+                const double cs0 = sound_speed(gam, C0.r, C0.p);
+                const double flat = flatten(C0.p, row[-9], row[-4], row[6], row[11], row[-3], C0.u, row[7]);
+                const Par R = field(0, flat), P = field(1, flat), U = field(2, flat);
+                // angular momentum (geomx 1)
+                const Par A = recon(w, row[-7] * rad[0], row[-2] * rad[1], C0.v * rad[2], row[8] * rad[3],
+                                    row[13] * rad[4], flat);
+                Par Z{0.0, 0.0, 0.0};
+                if (!ISO && d.ndim != 2) Z = field(4, flat);  // in 2D the z-velocity is identically zero
+                const Half eL = state_at_left_edge(gam, sx, cs0, C0.r, C0.p, C0.u, R, P, U, A, Z);
+                const Half eR = state_at_right_edge(gam, sx, cs0, C0.r, C0.p, C0.u, R, P, U, A, Z);
+                const Half L{up1(eR.r), up1(eR.p), up1(eR.u), up1(eR.v), ISO ? 0.0 : up1(eR.w)};
+                const Flux F = hllc(eos, d.ie, gam, L, eL);
+                // net_source (src/solver/riemann/riemann.cu:40-87) and the flux differences
+                auto net = [&](double x) { return x * g0 - down1(x) * g1; };
+                const double pres1 = down1(F.pres);
+                Cell D;
+                D.r = net(F.r) * f;
+                D.u = (net(F.u) + 0.5 * (g0 + g1) * (F.pres - pres1)) * f;
+                D.v = net(F.v) * f * irad;
+                D.w = D.p = 0.0;
+                if (!ISO) {
+                    D.w = net(F.w) * f;
+                    double de = net(F.uprs);
+                    if (d.ie != 0) de *= 0.5 * (F.pres + pres1);
+                    D.p = (net(F.p) + (eos == 2 ? de : 0.0)) * f;
+                }
+                if (output) {
+                    const Cell Q = update_cell<ISO>(eos, d.ie, gam, cs2, C0, D, &sc->floor_hits);
+                    if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                    emit_to(d, out, o, i, jj, Q);
+                }
+                o += 5 * (size_t)d.xarr;
+            }
+            __syncwarp();  // the copy's reads are done
+            if (lane == 0 && j + 2 * RX_ROWS < j1) issue(j + 2 * RX_ROWS, k + 2);
+        }
+    }
+}
 
-    if (DIR == 1 && tid < SW_W) {
+// r, p, u, v of one cell of a column
+__device__ __forceinline__ void load4(const double* c, double* q) {
+#pragma unroll
+    for (int m = 0; m < 4; ++m) q[m] = c[m];
+}
+
+// Azimuthal sweep (sweeps.cu:361-433) with the orbital shift (orbit.cu:17-99): a lane
+// marches along its own column.  Five rows of it are in registers, the next one in
+// flight; each row costs one reconstruction, one trace of both edges, the flux at the
+// face below it and the update of the cell below that, written len rows long at its
+// shifted place.  The per-radius factors are loop constants and the per-row tables
+// the same for the whole warp.
+template <bool ISO>
+__global__ void __launch_bounds__(32 * SW_WARPS, 3)
+    k_sweep_y(const Cell* __restrict__ in, const DiskView d, Cell* __restrict__ out, int ncol, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Scalars* sc = d.sc;
+    pdl_enter();
+    if (sc->done) return;
+    const double dt = sc->dt, gam = d.gam;
+    const int eos = ISO ? 0 : d.eos;
+    for (int item = blockIdx.x * SW_WARPS + warp; item < nitems; item += gridDim.x * SW_WARPS) {
+        const int i = NPAD + 32 * (item % ncol) + lane;
+        const bool active = i < NPAD + d.xres;
+        const int ic = min(i, NPAD + d.xres - 1);
+        const int s0 = NPAD + len * (item / ncol), s1 = min(s0 + len, NPAD + d.yres);
+        const double rad = (d.geomy == 3) ? d.radx[ic] : 1.0, irad = (d.geomy == 3) ? d.irad[ic] : 1.0;
+        const double rot = d.rot[ic], cs2 = d.cs2x[ic];
+        const double v0 = (d.geomy == 3) ? rot + rad * d.frame_omega : rot;
         // set_orbital_advection (src/orbit/orbit.cu:74-99) for this column
-        const int i = q0 + tid;
         int shift = 0;
-        if (d.orbadv && i < NPAD + d.xres) {
-            const double rad = d.radx[i];
-            const double dy = d.dy0 * rad;
-            const double rot = d.rot[i];
+        if (d.orbadv) {
+            const double dy = d.dy0 * d.radx[ic];
             shift = __double2int_rd(rot * dt / dy + 0.5);
             double speed = shift * dy / dt;
             speed = rot - speed;
-            if (s0 == NPAD) {
+            if (s0 == NPAD && active) {
                 d.res[i] = speed;
                 d.inc[i] = shift;
             }
         }
-        s_inc[tid] = shift;
-    }
-    if (!pipe_wait<NS>(bar, kt, sc)) {
-        pipe_drain<NS>(bar, kt, ahead, sc);
-        return;
-    }
-
-    // ---- P1: reconstruction + both edge states of every cell
-    for (int it = tid; it < SW_NST; it += NT) {
-        const int q = (DIR == 0) ? it / SW_P1 : it % SW_W;
-        const int t = 2 + ((DIR == 0) ? it % SW_P1 : it / SW_W);
-        const int s = s0 - NPAD + t;
-        const int qq = q0 + q;
-        // sweep order: r, p, u, then for DIR 0 v (angular momentum) and w, for DIR 1 w and v_r
-        double r[5], p[5], u[5], a[5], z[5];
-        double v0 = 0.0, irad_q = 1.0;
-        if (DIR == 1) {  // the azimuthal velocity relative to the disk's rotation
-            const int i = min(qq, d.xarr - 1);
-            irad_q = (d.geomy == 3) ? d.irad[i] : 1.0;
-            v0 = d.rot[i];
-            if (d.geomy == 3) v0 += d.radx[i] * d.frame_omega;
-        }
+        const double sdt = dt * irad;
+        // row the first output goes to: T[(j+inc) mod N] = C[j] (orbit.cu:30-46)
+        int js = (s0 - d.ypad + shift) % d.yres;
+        if (js < 0) js += d.yres;
+        const double* col = reinterpret_cast<const double*>(in + ic);
+        const size_t pitch = 5 * (size_t)d.xarr;
+        const Emitter emit_to(d, i);
+        double* o = cell_at(d, out, ic, js + d.ypad);
+        const double* next = col + pitch * (s0 - NPAD);
+        double q[5][4], nx[4];  // rows t-2 .. t+2 and t+3: r, p, v_r, v_phi
 #pragma unroll
-        for (int k = 0; k < 5; ++k) {
-            const double* c = (DIR == 0) ? tile + (q * SW_TL + (t - 2 + k)) * 5
-                                         : tile + ((t - 2 + k) * SWY_COLS + (q + 1)) * 5;
-            r[k] = c[0];
-            p[k] = c[1];
-            if (DIR == 0) {
-                u[k] = c[2];
-                a[k] = c[3];
-                if (d.geomx == 1) a[k] *= d.radx[min(max(s - 2 + k, 0), d.xarr - 1)];
-                if (!ISO) z[k] = c[4];
-            } else {
-                u[k] = c[3] - v0;
-                a[k] = c[2];
-                if (!ISO) z[k] = c[4];
-            }
-        }
-        const double cs0 = sound_speed(gam, r[2], p[2]);
-        const double flat = flatten(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3]);
-        const int sc_ = (DIR == 0) ? min(s, d.xarr - 1) : min(s, d.yarr - 1);
-        const double* wt = ((DIR == 0) ? d.wx : d.wy) + 6 * sc_;
-        const double sx = dt * irad_q * ((DIR == 0) ? d.idx_x : d.idx_y)[sc_];
-        const Par R = recon(wt, r[0], r[1], r[2], r[3], r[4], flat);
-        const Par P = recon(wt, p[0], p[1], p[2], p[3], p[4], flat);
-        const Par U = recon(wt, u[0], u[1], u[2], u[3], u[4], flat);
-        const Par A = recon(wt, a[0], a[1], a[2], a[3], a[4], flat);
-        // the z-velocity, identically zero in 2D: a zero field's parabola is {0, 0, 0}
-        Par Z{0.0, 0.0, 0.0};
-        if (!ISO && d.ndim != 2) Z = recon(wt, z[0], z[1], z[2], z[3], z[4], flat);
-        else if (!ISO) Z.a = z[2];
-        const Half eL = state_at_left_edge(gam, sx, cs0, r[2], p[2], u[2], R, P, U, A, Z);
-        const Half eR = state_at_right_edge(gam, sx, cs0, r[2], p[2], u[2], R, P, U, A, Z);
-        double* o = st + it;
-        o[0] = eL.r;
-        o[1 * SW_NST] = eL.p;
-        o[2 * SW_NST] = eL.u;
-        o[3 * SW_NST] = eL.v;
-        if (!ISO) o[4 * SW_NST] = eL.w;
-        o += NH * SW_NST;
-        o[0] = eR.r;
-        o[1 * SW_NST] = eR.p;
-        o[2 * SW_NST] = eR.u;
-        o[3 * SW_NST] = eR.v;
-        if (!ISO) o[4 * SW_NST] = eR.w;
-    }
-    __syncthreads();
-
-    // ---- P2: HLLC flux at every face (left state from cell t-1, right from cell t)
-    for (int it = tid; it < SW_NFX; it += NT) {
-        const int q = (DIR == 0) ? it / SW_P2 : it % SW_W;
-        const int t = 3 + ((DIR == 0) ? it % SW_P2 : it / SW_W);
-        const double* pL = st + NH * SW_NST + ((DIR == 0) ? q * SW_P1 + (t - 3) : (t - 3) * SW_W + q);
-        const double* pR = st + ((DIR == 0) ? q * SW_P1 + (t - 2) : (t - 2) * SW_W + q);
-        Half L{pL[0], pL[SW_NST], pL[2 * SW_NST], pL[3 * SW_NST], 0.0};
-        Half R{pR[0], pR[SW_NST], pR[2 * SW_NST], pR[3 * SW_NST], 0.0};
-        if (!ISO) {
-            L.w = pL[4 * SW_NST];
-            R.w = pR[4 * SW_NST];
-        }
-        const Flux F = hllc(eos, d.ie, gam, L, R);
-        double* o = fl + it;
-        o[0] = F.r;
-        o[1 * SW_NFX] = F.u;
-        o[2 * SW_NFX] = F.v;
-        o[3 * SW_NFX] = F.pres;
-        if (!ISO) {
-            o[4 * SW_NFX] = F.w;
-            o[5 * SW_NFX] = F.p;
-            o[6 * SW_NFX] = F.uprs;
-        }
-    }
-    __syncthreads();
-
-    // ---- P3: flux differences, geometric sources, conservative update
-    for (int it = tid; it < SW_LEN * SW_W; it += NT) {
-        const int q = (DIR == 0) ? it / SW_LEN : it % SW_W;
-        const int t = 3 + ((DIR == 0) ? it % SW_LEN : it / SW_W);
-        const int s = s0 - NPAD + t;
-        const int qq = q0 + q;
-        const bool valid = (DIR == 0) ? (s < NPAD + d.xres && qq < d.ypad + d.yres)
-                                      : (s < NPAD + d.yres && qq < NPAD + d.xres);
-        if (valid) {
-            const double* f0 = fl + ((DIR == 0) ? q * SW_P2 + (t - 3) : (t - 3) * SW_W + q);
-            const double* f1 = f0 + ((DIR == 0) ? 1 : SW_W);
-            const double g0 = (DIR == 0 && d.geomx == 1) ? d.xa[s] : 1.0;  // eval_gfac (riemann.cu:5-11)
-            const double g1 = (DIR == 0 && d.geomx == 1) ? d.xa[s + 1] : 1.0;
-            auto net = [&](int k) { return f0[k * SW_NFX] * g0 - f1[k * SW_NFX] * g1; };
-            const double pres0 = f0[3 * SW_NFX], pres1 = f1[3 * SW_NFX];
-            // net_source (src/solver/riemann/riemann.cu:40-87): along the sweep, and the energy's
-            const double f = (DIR == 0) ? dt * d.ixv[s] : dt * d.iyv[s] * ((d.geomy == 3) ? d.irad[qq] : 1.0);
-            const double Dr = net(0) * f;
-            double Du = (net(1) + 0.5 * (g0 + g1) * (pres0 - pres1)) * f;
-            double Da = net(2) * f;
-            double Dz = 0.0, Dp = 0.0;
-            if (!ISO) {
-                Dz = net(4) * f;
-                double de = 0.0;
-                if (eos == 2) de = (d.ie == 0) ? net(6) : 0.5 * (pres0 + pres1) * net(6);
-                Dp = (net(5) + de) * f;
-            }
-            const double* c = (DIR == 0) ? tile + (q * SW_TL + t) * 5 : tile + (t * SWY_COLS + (q + 1)) * 5;
-            const Cell C0{c[0], c[1], c[2], c[3], c[4]};
-            Cell D;
-            int i, j;
-            if (DIR == 0) {
-                if (d.geomx == 1) Da *= d.irad[s];
-                D = Cell{Dr, Dp, Du, Da, Dz};
-                i = s;
-                j = qq;
-            } else {
-                double v0 = d.rot[qq];
-                if (d.geomy == 3) v0 += d.radx[qq] * d.frame_omega;
-                Du += v0 * Dr;
-                D = Cell{Dr, Dp, Da, Du, Dz};
-                i = qq;
-                j = s;
-                if (d.orbadv) {  // orbital shift T[(j+inc) mod N] = C[j] (orbit.cu:30-46)
-                    int js = (s - d.ypad + s_inc[q]) % d.yres;
-                    if (js < 0) js += d.yres;
-                    j = js + d.ypad;
+        for (int m = 0; m < 5; ++m, next += pitch) load4(next, q[m]);
+        Half pr{};   // the state at the right edge of the cell below
+        Flux pf{};   // the flux at the face below it
+#pragma unroll 1
+        for (int t = s0 - 1; t <= s1; ++t) {
+            if (t < s1) load4(next, nx);
+            next += pitch;
+            double u[5];
+#pragma unroll
+            for (int m = 0; m < 5; ++m) u[m] = q[m][3] - v0;
+            const double* w = d.wy + 6 * t;
+            auto field = [&](int m, double flat) { return recon(w, q[0][m], q[1][m], q[2][m], q[3][m], q[4][m], flat); };
+            const double cs0 = sound_speed(gam, q[2][0], q[2][1]);
+            const double flat = flatten(q[2][1], q[0][1], q[1][1], q[3][1], q[4][1], u[1], u[2], u[3]);
+            const double sx = sdt * d.idx_y[t];
+            const Par R = field(0, flat), P = field(1, flat), A = field(2, flat);
+            const Par U = recon(w, u[0], u[1], u[2], u[3], u[4], flat);
+            const Par Z{0.0, 0.0, 0.0};
+            const Half eL = state_at_left_edge(gam, sx, cs0, q[2][0], q[2][1], u[2], R, P, U, A, Z);
+            const Half eR = state_at_right_edge(gam, sx, cs0, q[2][0], q[2][1], u[2], R, P, U, A, Z);
+            Flux F{};
+            if (t >= s0) F = hllc(eos, d.ie, gam, pr, eL);
+            if (t > s0) {  // the cell below has both its fluxes
+                const double f = sdt * d.iyv[t - 1];
+                Cell D;
+                D.r = (pf.r - F.r) * f;
+                D.v = ((pf.u - F.u) + (pf.pres - F.pres)) * f + v0 * D.r;
+                D.u = (pf.v - F.v) * f;
+                D.w = D.p = 0.0;
+                if (!ISO) {
+                    double de = pf.uprs - F.uprs;
+                    if (d.ie != 0) de *= 0.5 * (pf.pres + F.pres);
+                    D.p = ((pf.p - F.p) + (eos == 2 ? de : 0.0)) * f;
+                }
+                if (active) {
+                    const Cell C0{q[1][0], q[1][1], q[1][2], q[1][3], 0.0};
+                    const Cell Q = update_cell<ISO>(eos, d.ie, gam, cs2, C0, D, &sc->floor_hits);
+                    if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                    emit_to(d, out, o, i, js + d.ypad, Q);
+                }
+                o += pitch;
+                if (++js == d.yres) {
+                    js = 0;
+                    o -= pitch * d.yres;
                 }
             }
-            const Cell Q = update_cell<ISO>(eos, d.ie, gam, d.cs2x[i], C0, D, &sc->floor_hits);
-            if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-            emit(d, out, i, j, Q);
+            pr = eR;
+            pf = F;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                q[0][m] = q[1][m];
+                q[1][m] = q[2][m];
+                q[2][m] = q[3][m];
+                q[3][m] = q[4][m];
+                q[4][m] = nx[m];
+            }
         }
-    }
-    __syncthreads();  // stage k % NS, the state / flux arrays and s_inc are free again
     }
 }
 
 // ===================================================== residual advection
-// ISO as in k_sweep: without the pressure (reset from the density after the
-// update) and the z-velocity.
-template <class G, bool ISO>
-__global__ void __launch_bounds__(G::THREADS, G::MINB)
-    k_advect(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out, int ntx, int ntiles) {
-    constexpr int SW_W = G::W, SW_LEN = G::L, SW_TL = G::TL, SW_TILE_MAX = G::TILE_MAX, SW_NST = G::NST;
-    constexpr int SWY_COLS = G::YCOLS, SWY_TILE = G::YTILE, NS = G::NS, NT = G::THREADS;
-    extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n % NS) * SW_TILE_MAX; };
-    double* fl = smem + NS * SW_TILE_MAX;  // [ISO ? 3 : 5][SW_TL * SW_W] face fluxes, indexed by face t
-    uint64_t* bar = reinterpret_cast<uint64_t*>(fl + (ISO ? 3 : 5) * SW_TL * SW_W);
+// advection.cu:1-173, marching like the azimuthal sweep.  The residual speed of a column
+// has one sign, so every cell feeds one face, the same of its two for the whole column:
+// with this row's flux and the last one's the update of this row (upwards) or of the
+// last (downwards) is complete.
+template <bool ISO>
+__global__ void __launch_bounds__(32 * SW_WARPS, 4)
+    k_advect(const Cell* __restrict__ in, const DiskView d, Cell* __restrict__ out, int ncol, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
+    pdl_enter();
     if (sc->done) return;
-    const int tid = threadIdx.x;
     const double dt = sc->dt;
-    constexpr int NFL = SW_TL * SW_W;
-    auto origin = [&](int tile, int& s0, int& q0) {
-        s0 = NPAD + SW_LEN * (tile % ntx);
-        q0 = NPAD + SW_W * (tile / ntx);
-    };
-    auto issue = [&](int tile, int k) {
-        int s0, q0;
-        origin(tile, s0, q0);
-        issue_begin(&bar[k % NS], SWY_TILE * 8);
-        issue_box(stage(k), &tm, 5 * (q0 - 1), s0 - NPAD, &bar[k % NS]);
-    };
-    pipe_init<NS>(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0)
-        for (int m = 0; m < NS - 1; ++m)
-            if ((int)blockIdx.x + m * (int)gridDim.x < ntiles) issue(blockIdx.x + m * gridDim.x, m);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-    int ahead = 0;
-    while (ahead < NS - 1 && tile_id + (ahead + 1) * (int)gridDim.x < ntiles) ++ahead;
-    if (tid == 0 && ahead == NS - 1) issue(tile_id + (NS - 1) * gridDim.x, kt + NS - 1);
-    int s0, q0;
-    origin(tile_id, s0, q0);
-    double* tile = stage(kt);
-    if (!pipe_wait<NS>(bar, kt, sc)) {
-        pipe_drain<NS>(bar, kt, ahead, sc);
-        return;
-    }
-
-    // ---- P1: upwind PPM average over the swept fraction (advection.cu:20-67)
-    for (int it = tid; it < SW_NST; it += NT) {
-        const int q = it % SW_W;
-        const int t = 2 + it / SW_W;
-        const int s = min(s0 - NPAD + t, d.yarr - 1);
-        const int i = min(q0 + q, d.xarr - 1);
-        const double speed = d.res[i];
-        const double sdt = dt * ((d.geomy == 3) ? d.irad[i] : 1.0);
-        const double* wt = d.wy + 6 * s;
-        const Frac x = frac(lesser(fabs(speed) * (sdt * d.idx_y[s]), 1.0));
-        const bool up = speed > 0.0;  // this cell is upwind of its upper face, else of its lower one
-        // average of field k of the cells over the swept part
-        const double* c0 = tile + ((t - 2) * SWY_COLS + (q + 1)) * 5;
-        auto ave = [&](int k) {
-            const double* c = c0 + k;
-            const Par A = recon(wt, c[0], c[5 * SWY_COLS], c[10 * SWY_COLS], c[15 * SWY_COLS], c[20 * SWY_COLS], 0.0);
-            return up ? aveR(x, A) : aveL(x, A);
-        };
-        const double fr = ave(0);
-        const double m = fr * speed;
-        double* o = fl + (t + (up ? 1 : 0)) * SW_W + q;
-        o[0] = m;
-        o[1 * NFL] = ave(2) * m;
-        o[2 * NFL] = ave(3) * m;
-        if (!ISO) {
-            o[3 * NFL] = d.ndim != 2 ? ave(4) * m : 0.0;
-            o[4 * NFL] = d.eos != 0 ? ave(1) * speed : 0.0;
-        }
-    }
-    __syncthreads();
-
-    // ---- P2: flux difference and update_Cell_advect (advection.cu:88-105, 153-170)
-    for (int it = tid; it < SW_LEN * SW_W; it += NT) {
-        const int q = it % SW_W;
-        const int t = 3 + it / SW_W;
-        const int s = s0 - NPAD + t;
-        const int i = q0 + q;
-        if (s < NPAD + d.yres && i < NPAD + d.xres) {
-            const double* f0 = fl + t * SW_W + q;
-            double f = dt * d.iyv[s];
-            if (d.geomy > 2) f *= d.irad[i];
-            auto net = [&](int k) { return (f0[k * NFL] - f0[k * NFL + SW_W]) * f; };
-            const double* c = tile + (t * SWY_COLS + (q + 1)) * 5;
-            Cell Q{c[0], c[1], c[2], c[3], c[4]};
-            const double r = Q.r + net(0);
-            const double ir = inv(r);
-            Q.u = (Q.u * Q.r + net(1)) * ir;
-            Q.v = (Q.v * Q.r + net(2)) * ir;
-            if (!ISO) {
-                Q.w = (Q.w * Q.r + net(3)) * ir;
-                Q.p += net(4);
+    for (int item = blockIdx.x * SW_WARPS + warp; item < nitems; item += gridDim.x * SW_WARPS) {
+        const int i = NPAD + 32 * (item % ncol) + lane;
+        const bool active = i < NPAD + d.xres;
+        const int ic = min(i, NPAD + d.xres - 1);
+        const int s0 = NPAD + len * (item / ncol), s1 = min(s0 + len, NPAD + d.yres);
+        const double speed = d.res[ic], cs2 = d.cs2x[ic];
+        const double sdt = dt * ((d.geomy == 3) ? d.irad[ic] : 1.0);
+        const double sx = fabs(speed) * sdt;
+        const bool up = speed > 0.0;
+        const size_t pitch = 5 * (size_t)d.xarr;
+        const double* next = reinterpret_cast<const double*>(in + ic) + pitch * (s0 - NPAD);
+        const Emitter emit_to(d, i);
+        double* o = cell_at(d, out, ic, up ? s0 - 1 : s0 - 2);  // the row updated at t = s0 - 1
+        double q[5][4], nx[4];
+#pragma unroll
+        for (int m = 0; m < 5; ++m, next += pitch) load4(next, q[m]);
+        double pm = 0.0, pu = 0.0, pv = 0.0, pp = 0.0;  // what the row before carries through its face
+#pragma unroll 1
+        for (int t = s0 - 1; t <= s1; ++t) {
+            if (t < s1) load4(next, nx);
+            next += pitch;
+            const double* w = d.wy + 6 * t;
+            const Frac x = frac(lesser(sx * d.idx_y[t], 1.0));
+            auto ave = [&](int m) {
+                const Par a = recon(w, q[0][m], q[1][m], q[2][m], q[3][m], q[4][m], 0.0);
+                return up ? aveR(x, a) : aveL(x, a);
+            };
+            const double fm = ave(0) * speed, fu = ave(2) * fm, fv = ave(3) * fm;
+            const double fp = (!ISO && d.eos != 0) ? ave(1) * speed : 0.0;
+            const int row = up ? t : t - 1;
+            if (active && row >= s0 && row < s1) {
+                const double f = sdt * d.iyv[row];
+                Cell Q{up ? q[2][0] : q[1][0], up ? q[2][1] : q[1][1], up ? q[2][2] : q[1][2], up ? q[2][3] : q[1][3],
+                       0.0};
+                const double r = Q.r + (pm - fm) * f;
+                const double ir = inv(r);
+                Q.u = (Q.u * Q.r + (pu - fu) * f) * ir;
+                Q.v = (Q.v * Q.r + (pv - fv) * f) * ir;
+                if (!ISO) Q.p += (pp - fp) * f;
+                Q.r = r;
+                if (ISO || d.eos == 0) Q.p = cs2 * r;
+                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+                emit_to(d, out, o, i, row, Q);
             }
-            Q.r = r;
-            if (ISO || d.eos == 0) Q.p = d.cs2x[i] * r;
-            if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-            emit(d, out, i, s, Q);
+            o += pitch;
+            pm = fm;
+            pu = fu;
+            pv = fv;
+            pp = fp;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+                q[0][m] = q[1][m];
+                q[1][m] = q[2][m];
+                q[2][m] = q[3][m];
+                q[3][m] = q[4][m];
+                q[4][m] = nx[m];
+            }
         }
-    }
-    __syncthreads();
     }
 }
 
-// ====================================================== kick 1 (+ stress)
-// 4 CTAs per SM (64 registers, a few bytes of spills with the stress): 32 warps
-// hide the table and tile loads better than 24 (0.120 -> 0.106 ms)
+// ================================================================== kicks
+// Both half-kicks march along the rows like the azimuthal passes, lanes along the
+// radius with one halo cell a side (30 outputs of 32): a row is loaded, predicted
+// (kick 2) and exchanged with the neighbouring lanes once and stays in registers while
+// it is the upper, the middle and the lower row of the 3 x 3 stress stencil.  The
+// 32 x 8 tiles they replace predicted 340 cells for 256 outputs in two rounds and
+// spent 460 (kick 1) and 880 (kick 2) instructions a cell, mostly on table loads and
+// shared-memory addresses.
+struct Column {  // the per-radius factors of a lane
+    int i, ic;   // cell index, and clamped to the array for loads
+    double rad, irad, gstar, nu;
+    bool inside, output;
+};
+__device__ __forceinline__ Column column(const DiskView& d, int seg, int lane) {
+    Column c;
+    c.i = NPAD - 1 + KK_OUT * seg + lane;
+    c.ic = min(c.i, d.xarr - 1);
+    c.inside = c.i >= NPAD && c.i < NPAD + d.xres;
+    c.output = c.inside && lane >= 1 && lane <= KK_OUT;
+    c.rad = d.radx[c.ic];
+    c.irad = d.irad[c.ic];
+    c.gstar = d.geomx == 1 ? d.gstar[c.ic] : 0.0;
+    c.nu = d.nux[c.ic];
+    return c;
+}
+__device__ __forceinline__ Grav row_gravity(const DiskView& d, const Column& c, int j, int which, const pg_body& pl,
+                                            const pg_body& st) {
+    if (d.twobd) return body_gravity(d, c.ic, j, which, pl, st);
+    const double* tr = d.trig + 4 * j + 2 * which;
+    return gravity_at(d, c.gstar, c.rad, tr[0], tr[1], d.trig[4 * d.yarr + which], pl);
+}
+// u and v of one row at the lane's column and its two neighbours'
+struct Row3 {
+    double u[3], v[3], nr;  // left, own, right; own density times viscosity
+};
+__device__ __forceinline__ Row3 row3(double u, double v, double nr) {
+    return Row3{{up1(u), u, down1(u)}, {up1(v), v, down1(v)}, nr};
+}
+// viscous force of the middle of three rows (viscous' stencil order: middle, lower, upper)
+__device__ __forceinline__ void row_stress(const DiskView& d, const Column& c, int j, const Row3& lo, const Row3& mid,
+                                           const Row3& hi, double& vx, double& vy) {
+    const double u[9] = {mid.u[0], mid.u[1], mid.u[2], lo.u[0], lo.u[1], lo.u[2], hi.u[0], hi.u[1], hi.u[2]};
+    const double v[9] = {mid.v[0], mid.v[1], mid.v[2], lo.v[0], lo.v[1], lo.v[2], hi.v[0], hi.v[1], hi.v[2]};
+    const double nr[9] = {up1(mid.nr), mid.nr, down1(mid.nr), 0.0, lo.nr, 0.0, 0.0, hi.nr, 0.0};
+    viscous(d.visx + 5 * c.ic, d.visy + 4 * j, u, v, nr, vx, vy);
+}
+
 template <bool VISC>
-__global__ void __launch_bounds__(ST_THREADS, 4)
-    k_kick1(const __grid_constant__ CUtensorMap tm, const DiskView d, Cell* __restrict__ out,
-            double* __restrict__ vis, int ntx, int ntiles, const pg_dust* __restrict__ din,
-            pg_dust* __restrict__ dout) {
-    extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n & 1) * ST_TILE; };
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * ST_TILE);
+__global__ void __launch_bounds__(32 * SW_WARPS, 4)
+    k_kick1(const Cell* __restrict__ in, const DiskView d, Cell* __restrict__ out, double* __restrict__ vis,
+            const pg_dust* __restrict__ din, pg_dust* __restrict__ dout, int nseg, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
+    pdl_enter();
     if (sc->done) return;
-    const int tid = threadIdx.x;
     const double hdt = 0.5 * sc->dt;
-    auto origin = [&](int tile, int& i0, int& j0) {
-        i0 = NPAD + ST_TX * (tile % ntx);
-        j0 = d.ypad + ST_TY * (tile / ntx);
-    };
-    auto issue = [&](int tile, int k) {
-        int i0, j0;
-        origin(tile, i0, j0);
-        issue_begin(&bar[k & 1], ST_TILE_N * 8);
-        issue_box(stage(k), &tm, 5 * (i0 - 1), j0 - 1, &bar[k & 1]);
-    };
-    pipe_init(bar);
-    if ((int)blockIdx.x >= ntiles) return;
-    if (tid == 0) issue(blockIdx.x, 0);
-    int kt = 0;
-    for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-        if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-        int i0, j0;
-        origin(tile_id, i0, j0);
-        const double* tile = stage(kt);
-        if (!pipe_wait(bar, kt, sc)) {
-        pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-        return;
-    }
-        const int hx = 1 + tid % ST_TX, hy = 1 + tid / ST_TX;
-        const int i = i0 + hx - 1, j = j0 + hy - 1;
-        if (i < NPAD + d.xres && j < d.ypad + d.yres) {
-            const double* c = tile + (hy * ST_HX + hx) * 5;
-            const Cell C{c[0], c[1], c[2], c[3], c[4]};
+    const pg_body pl = sc->planet_cur, star = sc->star_cur;
+    const size_t pitch = 5 * (size_t)d.xarr;
+    for (int item = blockIdx.x * SW_WARPS + warp; item < nitems; item += gridDim.x * SW_WARPS) {
+        const Column c = column(d, item % nseg, lane);
+        const int j0 = d.ypad + len * (item / nseg), j1 = min(j0 + len, d.ypad + d.yres);
+        const double* next = reinterpret_cast<const double*>(in + c.ic) + pitch * (VISC ? j0 - 1 : j0);
+        const Emitter emit_to(d, c.i);
+        double* o = cell_at(d, out, c.ic, j0);
+        double q[4], up[4], nx[4];  // the middle row, the one above and the next in flight: r, p, v_r, v_phi
+        Row3 lo{}, mid{}, hi{};
+        int jl = VISC ? j0 - 1 : j0;             // the next row to load, and the last one
+        const int jlast = VISC ? j1 : j1 - 1;
+        auto fetch = [&]() {
+            if (jl <= jlast) load4(next, nx);
+            next += pitch;
+            ++jl;
+        };
+        auto enter = [&]() {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) up[m] = nx[m];
+            fetch();
+            if (VISC) hi = row3(up[2], up[3], up[0] * c.nu);
+        };
+        fetch();
+        if (VISC) {
+            enter();
+            mid = hi;
+        }
+        enter();
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) q[m] = up[m];
+            const Grav g = row_gravity(d, c, j, 0, pl, star);
             double vx = 0.0, vy = 0.0;
             if (VISC) {
-                double nu[3], u[9], v[9], nr[9];
-#pragma unroll
-                for (int n = 0; n < 3; ++n) nu[n] = d.nux[i + n - 1];
-                gather9(tile, hx, hy, nu, u, v, nr);
-                viscous(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, vx, vy);
-                // the stress is kept for the predictor of kick2, with its periodic images
-                const size_t m0 = (size_t)i + (size_t)d.xarr * j;
-                vis[2 * m0] = vx;
-                vis[2 * m0 + 1] = vy;
-                int jimg = -1;
-                if (j < 2 * NPAD) jimg = j + d.yres;
-                else if (j >= d.yres) jimg = j - d.yres;
-                if (jimg >= 0) {
-                    const size_t m = (size_t)i + (size_t)d.xarr * jimg;
-                    vis[2 * m] = vx;
-                    vis[2 * m + 1] = vy;
-                }
+                lo = mid;
+                mid = hi;
             }
-            const Grav g = body_gravity(d, i, j, 0, sc->planet_cur, sc->star_cur);
-            Cell Q = kick<VISC>(d, C, d.irad[i], g, vx, vy, 0.0, hdt);
-            if (d.cool) Q.p = p_cool(d, i, C.p, C.r, hdt);  // sweeps.cu:695-699
-            emit(d, out, i, j, Q);
-            if (d.ave) accumulate_average(d, i, j, C, hdt);  // averaging(dev, 0.5 dt, T) before solve
+            enter();
+            if (VISC) {
+                row_stress(d, c, j, lo, mid, hi, vx, vy);
+            }
+            double* const oj = o;
+            o += pitch;
+            if (!c.output) continue;
+            if (VISC) {
+                // the stress is kept for the predictor of kick2, with its periodic images
+                double2* s = reinterpret_cast<double2*>(vis) + (size_t)c.i + (size_t)d.xarr * j;
+                *s = double2{vx, vy};
+                if (j < 2 * NPAD) s[(size_t)d.xarr * d.yres] = double2{vx, vy};
+                else if (j >= d.yres) *(s - (size_t)d.xarr * d.yres) = double2{vx, vy};
+            }
+            const Cell C{q[0], q[1], q[2], q[3], 0.0};
+            Cell Q = kick<VISC>(d, C, c.irad, g, vx, vy, 0.0, hdt);
+            if (d.cool) Q.p = p_cool(d, c.i, C.p, C.r, hdt);  // sweeps.cu:695-699
+            emit_to(d, out, oj, c.i, j, Q);
+            if (d.ave) accumulate_average(d, c.i, j, C, hdt);  // averaging(dev, 0.5 dt, T) before solve
             if (din) {  // dust half-kick: drag towards the gas cell C (sweeps.cu:626-707, mdt = 0)
-                const DCell D = dust_kick(d, C, C.u, C.v, C.p, load_dust(din, d.xarr, i, j), g.gx, g.gy, g.gz,
-                                          d.irad[i], 0.0, hdt);
-                emit_dust(d, dout, i, j, D);
+                const DCell D = dust_kick(d, C, C.u, C.v, C.p, load_dust(din, d.xarr, c.i, j), g.gx, g.gy, g.gz,
+                                          c.irad, 0.0, hdt);
+                emit_dust(d, dout, c.i, j, D);
             }
         }
-        __syncthreads();
     }
 }
 
-// ============================================ kick 2 + damping + CFL speed
-// 3 CTAs per SM (80 registers, no spills; 65 KB of shared memory each): the
-// pass waits on table and tile loads, and 24 warps per SM hide them better than
-// the 16 its natural 102 registers allow (0.222 -> 0.181 ms on the 1024x3072 disk)
+// Kick 2 with damping and the CFL rate.  A row is predicted (sweeps.cu:713-729 with
+// mdt = dt = dt/2) when it enters, with kick 1's stress and the bodies at t + dt; the
+// corrector re-uses its gravity.
 template <bool VISC>
-__global__ void __launch_bounds__(ST_THREADS, 3)
-    k_kick2(const __grid_constant__ CUtensorMap tm, const __grid_constant__ CUtensorMap tv, const DiskView d,
-            Cell* __restrict__ out, int ntx, int ntiles, const pg_dust* __restrict__ din,
-            pg_dust* __restrict__ dout) {
-    extern __shared__ __align__(128) double smem_raw[];
-    double* smem = smem_base128(smem_raw);
-    auto stage = [&](int n) { return smem + (n & 1) * ST_TILE; };                   // C with 1 halo
-    auto vstage = [&](int n) { return smem + 2 * ST_TILE + (n & 1) * ST_VIS; };  // stress of the first evaluation
-    double* tp = smem + 2 * ST_TILE + 2 * ST_VIS;                      // predicted state with 1 halo
-    double* gc = tp + ST_TILE;  // gravity at the predictor's cells: the corrector's is the same (time `next`)
-    double* tb = gc + ST_GRAV;  // the tile's tables: [KR_N][ST_HX] per radius, then [KY_N][ST_HY] per row
-    double* ty = tb + KR_N * ST_HX;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(tb + ST_TAB);
+__global__ void __launch_bounds__(32 * SW_WARPS, 3)
+    k_kick2(const Cell* __restrict__ in, const double* __restrict__ vis, const DiskView d, Cell* __restrict__ out,
+            const pg_dust* __restrict__ din, pg_dust* __restrict__ dout, int nseg, int len, int nitems) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
+    pdl_enter();
     if (sc->done) return;
-    const int tid = threadIdx.x;
     const double dt = sc->dt, hdt = 0.5 * dt;
-    const pg_body pl = sc->planet_next;
-    const pg_body st = sc->star_next;
-    // the disk's gravity comes from the staged tables; the two-body frame reads its own
-    const bool disk_grav = !d.twobd;
-    const double iplx2 = disk_grav ? d.trig[4 * d.yarr + 1] : 0.0;
-    auto origin = [&](int tile, int& i0, int& j0) {
-        i0 = NPAD + ST_TX * (tile % ntx);
-        j0 = d.ypad + ST_TY * (tile / ntx);
-    };
-    // Per-radius and per-row table entries of the tile and its halo, read once per
-    // tile (coalesced) instead of once per cell: the pass is bound by the latency of
-    // those loads.  Indices past the grid are clamped; those cells are not used.
-    auto stage_tables = [&](int i0, int j0) {
-        for (int it = tid; it < KR_N * ST_HX; it += ST_THREADS) {
-            const int f = it / ST_HX, hx = it % ST_HX;
-            const int i = min(max(i0 - 1 + hx, 0), d.xarr - 1);
-            double v = 0.0;
-            if (f == KR_RAD) v = d.radx[i];
-            else if (f == KR_IRAD) v = d.irad[i];
-            else if (f == KR_GSTAR) v = d.geomx == 1 ? d.gstar[i] : 0.0;
-            else if (f == KR_NU) v = VISC ? d.nux[i] : 0.0;
-            else if (f == KR_IDX) v = d.idx_x[i];
-            else if (f == KR_ROT) v = d.ndim > 1 ? d.rot[i] : 0.0;
-            else if (f < KR_KILL) v = VISC ? d.visx[5 * i + (f - KR_VX)] : 0.0;
-            else v = d.kill ? d.killx[4 * i + (f - KR_KILL)] : 0.0;
-            tb[it] = v;
-        }
-        for (int it = tid; it < KY_N * ST_HY; it += ST_THREADS) {
-            const int f = it / ST_HY, hy = it % ST_HY;
-            const int j = min(max(j0 - 1 + hy, 0), d.yarr - 1);  // 1D: one row, no ghost rows
-            double v = 0.0;
-            if (f == KY_SIN) v = disk_grav ? d.trig[4 * j + 2] : 0.0;
-            else if (f == KY_COS) v = disk_grav ? d.trig[4 * j + 3] : 0.0;
-            else if (f == KY_IDY) v = d.ndim > 1 ? d.idx_y[j] : 0.0;
-            else v = VISC ? d.visy[4 * j + (f - KY_VY)] : 0.0;
-            ty[it] = v;
-        }
-    };
-    // gravity at tile cell (hx, hy), bodies at t + dt
-    auto grav = [&](int hx, int hy, int i, int j) {
-        if (disk_grav)
-            return gravity_at(d, tb[KR_GSTAR * ST_HX + hx], tb[KR_RAD * ST_HX + hx], ty[KY_SIN * ST_HY + hy],
-                              ty[KY_COS * ST_HY + hy], iplx2, pl);
-        return body_gravity(d, i, j, 1, pl, st);
-    };
-    auto issue = [&](int tile, int k) {
-        int i0, j0;
-        origin(tile, i0, j0);
-        issue_begin(&bar[k & 1], (ST_TILE_N + (VISC ? ST_VIS_N : 0)) * 8);
-        issue_box(stage(k), &tm, 5 * (i0 - 1), j0 - 1, &bar[k & 1]);
-        if (VISC) issue_box(vstage(k), &tv, 2 * (i0 - 1), j0 - 1, &bar[k & 1]);
-    };
-    pipe_init(bar);
+    const pg_body pl = sc->planet_next, star = sc->star_next;
+    const size_t pitch = 5 * (size_t)d.xarr;
     double vmax = 0.0;
-    if ((int)blockIdx.x < ntiles) {
-        if (tid == 0) issue(blockIdx.x, 0);
-        int kt = 0;
-        for (int tile_id = blockIdx.x; tile_id < ntiles; tile_id += gridDim.x, ++kt) {
-            if (tid == 0 && tile_id + (int)gridDim.x < ntiles) issue(tile_id + gridDim.x, kt + 1);
-            int i0, j0;
-            origin(tile_id, i0, j0);
-            const double* tile = stage(kt);
-            const double* tvis = vstage(kt);
-            stage_tables(i0, j0);  // while the tile's copy is in flight
-            __syncthreads();
-            if (!pipe_wait(bar, kt, sc)) {
-        pipe_drain(bar, kt, tile_id + (int)gridDim.x < ntiles, sc);
-        return;
-    }
-
+    for (int item = blockIdx.x * SW_WARPS + warp; item < nitems; item += gridDim.x * SW_WARPS) {
+        const Column c = column(d, item % nseg, lane);
+        const int j0 = d.ypad + len * (item / nseg), j1 = min(j0 + len, d.ypad + d.yres);
+        int jn = VISC ? j0 - 1 : j0;  // the next row to enter
+        const double* next = reinterpret_cast<const double*>(in + c.ic) + pitch * jn;
+        const double2* nvis = reinterpret_cast<const double2*>(vis) + (size_t)c.ic + (size_t)d.xarr * jn;
+        const Emitter emit_to(d, c.i);
+        double* o = cell_at(d, out, c.ic, j0);
+        const int jlast = VISC ? j1 : j1 - 1;
+        double q[4], up[4], nx[4];  // the middle row, the one above, the next in flight (with its stress)
+        double2 nf{0.0, 0.0};
+        auto fetch = [&](int j) {
+            if (j <= jlast) {
+                load4(next, nx);
+                if (VISC) nf = *nvis;
+            }
+            next += pitch;
+            nvis += d.xarr;
+        };
+        Grav g{}, gup{};
+        Row3 lo{}, mid{}, hi{};
+        auto enter = [&]() {  // row jn into `up`, its prediction into `hi`
+#pragma unroll
+            for (int m = 0; m < 4; ++m) up[m] = nx[m];
+            const double2 f = nf;
+            fetch(jn + 1);
+            gup = row_gravity(d, c, jn, 1, pl, star);
+            ++jn;
+            if (!VISC) return;
+            double u = up[2], v = up[3];
+            if (c.inside) {
+                const Cell P = kick<true>(d, Cell{up[0], up[1], u, v, 0.0}, c.irad, gup, f.x, f.y, hdt, hdt);
+                u = P.u;
+                v = P.v;
+            }
+            // radial ghosts of the predicted state (boundx2, src/boundary/boundary.cu:722-820): bound 0
+            // keeps the analytic state; a copy or a reflection of the edge cell otherwise
+            if (d.bound_lft != 0) {
+                const double a = down1(u), b = down1(v);
+                if (c.i == NPAD - 1) {
+                    u = d.bound_lft == 2 ? -a : a;
+                    v = b;
+                }
+            }
+            if (d.bound_rgh != 0) {
+                const double a = up1(u), b = up1(v);
+                if (c.i == NPAD + d.xres) {
+                    u = d.bound_rgh == 2 ? -a : a;
+                    v = b;
+                }
+            }
+            hi = row3(u, v, up[0] * c.nu);
+        };
+        fetch(jn);
+        enter();
+        if (VISC) {
+            mid = hi;
+            enter();
+        }
+#pragma unroll 1
+        for (int j = j0; j < j1; ++j) {
+#pragma unroll
+            for (int m = 0; m < 4; ++m) q[m] = up[m];
+            g = gup;
+            double vx = 0.0, vy = 0.0;
             if (VISC) {
-                // predictor (sweeps.cu:713-729 with mdt = dt = dt/2) on the tile and its halo
-                for (int it = tid; it < ST_HX * ST_HY; it += ST_THREADS) {
-                    const int hx = it % ST_HX, hy = it / ST_HX;
-                    const int i = i0 - 1 + hx, j = j0 - 1 + hy;
-                    if (i < NPAD || i >= NPAD + d.xres || j < 0 || j >= d.yarr) continue;
-                    const double* c = tile + it * 5;
-                    const Cell C{c[0], c[1], c[2], c[3], c[4]};
-                    const Grav g = grav(hx, hy, i, j);
-                    gc[3 * it] = g.gx;
-                    gc[3 * it + 1] = g.gy;
-                    gc[3 * it + 2] = g.gz;
-                    const Cell Q = kick<true>(d, C, tb[KR_IRAD * ST_HX + hx], g, tvis[2 * it], tvis[2 * it + 1], hdt,
-                                              hdt);
-                    double* o = tp + it * 5;
-                    o[0] = Q.r; o[1] = Q.p; o[2] = Q.u; o[3] = Q.v; o[4] = Q.w;
-                }
-                __syncthreads();
-                // radial ghosts of the predicted state (boundx2, src/boundary/boundary.cu:722-820):
-                // the stencil only reaches the innermost ghost column on either side, which
-                // only tiles at the radial edges hold (a CTA-uniform test, so the barrier
-                // below is skipped by all threads or none)
-                const bool redge = i0 - 1 <= NPAD - 1 || i0 - 2 + ST_HX >= NPAD + d.xres;
-                if (redge) {
-                for (int it = tid; it < ST_HX * ST_HY; it += ST_THREADS) {
-                    const int hx = it % ST_HX, hy = it / ST_HX;
-                    const int i = i0 - 1 + hx;
-                    const int side = (i == NPAD - 1) ? 0 : ((i == NPAD + d.xres) ? 1 : -1);
-                    if (side < 0) continue;
-                    const int bnd = side == 0 ? d.bound_lft : d.bound_rgh;
-                    double* o = tp + (hy * ST_HX + hx) * 5;
-                    const double* src;
-                    if (bnd == 0) src = tile + (hy * ST_HX + hx) * 5;  // constant analytic state
-                    else {
-                        // the adjacent interior cell is both the copy and the reflection source
-                        const int hs = side == 0 ? hx + 1 : hx - 1;
-                        src = tp + (hy * ST_HX + hs) * 5;
-                    }
-                    o[0] = src[0]; o[1] = src[1]; o[2] = src[2]; o[3] = src[3]; o[4] = src[4];
-                    if (bnd == 2) o[2] = -o[2];
-                }
-                __syncthreads();
-                }
+                lo = mid;
+                mid = hi;
+                enter();
+                row_stress(d, c, j, lo, mid, hi, vx, vy);
+            } else {
+                enter();
             }
-
-            const int hx = 1 + tid % ST_TX, hy = 1 + tid / ST_TX;
-            const int i = i0 + hx - 1, j = j0 + hy - 1;
-            if (i < NPAD + d.xres && j < d.ypad + d.yres) {
-                const double* c = tile + (hy * ST_HX + hx) * 5;
-                const Cell C{c[0], c[1], c[2], c[3], c[4]};
-                double vx = 0.0, vy = 0.0;
-                const double irad = tb[KR_IRAD * ST_HX + hx];
-                if (VISC) {
-                    double nu[3], u[9], v[9], nr[9], X[5], Y[4];
+            double* const oj = o;
+            o += pitch;
+            if (!c.output) continue;
+            const int i = c.i;
+            const Cell C{q[0], q[1], q[2], q[3], 0.0};
+            double Tu = C.u, Tv = C.v;
+            Cell Q = kick<VISC>(d, C, c.irad, g, vx, vy, hdt, hdt, &Tu, &Tv);
+            // cooling over dt/2; the predictor cools over mdt = dt/2 as well, so Q.p is also
+            // the predicted pressure the dust's second stopping time reads (sweeps.cu:668-699)
+            if (d.cool) Q.p = p_cool(d, i, C.p, C.r, hdt);
+            const double Tp = Q.p;
+            if (d.kill) {
+                // killwave (src/killwave/killwave.cu:48-100): relax towards init_C
+                const double* I = d.initx + 5 * i;
 #pragma unroll
-                    for (int n = 0; n < 3; ++n) nu[n] = tb[KR_NU * ST_HX + hx + n - 1];
-#pragma unroll
-                    for (int n = 0; n < 5; ++n) X[n] = tb[(KR_VX + n) * ST_HX + hx];
-#pragma unroll
-                    for (int n = 0; n < 4; ++n) Y[n] = ty[(KY_VY + n) * ST_HY + hy];
-                    gather9(tp, hx, hy, nu, u, v, nr);
-                    viscous(X, Y, u, v, nr, vx, vy);
-                }
-                const int ic = 3 * (hy * ST_HX + hx);
-                const Grav g = VISC ? Grav{gc[ic], gc[ic + 1], gc[ic + 2]} : grav(hx, hy, i, j);
-                double Tu = C.u, Tv = C.v;
-                Cell Q = kick<VISC>(d, C, irad, g, vx, vy, hdt, hdt, &Tu, &Tv);
-                // cooling over dt/2; the predictor cools over mdt = dt/2 as well, so Q.p is also
-                // the predicted pressure the dust's second stopping time reads (sweeps.cu:668-699)
-                if (d.cool) Q.p = p_cool(d, i, C.p, C.r, hdt);
-                const double Tp = Q.p;
-                if (d.kill) {
-                    // killwave (src/killwave/killwave.cu:48-100): relax towards init_C
-                    const double* I = d.initx + 5 * i;
-#pragma unroll
-                    for (int side = 0; side < 2; ++side) {
-                        const double tau = tb[(KR_KILL + 2 * side + 1) * ST_HX + hx];
-                        if (tau > 0.0) {
-                            double f = tb[(KR_KILL + 2 * side) * ST_HX + hx];
-                            f *= dt / tau;
-                            Q.r += f * (I[0] - Q.r);
-                            Q.p += f * (I[1] - Q.p);
-                            Q.u += f * (I[2] - Q.u);
-                            Q.v += f * (I[3] - Q.v);
-                            Q.w += f * (I[4] - Q.w);
-                        }
+                for (int side = 0; side < 2; ++side) {
+                    const double tau = d.killx[4 * i + 2 * side + 1];
+                    if (tau > 0.0) {
+                        const double f = d.killx[4 * i + 2 * side] * (dt / tau);
+                        Q.r += f * (I[0] - Q.r);
+                        Q.p += f * (I[1] - Q.p);
+                        Q.u += f * (I[2] - Q.u);
+                        Q.v += f * (I[3] - Q.v);
                     }
                 }
-                if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-                if (din) {  // dust corrector half-kick towards the predicted gas velocity (sweeps.cu:663-707)
-                    const DCell D = dust_kick(d, C, Tu, Tv, Tp, load_dust(din, d.xarr, i, j), g.gx, g.gy, g.gz,
-                                              irad, hdt, hdt);
-                    emit_dust(d, dout, i, j, D);
-                    vmax = fmax(vmax, signal_rate_at(d, Q, tb[KR_RAD * ST_HX + hx], tb[KR_IDX * ST_HX + hx],
-                                                     tb[KR_ROT * ST_HX + hx], ty[KY_IDY * ST_HY + hy], irad, &D));
-                } else {
-                    vmax = fmax(vmax, signal_rate_at(d, Q, tb[KR_RAD * ST_HX + hx], tb[KR_IDX * ST_HX + hx],
-                                                     tb[KR_ROT * ST_HX + hx], ty[KY_IDY * ST_HY + hy], irad));
-                }
-                emit(d, out, i, j, Q);
-                if (d.ave) accumulate_average(d, i, j, Q, hdt);  // ... and after it
             }
-            __syncthreads();
+            if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
+            if (din) {  // dust corrector half-kick towards the predicted gas velocity (sweeps.cu:663-707)
+                const DCell D = dust_kick(d, C, Tu, Tv, Tp, load_dust(din, d.xarr, i, j), g.gx, g.gy, g.gz, c.irad,
+                                          hdt, hdt);
+                emit_dust(d, dout, i, j, D);
+                vmax = fmax(vmax, signal_rate(d, Q, i, j, &D));
+            } else {
+                vmax = fmax(vmax, signal_rate(d, Q, i, j));
+            }
+            emit_to(d, out, oj, i, j, Q);
+            if (d.ave) accumulate_average(d, i, j, Q, hdt);  // ... and after it
         }
     }
-    block_max_to<ST_THREADS>(&sc->vmax_bits, vmax);
+    block_max_to<32 * SW_WARPS>(&sc->vmax_bits, vmax);
 }
 
 // ================================================================ misc
@@ -892,22 +795,60 @@ __global__ void k_run_begin(Scalars* sc, double end_time, int fresh) {
     sc->pad_ = 0;
 }
 
+// Per row, sin and cos of (azimuth - planet angle) for the planet of the first
+// half-kick and for the planet at t+dt, and 1/x_p^2 of both (forces.cu:41-58).  By the
+// one block whose first thread has just set the clock: as a launch of its own the table
+// cost a step of the 126x389 disk 2 us.
+__device__ __forceinline__ void planet_rows(const DiskView& d) {
+    __syncthreads();
+    const Scalars* sc = d.sc;
+    const pg_body& a = sc->planet_cur;
+    const pg_body& b = sc->planet_next;
+    const double ya = a.y + 0.0 * a.vy, yb = b.y + 0.0 * b.vy;
+    for (int j = threadIdx.x; j < d.yarr; j += blockDim.x) {
+        double* t = d.trig + 4 * j;
+        sincos(d.ycj[j] - ya, &t[0], &t[1]);
+        sincos(d.ycj[j] - yb, &t[2], &t[3]);
+        if (d.twobd) {
+            double* u = d.strig + 4 * j;
+            sincos(d.ycj[j] - (sc->star_cur.y + 0.0 * sc->star_cur.vy), &u[0], &u[1]);
+            sincos(d.ycj[j] - (sc->star_next.y + 0.0 * sc->star_next.vy), &u[2], &u[3]);
+        }
+    }
+    if (threadIdx.x == 0) {
+        d.trig[4 * d.yarr] = 1.0 / a.x / a.x;
+        d.trig[4 * d.yarr + 1] = 1.0 / b.x / b.x;
+    }
+}
+
 // Host-supplied t, dt (pg_*_solve): planet for this step, reset of the signal-speed max.
-__global__ void k_set_time(const DiskView d, double t, double dt) {
-    Scalars* sc = d.sc;
-    sc->done = 0;
-    sc->dt = dt;
-    sc->planet_cur = sc->planet_next;
-    sc->star_cur = sc->star_next;
-    evolve_bodies(d, sc, t + dt);  // evolve_planet (solve.cu:264)
-    sc->t = t + dt;
-    sc->dt_prev = dt;
-    sc->vmax_bits = 0ull;
-    sc->steps += 1;
+__global__ void __launch_bounds__(1024) k_set_time(const DiskView d, double t, double dt, pg_body* planets) {
+    pdl_enter();
+    if (threadIdx.x == 0) {
+        Scalars* sc = d.sc;
+        sc->done = 0;
+        sc->dt = dt;
+        sc->planet_cur = sc->planet_next;
+        sc->star_cur = sc->star_next;
+        evolve_bodies(d, sc, t + dt);  // evolve_planet (solve.cu:264)
+        sc->t = t + dt;
+        sc->dt_prev = dt;
+        sc->vmax_bits = 0ull;
+        sc->steps += 1;
+        if (planets) {  // recorded for the adjoint
+            planets[0] = sc->planet_cur;
+            planets[1] = sc->planet_next;
+        }
+    }
+    planet_rows(d);
 }
 
 // Device-resident loop step of one disk (advance_clock).
-__global__ void k_time_step(const DiskView d) { advance_clock(d); }
+__global__ void __launch_bounds__(1024) k_time_step(const DiskView d) {
+    pdl_enter();
+    if (threadIdx.x == 0) advance_clock(d);
+    planet_rows(d);
+}
 
 __global__ void k_init_planet(const DiskView d, double a, double e, double rs, double t) {
     // init_planet (src/planet/planet.cu:319-402): one planet, or the star-planet
@@ -1045,30 +986,8 @@ __global__ void k_init_tables(const DiskView d, TabArgs a, double* radx, double*
     }
 }
 
-// Per row, sin and cos of (azimuth - planet angle) for the planet of the first
-// half-kick and for the planet at t+dt, and 1/x_p^2 of both (forces.cu:41-58).
-__global__ void k_planet_trig(const DiskView d) {
-    const Scalars* sc = d.sc;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const pg_body& a = sc->planet_cur;
-    const pg_body& b = sc->planet_next;
-    if (j < d.yarr) {
-        double* t = d.trig + 4 * j;
-        sincos(d.ycj[j] - (a.y + 0.0 * a.vy), &t[0], &t[1]);
-        sincos(d.ycj[j] - (b.y + 0.0 * b.vy), &t[2], &t[3]);
-        if (d.twobd) {
-            double* u = d.strig + 4 * j;
-            sincos(d.ycj[j] - (sc->star_cur.y + 0.0 * sc->star_cur.vy), &u[0], &u[1]);
-            sincos(d.ycj[j] - (sc->star_next.y + 0.0 * sc->star_next.vy), &u[2], &u[3]);
-        }
-    }
-    if (j == 0) {
-        d.trig[4 * d.yarr] = 1.0 / a.x / a.x;
-        d.trig[4 * d.yarr + 1] = 1.0 / b.x / b.x;
-    }
-}
-
-// Bound-0 radial ghosts hold init_C (src/boundary/boundary.cu:30-33, 56-59) in every row.
+// Bound-0 radial ghosts hold init_C (src/boundary/boundary.cu:30-33, 56-59) in every
+// row, of blockIdx.y consecutive buffers.
 __global__ void k_init_xghosts(const DiskView d, Cell* buf) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= 2 * NPAD * d.yarr) return;
@@ -1078,7 +997,7 @@ __global__ void k_init_xghosts(const DiskView d, Cell* buf) {
     const int bnd = n < NPAD ? d.bound_lft : d.bound_rgh;
     if (bnd != 0) return;
     const double* I = d.initx + 5 * i;
-    store_cell(buf, d.xarr, i, j, Cell{I[0], I[1], I[2], I[3], I[4]});
+    store_cell(buf + (size_t)blockIdx.y * d.xarr * d.yarr, d.xarr, i, j, Cell{I[0], I[1], I[2], I[3], I[4]});
 }
 
 // boundy then boundx (src/boundary/boundary.cu:141-209, 13-62) on one buffer.
@@ -1156,31 +1075,8 @@ cudaError_t set_kernel_attributes() {
         r = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         if (r != cudaSuccess) e = r;
     };
-    auto set_v = [&](auto tag) {
-        using G = typename decltype(tag)::G;
-        if constexpr (G::X_OK) {
-            set((const void*)k_sweep<0, G, true>, G::template smem<true>());
-            set((const void*)k_sweep<0, G, false>, G::template smem<false>());
-        }
-        set((const void*)k_sweep<1, G, true>, G::template smem<true>());
-        set((const void*)k_sweep<1, G, false>, G::template smem<false>());
-        set((const void*)k_advect<G, true>, G::template ad_smem<true>());
-        set((const void*)k_advect<G, false>, G::template ad_smem<false>());
-    };
-    set_v(SV<0>{});
-    set_v(SV<1>{});
-    set_v(SV<2>{});
-    set_v(SV<3>{});
-    set_v(SV<4>{});
-    set_v(SV<5>{});
-    set_v(SV<6>{});
-    set_v(SV<7>{});
-    set_v(SV<8>{});
-    set_v(SV<9>{});
-    set((const void*)k_kick1<true>, K1_SMEM);
-    set((const void*)k_kick1<false>, K1_SMEM);
-    set((const void*)k_kick2<true>, K5_SMEM);
-    set((const void*)k_kick2<false>, K5_SMEM);
+    set((const void*)k_sweep_x<true>, RX_SMEM);
+    set((const void*)k_sweep_x<false>, RX_SMEM);
     return e;
 }
 
@@ -1207,8 +1103,8 @@ void launch_torque(const DiskView& d, const Cell* buf, double* part, int nblocks
     k_torque<<<nblocks, 256, 0, s>>>(d, buf, part);
 }
 
-void launch_init_xghosts(const DiskView& d, Cell* buf, cudaStream_t s) {
-    k_init_xghosts<<<cdiv(2 * NPAD * d.yarr, 256), 256, 0, s>>>(d, buf);
+void launch_init_xghosts(const DiskView& d, Cell* buf, cudaStream_t s, int nbuf) {
+    k_init_xghosts<<<dim3(cdiv(2 * NPAD * d.yarr, 256), nbuf), 256, 0, s>>>(d, buf);
 }
 
 void launch_bound(const DiskView& d, Cell* buf, cudaStream_t s) {
@@ -1224,23 +1120,17 @@ void launch_cfl(const DiskView& d, const Cell* buf, cudaStream_t s, const pg_dus
     k_cfl<<<blocks, 256, 0, s>>>(d, buf, dbuf);
 }
 
-void launch_set_time(const DiskView& d, double t, double dt, cudaStream_t s) {
-    launch_set_time_only(d, t, dt, s);
-    launch_planet_trig(d, s);
-}
-void launch_set_time_only(const DiskView& d, double t, double dt, cudaStream_t s) {
-    k_set_time<<<1, 1, 0, s>>>(d, t, dt);
-}
-void launch_planet_trig(const DiskView& d, cudaStream_t s) {
-    k_planet_trig<<<cdiv(d.yarr, 256), 256, 0, s>>>(d);
+// threads of the clock's block: up to 1024, the rows of the planet table
+static unsigned clock_threads(const DiskView& d) { return d.yarr < 1024 ? (unsigned)(d.yarr + 31) / 32 * 32 : 1024; }
+void launch_set_time(const DiskView& d, double t, double dt, cudaStream_t s, pg_body* planets) {
+    launch_step(k_set_time, 1, clock_threads(d), 0, s, d, t, dt, planets);
 }
 void launch_run_begin(Scalars* sc, double end_time, bool fresh, cudaStream_t s) {
     k_run_begin<<<1, 1, 0, s>>>(sc, end_time, fresh ? 1 : 0);
 }
 
 void launch_time_step(const DiskView& d, cudaStream_t s) {
-    k_time_step<<<1, 1, 0, s>>>(d);
-    k_planet_trig<<<cdiv(d.yarr, 256), 256, 0, s>>>(d);
+    launch_step(k_time_step, 1, clock_threads(d), 0, s, d);
 }
 
 void launch_init_planet(const DiskView& d, const pg_params& P, double t, cudaStream_t s) {
@@ -1249,12 +1139,9 @@ void launch_init_planet(const DiskView& d, const pg_params& P, double t, cudaStr
     k_init_planet<<<1, 1, 0, s>>>(d, a, P.planet_ecc, rs, t);
 }
 
-// Persistent grid: as many CTAs as fit on the GPU at once, each looping over tiles.
 static int kernel_occupancy(const void* kernel, int threads, size_t smem);
 
-// Persistent grid: as many CTAs as fit on the GPU at once (at most cps per SM
-// when cps > 0), each looping over tiles.
-static unsigned persistent_grid(const void* kernel, int threads, size_t smem, long long ntiles, int cps = 0) {
+static int sm_count() {
     static int nsm = 0;
     if (nsm == 0) {
         int dev = 0;
@@ -1262,9 +1149,15 @@ static unsigned persistent_grid(const void* kernel, int threads, size_t smem, lo
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
         if (nsm <= 0) nsm = 148;
     }
+    return nsm;
+}
+
+// Persistent grid: as many CTAs as fit on the GPU at once (at most cps per SM
+// when cps > 0), each looping over its work.
+static unsigned persistent_grid(const void* kernel, int threads, size_t smem, long long ntiles, int cps = 0) {
     int per_sm = kernel_occupancy(kernel, threads, smem);
     if (cps > 0 && cps < per_sm) per_sm = cps;
-    long long g = (long long)per_sm * nsm;
+    long long g = (long long)per_sm * sm_count();
     if (g > ntiles) g = ntiles;
     return (unsigned)(g < 1 ? 1 : g);
 }
@@ -1290,149 +1183,83 @@ static int kernel_occupancy(const void* kernel, int threads, size_t smem) {
     return per_sm;
 }
 
-void launch_kick1(const DiskView& d, const CellMaps& in, Cell* out, double* vis, cudaStream_t s, const pg_dust* din,
-                  pg_dust* dout, const Tune* t) {
-    const int ntx = (int)cdiv(d.xres, ST_TX), nt = ntx * (int)cdiv(d.yres, ST_TY);
-    const int cps = t ? t->cps[0] : 0;
-    if (d.visc && d.ndim == 2) {
-        const unsigned g = persistent_grid((const void*)k_kick1<true>, ST_THREADS, K1_SMEM, nt, cps);
-        k_kick1<true><<<g, ST_THREADS, K1_SMEM, s>>>(in.stencil, d, out, vis, ntx, nt, din, dout);
-    } else {
-        const unsigned g = persistent_grid((const void*)k_kick1<false>, ST_THREADS, K1_SMEM, nt, cps);
-        k_kick1<false><<<g, ST_THREADS, K1_SMEM, s>>>(in.stencil, d, out, vis, ntx, nt, din, dout);
-    }
-}
-
 // the 2D isothermal instances of the sweeps and the advection apply
 static bool iso_2d(const DiskView& d) { return d.eos == 0 && d.ndim == 2; }
 
-template <int DIR, class G, bool ISO>
-static void sweep_g(const DiskView& d, const CUtensorMap& m, Cell* out, cudaStream_t s, int cps) {
-    if constexpr (DIR == 0 && !G::X_OK) {
-        return;  // never chosen: the autotuner skips radial variants whose box does not fit
-    } else {
-        const int ntx = (int)cdiv(DIR == 0 ? d.xres : d.yres, G::L);
-        const int nt = ntx * (int)cdiv(DIR == 0 ? d.yres : d.xres, G::W);
-        constexpr size_t smem = G::template smem<ISO>();
-        const unsigned g = persistent_grid((const void*)k_sweep<DIR, G, ISO>, G::THREADS, smem, nt, cps);
-        k_sweep<DIR, G, ISO><<<g, G::THREADS, smem, s>>>(m, d, out, ntx, nt);
-    }
+// Rows a warp of a pass takes one after the other: the tuned length, or the one of least
+// run_cost (pg_internal.h).  1024x3072, us a pass at 4 / 16 / 32 / 48 / 96 rows: radial
+// sweep 124 / 127 / 143 / 128 / 159, azimuthal 175 / 154 / 175 / 153 / 223 (2368 warps
+// fit: 48 rows are 2048 runs, 32 rows one and a third wave).
+static int pass_length(const Tune* t, int k, const void* kernel, size_t smem, int lines, int rows, double extra) {
+    const int len = (t && k >= 0) ? SWEEP_LENGTHS[t->v[k]] : 0;
+    if (len > 0) return len;
+    const long long resident = (long long)SW_WARPS * sm_count() * kernel_occupancy(kernel, 32 * SW_WARPS, smem);
+    return run_length(lines, rows, resident, extra);
+}
+// CTAs for `items` warps of work, at most what fits at once (cps > 0: at most cps per SM)
+static unsigned sweep_grid(const void* kernel, size_t smem, long long items, int cps) {
+    return persistent_grid(kernel, 32 * SW_WARPS, smem, (items + SW_WARPS - 1) / SW_WARPS, cps);
 }
 
-template <class G, bool ISO>
-static void advect_g(const DiskView& d, const CUtensorMap& m, Cell* out, cudaStream_t s, int cps) {
-    const int ntx = (int)cdiv(d.yres, G::L), nt = ntx * (int)cdiv(d.xres, G::W);
-    constexpr size_t smem = G::template ad_smem<ISO>();
-    const unsigned g = persistent_grid((const void*)k_advect<G, ISO>, G::THREADS, smem, nt, cps);
-    k_advect<G, ISO><<<g, G::THREADS, smem, s>>>(m, d, out, ntx, nt);
-}
-
-// calls f(SV<v>{}) for the variant id v
-template <class F>
-static void with_variant(int v, F&& f) {
-    switch (v) {
-        case 1: f(SV<1>{}); break;
-        case 2: f(SV<2>{}); break;
-        case 3: f(SV<3>{}); break;
-        case 4: f(SV<4>{}); break;
-        case 5: f(SV<5>{}); break;
-        case 6: f(SV<6>{}); break;
-        case 7: f(SV<7>{}); break;
-        case 8: f(SV<8>{}); break;
-        case 9: f(SV<9>{}); break;
-        default: f(SV<0>{}); break;
-    }
-}
-
-static int variant_of(const Tune* t, int k, int dir) {
-    const int v = t ? t->v[k] : 0;
-    if (v < 0 || v >= NSWEEP_VARIANTS || (dir == 0 && !sweep_variant_x_ok(v))) return 0;
-    return v;
+// one marching pass: runs of `lines` warps across the radius
+template <class K, class... A>
+static void march(const Tune* t, int k, int cps, K kernel, size_t smem, const DiskView& d, int lines, double extra,
+                  cudaStream_t s, A... a) {
+    const int len = pass_length(t, k, (const void*)kernel, smem, lines, d.yres, extra);
+    const int items = lines * (int)cdiv(d.yres, len);
+    launch_step(kernel, sweep_grid((const void*)kernel, smem, items, t ? t->cps[cps] : 0), 32 * SW_WARPS, smem, s, a...,
+                lines, len, items);
 }
 
 void launch_sweep_x(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
-    const int v = variant_of(t, 0, 0);
-    with_variant(v, [&](auto tag) {
-        using G = typename decltype(tag)::G;
-        if (iso_2d(d)) sweep_g<0, G, true>(d, in.sx[v], out, s, t ? t->cps[1] : 0);
-        else sweep_g<0, G, false>(d, in.sx[v], out, s, t ? t->cps[1] : 0);
-    });
+    const int n = (int)cdiv(d.xres, RX_OUT);
+    if (iso_2d(d)) march(t, 0, 1, k_sweep_x<true>, RX_SMEM, d, n, 1.5, s, in.sx, d, out);
+    else march(t, 0, 1, k_sweep_x<false>, RX_SMEM, d, n, 1.5, s, in.sx, d, out);
+}
+void launch_sweep_y(const DiskView& d, const Cell* in, Cell* out, cudaStream_t s, const Tune* t) {
+    const int n = (int)cdiv(d.xres, 32);
+    if (iso_2d(d)) march(t, 1, 2, k_sweep_y<true>, 0, d, n, 3.5, s, in, d, out);
+    else march(t, 1, 2, k_sweep_y<false>, 0, d, n, 3.5, s, in, d, out);
+}
+void launch_advect(const DiskView& d, const Cell* in, Cell* out, cudaStream_t s, const Tune* t) {
+    const int n = (int)cdiv(d.xres, 32);
+    if (iso_2d(d)) march(t, 2, 3, k_advect<true>, 0, d, n, 3.5, s, in, d, out);
+    else march(t, 2, 3, k_advect<false>, 0, d, n, 3.5, s, in, d, out);
+}
+void launch_kick1(const DiskView& d, const Cell* in, Cell* out, double* vis, cudaStream_t s, const pg_dust* din,
+                  pg_dust* dout, const Tune* t) {
+    const int n = (int)cdiv(d.xres, KK_OUT);
+    if (d.visc && d.ndim == 2) march(t, -1, 0, k_kick1<true>, 0, d, n, 2.0, s, in, d, out, vis, din, dout);
+    else march(t, -1, 0, k_kick1<false>, 0, d, n, 1.0, s, in, d, out, vis, din, dout);
+}
+void launch_kick2(const DiskView& d, const Cell* in, const double* vis, Cell* out, cudaStream_t s, const pg_dust* din,
+                  pg_dust* dout, const Tune* t) {
+    const int n = (int)cdiv(d.xres, KK_OUT);
+    if (d.visc && d.ndim == 2) march(t, -1, 4, k_kick2<true>, 0, d, n, 2.5, s, in, vis, d, out, din, dout);
+    else march(t, -1, 4, k_kick2<false>, 0, d, n, 1.0, s, in, vis, d, out, din, dout);
 }
 
-void launch_sweep_y(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
-    const int v = variant_of(t, 1, 1);
-    with_variant(v, [&](auto tag) {
-        using G = typename decltype(tag)::G;
-        if (iso_2d(d)) sweep_g<1, G, true>(d, in.sy[v], out, s, t ? t->cps[2] : 0);
-        else sweep_g<1, G, false>(d, in.sy[v], out, s, t ? t->cps[2] : 0);
-    });
-}
-
-void launch_advect(const DiskView& d, const CellMaps& in, Cell* out, cudaStream_t s, const Tune* t) {
-    const int v = variant_of(t, 2, 1);
-    with_variant(v, [&](auto tag) {
-        using G = typename decltype(tag)::G;
-        if (iso_2d(d)) advect_g<G, true>(d, in.sy[v], out, s, t ? t->cps[3] : 0);
-        else advect_g<G, false>(d, in.sy[v], out, s, t ? t->cps[3] : 0);
-    });
-}
-
-void launch_kick2(const DiskView& d, const CellMaps& in, const VisMaps& vis, Cell* out, cudaStream_t s,
-                  const pg_dust* din, pg_dust* dout, const Tune* t) {
-    const int ntx = (int)cdiv(d.xres, ST_TX), nt = ntx * (int)cdiv(d.yres, ST_TY);
-    const int cps = t ? t->cps[4] : 0;
-    if (d.visc && d.ndim == 2) {
-        const unsigned g = persistent_grid((const void*)k_kick2<true>, ST_THREADS, K5_SMEM, nt, cps);
-        k_kick2<true><<<g, ST_THREADS, K5_SMEM, s>>>(in.stencil, vis.stencil, d, out, ntx, nt, din, dout);
-    } else {
-        const unsigned g = persistent_grid((const void*)k_kick2<false>, ST_THREADS, K5_SMEM, nt, cps);
-        k_kick2<false><<<g, ST_THREADS, K5_SMEM, s>>>(in.stencil, vis.stencil, d, out, ntx, nt, din, dout);
-    }
-}
-
-// CTAs per SM that fit for a pass (0 kick1, 1 sweep_x, 2 sweep_y, 3 advect, 4 kick2) with tile variant v
-int pass_occupancy(const DiskView& d, int pass, int v) {
+// CTAs per SM that fit for a pass (0 kick1, 1 sweep_x, 2 sweep_y, 3 advect, 4 kick2)
+int pass_occupancy(const DiskView& d, int pass) {
     const bool vis = d.visc && d.ndim == 2, iso = iso_2d(d);
-    int occ = 1;
+    constexpr int nt = 32 * SW_WARPS;
     switch (pass) {
-        case 0: return kernel_occupancy(vis ? (const void*)k_kick1<true> : (const void*)k_kick1<false>, ST_THREADS, K1_SMEM);
-        case 4: return kernel_occupancy(vis ? (const void*)k_kick2<true> : (const void*)k_kick2<false>, ST_THREADS, K5_SMEM);
-        case 1:
-            with_variant(v, [&](auto tag) {
-                using G = typename decltype(tag)::G;
-                if constexpr (G::X_OK)
-                    occ = iso ? kernel_occupancy((const void*)k_sweep<0, G, true>, G::THREADS, G::template smem<true>())
-                              : kernel_occupancy((const void*)k_sweep<0, G, false>, G::THREADS, G::template smem<false>());
-            });
-            return occ;
-        case 2:
-            with_variant(v, [&](auto tag) {
-                using G = typename decltype(tag)::G;
-                occ = iso ? kernel_occupancy((const void*)k_sweep<1, G, true>, G::THREADS, G::template smem<true>())
-                          : kernel_occupancy((const void*)k_sweep<1, G, false>, G::THREADS, G::template smem<false>());
-            });
-            return occ;
-        default:
-            with_variant(v, [&](auto tag) {
-                using G = typename decltype(tag)::G;
-                occ = iso ? kernel_occupancy((const void*)k_advect<G, true>, G::THREADS, G::template ad_smem<true>())
-                          : kernel_occupancy((const void*)k_advect<G, false>, G::THREADS, G::template ad_smem<false>());
-            });
-            return occ;
+        case 0: return kernel_occupancy(vis ? (const void*)k_kick1<true> : (const void*)k_kick1<false>, nt, 0);
+        case 1: return kernel_occupancy(iso ? (const void*)k_sweep_x<true> : (const void*)k_sweep_x<false>, nt, RX_SMEM);
+        case 2: return kernel_occupancy(iso ? (const void*)k_sweep_y<true> : (const void*)k_sweep_y<false>, nt, 0);
+        case 3: return kernel_occupancy(iso ? (const void*)k_advect<true> : (const void*)k_advect<false>, nt, 0);
+        default: return kernel_occupancy(vis ? (const void*)k_kick2<true> : (const void*)k_kick2<false>, nt, 0);
     }
 }
 
-// threads per CTA and the CTAs per SM its registers were compiled for, of a tile variant
-void sweep_variant_launch(int v, int* threads, int* minb) {
-    with_variant(v, [&](auto tag) {
-        using G = typename decltype(tag)::G;
-        *threads = G::THREADS;
-        *minb = G::MINB;
-    });
+// threads per CTA of the sweeps and the CTAs per SM their registers were compiled for
+void sweep_launch_shape(int* threads, int* minb) {
+    *threads = 32 * SW_WARPS;
+    *minb = 3;
 }
 
 int kernels_per_step(const DiskView& d) {
-    int n = 2 /*time, planet trig*/ + 1 /*kick1*/ + 1 /*sweep x*/ + 1 /*kick2*/;
+    int n = 1 /*clock and planet table*/ + 1 /*kick1*/ + 1 /*sweep x*/ + 1 /*kick2*/;
     if (d.ndim > 1) n += 1;
     if (d.ndim > 1 && d.orbadv) n += 1;
     if (d.dust) n += 1 + (d.ndim > 1 ? 1 : 0) + (d.ndim > 1 && d.orbadv ? 1 : 0);  // dust sweeps, advection

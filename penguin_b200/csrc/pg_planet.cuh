@@ -39,6 +39,18 @@ template <class D>
 __device__ inline void orbit_solution(const D& d, pg_body& b, double t) {  // planet.cu:105-133
     const double a = b.a, e = b.e;
     const double n = sqrt(1.0 / a / a / a);
+    b.m = ramp_function(t, d.ramp_time, d.planet_mass);
+    b.z = HPI;
+    b.vz = 0.0;
+    if (e == 0.0) {
+        // a circular orbit: the expressions below at e = 0, without their two sincos and
+        // atan (this runs in one thread on the step's critical path)
+        b.x = a;
+        b.y = fmod(n * t, TWOPI) - fmod(d.frame_omega * t, TWOPI) + PI;
+        b.vx = 0.0;
+        b.vy = n;
+        return;
+    }
     const double efac = sqrt(1.0 - e * e);
     const double B = e / (1.0 + efac);
     double u, cosu, sinu;
@@ -49,13 +61,10 @@ __device__ inline void orbit_solution(const D& d, pg_body& b, double t) {  // pl
     sincos(f, &esinf, &ecosf);
     esinf *= e;
     ecosf *= e;
-    b.m = ramp_function(t, d.ramp_time, d.planet_mass);
     b.x = a * efac * efac / (1.0 + ecosf);
     b.y = f - fmod(d.frame_omega * t, TWOPI) + PI;
-    b.z = HPI;
     b.vx = n * a * esinf / efac;
     b.vy = n * (1.0 + ecosf) * (1.0 + ecosf) / efac / efac / efac;
-    b.vz = 0.0;
 }
 
 // The star-planet pair on the reduced orbit (src/planet/planet.cu:135-175),

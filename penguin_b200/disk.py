@@ -184,7 +184,8 @@ class Disk:
 
 
 def sweep_variant(v: int) -> dict:
-    """Knobs of tile variant v of the sweeps and the residual advection."""
+    """Knobs of variant v of the sweeps and the residual advection (pencil_length, the rows
+    a warp takes one after the other: 0, by the grid's size)."""
     out = (ctypes.c_int * 6)()
     check(lib().pg_sweep_variant(v, out))
     return {"pencils_per_tile": out[0], "pencil_length": out[1], "cells_per_thread": out[2],
@@ -198,8 +199,8 @@ def describe_tuning(choice: dict) -> dict:
         k = {"ctas_per_sm": choice["cps_" + p] or "all that fit"}
         if p in ("sweep_x", "sweep_y", "advect"):
             k.update(sweep_variant(choice["v_" + p]))
-        else:  # the stencil passes: 32 x 8 cells per tile, one cell per thread, two TMA stages
-            k.update({"tile": "32x8", "cells_per_thread": 1, "tma_stages": 2})
+        else:  # the kicks: 30 outputs of a warp's 32 radii, runs of rows by the grid's size
+            k.update({"pencils_per_tile": 30, "pencil_length": 0})
         out[p] = k
     return out
 
