@@ -222,7 +222,7 @@ __device__ __forceinline__ S3<T> update_iso(S3<T> Q, T Dr, T Du, T Dv) {
     Q.r += Dr;
     Q.u += Du;
     Q.v += Dv;
-    const T ir = 1.0 / Q.r;
+    const T ir = inv(Q.r);
     Q.u *= ir;
     Q.v *= ir;
     if (Q.r < r_min) {
@@ -286,23 +286,12 @@ __device__ __forceinline__ void adv_face(const Args& a, const Seed& s, int i, in
     const ParT<T> R = recon<T>(wt, r[0], r[1], r[2], r[3], r[4], T(0.0));
     const ParT<T> U = recon<T>(wt, u[0], u[1], u[2], u[3], u[4], T(0.0));
     const ParT<T> W = recon<T>(wt, w[0], w[1], w[2], w[3], w[4], T(0.0));
-    const double xl = d.ya[c], xr = d.ya[c + 1];
-    const double sdt = a.dt * d.irad[i];
-    const double idx = d.idx_y[c];
-    T vr, vu, vw;
-    if (val(speed) > 0.0) {
-        const T x0 = xr - speed * sdt;
-        const FracT<T> q = frac_right(lim01((x0 - xl) * idx));
-        vr = aveR(q, R);
-        vu = aveR(q, U) * vr;
-        vw = aveR(q, W) * vr;
-    } else {
-        const T x0 = xl - speed * sdt;
-        const FracT<T> q = frac_left(lim01((x0 - xl) * idx));
-        vr = aveL(q, R);
-        vu = aveL(q, U) * vr;
-        vw = aveL(q, W) * vr;
-    }
+    const bool up = val(speed) > 0.0;
+    const T x = (up ? speed : -speed) * (a.dt * d.irad[i] * d.idx_y[c]);
+    const FracT<T> q = frac(lesser(x, T(1.0)));
+    const T vr = up ? aveR(q, R) : aveL(q, R);
+    const T vu = (up ? aveR(q, U) : aveL(q, U)) * vr;
+    const T vw = (up ? aveR(q, W) : aveL(q, W)) * vr;
     fr = vr * speed;
     fu = vu * speed;
     fw = vw * speed;
@@ -331,7 +320,7 @@ __device__ __forceinline__ S3<T> eval_adv(const Args& a, const Seed& s, int i, i
     Q.r += Dr;
     Q.u += Dw;
     Q.v += Du;
-    const T ir = 1.0 / Q.r;
+    const T ir = inv(Q.r);
     Q.u *= ir;
     Q.v *= ir;
     return Q;
@@ -353,8 +342,7 @@ __device__ __forceinline__ void gravity(const Args& a, const Seed& s, int i, int
         const double sinfac = a.trig[4 * j + 2 * which], cosfac = a.trig[4 * j + 2 * which + 1];
         const double iplx2 = 1.0 / p.x / p.x;
         const double rad = d.radx[i], plx = p.x;
-        const T Rp = sqrt(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + rs * rs);
-        const T ir = 1.0 / Rp;
+        const T ir = rsq(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + rs * rs);
         const T rs_fac = ir * ir * ir;
         gx += -plm * (rad - plx * cosfac) * rs_fac - plm * cosfac * iplx2;
         gy += -plm * plx * sinfac * rs_fac + plm * sinfac * iplx2;
@@ -363,6 +351,7 @@ __device__ __forceinline__ void gravity(const Args& a, const Seed& s, int i, int
 
 // the per-row angles of the step's two planets that gravity() reads
 __global__ void k_adj_trig(const DiskView d, pg_body p0, pg_body p1, double* trig) {
+    pdl_enter();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= d.yarr) return;
     sincos(d.ycj[j] - (p0.y + 0.0 * p0.vy), &trig[4 * j], &trig[4 * j + 1]);
@@ -373,7 +362,7 @@ __global__ void k_adj_trig(const DiskView d, pg_body p0, pg_body p1, double* tri
 template <class T>
 __device__ __forceinline__ S3<T> kick(const DiskView& d, const S3<T>& C, T gx, T gy, T vx, T vy, double ix,
                                       double mdt, double dt) {
-    const T ir = d.visc ? 1.0 / C.r : T(0.0);
+    const T ir = d.visc ? inv(C.r) : T(0.0);
     T fx = C.v * C.v * ix;
     T fy = 0.0;
     if (d.visc) {
@@ -511,6 +500,7 @@ constexpr int ADJ_THREADS = 128;
 // lambda_in(cell, field) = sum over the outputs whose stencil holds the cell.
 template <int PASS>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_state(const Args a) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -543,21 +533,26 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_state(const Args a) {
 // d loss / d theta: each output cell contracted with its derivative along
 // every parameter, summed over the grid.
 // sum of acc[3] over the block (ADJ_THREADS threads, all arriving) into gth
-__device__ __forceinline__ void block_add3(const double* acc, double* gth) {
-    __shared__ double red[3][ADJ_THREADS];
-    for (int th = 0; th < 3; ++th) red[th][threadIdx.x] = acc[th];
-    __syncthreads();
-    for (int w = ADJ_THREADS / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w)
-            for (int th = 0; th < 3; ++th) red[th][threadIdx.x] += red[th][threadIdx.x + w];
-        __syncthreads();
+__device__ __forceinline__ void block_add3(double* acc, double* gth) {
+    constexpr int WARPS = ADJ_THREADS / 32;
+    __shared__ double red[3][WARPS];
+#pragma unroll
+    for (int th = 0; th < 3; ++th) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) acc[th] += __shfl_down_sync(0xffffffffu, acc[th], o);
+        if ((threadIdx.x & 31) == 0) red[th][threadIdx.x >> 5] = acc[th];
     }
-    if (threadIdx.x == 0)
-        for (int th = 0; th < 3; ++th) atomicAdd(&gth[th], red[th][0]);
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double v = 0.0;
+        for (int w = 0; w < WARPS; ++w) v += red[threadIdx.x][w];
+        atomicAdd(&gth[threadIdx.x], v);
+    }
 }
 
 template <int PASS>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_theta(const Args a) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     double acc[3] = {0.0, 0.0, 0.0};
@@ -632,6 +627,7 @@ __device__ __forceinline__ FluxT<double> face_lambda(const Args& a, const double
 
 template <int DIR>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_flux(const Args a, const double* lslot) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -740,7 +736,8 @@ __device__ __forceinline__ void rev_thread(long long t, int per, int npen, int c
 
 // the half-states of the cells that have them (see k_rev_face)
 template <int DIR>
-__global__ void __launch_bounds__(ADJ_THREADS) k_rev_states(const Args a, double* buf) {
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_rev_states(const Args a, double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -775,7 +772,8 @@ __device__ __forceinline__ int rev_below(const DiskView& d, int f) {
 
 // HLLC at every face of the pencils from the stored half-states
 template <int DIR>
-__global__ void __launch_bounds__(ADJ_THREADS) k_rev_flux(const Args a, double* buf) {
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_rev_flux(const Args a, double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -814,9 +812,10 @@ __device__ __forceinline__ FluxT<double> rev_flux(const DiskView& d, const doubl
 // adjoint of Q into lam_in and lambda_D of the slots into lslot (3 planes)
 // theta: with the hand-written reverse, also the theta derivative of the update
 // itself (DIR 1: (rot + r Omega) D_Sigma in the v_phi slot).  rbuf: the face
-// fluxes kept by k_rev_flux, or null to evaluate them here.
-template <int DIR>
-__global__ void __launch_bounds__(ADJ_THREADS) k_adj_upd(const Args a, double* lslot, bool theta, const double* rbuf) {
+// fluxes kept by k_rev_flux; without HAND they are evaluated here.
+template <int DIR, bool HAND>
+__global__ void __launch_bounds__(ADJ_THREADS, 3) k_adj_upd(const Args a, double* lslot, bool theta, const double* rbuf) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -827,22 +826,20 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_upd(const Args a, double* l
         const size_t mo = (DIR == 1) ? pidx(d, i, sy_post_row(d, a.inc, i, j)) : (size_t)m;
         const double lr = a.lam[mo], lu = a.lam[P + mo], lv = a.lam[2 * P + mo];
         FluxT<double> F0, F1;
-        if (rbuf) {
+        if constexpr (HAND) {
             const int c = (DIR == 0) ? i : j, q = (DIR == 0) ? j : i;
             F0 = rev_flux<DIR>(d, rbuf, c, q);
             F1 = rev_flux<DIR>(d, rbuf, c + 1, q);
-        } else if (DIR == 0) {
-            F0 = face_flux<double, 0>(a, s0, i, j);
-            F1 = face_flux<double, 0>(a, s0, i + 1, j);
         } else {
-            F0 = face_flux<double, 1>(a, s0, j, i);
-            F1 = face_flux<double, 1>(a, s0, j + 1, i);
+            const int c = (DIR == 0) ? i : j, q = (DIR == 0) ? j : i;
+            F0 = face_flux<double, DIR>(a, s0, c, q);
+            F1 = face_flux<double, DIR>(a, s0, c + 1, q);
         }
         double Dr, D1, D2;
         sweep_D<DIR>(a, i, j, F0, F1, Dr, D1, D2);
         const S3<double> Q = ld<double>(a, s0, i, j);
         double g[6];
-        if (rbuf) {
+        if constexpr (HAND) {
             // update_iso in reverse: r' = r + D_r, u' = (u r + D_1) / r', v' = (v r + D_2) / r',
             // or the floor r' = max(1e-10 r, smallr) with u, v kept
             const S3<double> O = update_iso<double>(Q, Dr, D1, D2);
@@ -853,7 +850,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_upd(const Args a, double* l
                 g[2] = lv;
                 g[3] = g[4] = g[5] = 0.0;
             } else {
-                const double iR = 1.0 / O.r;
+                const double iR = inv(O.r);
                 g[0] = lr + (lu * (Q.u - O.u) + lv * (Q.v - O.v)) * iR;
                 g[1] = lu * Q.r * iR;
                 g[2] = lv * Q.r * iR;
@@ -899,7 +896,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_upd(const Args a, double* l
 template <int DIR>
 struct EdgeFwd {
     double r[5], p[5], u[5], v[5];
-    double rad, irad_q, cs0, flat, idx, xl, xr, sdt;
+    double rad, irad_q, cs0, flat, sx;
     const double* wt;
     rev::FlatTape ft;
     rev::ReconTape tR, tP, tU, tV;
@@ -929,18 +926,14 @@ struct EdgeFwd {
                 v[k] = C.u;
             }
         }
-        cs0 = sqrt(d.gam * p[2] / r[2]);
-        flat = rev::flatten_tape(1.0 / cs0, p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3], ft);
+        cs0 = sound_speed(d.gam, r[2], p[2]);
+        flat = rev::flatten_tape(p[2], p[0], p[1], p[3], p[4], u[1], u[2], u[3], ft);
         wt = ((DIR == 0) ? d.wx : d.wy) + 6 * c;
-        const double* fa = (DIR == 0) ? d.xa : d.ya;
-        idx = ((DIR == 0) ? d.idx_x : d.idx_y)[c];
+        sx = a.dt * irad_q * ((DIR == 0) ? d.idx_x : d.idx_y)[c];
         R = rev::recon_tape(wt, r[0], r[1], r[2], r[3], r[4], flat, tR);
         P = rev::recon_tape(wt, p[0], p[1], p[2], p[3], p[4], flat, tP);
         U = rev::recon_tape(wt, u[0], u[1], u[2], u[3], u[4], flat, tU);
         V = rev::recon_tape(wt, v[0], v[1], v[2], v[3], v[4], flat, tV);
-        xl = fa[c];
-        xr = fa[c + 1];
-        sdt = (DIR == 0) ? a.dt : a.dt * irad_q;
     }
 };
 
@@ -953,22 +946,13 @@ __device__ __forceinline__ void edge_rev_states(const Args& a, int c, int q, con
                                                 double* mid) {
     const DiskView& d = a.d;
     const EdgeFwd<DIR> F(a, c, q);
-    const Par Z{0.0, 0.0, 0.0};
-    const Half bsl{bl[0], bl[1], bl[2], DIR == 0 ? bl[3] : 0.0, DIR == 0 ? 0.0 : bl[3]};
-    const Half bsr{br[0], br[1], br[2], DIR == 0 ? br[3] : 0.0, DIR == 0 ? 0.0 : br[3]};
+    const Half bsl{bl[0], bl[1], bl[2], 0.0, 0.0}, bsr{br[0], br[1], br[2], 0.0, 0.0};
     double bcs0 = 0.0, br0c = 0.0, bp0c = 0.0, bu0c = 0.0;
-    Par bR{0.0, 0.0, 0.0}, bP{0.0, 0.0, 0.0}, bU{0.0, 0.0, 0.0}, bV{0.0, 0.0, 0.0}, bZ{0.0, 0.0, 0.0};
-    if (DIR == 0) {
-        rev::state_left_rev(d.gam, F.xl, F.idx, F.sdt, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, F.V, Z, bsl,
-                            bcs0, br0c, bp0c, bu0c, bR, bP, bU, bV, bZ);
-        rev::state_right_rev(d.gam, F.xl, F.xr, F.idx, F.sdt, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, F.V, Z,
-                             bsr, bcs0, br0c, bp0c, bu0c, bR, bP, bU, bV, bZ);
-    } else {
-        rev::state_left_rev(d.gam, F.xl, F.idx, F.sdt, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, Z, F.V, bsl,
-                            bcs0, br0c, bp0c, bu0c, bR, bP, bU, bZ, bV);
-        rev::state_right_rev(d.gam, F.xl, F.xr, F.idx, F.sdt, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, Z, F.V,
-                             bsr, bcs0, br0c, bp0c, bu0c, bR, bP, bU, bZ, bV);
-    }
+    Par bR{0.0, 0.0, 0.0}, bP{0.0, 0.0, 0.0}, bU{0.0, 0.0, 0.0}, bV{0.0, 0.0, 0.0};
+    rev::state_rev<0>(d.gam, F.sx, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, F.V, bsl, bl[3], bcs0, br0c, bp0c,
+                      bu0c, bR, bP, bU, bV);
+    rev::state_rev<1>(d.gam, F.sx, F.cs0, F.r[2], F.p[2], F.u[2], F.R, F.P, F.U, F.V, bsr, br[3], bcs0, br0c, bp0c,
+                      bu0c, bR, bP, bU, bV);
     const Par* bs[4] = {&bR, &bP, &bU, &bV};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -1004,25 +988,35 @@ __device__ __forceinline__ void edge_rev_recon(const Args& a, int c, int q, cons
     rev::recon_rev(F.wt, F.tV, F.flat, bV, av, bflat);
     rev::flatten_rev(F.ft, bflat, ap);
     // cs0 = sqrt(gam p / r) of the middle cell, which also enters the states directly
-    const double bA = rev::dsqrt(F.cs0, bcs0);
-    ap[2] += bA * d.gam / F.r[2] + bp0c;
-    ar[2] += br0c - bA * d.gam * F.p[2] / (F.r[2] * F.r[2]);
+    const double ir = inv(F.r[2]), bA = 0.5 * bcs0 * d.gam * inv(F.cs0) * ir;
+    ap[2] += bA + bp0c;
+    ar[2] += br0c - bA * F.p[2] * ir;
     au[2] += bu0c;
     if (g3) {
-        for (int th = 0; th < 3; ++th) {
-            const double* dt = a.dtab + (size_t)th * NTAB * d.xarr;
-            double g = 0.0;
-            for (int k = 0; k < 5; ++k) {
-                const int ik = (DIR == 0) ? c - 2 + k : q;
-                if (ik >= NPAD && ik < NPAD + d.xres) {
-                    g += ap[k] * F.r[k] * dt[T_CS2 * d.xarr + ik];
-                } else {  // radial ghost: init_C of the disk
-                    g += ap[k] * dt[T_P0 * d.xarr + ik] + au[k] * dt[T_U0 * d.xarr + ik] +
-                         av[k] * d.radx[ik] * dt[T_V0 * d.xarr + ik];
-                }
-                if (DIR == 1) g -= au[k] * dt[T_ROT * d.xarr + q];
+        double w[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) w[k] = ap[k] * F.r[k];
+        if (DIR == 1) {  // one radius
+            const double sp = ((w[0] + w[1]) + (w[2] + w[3])) + w[4];
+            const double su = ((au[0] + au[1]) + (au[2] + au[3])) + au[4];
+            for (int th = 0; th < 3; ++th) {
+                const double* dt = a.dtab + (size_t)th * NTAB * d.xarr + q;
+                g3[th] += sp * dt[T_CS2 * d.xarr] - su * dt[T_ROT * d.xarr];
             }
-            g3[th] += g;
+        } else {
+            for (int th = 0; th < 3; ++th) {
+                const double* dt = a.dtab + (size_t)th * NTAB * d.xarr + c - 2;
+                double g = 0.0;
+#pragma unroll
+                for (int k = 0; k < 5; ++k) {
+                    if (c - 2 + k >= NPAD && c - 2 + k < NPAD + d.xres)
+                        g += w[k] * dt[T_CS2 * d.xarr + k];
+                    else  // radial ghost: init_C of the disk
+                        g += ap[k] * dt[T_P0 * d.xarr + k] + au[k] * dt[T_U0 * d.xarr + k] +
+                             av[k] * d.radx[c - 2 + k] * dt[T_V0 * d.xarr + k];
+                }
+                g3[th] += g;
+            }
         }
     }
 #pragma unroll
@@ -1041,6 +1035,7 @@ __device__ __forceinline__ void edge_rev_recon(const Args& a, int c, int q, cons
 
 template <int DIR>
 __global__ void __launch_bounds__(ADJ_THREADS) k_rev_face(const Args a, const double* lslot, double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -1075,7 +1070,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rev_face(const Args a, const do
 }
 
 template <int DIR>
-__global__ void __launch_bounds__(ADJ_THREADS, 3) k_rev_cell_a(const Args a, double* buf) {
+__global__ void __launch_bounds__(ADJ_THREADS, 4) k_rev_cell_a(const Args a, double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -1101,6 +1097,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_rev_cell_a(const Args a, dou
 
 template <int DIR>
 __global__ void __launch_bounds__(ADJ_THREADS, 3) k_rev_cell_b(const Args a, double* buf, bool theta) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -1129,6 +1126,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, 3) k_rev_cell_b(const Args a, dou
 
 template <int DIR>
 __global__ void __launch_bounds__(ADJ_THREADS) k_rev_gather(const Args a, const double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     int n, npen, p0;
     rev_dims<DIR>(d, n, npen, p0);
@@ -1169,6 +1167,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rev_gather(const Args a, const 
 // derivative.  Per cell (k_radv_gather): the stencil adjoints of the faces
 // whose upwind stencil holds it.
 __global__ void __launch_bounds__(ADJ_THREADS) k_radv_upd(const Args a, double* lslot) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1178,7 +1177,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_radv_upd(const Args a, double* 
         const S3<double> Q = ld<double>(a, s0, i, j);
         const S3<double> O = eval_adv<double>(a, s0, i, j);
         const double lr = a.lam[m], lu = a.lam[P + m], lv = a.lam[2 * P + m];
-        const double iR = 1.0 / O.r;  // 1 / (Q.r + D_r)
+        const double iR = inv(O.r);  // 1 / (Q.r + D_r)
         a.lam_in[m] = lr + (lu * (Q.u - O.u) + lv * (Q.v - O.v)) * iR;
         a.lam_in[P + m] = lu * Q.r * iR;
         a.lam_in[2 * P + m] = lv * Q.r * iR;
@@ -1191,6 +1190,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_radv_upd(const Args a, double* 
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_radv_face(const Args a, const double* lslot, double* buf,
                                                            bool theta) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1217,30 +1217,19 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_radv_face(const Args a, const d
         const Par R = rev::recon_tape(wt, r[0], r[1], r[2], r[3], r[4], 0.0, tR);
         const Par U = rev::recon_tape(wt, u[0], u[1], u[2], u[3], u[4], 0.0, tU);
         const Par W = rev::recon_tape(wt, w[0], w[1], w[2], w[3], w[4], 0.0, tW);
-        const double xl = d.ya[c], xr = d.ya[c + 1];
-        const double sdt = a.dt * d.irad[i];
-        const double idx = d.idx_y[c];
-        const double x0 = (speed > 0.0) ? xr - speed * sdt : xl - speed * sdt;
-        const double ax = (x0 - xl) * idx;
-        const double x = lim01(ax);
-        double aR, aU, aW;
-        if (speed > 0.0) {
-            const Frac q = frac_right(x);
-            aR = aveR(q, R);
-            aU = aveR(q, U);
-            aW = aveR(q, W);
-        } else {
-            const Frac q = frac_left(x);
-            aR = aveL(q, R);
-            aU = aveL(q, U);
-            aW = aveL(q, W);
-        }
+        const bool up = speed > 0.0;
+        const double sx = a.dt * d.irad[i] * d.idx_y[c];
+        const double xr = fabs(speed) * sx;  // the swept fraction
+        const double x = lesser(xr, 1.0);
+        const Frac q = frac(x);
+        const double aR = up ? aveR(q, R) : aveL(q, R), aU = up ? aveR(q, U) : aveL(q, U);
+        const double aW = up ? aveR(q, W) : aveL(q, W);
         // fr = aR speed, fu = (aU aR) speed, fw = (aW aR) speed
         const double b_aR = speed * (bFr + bFu * aU + bFw * aW);
         const double b_aU = speed * bFu * aR, b_aW = speed * bFw * aR;
         Par bR{0.0, 0.0, 0.0}, bU{0.0, 0.0, 0.0}, bW{0.0, 0.0, 0.0};
         double bx;
-        if (speed > 0.0) {
+        if (up) {
             bx = rev::aveR_rev(x, R, b_aR, bR) + rev::aveR_rev(x, U, b_aU, bU) + rev::aveR_rev(x, W, b_aW, bW);
         } else {
             bx = rev::aveL_rev(x, R, b_aR, bR) + rev::aveL_rev(x, U, b_aU, bU) + rev::aveL_rev(x, W, b_aW, bW);
@@ -1256,9 +1245,9 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_radv_face(const Args a, const d
             buf[(size_t)(3 * k + 2) * n + m] = au[k];  // v_phi
         }
         if (theta) {
-            // d/d speed: the flux factor and, through x0, the swept fraction
+            // d/d speed: the flux factor and the swept fraction
             double bs = bFr * aR + bFu * aU * aR + bFw * aW * aR;
-            if (rev::lim_pass(ax)) bs -= bx * sdt * idx;
+            if (!(1.0 < xr)) bs += up ? bx * sx : -bx * sx;
             for (int th = 0; th < 3; ++th) acc[th] += bs * a.dtab[((size_t)th * NTAB + T_ROT) * d.xarr + i];
         }
     }
@@ -1266,6 +1255,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_radv_face(const Args a, const d
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_radv_gather(const Args a, const double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1295,7 +1285,7 @@ struct KickAdj {
 __device__ __forceinline__ KickAdj kick_rev(bool visc, const S3<double>& C, double gy, double vx, double vy, double ix,
                                             double mdt, double dt, double lr, double lu, double lv) {
     KickAdj b{0.0, lu, lv, 0.0, 0.0, lu * dt, lv * dt};
-    const double ir = visc ? 1.0 / C.r : 0.0;
+    const double ir = visc ? inv(C.r) : 0.0;
     double b_ir = 0.0;
     const double b_fx = lu * dt, b_fy = lv * dt;
     if (mdt != 0.0) {
@@ -1323,23 +1313,23 @@ __device__ __forceinline__ KickAdj kick_rev(bool visc, const S3<double>& C, doub
 }
 
 // theta derivative of a viscous force through nu (tab T_NU) and the bound-0
-// ghosts' init_C in its 3x3 stencil around column i, contracted with the
-// stencil adjoints bu, bv, bn (of u, v and nr = Sigma nu); rX: the stencil's Sigma
-__device__ __forceinline__ void stencil_theta(const Args& a, int i, const double* bu, const double* bv,
-                                              const double* bn, const double* rX, double* acc) {
+// ghosts' init_C in its 3x3 stencil around column i; rX: the stencil's Sigma.  In
+// a neighbour column only the middle row counts: the corners' adjoints cancel.
+__device__ __forceinline__ void stencil_theta(const Args& a, int i, int j, const rev::StressAdj& S, const double* rX,
+                                              double* acc) {
     const DiskView& d = a.d;
+    const double *X = d.visx + 5 * i, *Y = d.visy + 4 * j;
+    const double e = S.nx * X[0], w = S.ny * Y[0] * X[4];
+    const double nu[3] = {-e * rX[0], S.n * rX[1] + w * (rX[7] - rX[4]), e * rX[2]};
     for (int th = 0; th < 3; ++th) {
         const double* dt = a.dtab + (size_t)th * NTAB * d.xarr;
-        double g = 0.0;
-        for (int k = 0; k < 9; ++k) {
-            int dx, dy;
-            nb(k, dx, dy);
-            const int ii = i + dx;
-            g += bn[k] * rX[k] * dt[T_NU * d.xarr + ii];
-            if (ii < NPAD || ii >= NPAD + d.xres)  // radial ghost: init_C
-                g += bu[k] * dt[T_U0 * d.xarr + ii] + bv[k] * dt[T_V0 * d.xarr + ii];
-        }
-        acc[th] += g;
+        acc[th] += nu[0] * dt[T_NU * d.xarr + i - 1] + nu[1] * dt[T_NU * d.xarr + i] + nu[2] * dt[T_NU * d.xarr + i + 1];
+        if (i == NPAD)
+            acc[th] += (-S.ux * X[0] + 2.0 * S.p * X[2] * X[3]) * dt[T_U0 * d.xarr + i - 1] +
+                       (-S.vx * X[0] + S.q * X[2] * X[3]) * dt[T_V0 * d.xarr + i - 1];
+        if (i == NPAD + d.xres - 1)
+            acc[th] += (S.ux * X[0] + 2.0 * S.p * X[1] * X[3]) * dt[T_U0 * d.xarr + i + 1] +
+                       (S.vx * X[0] + S.q * X[1] * X[3]) * dt[T_V0 * d.xarr + i + 1];
     }
 }
 
@@ -1354,8 +1344,7 @@ __device__ __forceinline__ void gravity_theta(const Args& a, int i, int j, int w
     const double sinfac = a.trig[4 * j + 2 * which], cosfac = a.trig[4 * j + 2 * which + 1];
     const double iplx2 = 1.0 / p.x / p.x;
     const double rad = d.radx[i], plx = p.x;
-    const double Rp = sqrt(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + p.rs * p.rs);
-    const double ir = 1.0 / Rp;
+    const double ir = rsq(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + p.rs * p.rs);
     const double rs_fac = ir * ir * ir;
     const double ax = rad - plx * cosfac, ay = plx * sinfac;
     // d/dm
@@ -1370,13 +1359,53 @@ __device__ __forceinline__ void gravity_theta(const Args& a, int i, int j, int w
 // kick1 in reverse mode (same buffer).  Per output cell (k_rk1_cell): the
 // pointwise adjoint of the half-kick (mdt = 0) into lam_in, and the adjoint of
 // its viscous force (from the kick and from kick2's use of the force, lamv)
-// through the reverse of the viscous stencil: 9 cells x 3 state variables per
-// output cell.  Per input cell (k_rk1_gather): the stencil adjoints of the 9
-// outputs whose stencil holds it (periodic rows wrap; the constant bound-0
-// ghost columns drop out).  theta: gravity (q, h), nu, the ghosts' init_C.
-constexpr int RK1_STEN = 27;
+// through the reverse of the viscous stencil, eleven planes (StressAdj).  Per
+// input cell (k_rk1_gather): the stencil adjoints of the 9 outputs whose
+// stencil holds it (periodic rows wrap; the constant bound-0 ghost columns drop
+// out).  theta: gravity (q, h), nu, the ghosts' init_C.
+constexpr int RK1_STEN = 11;
+
+// planar: plane k of output m at buf[k n + m]
+__device__ __forceinline__ void put_stress(double* buf, long long n, long long m, const rev::StressAdj& S) {
+    const double f[RK1_STEN] = {S.nx, S.ny, S.ux, S.uy, S.vx, S.vy, S.p, S.q, S.n, S.u, S.v};
+#pragma unroll
+    for (int k = 0; k < RK1_STEN; ++k) buf[k * n + m] = f[k];
+}
+// the adjoint (nr, u, v) of cell (i, j) through the stress of every output that reads it
+__device__ __forceinline__ void gather_stress(const DiskView& d, const double* buf, int i, int j, double* acc) {
+    const long long n = (long long)d.xres * d.yres;
+    const int jd = wrap_row(d, j - 1), ju = wrap_row(d, j + 1);
+    const double *Yd = d.visy + 4 * jd, *Yu = d.visy + 4 * ju;
+    const double* c = buf + pidx(d, i, j);
+    double an = c[8 * n], au = c[9 * n], av = c[10 * n];
+    {  // the outputs below and above this cell
+        const double* X = d.visx + 5 * i;
+        const double *b = buf + pidx(d, i, jd), *t = buf + pidx(d, i, ju);
+        const double i_r1 = X[4], M0 = Yd[0] * i_r1, M1 = Yu[0] * i_r1;
+        const double K0 = Yd[1] * Yd[3] * i_r1 * i_r1, K1 = Yu[2] * Yu[3] * i_r1 * i_r1;
+        an += b[n] * M0 - t[n] * M1;
+        au += b[3 * n] * M0 + b[6 * n] * K0 - t[3 * n] * M1 + t[6 * n] * K1;
+        av += b[5 * n] * M0 + 2.0 * b[7 * n] * K0 - t[5 * n] * M1 + 2.0 * t[7 * n] * K1;
+    }
+#pragma unroll
+    for (int side = -1; side <= 1; side += 2) {  // the outputs of the column to its left (-1), right
+        const int oi = i + side;
+        if (oi < NPAD || oi >= NPAD + d.xres) continue;
+        const double* X = d.visx + 5 * oi;
+        const double *m = buf + pidx(d, oi, j), *b = buf + pidx(d, oi, jd), *t = buf + pidx(d, oi, ju);
+        const double e = -side * X[0], D = X[side < 0 ? 1 : 2] * X[3];
+        const double L0 = Yd[0] * X[4] * e, L1 = Yu[0] * X[4] * e;
+        an += m[0] * e;
+        au += m[2 * n] * e + 2.0 * m[6 * n] * D + b[7 * n] * L0 - t[7 * n] * L1;
+        av += m[4 * n] * e + m[7 * n] * D + b[6 * n] * L0 - t[6 * n] * L1;
+    }
+    acc[0] = an * d.nux[i];
+    acc[1] = au;
+    acc[2] = av;
+}
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_cell(const Args a, double* buf, bool theta) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1401,7 +1430,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_cell(const Args a, double* 
             viscous<double>(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, vx, vy);
         }
         const double ix = d.irad[i];
-        const double ir = d.visc ? 1.0 / C.r : 0.0;
+        const double ir = d.visc ? inv(C.r) : 0.0;
         const double lr = a.lam[m], lu = a.lam[P + m], lv = a.lam[2 * P + m];
         if (theta) gravity_theta(a, i, j, 0, lu * dt, lv * dt, acc);
         // o.r = C.r, o.u = C.u + (C.v^2 ix + vx ir + gx) dt, o.v = C.v + (vy ir + gy) dt
@@ -1410,36 +1439,23 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_cell(const Args a, double* 
         a.lam_in[2 * P + m] = lv + lu * dt * 2.0 * C.v * ix;
         if (d.visc) {
             const double bvx = lu * dt * ir + a.lamv[m], bvy = lv * dt * ir + a.lamv[P + m];
-            double bu[9] = {}, bv[9] = {}, bn[9] = {};
-            rev::viscous_rev(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, bvx, bvy, bu, bv, bn);
-            for (int k = 0; k < 9; ++k) {  // planar: field 3 k + f of output m at buf[(3 k + f) n + m]
-                buf[(size_t)(3 * k) * n + m] = bn[k] * nu[k % 3];
-                buf[(size_t)(3 * k + 1) * n + m] = bu[k];
-                buf[(size_t)(3 * k + 2) * n + m] = bv[k];
-            }
-            if (theta) stencil_theta(a, i, bu, bv, bn, rX, acc);
+            const rev::StressAdj S = rev::viscous_rev(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, bvx, bvy);
+            put_stress(buf, n, m, S);
+            if (theta) stencil_theta(a, i, j, S, rX, acc);
         }
     }
     if (theta) block_add3(acc, a.gth);
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_gather(const Args a, const double* buf) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
     for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < n; m += (long long)gridDim.x * blockDim.x) {
         const int i = NPAD + (int)(m % d.xres), j = d.ypad + (int)(m / d.xres);
-        double acc[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < 9; ++k) {
-            int dx, dy;
-            nb(k, dx, dy);
-            const int oi = i - dx;  // the output whose stencil slot k is this cell
-            if (oi < NPAD || oi >= NPAD + d.xres) continue;
-            const size_t mo = pidx(d, oi, wrap_row(d, j - dy));
-            acc[0] += buf[(size_t)(3 * k) * n + mo];
-            acc[1] += buf[(size_t)(3 * k + 1) * n + mo];
-            acc[2] += buf[(size_t)(3 * k + 2) * n + mo];
-        }
+        double acc[3];
+        gather_stress(d, buf, i, j, acc);
         a.lam_in[m] += acc[0];
         a.lam_in[P + m] += acc[1];
         a.lam_in[2 * P + m] += acc[2];
@@ -1448,8 +1464,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_gather(const Args a, const 
 
 // kick2 in reverse mode (same buffer).  Per output cell (k_rk2_cell): the
 // corrector's adjoint into lam_in; with viscosity, the reverse of the viscous
-// force over the 3x3 stencil of predicted states: their adjoints, 27 values per
-// output.  Per input cell (k_rk2_gather): the predicted-state adjoint gathered
+// force over the 3x3 stencil of predicted states: their adjoints, eleven planes.  Per input cell (k_rk2_gather): the predicted-state adjoint gathered
 // from the 9 outputs, then the reverse of the predictor: lam_in of the cell and
 // lamv_in of kick1's force.  theta: gravity (q, h) of both half-kicks, nu in the
 // force, the bound-0 ghosts' init_C.
@@ -1457,6 +1472,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk1_gather(const Args a, const 
 // one ring of ghosts; bound-0 radial ghosts keep init_C): (xres+2) x (yres+2)
 // cells, 3 values each
 __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_pred(const Args a, double* pred) {
+    pdl_enter();
     const DiskView& d = a.d;
     const int W = d.xres + 2;
     const long long n = (long long)W * (d.yres + 2);
@@ -1478,6 +1494,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_pred(const Args a, double* 
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_cell(const Args a, double* buf, const double* pred, bool theta) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1510,20 +1527,16 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_cell(const Args a, double* 
         a.lam_in[2 * P + m] = b.v;
         if (theta) gravity_theta(a, i, j, 1, b.gx, b.gy, acc);
         if (d.visc) {
-            double bu[9] = {}, bv[9] = {}, bn[9] = {};
-            rev::viscous_rev(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, b.vx, b.vy, bu, bv, bn);
-            for (int k = 0; k < 9; ++k) {
-                buf[(size_t)(3 * k) * n + m] = bn[k] * nu[k % 3];
-                buf[(size_t)(3 * k + 1) * n + m] = bu[k];
-                buf[(size_t)(3 * k + 2) * n + m] = bv[k];
-            }
-            if (theta) stencil_theta(a, i, bu, bv, bn, rX, acc);
+            const rev::StressAdj S = rev::viscous_rev(d.visx + 5 * i, d.visy + 4 * j, u, v, nr, b.vx, b.vy);
+            put_stress(buf, n, m, S);
+            if (theta) stencil_theta(a, i, j, S, rX, acc);
         }
     }
     if (theta) block_add3(acc, a.gth);
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_gather(const Args a, const double* buf, bool theta) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1532,17 +1545,8 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_rk2_gather(const Args a, const 
     double acc[3] = {0.0, 0.0, 0.0};
     for (long long m = blockIdx.x * (long long)blockDim.x + threadIdx.x; m < n; m += (long long)gridDim.x * blockDim.x) {
         const int i = NPAD + (int)(m % d.xres), j = d.ypad + (int)(m / d.xres);
-        double bX[3] = {0.0, 0.0, 0.0};
-        for (int k = 0; k < 9; ++k) {
-            int dx, dy;
-            nb(k, dx, dy);
-            const int oi = i - dx;
-            if (oi < NPAD || oi >= NPAD + d.xres) continue;
-            const size_t mo = pidx(d, oi, wrap_row(d, j - dy));
-            bX[0] += buf[(size_t)(3 * k) * n + mo];
-            bX[1] += buf[(size_t)(3 * k + 1) * n + mo];
-            bX[2] += buf[(size_t)(3 * k + 2) * n + mo];
-        }
+        double bX[3];
+        gather_stress(d, buf, i, j, bX);
         // the predictor X = kick(C, g, kick1's force, dt/2, dt/2)
         const S3<double> C = ld<double>(a, s0, i, j);
         double ox, oy, gx, gy;
@@ -1578,6 +1582,7 @@ __device__ __forceinline__ S3<T> predicted(const Args& a, const Seed& s, int i, 
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_k2a(const Args a, double* ls) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1620,6 +1625,7 @@ __global__ void __launch_bounds__(ADJ_THREADS) k_adj_k2a(const Args a, double* l
 }
 
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_k2b(const Args a, const double* ls) {
+    pdl_enter();
     const DiskView& d = a.d;
     const long long n = (long long)d.xres * d.yres;
     const size_t P = plane(d);
@@ -1898,40 +1904,40 @@ static void launch_pass(const Args& a, bool theta, double* scratch, double* rev,
         constexpr int DIR = (PASS == P_SX) ? 0 : 1;
         if (rev) {
             const long long pen = (DIR == 0) ? a.d.yres : a.d.xres, len = (DIR == 0) ? a.d.xres + 2 : a.d.yres;
-            k_rev_states<DIR><<<grid_for(pen * len), ADJ_THREADS, 0, s>>>(a, rev);
-            k_rev_flux<DIR><<<grid_for(pen * len), ADJ_THREADS, 0, s>>>(a, rev);
-            k_adj_upd<DIR><<<g, ADJ_THREADS, 0, s>>>(a, scratch, theta, rev);
-            k_rev_face<DIR><<<grid_for(pen * len), ADJ_THREADS, 0, s>>>(a, scratch, rev);
-            k_rev_cell_a<DIR><<<grid_for(pen * len), ADJ_THREADS, 0, s>>>(a, rev);
-            k_rev_cell_b<DIR><<<grid_for(pen * len), ADJ_THREADS, 0, s>>>(a, rev, theta);
-            k_rev_gather<DIR><<<g, ADJ_THREADS, 0, s>>>(a, rev);
+            launch_step(k_rev_states<DIR>, grid_for(pen * len), ADJ_THREADS, 0, s, a, rev);
+            launch_step(k_rev_flux<DIR>, grid_for(pen * len), ADJ_THREADS, 0, s, a, rev);
+            launch_step(k_adj_upd<DIR, true>, g, ADJ_THREADS, 0, s, a, scratch, theta, rev);
+            launch_step(k_rev_face<DIR>, grid_for(pen * len), ADJ_THREADS, 0, s, a, scratch, rev);
+            launch_step(k_rev_cell_a<DIR>, grid_for(pen * len), ADJ_THREADS, 0, s, a, rev);
+            launch_step(k_rev_cell_b<DIR>, grid_for(pen * len), ADJ_THREADS, 0, s, a, rev, theta);
+            launch_step(k_rev_gather<DIR>, g, ADJ_THREADS, 0, s, a, rev);
             return;  // theta done by the reverse kernels
         }
-        k_adj_upd<DIR><<<g, ADJ_THREADS, 0, s>>>(a, scratch, false, nullptr);
-        k_adj_flux<DIR><<<g, ADJ_THREADS, 0, s>>>(a, scratch);
+        launch_step(k_adj_upd<DIR, false>, g, ADJ_THREADS, 0, s, a, scratch, false, nullptr);
+        launch_step(k_adj_flux<DIR>, g, ADJ_THREADS, 0, s, a, scratch);
     } else if (PASS == P_K1 && rev) {
-        k_rk1_cell<<<g, ADJ_THREADS, 0, s>>>(a, rev, theta);
-        if (a.d.visc) k_rk1_gather<<<g, ADJ_THREADS, 0, s>>>(a, rev);
+        launch_step(k_rk1_cell, g, ADJ_THREADS, 0, s, a, rev, theta);
+        if (a.d.visc) launch_step(k_rk1_gather, g, ADJ_THREADS, 0, s, a, rev);
         return;  // theta done by k_rk1_cell
     } else if (PASS == P_K2 && rev) {
-        double* pred = rev + (size_t)a.d.xres * a.d.yres * RK1_STEN;  // after the 27 stencil adjoints per cell
+        double* pred = rev + (size_t)a.d.xres * a.d.yres * RK1_STEN;  // after the stencil adjoints
         if (a.d.visc)
-            k_rk2_pred<<<grid_for((long long)(a.d.xres + 2) * (a.d.yres + 2)), ADJ_THREADS, 0, s>>>(a, pred);
-        k_rk2_cell<<<g, ADJ_THREADS, 0, s>>>(a, rev, pred, theta);
-        if (a.d.visc) k_rk2_gather<<<g, ADJ_THREADS, 0, s>>>(a, rev, theta);
+            launch_step(k_rk2_pred, grid_for((long long)(a.d.xres + 2) * (a.d.yres + 2)), ADJ_THREADS, 0, s, a, pred);
+        launch_step(k_rk2_cell, g, ADJ_THREADS, 0, s, a, rev, pred, theta);
+        if (a.d.visc) launch_step(k_rk2_gather, g, ADJ_THREADS, 0, s, a, rev, theta);
         return;  // theta done by the reverse kernels
     } else if (PASS == P_ADV && rev) {
-        k_radv_upd<<<g, ADJ_THREADS, 0, s>>>(a, scratch);
-        k_radv_face<<<g, ADJ_THREADS, 0, s>>>(a, scratch, rev, theta);
-        k_radv_gather<<<g, ADJ_THREADS, 0, s>>>(a, rev);
+        launch_step(k_radv_upd, g, ADJ_THREADS, 0, s, a, scratch);
+        launch_step(k_radv_face, g, ADJ_THREADS, 0, s, a, scratch, rev, theta);
+        launch_step(k_radv_gather, g, ADJ_THREADS, 0, s, a, rev);
         return;  // theta done by k_radv_face
     } else if (PASS == P_K2 && a.d.visc) {
-        k_adj_k2a<<<g, ADJ_THREADS, 0, s>>>(a, scratch);
-        k_adj_k2b<<<g, ADJ_THREADS, 0, s>>>(a, scratch);
+        launch_step(k_adj_k2a, g, ADJ_THREADS, 0, s, a, scratch);
+        launch_step(k_adj_k2b, g, ADJ_THREADS, 0, s, a, scratch);
     } else {
-        k_adj_state<PASS><<<g, ADJ_THREADS, 0, s>>>(a);
+        launch_step(k_adj_state<PASS>, g, ADJ_THREADS, 0, s, a);
     }
-    if (theta) k_adj_theta<PASS><<<g, ADJ_THREADS, 0, s>>>(a);
+    if (theta) launch_step(k_adj_theta<PASS>, g, ADJ_THREADS, 0, s, a);
 }
 
 template <int PASS>
@@ -2297,7 +2303,7 @@ static Args base_args(pg_adj* a, int n, int slot, const pg_body* pl, int bank = 
     g.dtab = a->dtab;
     g.gth = a->gth;
     g.trig = a->trig;
-    k_adj_trig<<<(g.d.yarr + 127) / 128, 128, 0, a->stream>>>(g.d, g.pl[0], g.pl[1], a->trig);
+    launch_step(k_adj_trig, (g.d.yarr + 127) / 128, 128, 0, a->stream, g.d, g.pl[0], g.pl[1], a->trig);
     return g;
 }
 

@@ -17,34 +17,31 @@
 namespace pg {
 namespace rev {
 
-// adjoint of sqrt(a) at s = sqrt(a) (zero at a = 0, like the dual sqrt)
-__device__ __forceinline__ double dsqrt(double s, double bs) { return s == 0.0 ? 0.0 : 0.5 * bs / s; }
-
 // ------------------------------------------------------------- HLLC (EOS 0)
 // Adjoint of hllc(0, ie, gam, L, R) for the flux components r, u, v, w and pres
-// (the energy fluxes vanish for EOS 0).  bF: {r, u, v, w, pres}.
+// (the energy fluxes vanish for EOS 0).  bF: {r, u, v, w, pres}.  The reciprocals of the
+// replay serve the reverse as well, which has no division of its own.
 __device__ __forceinline__ void hllc_rev(double gam, const Half& L, const Half& R, const double* bF, Half& bL,
                                          Half& bR) {
-    const double cl = sqrt(gam * L.p / L.r);
-    const double cr = sqrt(gam * R.p / R.r);
-    const double c_ = 0.5 * (cr + cl);
+    const double sL = rsq(gam * L.p * L.r), sR = rsq(gam * R.p * R.r);  // c = gam p s, 1 / c = r s
+    const double cl = __dmul_rn(gam * L.p, sL), cr = __dmul_rn(gam * R.p, sR);
+    const double ic = inv(cl + cr);
     const double p_ = 0.5 * (R.p + L.p);
-    const double xe = 0.5 * gam * (L.u - R.u) / c_;
+    const double xe = gam * (L.u - R.u) * ic;
     const double el = exp_lim(xe);
     const double pm = p_ * el;
-    const double srl = sqrt(L.r), srr = sqrt(R.r);
-    const double is = 1.0 / (srl + srr);
-    const double u_ = (srl * L.u + srr * R.u) * is;
-    const double n2 = 0.5 * srl * srr * (is * is);
+    const double w = rsq(L.r * R.r), q = R.r * w, iq = inv(1.0 + q);
+    const double K = L.u + q * R.u, u_ = K * iq;
     const double du = R.u - L.u;
-    const double H = cl * cl * srl + cr * cr * srr;
-    const double cc = sqrt(H * is + n2 * du * du);
+    const double H = cl * cl + cr * cr * q;
+    const double n2 = 0.5 * q * (iq * iq);
+    const double c2 = H * iq + n2 * (du * du);
+    const double icc = rsq(c2), cc = c2 * icc;
     const double sl = u_ - cc, sr = u_ + cc;
-    const double num = L.r * L.u * cl + R.r * R.u * cr;
-    const double den = L.r * cl + R.r * cr;
-    const double q1 = num / den;
-    const double E = (L.r + R.r) * (0.5 * (cl + cr));
-    const double q2 = (L.p - R.p) / E;
+    const double ml = L.r * cl, mr = R.r * cr;
+    const double num = ml * L.u + mr * R.u, id = inv(ml + mr);
+    const double iS = inv(L.r + R.r), dp = L.p - R.p;
+    const double q1 = num * id, q2 = 2.0 * dp * (iS * ic);
     const double sm = q1 + q2;
     const bool left = (std::signbit(sl) == 0) || (std::signbit(sr) == 0 && std::signbit(sm) == 0);
     const Half& S = left ? L : R;
@@ -52,15 +49,15 @@ __device__ __forceinline__ void hllc_rev(double gam, const Half& L, const Half& 
     const bool super = (std::signbit(sl) == 0 || std::signbit(sr) != 0);
     double Fr;
     double b_sl = 0.0, b_sr = 0.0, b_sm = 0.0, b_pm = 0.0;
-    double s_ = 0.0, inv = 0.0, A = 0.0, B = 0.0;
+    double s_ = 0.0, is = 0.0, A = 0.0, B = 0.0;
     if (super) {
         Fr = S.u * S.r;
     } else {
         s_ = left ? sl : sr;
-        inv = 1.0 / (s_ - sm);
+        is = inv(s_ - sm);
         A = sm * S.r * (s_ - S.u);
         B = s_ * pm - sm * S.p;
-        Fr = A * inv;
+        Fr = A * is;
     }
     // F.u = S.u F.r, F.v = S.v F.r, F.w = S.w F.r
     const double bFr = bF[0] + bF[1] * S.u + bF[2] * S.v + bF[3] * S.w;
@@ -72,102 +69,85 @@ __device__ __forceinline__ void hllc_rev(double gam, const Half& L, const Half& 
         bS.r += bFr * S.u;
         bS.p += bF[4];
     } else {
-        const double b_inv = bFr * A + bF[4] * B;
-        const double bA = bFr * inv, bB = bF[4] * inv;
-        double b_s = -inv * inv * b_inv;
-        b_sm += inv * inv * b_inv;
-        b_sm += bA * S.r * (s_ - S.u);
+        const double b_is = (bFr * A + bF[4] * B) * (is * is);
+        const double bA = bFr * is, bB = bF[4] * is;
+        double b_s = -b_is;
+        b_sm += b_is + bA * S.r * (s_ - S.u) - bB * S.p;
         bS.r += bA * sm * (s_ - S.u);
-        b_s += bA * sm * S.r;
+        b_s += bA * sm * S.r + bB * pm;
         bS.u -= bA * sm * S.r;
-        b_s += bB * pm;
         b_pm += bB * s_;
-        b_sm -= bB * S.p;
         bS.p -= bB * sm;
         if (left) b_sl += b_s;
         else b_sr += b_s;
     }
-    double b_cl = 0.0, b_cr = 0.0, b_srl = 0.0, b_srr = 0.0, b_is = 0.0;
     // sl = u_ - cc, sr = u_ + cc
     const double b_u = b_sl + b_sr;
-    const double b_cc = b_sr - b_sl;
-    // sm = num / den + (L.p - R.p) / E
+    const double b_c2 = 0.5 * (b_sr - b_sl) * icc;
+    double b_cl, b_cr, b_q, b_iq, b_ic;
+    // sm = num id + 2 dp iS ic
     {
-        const double b_num = b_sm / den, b_den = -b_sm * q1 / den;
-        bL.r += b_num * L.u * cl;
-        bL.u += b_num * L.r * cl;
-        b_cl += b_num * L.r * L.u;
-        bR.r += b_num * R.u * cr;
-        bR.u += b_num * R.r * cr;
-        b_cr += b_num * R.r * R.u;
-        bL.r += b_den * cl;
-        b_cl += b_den * L.r;
-        bR.r += b_den * cr;
-        b_cr += b_den * R.r;
-        const double b_dp = b_sm / E, b_E = -b_sm * q2 / E;
+        const double b_num = b_sm * id, b_den = -b_num * q1;
+        const double b_ml = b_num * L.u + b_den, b_mr = b_num * R.u + b_den;
+        bL.u += b_num * ml;
+        bR.u += b_num * mr;
+        bL.r += b_ml * cl;
+        b_cl = b_ml * L.r;
+        bR.r += b_mr * cr;
+        b_cr = b_mr * R.r;
+        const double b_dp = 2.0 * b_sm * (iS * ic);
         bL.p += b_dp;
         bR.p -= b_dp;
-        const double b_LR = b_E * (0.5 * (cl + cr)), b_ch = b_E * (L.r + R.r);
-        bL.r += b_LR;
-        bR.r += b_LR;
-        b_cl += 0.5 * b_ch;
-        b_cr += 0.5 * b_ch;
+        const double b_S = -b_sm * q2 * iS;
+        bL.r += b_S;
+        bR.r += b_S;
+        b_ic = 2.0 * b_sm * dp * iS;
     }
-    // cc = sqrt(H is + n2 du^2)
+    // c2 = H iq + n2 du^2, H = cl^2 + cr^2 q, n2 = q iq^2 / 2; u_ = (L.u + q R.u) iq
     {
-        const double b_G = dsqrt(cc, b_cc);
-        const double b_H = b_G * is;
-        b_is += b_G * H;
-        b_cl += b_H * 2.0 * cl * srl;
-        b_srl += b_H * cl * cl;
-        b_cr += b_H * 2.0 * cr * srr;
-        b_srr += b_H * cr * cr;
-        const double b_n2 = b_G * du * du;
-        const double b_du = b_G * 2.0 * n2 * du;
+        const double b_H = b_c2 * iq;
+        b_iq = b_c2 * H;
+        b_cl += 2.0 * b_H * cl;
+        b_cr += 2.0 * b_H * cr * q;
+        b_q = b_H * cr * cr;
+        const double b_n2 = b_c2 * (du * du), b_du = 2.0 * b_c2 * n2 * du;
         bR.u += b_du;
         bL.u -= b_du;
-        // n2 = 0.5 srl srr is^2
-        b_srl += b_n2 * 0.5 * srr * (is * is);
-        b_srr += b_n2 * 0.5 * srl * (is * is);
-        b_is += b_n2 * 0.5 * srl * srr * 2.0 * is;
+        b_q += 0.5 * b_n2 * (iq * iq);
+        b_iq += b_n2 * q * iq;
+        const double b_K = b_u * iq;
+        b_iq += b_u * K;
+        bL.u += b_K;
+        bR.u += b_K * q;
+        b_q += b_K * R.u;
+        b_q -= b_iq * (iq * iq);
+        // q = sqrt(R.r / L.r): dq = q / 2 (dR.r / R.r - dL.r / L.r), and 1 / R.r = w q / (...)
+        // taken from w = (L.r R.r)^-1/2: 1 / R.r = L.r w^2, 1 / L.r = R.r w^2
+        const double hq = 0.5 * b_q * q * (w * w);
+        bR.r += hq * L.r;
+        bL.r -= hq * R.r;
     }
-    // u_ = (srl L.u + srr R.u) is
+    // pm = p_ exp_lim(xe), xe = gam (L.u - R.u) ic, ic = 1 / (cl + cr)
     {
-        const double K = srl * L.u + srr * R.u;
-        const double b_K = b_u * is;
-        b_is += b_u * K;
-        b_srl += b_K * L.u;
-        bL.u += b_K * srl;
-        b_srr += b_K * R.u;
-        bR.u += b_K * srr;
+        const double b_p = 0.5 * b_pm * el;
+        const double b_xe = (1.0e-6 > 1.0 + xe) ? 0.0 : b_pm * p_;
+        const double g = b_xe * gam * ic;
+        bL.u += g;
+        bR.u -= g;
+        b_ic += b_xe * gam * (L.u - R.u);
+        bR.p += b_p;
+        bL.p += b_p;
+        const double b_c = -b_ic * (ic * ic);
+        b_cl += b_c;
+        b_cr += b_c;
     }
-    // is = 1 / (srl + srr)
-    b_srl -= b_is * is * is;
-    b_srr -= b_is * is * is;
-    bL.r += dsqrt(srl, b_srl);
-    bR.r += dsqrt(srr, b_srr);
-    // pm = p_ exp_lim(xe), xe = 0.5 gam (L.u - R.u) / c_
+    // c = sqrt(gam p / r): dc = c / 2 (dp / p - dr / r) = gam s / 2 (dp - p s^2 gam p dr)
     {
-        const double b_p = b_pm * el;
-        const double b_el = b_pm * p_;
-        const double b_xe = (1.0e-6 > 1.0 + xe) ? 0.0 : b_el;
-        const double g = 0.5 * gam / c_;
-        bL.u += b_xe * g;
-        bR.u -= b_xe * g;
-        const double b_c = -b_xe * xe / c_;
-        bR.p += 0.5 * b_p;
-        bL.p += 0.5 * b_p;
-        b_cr += 0.5 * b_c;
-        b_cl += 0.5 * b_c;
-    }
-    // cl = sqrt(gam L.p / L.r)
-    {
-        const double ba = dsqrt(cl, b_cl);
-        bL.p += ba * gam / L.r;
-        bL.r -= ba * gam * L.p / (L.r * L.r);
-        const double bb = dsqrt(cr, b_cr);
-        bR.p += bb * gam / R.r;
-        bR.r -= bb * gam * R.p / (R.r * R.r);
+        const double a = 0.5 * gam * b_cl * sL, b = 0.5 * gam * b_cr * sR;
+        bL.p += a;
+        bL.r -= a * L.p * (cl * sL);
+        bR.p += b;
+        bR.r -= b * R.p * (cr * sR);
     }
 }
 
@@ -209,14 +189,12 @@ __device__ __forceinline__ Par recon_tape(const double* __restrict__ w, double a
     t.sR2 = sR;
     sR *= (1.0 - flat);
     sL *= (1.0 - flat);
-    const double t3 = sR + sL;
-    const double t2 = t3 * t3;
-    const double t1 = t3 * 3.0 * (sL - sR);
+    // slopes of one sign: each at most twice the other in size (recon, pg_hydro.cuh)
     t.mono = 0;
-    if (t2 < t1) {
+    if (fabs(sL) > 2.0 * fabs(sR)) {
         sL = 2.0 * sR;
         t.mono = 1;
-    } else if (t2 < -t1) {
+    } else if (fabs(sR) > 2.0 * fabs(sL)) {
         sR = 2.0 * sL;
         t.mono = 2;
     }
@@ -266,68 +244,61 @@ __device__ __forceinline__ void recon_rev(const double* __restrict__ w, const Re
 }
 
 // ---------------------------------------------------------------- flattening
+// Tape of flatten() (pg_hydro.cuh): f = 10 num big / (den p0) of the steeper side.
 struct FlatTape {
-    double p0, dp1f, dp2f, dp1b, dp2b, rf, rb, fpre, mx, g;
-    signed char active, pf, pb, selpre, selmx, cap, sgf, sgb, smf, smb;
+    double p0, num, den, big, iD, f;
+    signed char live, back, bigb;    // the coefficient is not constant; side; which |dp1| is the larger
+    signed char s1, s2, sb;          // signs of dp1 - dp2 / 2, of dp2 and of the larger dp1
 };
 
-__device__ __forceinline__ double flatten_tape(double inv_cs, double p0, double pm2, double pm1, double pp1,
-                                               double pp2, double um1, double u0, double up1, FlatTape& t) {
+__device__ __forceinline__ double flatten_tape(double p0, double pm2, double pm1, double pp1, double pp2, double um1,
+                                               double u0, double up1, FlatTape& t) {
+    const double dp1f = pp1 - p0, dp2f = pp2 - pm1;
+    const double dp1b = p0 - pm1, dp2b = pp1 - pm2;
+    const double wf = fabs(dp2f), wb = fabs(dp2b);
+    const double ef = dp1f - 0.5 * dp2f, eb = dp1b - 0.5 * dp2b;
+    const double nf = fabs(ef) - 0.25 * wf;
+    const double nb = fabs(eb) - 0.25 * wb;
+    t.live = 0;
+    if (!((u0 > up1 || um1 > u0) && wf > 0.0 && wb > 0.0 && (nf > 0.0 || nb > 0.0))) return 0.0;
+    const bool back = nb * wf > nf * wb;
+    const bool bigb = fabs(dp1b) > fabs(dp1f);
     t.p0 = p0;
-    t.dp1f = pp1 - p0;
-    t.dp2f = pp2 - pm1;
-    t.dp1b = p0 - pm1;
-    t.dp2b = pp1 - pm2;
-    (void)inv_cs;  // the branch of flatten (pg_hydro.cuh): signs of the velocity differences
-    const double Mf = u0 - up1;
-    const double Mb = um1 - u0;
-    double f = 0.0;
-    t.active = ((Mf > 0.0 || Mb > 0.0) && t.dp2f != 0.0 && t.dp2b != 0.0) ? 1 : 0;
-    if (t.active) {
-        t.rf = t.dp1f / t.dp2f;
-        const double xf = fabs(t.rf - 0.5) - 0.25;
-        t.sgf = (signed char)fabs_factor(t.rf - 0.5);
-        t.pf = (xf > 0.0) ? 1 : 0;
-        const double ddpf = 10.0 * (t.pf ? xf : 0.0);
-        t.rb = t.dp1b / t.dp2b;
-        const double xb = fabs(t.rb - 0.5) - 0.25;
-        t.sgb = (signed char)fabs_factor(t.rb - 0.5);
-        t.pb = (xb > 0.0) ? 1 : 0;
-        const double ddpb = 10.0 * (t.pb ? xb : 0.0);
-        t.selpre = (ddpb > ddpf) ? 1 : 0;
-        t.fpre = t.selpre ? ddpb : ddpf;
-        const double af = fabs(t.dp1f), ab = fabs(t.dp1b);
-        t.smf = (signed char)fabs_factor(t.dp1f);
-        t.smb = (signed char)fabs_factor(t.dp1b);
-        t.selmx = (ab > af) ? 1 : 0;
-        t.mx = t.selmx ? ab : af;
-        t.g = t.fpre * t.mx / p0;
-        t.cap = (t.g < 0.5) ? 0 : 1;
-        f = t.cap ? 0.5 : t.g;
-    }
-    return f;
+    t.num = back ? nb : nf;
+    t.den = back ? wb : wf;
+    t.big = bigb ? fabs(dp1b) : fabs(dp1f);
+    t.iD = inv(t.den * p0);
+    t.back = back;
+    t.bigb = bigb;
+    t.s1 = (signed char)fabs_factor(back ? eb : ef);
+    t.s2 = (signed char)fabs_factor(back ? dp2b : dp2f);
+    t.sb = (signed char)fabs_factor(bigb ? dp1b : dp1f);
+    t.f = 10.0 * t.num * t.big * t.iD;
+    if (!(t.f < 0.5)) return 0.5;
+    t.live = 1;
+    return t.f;
 }
 
 // accumulates into bp[5] = (pm2, pm1, p0, pp1, pp2)
 __device__ __forceinline__ void flatten_rev(const FlatTape& t, double bf, double* bp) {
-    if (!t.active || t.cap) return;
-    const double b_fpre = bf * t.mx / t.p0;
-    const double b_mx = bf * t.fpre / t.p0;
-    bp[2] -= bf * t.g / t.p0;
+    if (!t.live) return;
+    const double g = 10.0 * bf * t.iD;
+    const double b_num = g * t.big, b_big = g * t.num;
+    const double b_D = -bf * t.f * t.iD;  // f = 10 num big / D, D = den p0
+    bp[2] += b_D * t.den;
+    const double b_den = b_D * t.p0 - 0.25 * b_num;  // num = |dp1 - dp2 / 2| - |dp2| / 4, den = |dp2|
+    const double b_e = b_num * t.s1;
+    const double b1 = b_e, b2 = b_den * t.s2 - 0.5 * b_e;
     double b_dp1f = 0.0, b_dp1b = 0.0, b_dp2f = 0.0, b_dp2b = 0.0;
-    if (t.selmx) b_dp1b += b_mx * t.smb;
-    else b_dp1f += b_mx * t.smf;
-    if (t.selpre) {
-        if (t.pb) {
-            const double b_r = 10.0 * b_fpre * t.sgb;
-            b_dp1b += b_r / t.dp2b;
-            b_dp2b -= b_r * t.rb / t.dp2b;
-        }
-    } else if (t.pf) {
-        const double b_r = 10.0 * b_fpre * t.sgf;
-        b_dp1f += b_r / t.dp2f;
-        b_dp2f -= b_r * t.rf / t.dp2f;
+    if (t.back) {
+        b_dp1b = b1;
+        b_dp2b = b2;
+    } else {
+        b_dp1f = b1;
+        b_dp2f = b2;
     }
+    if (t.bigb) b_dp1b += b_big * t.sb;
+    else b_dp1f += b_big * t.sb;
     // dp1f = pp1 - p0, dp2f = pp2 - pm1, dp1b = p0 - pm1, dp2b = pp1 - pm2
     bp[3] += b_dp1f + b_dp2b;
     bp[2] += b_dp1b - b_dp1f;
@@ -337,197 +308,132 @@ __device__ __forceinline__ void flatten_rev(const FlatTape& t, double bf, double
 }
 
 // --------------------------------------------------- parabola averages
-// Adjoints of aveL / aveR at fraction x (frac_left / frac_right): accumulate the
-// Par adjoint and return d(ave)/dx.
+// Adjoints of aveL / aveR at the swept fraction x (frac): accumulate the Par adjoint and
+// return the adjoint of x.
 __device__ __forceinline__ double aveL_rev(double x, const Par& p, double b, Par& bp) {
-    const double h = x / 2.0, g = 1.0 - div_1p5(x);
+    const double h = 0.5 * x, g = 1.0 - x * (2.0 / 3.0);
     const double a6 = 3.0 * (p.sL - p.sR);
     const double S = p.sR + p.sL;
     // aL + h (S + g a6), aL = a - sL
+    const double bh = b * h;
     bp.a += b;
-    bp.sL += b * (-1.0 + h * (1.0 + 3.0 * g));
-    bp.sR += b * (h * (1.0 - 3.0 * g));
-    return b * ((S + g * a6) / 2.0 + h * a6 * (-1.0 / 1.5));
+    bp.sL += bh * (1.0 + 3.0 * g) - b;
+    bp.sR += bh * (1.0 - 3.0 * g);
+    return b * (0.5 * (S + g * a6) - h * a6 * (2.0 / 3.0));
 }
 __device__ __forceinline__ double aveR_rev(double x, const Par& p, double b, Par& bp) {
-    const double y = 1.0 - x;
-    const double h = y / 2.0, g = 1.0 - div_1p5(y);
+    const double h = 0.5 * x, g = 1.0 - x * (2.0 / 3.0);
     const double a6 = 3.0 * (p.sL - p.sR);
     const double S = p.sR + p.sL;
     // aR - h (S - g a6), aR = a + sR
+    const double bh = b * h;
     bp.a += b;
-    bp.sL += b * (-h * (1.0 - 3.0 * g));
-    bp.sR += b * (1.0 - h * (1.0 + 3.0 * g));
-    const double dy = -(S - g * a6) / 2.0 + h * a6 * (-1.0 / 1.5);  // d/dy
-    return -b * dy;
+    bp.sL -= bh * (1.0 - 3.0 * g);
+    bp.sR += b - bh * (1.0 + 3.0 * g);
+    return -b * (0.5 * (S - g * a6) + h * a6 * (2.0 / 3.0));
 }
 
 // ------------------------------------------------------- interface states
-// lim01 passes the derivative iff 0 <= a <= 1 (the dual fmax/fmin selections)
-__device__ __forceinline__ bool lim_pass(double a) { return !(0.0 > a) && !(1.0 < a); }
-
-// Adjoint of state_at_left_edge (states.cu:151-206) given bs, the adjoint of the
-// returned state.  Accumulates into bcs0, br0c, bp0c, bu0c and the Par adjoints.
-__device__ __forceinline__ void state_left_rev(double gam, double xl, double idx, double sdt, double cs0, double r0c,
-                                               double p0c, double u0c, const Par& R, const Par& Pp, const Par& U,
-                                               const Par& V, const Par& W, const Half& bs, double& bcs0,
-                                               double& br0c, double& bp0c, double& bu0c, Par& bR, Par& bP, Par& bU,
-                                               Par& bV, Par& bW) {
-    const double hdt = 0.5 * sdt;
-    // forward replay (the expressions of state_at_left_edge)
-    const bool t0pass = !(0.0 < u0c);
-    double tmp = fmin(u0c, 0.0);
-    tmp = xl - tmp * sdt + cs0 * sdt;
-    const double a1 = (tmp - xl) * idx;
-    const double x1 = lim01(a1);
+// Adjoint of state_at_left_edge (SIDE 0) or state_at_right_edge (SIDE 1)
+// (states.cu:151-264) given bs, the adjoint of the returned state: the forward's
+// expressions (pg_hydro.cuh), then back through the branches they took.  V is the one
+// transported field (v or w, adjoint bt).  Accumulates into bcs0, br0c, bp0c, bu0c and the
+// Par adjoints.
+template <int SIDE>
+__device__ __forceinline__ double ave(double x, const Par& p) {
+    return SIDE == 0 ? aveL(frac(x), p) : aveR(frac(x), p);
+}
+template <int SIDE>
+__device__ __forceinline__ double ave_rev(double x, const Par& p, double b, Par& bp) {
+    return SIDE == 0 ? aveL_rev(x, p, b, bp) : aveR_rev(x, p, b, bp);
+}
+template <int SIDE>
+__device__ __forceinline__ void state_rev(double gam, double sx, double cs0, double r0c, double p0c, double u0c,
+                                          const Par& R, const Par& Pp, const Par& U, const Par& V, const Half& bs,
+                                          double bt, double& bcs0, double& br0c, double& bp0c, double& bu0c, Par& bR,
+                                          Par& bP, Par& bU, Par& bV) {
+    constexpr double sg = SIDE == 0 ? -1.0 : 1.0;  // the speed towards the edge is sg u
+    // forward replay
+    const bool t0pass = !(0.0 > sg * u0c);
+    const double x1r = (cs0 + (t0pass ? sg * u0c : 0.0)) * sx;
+    const bool pass1 = !(1.0 < x1r);
+    const double x1 = pass1 ? x1r : 1.0;
+    const double ue = ave<SIDE>(x1, U);
+    const bool dpass = !(0.0 > sg * ue);
+    const double m = dpass ? sg * ue : 0.0;  // >= 0
+    const double x2r = m * sx;
+    const bool pass2 = !(1.0 < x2r);
+    const double x2 = pass2 ? x2r : 1.0;
     const double rmin = r0c * 1.0e-10, pmin = p0c * 1.0e-10;
-    const double ur = aveL(frac_left(x1), U);
-    const bool dpass = !(0.0 < ur);
-    const double dis = fmin(ur, 0.0) * sdt;
-    tmp = xl - dis;
-    const double a2 = (tmp - xl) * idx;
-    const double x2 = lim01(a2);
-    const Frac q2 = frac_left(x2);
-    const double r0r = aveL(q2, R), p0r = aveL(q2, Pp);
-    const double u0 = aveL(q2, U);
+    const double r0r = ave<SIDE>(x2, R), p0r = ave<SIDE>(x2, Pp), u0 = ave<SIDE>(x2, U);
     const bool rsel = rmin > r0r, psel = pmin > p0r;
-    const double r0 = fmax(r0r, rmin);
-    const double p0 = fmax(p0r, pmin);
-    const double ir0 = 1.0 / r0;
-    const double cs = sqrt(gam * p0 * ir0);
-    tmp = xl - dis + cs * sdt;
-    const double a3 = (tmp - xl) * idx;
-    const double x3 = lim01(a3);
-    const Frac q3 = frac_left(x3);
-    const double uA = aveL(q3, U), pA = aveL(q3, Pp);
-    const double k = 2.0 / (cs * sdt);
-    const double u2 = ((uA - u0) * k) * -hdt;
-    const double p2 = ((pA - p0) * k) * -hdt;
-    const double E1 = exp_lim(u2), E2 = exp_lim(gam * u2);
-    // reverse
-    double bx3 = aveL_rev(x3, V, bs.v, bV) + aveL_rev(x3, W, bs.w, bW);
-    double b_u0 = bs.u, b_ir0 = bs.u * p2;
-    const double b_p2 = bs.u * ir0;
-    double b_p0 = bs.p * E2, b_r0 = bs.r * E1;
-    double b_u2 = 0.0;
-    if (!(1.0e-6 > 1.0 + gam * u2)) b_u2 += bs.p * p0 * gam;
-    if (!(1.0e-6 > 1.0 + u2)) b_u2 += bs.r * r0;
-    const double b_u1 = b_u2 * -hdt, b_pp1 = b_p2 * -hdt;
-    const double b_uA = b_u1 * k, b_pA = b_pp1 * k;
-    b_u0 -= b_u1 * k;
-    b_p0 -= b_pp1 * k;
-    const double b_k = b_u1 * (uA - u0) + b_pp1 * (pA - p0);
-    double b_cs = -b_k * k / cs;
-    bx3 += aveL_rev(x3, U, b_uA, bU) + aveL_rev(x3, Pp, b_pA, bP);
-    double b_dis = 0.0;
-    if (lim_pass(a3)) {
-        const double bt = bx3 * idx;
-        b_dis -= bt;
-        b_cs += bt * sdt;
+    const double r0 = rsel ? rmin : r0r, p0 = psel ? pmin : p0r;
+    const double g = gam * p0;
+    const double s = rsq(g * r0);
+    const double x3r = (g * s + m) * sx;
+    const bool pass3 = !(1.0 < x3r);
+    const double x3 = pass3 ? x3r : 1.0;
+    const double uA = ave<SIDE>(x3, U), pA = ave<SIDE>(x3, Pp);
+    const double ics = r0 * s;                        // 1 / cs
+    const double eu = sg * (uA - u0), du = eu * ics;  // u0 - uA on the left, uA - u0 on the right
+    const double dp = sg * (p0 - pA);
+    const double E1 = exp_lim(du), E2 = exp_lim(gam * du);
+    // reverse: r = r0 E1, p = p0 E2, u = u0 - dp s
+    double bx3 = ave_rev<SIDE>(x3, V, bt, bV);
+    double b_u0 = bs.u;
+    const double b_dp = -bs.u * s;
+    double b_s = -bs.u * dp;
+    double b_p0 = bs.p * E2 + sg * b_dp, b_r0 = bs.r * E1;
+    double b_du = 0.0;
+    if (!(1.0e-6 > 1.0 + gam * du)) b_du += bs.p * p0 * gam;
+    if (!(1.0e-6 > 1.0 + du)) b_du += bs.r * r0;
+    const double b_eu = b_du * ics * sg;
+    b_u0 -= b_eu;
+    b_r0 += b_du * eu * s;
+    b_s += b_du * eu * r0;
+    bx3 += ave_rev<SIDE>(x3, U, b_eu, bU) + ave_rev<SIDE>(x3, Pp, -sg * b_dp, bP);
+    double b_m = 0.0, b_g = 0.0;
+    if (pass3) {
+        const double b = bx3 * sx;
+        b_g = b * s;
+        b_s += b * g;
+        b_m = b;
     }
-    const double b_arg = dsqrt(cs, b_cs);
-    b_p0 += b_arg * gam * ir0;
-    b_ir0 += b_arg * gam * p0;
-    b_r0 -= b_ir0 * ir0 * ir0;
+    // s = (g r0)^-1/2
+    const double b_gr = -0.5 * b_s * s * (s * s);
+    b_g += b_gr * r0;
+    b_r0 += b_gr * g;
+    b_p0 += b_g * gam;
     double b_r0r = 0.0, b_p0r = 0.0;
     if (rsel) br0c += b_r0 * 1.0e-10;
     else b_r0r = b_r0;
     if (psel) bp0c += b_p0 * 1.0e-10;
     else b_p0r = b_p0;
-    double bx2 = aveL_rev(x2, R, b_r0r, bR) + aveL_rev(x2, Pp, b_p0r, bP) + aveL_rev(x2, U, b_u0, bU);
-    if (lim_pass(a2)) b_dis -= bx2 * idx;
-    const double b_ur = dpass ? b_dis * sdt : 0.0;
-    const double bx1 = aveL_rev(x1, U, b_ur, bU);
-    if (lim_pass(a1)) {
-        const double bt = bx1 * idx;
-        if (t0pass) bu0c -= bt * sdt;
-        bcs0 += bt * sdt;
+    const double bx2 =
+        ave_rev<SIDE>(x2, R, b_r0r, bR) + ave_rev<SIDE>(x2, Pp, b_p0r, bP) + ave_rev<SIDE>(x2, U, b_u0, bU);
+    if (pass2) b_m += bx2 * sx;
+    const double bx1 = ave_rev<SIDE>(x1, U, dpass ? sg * b_m : 0.0, bU);
+    if (pass1) {
+        const double b = bx1 * sx;
+        if (t0pass) bu0c += sg * b;
+        bcs0 += b;
     }
 }
 
-// Adjoint of state_at_right_edge (states.cu:210-264).
-__device__ __forceinline__ void state_right_rev(double gam, double xl, double xr, double idx, double sdt, double cs0,
-                                                double r0c, double p0c, double u0c, const Par& R, const Par& Pp,
-                                                const Par& U, const Par& V, const Par& W, const Half& bs,
-                                                double& bcs0, double& br0c, double& bp0c, double& bu0c, Par& bR,
-                                                Par& bP, Par& bU, Par& bV, Par& bW) {
-    const double hdt = 0.5 * sdt;
-    const bool t0pass = !(0.0 > u0c);
-    double tmp = fmax(u0c, 0.0);
-    tmp = xr - tmp * sdt - cs0 * sdt;
-    const double a1 = (tmp - xl) * idx;
-    const double x1 = lim01(a1);
-    const double rmin = r0c * 1.0e-10, pmin = p0c * 1.0e-10;
-    const double ul = aveR(frac_right(x1), U);
-    const bool dpass = !(0.0 > ul);
-    const double dis = fmax(ul, 0.0) * sdt;
-    tmp = xr - dis;
-    const double a2 = (tmp - xl) * idx;
-    const double x2 = lim01(a2);
-    const Frac q2 = frac_right(x2);
-    const double r0r = aveR(q2, R), p0r = aveR(q2, Pp);
-    const double u0 = aveR(q2, U);
-    const bool rsel = rmin > r0r, psel = pmin > p0r;
-    const double r0 = fmax(r0r, rmin);
-    const double p0 = fmax(p0r, pmin);
-    const double ir0 = 1.0 / r0;
-    const double cs = sqrt(gam * p0 * ir0);
-    tmp = xr - dis - cs * sdt;
-    const double a3 = (tmp - xl) * idx;
-    const double x3 = lim01(a3);
-    const Frac q3 = frac_right(x3);
-    const double uA = aveR(q3, U), pA = aveR(q3, Pp);
-    const double k = 2.0 / (cs * sdt);
-    const double u2 = ((u0 - uA) * k) * -hdt;
-    const double p2 = ((p0 - pA) * k) * -hdt;
-    const double E1 = exp_lim(u2), E2 = exp_lim(gam * u2);
-    double bx3 = aveR_rev(x3, V, bs.v, bV) + aveR_rev(x3, W, bs.w, bW);
-    double b_u0 = bs.u, b_ir0 = bs.u * p2;
-    const double b_p2 = bs.u * ir0;
-    double b_p0 = bs.p * E2, b_r0 = bs.r * E1;
-    double b_u2 = 0.0;
-    if (!(1.0e-6 > 1.0 + gam * u2)) b_u2 += bs.p * p0 * gam;
-    if (!(1.0e-6 > 1.0 + u2)) b_u2 += bs.r * r0;
-    const double b_u1 = b_u2 * -hdt, b_pp1 = b_p2 * -hdt;
-    const double b_uA = -b_u1 * k, b_pA = -b_pp1 * k;
-    b_u0 += b_u1 * k;
-    b_p0 += b_pp1 * k;
-    const double b_k = b_u1 * (u0 - uA) + b_pp1 * (p0 - pA);
-    double b_cs = -b_k * k / cs;
-    bx3 += aveR_rev(x3, U, b_uA, bU) + aveR_rev(x3, Pp, b_pA, bP);
-    double b_dis = 0.0;
-    if (lim_pass(a3)) {
-        const double bt = bx3 * idx;
-        b_dis -= bt;
-        b_cs -= bt * sdt;
-    }
-    const double b_arg = dsqrt(cs, b_cs);
-    b_p0 += b_arg * gam * ir0;
-    b_ir0 += b_arg * gam * p0;
-    b_r0 -= b_ir0 * ir0 * ir0;
-    double b_r0r = 0.0, b_p0r = 0.0;
-    if (rsel) br0c += b_r0 * 1.0e-10;
-    else b_r0r = b_r0;
-    if (psel) bp0c += b_p0 * 1.0e-10;
-    else b_p0r = b_p0;
-    double bx2 = aveR_rev(x2, R, b_r0r, bR) + aveR_rev(x2, Pp, b_p0r, bP) + aveR_rev(x2, U, b_u0, bU);
-    if (lim_pass(a2)) b_dis -= bx2 * idx;
-    const double b_ul = dpass ? b_dis * sdt : 0.0;
-    const double bx1 = aveR_rev(x1, U, b_ul, bU);
-    if (lim_pass(a1)) {
-        const double bt = bx1 * idx;
-        if (t0pass) bu0c -= bt * sdt;
-        bcs0 -= bt * sdt;
-    }
-}
-
-// ------------------------------------------------------------ viscosity
-// Adjoint of viscous() (viscosity.cu:84-194, 2D polar): the force is bilinear
-// in nr = Sigma nu and the velocity derivatives.  Accumulates into bu[9],
-// bv[9], bnr[9] (stencil order of viscous()).
-__device__ __forceinline__ void viscous_rev(const double* __restrict__ X, const double* __restrict__ Y, const double* u,
-                                            const double* v, const double* nr, double bfx, double bfy, double* bu,
-                                            double* bv, double* bnr) {
+// reverse of viscous(): the force is linear in the second derivatives and bilinear in
+// nr = Sigma nu and the first ones, so with (a, b) the adjoint of the force its stencil adjoints
+// are fixed by eleven numbers: those of the six first derivatives, p = a nr and q = b nr (every
+// second derivative's is p, 2 p, q or 2 q) and the middle cell's own.  Eleven planes from
+// the cells to their gather instead of the 27 adjoints of the stencil: 128 registers instead
+// of 254, kick1's and kick2's cells 29.7 and 29.7 -> 20.1 and 19.4 us at 256x768
+struct StressAdj {
+    double nx, ny, ux, uy, vx, vy;  // of d nr/dx, d nr/dy, du/dx, ...
+    double p, q;
+    double n, u, v;  // the middle cell's, through every path
+};
+__device__ __forceinline__ StressAdj viscous_rev(const double* __restrict__ X, const double* __restrict__ Y,
+                                                 const double* u, const double* v, const double* nr, double a,
+                                                 double b) {
     const double i_r20 = X[0], i_r21 = X[1], i_r10 = X[2], i_hr20 = X[3], i_r1 = X[4];
     const double i_t20 = Y[0], i_t21 = Y[1], i_t10 = Y[2], i_ht20 = Y[3];
     const double dudx = (u[2] - u[0]) * i_r20;
@@ -543,48 +449,22 @@ __device__ __forceinline__ void viscous_rev(const double* __restrict__ X, const 
     const double d2udxy = (u[8] - u[6] - u[5] + u[3]) * i_r20 * i_t20 * i_r1;
     const double dndy = (nr[7] - nr[4]) * i_t20 * i_r1;
     const double n1 = nr[1], u1 = u[1], v1 = v[1];
-    const double a = bfx, b = bfy;
-    // adjoints of the derivatives and of the middle values
-    const double b_dndx = a * 2.0 * dudx + b * ((dudy + dvdx) - v1 * i_r1);
-    const double b_dudx = a * (2.0 * dndx + 2.0 * n1 * i_r1);
-    const double b_d2udx2 = a * 2.0 * n1;
-    const double b_dndy = a * ((dudy + dvdx) - v1 * i_r1) + b * (2.0 * dvdy + 2.0 * u1 * i_r1);
-    const double b_dudy = a * dndy + b * (dndx + 4.0 * n1 * i_r1);
-    const double b_dvdx = a * dndy + b * (dndx + n1 * i_r1);
-    const double b_d2udy2 = a * n1, b_d2vdxy = a * n1;
-    const double b_dvdy = -3.0 * a * n1 * i_r1 + 2.0 * b * dndy;
-    const double b_d2vdy2 = b * 2.0 * n1;
-    const double b_d2udxy = b * n1, b_d2vdx2 = b * n1;
-    bnr[1] += a * (2.0 * d2udx2 + 2.0 * dudx * i_r1 + (d2udy2 + d2vdxy) - dvdy * i_r1 -
-                   2.0 * (dvdy + u1 * i_r1) * i_r1) +
-              b * (2.0 * d2vdy2 + 2.0 * dudy * i_r1 + (d2udxy + d2vdx2) - dvdx * i_r1 + v1 * i_r1 * i_r1 +
-                   2.0 * (dudy + dvdx - v1 * i_r1) * i_r1);
-    bu[1] += -a * 2.0 * n1 * i_r1 * i_r1 + b * 2.0 * dndy * i_r1;
-    bv[1] += -a * dndy * i_r1 + b * (-dndx * i_r1 - n1 * i_r1 * i_r1);
-    // the difference stencils
-    const double K = i_ht20 * i_r1 * i_r1, L = i_r20 * i_t20 * i_r1, M = i_t20 * i_r1;
-    bu[2] += b_dudx * i_r20 + b_d2udx2 * i_r21 * i_hr20;
-    bu[0] += -b_dudx * i_r20 + b_d2udx2 * i_r10 * i_hr20;
-    bu[1] += -b_d2udx2 * (i_r21 + i_r10) * i_hr20 - b_d2udy2 * (i_t21 + i_t10) * K;
-    bu[7] += b_dudy * M + b_d2udy2 * i_t21 * K;
-    bu[4] += -b_dudy * M + b_d2udy2 * i_t10 * K;
-    bu[8] += b_d2udxy * L;
-    bu[6] -= b_d2udxy * L;
-    bu[5] -= b_d2udxy * L;
-    bu[3] += b_d2udxy * L;
-    bv[2] += b_dvdx * i_r20 + b_d2vdx2 * i_r21 * i_hr20;
-    bv[0] += -b_dvdx * i_r20 + b_d2vdx2 * i_r10 * i_hr20;
-    bv[1] += -b_d2vdx2 * (i_r21 + i_r10) * i_hr20 - b_d2vdy2 * (i_t21 + i_t10) * K;
-    bv[7] += b_dvdy * M + b_d2vdy2 * i_t21 * K;
-    bv[4] += -b_dvdy * M + b_d2vdy2 * i_t10 * K;
-    bv[8] += b_d2vdxy * L;
-    bv[6] -= b_d2vdxy * L;
-    bv[5] -= b_d2vdxy * L;
-    bv[3] += b_d2vdxy * L;
-    bnr[2] += b_dndx * i_r20;
-    bnr[0] -= b_dndx * i_r20;
-    bnr[7] += b_dndy * M;
-    bnr[4] -= b_dndy * M;
+    StressAdj o;
+    o.p = a * n1;
+    o.q = b * n1;
+    o.nx = a * 2.0 * dudx + b * ((dudy + dvdx) - v1 * i_r1);
+    o.ny = a * ((dudy + dvdx) - v1 * i_r1) + b * (2.0 * dvdy + 2.0 * u1 * i_r1);
+    o.ux = a * (2.0 * dndx + 2.0 * n1 * i_r1);
+    o.uy = a * dndy + b * (dndx + 4.0 * n1 * i_r1);
+    o.vx = a * dndy + b * (dndx + n1 * i_r1);
+    o.vy = -3.0 * a * n1 * i_r1 + 2.0 * b * dndy;
+    o.n = a * (2.0 * d2udx2 + 2.0 * dudx * i_r1 + (d2udy2 + d2vdxy) - dvdy * i_r1 - 2.0 * (dvdy + u1 * i_r1) * i_r1) +
+          b * (2.0 * d2vdy2 + 2.0 * dudy * i_r1 + (d2udxy + d2vdx2) - dvdx * i_r1 + v1 * i_r1 * i_r1 +
+               2.0 * (dudy + dvdx - v1 * i_r1) * i_r1);
+    const double D = (i_r21 + i_r10) * i_hr20, K = (i_t21 + i_t10) * i_ht20 * i_r1 * i_r1;
+    o.u = -a * 2.0 * n1 * i_r1 * i_r1 + b * 2.0 * dndy * i_r1 - 2.0 * o.p * D - o.p * K;
+    o.v = -a * dndy * i_r1 + b * (-dndx * i_r1 - n1 * i_r1 * i_r1) - o.q * D - 2.0 * o.q * K;
+    return o;
 }
 
 }  // namespace rev

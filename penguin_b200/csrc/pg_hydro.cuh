@@ -106,10 +106,6 @@ __device__ __forceinline__ double div_1p5(double x) {
 template <class T>
 __device__ __forceinline__ FracT<T> frac(T y) { return {0.5 * y, 1.0 - y * (2.0 / 3.0)}; }
 template <class T>
-__device__ __forceinline__ FracT<T> frac_left(T x) { return frac(x); }
-template <class T>
-__device__ __forceinline__ FracT<T> frac_right(T x) { return frac<T>(1.0 - x); }
-template <class T>
 __device__ __forceinline__ T aveL(const FracT<T>& f, const ParT<T>& p) {
     const T a6 = 3.0 * (p.sL - p.sR);
     const T aL = p.a - p.sL;
@@ -124,8 +120,6 @@ __device__ __forceinline__ T aveR(const FracT<T>& f, const ParT<T>& p) {
     return aR - f.h * (S - f.g * a6);
 }
 
-template <class T>
-__device__ __forceinline__ T lim01(T a) { return fmin(fmax(a, T(0.0)), T(1.0)); }  // solve.cu:14
 template <class T>
 __device__ __forceinline__ T exp_lim(T x) { return larger(1.0 + x, T(1.0e-6)); }  // solve.cu:29
 
