@@ -1200,6 +1200,12 @@ pg_status pg_disk_solve(pg_disk* dk, double t, double dt) {
     PG_CUDA(cudaSetDevice(E.device));
     pg_status s0 = resolve_cur(E);
     if (s0 != PG_OK) return s0;
+    if (dt != 0.0 && tube_applies(E.view)) {  // the same kernel as the device loop's
+        PG_CUDA(launch_tube(E.view, E.buf[0], E.buf[1], E.buf[E.cur], 1, t, dt, E.stream));
+        if (passes_per_step(E.view) % 2) E.cur = 1 - E.cur;
+        E.fresh = false;
+        return PG_OK;
+    }
     // this step's t and dt go in as launch arguments of k_set_time; the five passes are one
     // captured graph per starting buffer, one launch instead of five behind the host's dt
     // read-back
@@ -1290,6 +1296,23 @@ pg_status pg_disk_run(pg_disk* dk, int nsteps, double end_time) {
     for (int k = 0; k < 2; ++k) {
         pg_status s = make_cell_maps(E.maps[k], E.buf[k], E.view.xarr, E.view.yarr);
         if (s != PG_OK) return s;
+    }
+    if (tube_applies(E.view)) {
+        // whole stretches of steps per launch; both buffers then hold the newest state.
+        // With a finite end_time the done flag is read between stretches.
+        constexpr int STRETCH = 2048;
+        for (long long step = 0; step < nsteps; step += STRETCH) {
+            if (may_finish && step > 0) {
+                int done = 0;
+                PG_CUDA(cudaMemcpyAsync(&done, &E.sc->done, sizeof(int), cudaMemcpyDeviceToHost, E.stream));
+                PG_CUDA(cudaStreamSynchronize(E.stream));
+                if (done) break;
+            }
+            const int k = nsteps - step < STRETCH ? (int)(nsteps - step) : STRETCH;
+            PG_CUDA(launch_tube(E.view, E.buf[0], E.buf[1], E.buf[E.cur], k, 0.0, 0.0, E.stream));
+        }
+        if (!may_finish && passes_per_step(E.view) % 2) E.cur = (E.cur + nsteps) & 1;
+        return PG_OK;
     }
     for (int step = 0; step < nsteps; ++step) {
         if (may_finish && step > 0 && step % 256 == 0) {

@@ -101,6 +101,10 @@ void launch_torque(const DiskView& d, const Cell* buf, double* part, int nblocks
 // compensated sum of n doubles in index order
 double compensated_sum(const double* a, int n);
 int kernels_per_step(const DiskView& d);
+// many steps of a 1D cartesian tube in one launch (pg_tube.cu)
+bool tube_applies(const DiskView& d);
+cudaError_t launch_tube(const DiskView& d, Cell* b0, Cell* b1, const Cell* in, int nsteps, double t, double dt,
+                        cudaStream_t s);
 void set_last_error(const char* msg);
 
 // `planes` planes of `count` doubles, back to back in device memory, to host arrays
