@@ -32,8 +32,8 @@ namespace pg {
 // passes).  Tiles of 32 x 8 cells whose phases met at __syncthreads and exchanged
 // states and fluxes through shared memory spent 900-1000 instructions a cell, 350 of
 // them FP64, and a quarter of their time at the barriers; the sweeps spend 720-770 now.
-// What is left to bound them is FP64 issue and latency: about half of the FP64 rate, a
-// third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1 108 -> 88, sweep_x 298 -> 123,
+// What is left to bound them is FP64 issue and latency: the FP64 pipe is 57-60 % busy in
+// the sweeps, at a third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1 108 -> 88, sweep_x 298 -> 123,
 // sweep_y 328 -> 123, advection 154 -> 72, kick2 177 -> 160.
 // Each kernel is compiled for the CTAs per SM that were fastest there: sweep_x at 3 / 4 / 5
 // 123 / 129 / 151, sweep_y 123 / 139 / 246, advection at 4 / 5 / 6 72 / 72 / 115 (adiabatic
