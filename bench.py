@@ -345,7 +345,7 @@ def measure_ensemble(job, local, stream, steps):
     out = {"disks": len(ps_all), "cells": cells_all, "steps": steps, "value": v_e, "ms_per_step": ms_e / steps,
            "gpu_launches": launches, "sequential_fp64": {"value": v_s, "ms_per_step": ms_s / steps},
            "over_sequential_fp64": v_e / v_s, "tuning": tuning,
-           "note": "both arms autotuned (ensemble: pass variants and CTA caps; each FP64 disk: pencils per tile, CTA caps)",
+           "note": "both arms autotuned (run lengths and CTA caps)",
            "config": "Nr in 32*[4,16], Nphi=3Nr, q log-U[1e-5,3e-3], alpha log-U[1e-4,1e-2], h/r U[0.03,0.08], seed 2024"}
     if job.world > 1:
         out["partition"] = {"ranks": job.world, "disks_per_rank": [len(g) for g in gathered] if gathered else None,

@@ -20,7 +20,9 @@ namespace pg {
 // or stay in registers from the row before (azimuthal passes), no barrier and no shared
 // memory.  Bound by FP64 issue and latency; with tiles of 32 x 4 cells whose phases met at
 // barriers the sweeps and the advection of gas and dust took 133 us at 384x1024, with these
-// 112.  The w velocity is identically zero (dust runs in 2D) and stays as it is.
+// 100.  Compiled for 4 CTAs per SM: at 5 the azimuthal sweep spills (38 -> 41 us with the
+// gas's, the advection 28 -> 30).  The w velocity is identically zero (dust runs in 2D) and
+// stays as it is.
 constexpr int DS_WARPS = 4;  // warps per CTA, independent of one another
 constexpr int DS_THREADS = 32 * DS_WARPS;
 constexpr int DS_OUT = 30;   // radial sweep: outputs of a warp's 32 cells
@@ -70,7 +72,7 @@ __device__ __forceinline__ void load3(const pg_dust* c, double& r, double& u, do
 
 // ============================================================ dust sweeps
 // Radial (fields r, u, r v): lane l holds cell 2 + 30 seg + l, lanes 1..30 update.
-__global__ void __launch_bounds__(DS_THREADS, 5)
+__global__ void __launch_bounds__(DS_THREADS, 4)
     k_dsweep_x(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int nseg, int len, int nitems) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
@@ -142,7 +144,7 @@ struct DColumn {
 };
 
 // Azimuthal (fields r, v - orb_rot - r Omega, u) and the orbital shift.
-__global__ void __launch_bounds__(DS_THREADS, 5)
+__global__ void __launch_bounds__(DS_THREADS, 4)
     k_dsweep_y(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int ncol, int len, int nitems) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
@@ -203,7 +205,7 @@ __global__ void __launch_bounds__(DS_THREADS, 5)
 // advection() on Dust (advection.cu:175-233) + advecty (:235-290): the gas's residual speed
 // orb_res, fields (r, v, u), update_Dust.  The speed of a column has one sign: every row
 // feeds the same one of its two faces.
-__global__ void __launch_bounds__(DS_THREADS, 5)
+__global__ void __launch_bounds__(DS_THREADS, 4)
     k_dadvect(const pg_dust* __restrict__ in, const DiskView d, pg_dust* __restrict__ out, int ncol, int len, int nitems) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Scalars* sc = d.sc;
@@ -302,32 +304,35 @@ __global__ void k_dust_extract(const DiskView d, const pg_dust* buf, double* r, 
 // ============================================================== launchers
 static inline unsigned dcdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
-// one marching pass: runs of `lines` warps across the radius, of the length of least run_cost
-template <class K>
-static void march_dust(K kernel, const DiskView& d, int lines, double extra, const pg_dust* in, pg_dust* out,
-                       cudaStream_t s) {
-    static int nsm = 0, per_sm = 0;  // of this kernel
-    if (per_sm == 0) {
-        int dev = 0, n = 0, k = 0;
+// CTAs of a kernel that fit on the device
+template <auto K>
+static int dust_resident() {
+    static const int n = [] {
+        int dev = 0, sms = 0, per_sm = 0;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        nsm = n > 0 ? n : 148;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, DS_THREADS, 0) != cudaSuccess || k < 1) k = 1;
-        per_sm = k;
-    }
-    const int len = run_length(lines, d.yres, (long long)DS_WARPS * nsm * per_sm, extra);
-    const int items = lines * (int)dcdiv(d.yres, len);
-    const unsigned most = (unsigned)(nsm * per_sm), all = dcdiv(items, DS_WARPS);
-    launch_step(kernel, all < most ? all : most, DS_THREADS, 0, s, in, d, out, lines, len, items);
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) sms = 148;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, DS_THREADS, 0) != cudaSuccess || per_sm < 1)
+            per_sm = 1;
+        return sms * per_sm;
+    }();
+    return n;
+}
+// one marching pass: runs of `lines` warps across the radius, of the length of least run_cost
+template <auto K>
+static void march_dust(const DiskView& d, int lines, double extra, const pg_dust* in, pg_dust* out, cudaStream_t s) {
+    const int fit = dust_resident<K>();
+    const int len = run_length(lines, d.yres, (long long)DS_WARPS * fit, extra);
+    const int items = lines * (int)dcdiv(d.yres, len), all = (int)dcdiv(items, DS_WARPS);
+    launch_step(K, (unsigned)(all < fit ? all : fit), DS_THREADS, 0, s, in, d, out, lines, len, items);
 }
 void launch_dsweep_x(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
-    march_dust(k_dsweep_x, d, (int)dcdiv(d.xres, DS_OUT), 1.5, in, out, s);
+    march_dust<k_dsweep_x>(d, (int)dcdiv(d.xres, DS_OUT), 1.5, in, out, s);
 }
 void launch_dsweep_y(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
-    march_dust(k_dsweep_y, d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
+    march_dust<k_dsweep_y>(d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
 }
 void launch_dadvect(const DiskView& d, const pg_dust* in, pg_dust* out, cudaStream_t s) {
-    march_dust(k_dadvect, d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
+    march_dust<k_dadvect>(d, (int)dcdiv(d.xres, 32), 3.5, in, out, s);
 }
 void launch_dust_init(const DiskView& d, pg_dust* buf, cudaStream_t s) { k_dust_init<<<592, 256, 0, s>>>(d, buf); }
 void launch_dust_xghosts(const DiskView& d, pg_dust* buf, cudaStream_t s) {
