@@ -34,7 +34,7 @@ namespace pg {
 // them FP64, and a quarter of their time at the barriers; the sweeps spend 720-770 now.
 // What is left to bound them is FP64 issue and latency: the FP64 pipe is 57-60 % busy in
 // the sweeps, at a third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1 108 -> 88, sweep_x 298 -> 123,
-// sweep_y 328 -> 123, advection 154 -> 72, kick2 177 -> 160.
+// sweep_y 328 -> 123, advection 154 -> 72, kick2 177 -> 147.
 // Each kernel is compiled for the CTAs per SM that were fastest there: sweep_x at 3 / 4 / 5
 // 123 / 129 / 151, sweep_y 123 / 139 / 246, advection at 4 / 5 / 6 72 / 72 / 115 (adiabatic
 // 512x1536: 26 / 32 / 43), kick1 at 3 / 4 / 5 106 / 88 / 104, kick2 at 2 / 3 / 4 201 / 160 / 182.
@@ -536,9 +536,10 @@ __device__ __forceinline__ Column column(const DiskView& d, int seg, int lane) {
     c.nu = d.nux[c.ic];
     return c;
 }
+template <bool PLAIN = false>
 __device__ __forceinline__ Grav row_gravity(const DiskView& d, const Column& c, int j, int which, const pg_body& pl,
                                             const pg_body& st) {
-    if (d.twobd) return body_gravity(d, c.ic, j, which, pl, st);
+    if (!PLAIN && d.twobd) return body_gravity(d, c.ic, j, which, pl, st);
     const double* tr = d.trig + 4 * j + 2 * which;
     return gravity_at(d, c.gstar, c.rad, tr[0], tr[1], d.trig[4 * d.yarr + which], pl);
 }
@@ -637,8 +638,11 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
 // Kick 2 with damping and the CFL rate.  A row is predicted (sweeps.cu:713-729 with
 // mdt = dt = dt/2) when it enters, with kick 1's stress and the bodies at t + dt; the
 // corrector re-uses its gravity.
-template <bool VISC>
-__global__ void __launch_bounds__(32 * SW_WARPS, 3)
+// PLAIN: no cooling, averages, dust or second body, whose code holds registers also where it
+// does not run: 1024x3072 158 us without that instance, 149 with it at 3 CTAs per SM, 147 at 4
+// (96 bytes spilled).  Kick 1, 87 us at 4 CTAs per SM either way and 92 at 5, has none.
+template <bool VISC, bool PLAIN>
+__global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
     k_kick2(const Cell* __restrict__ in, const double* __restrict__ vis, const DiskView d, Cell* __restrict__ out,
             const pg_dust* __restrict__ din, pg_dust* __restrict__ dout, int nseg, int len, int nitems) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -675,7 +679,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 3)
             for (int m = 0; m < 4; ++m) up[m] = nx[m];
             const double2 f = nf;
             fetch(jn + 1);
-            gup = row_gravity(d, c, jn, 1, pl, star);
+            gup = row_gravity<PLAIN>(d, c, jn, 1, pl, star);
             ++jn;
             if (!VISC) return;
             double u = up[2], v = up[3];
@@ -731,7 +735,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 3)
             Cell Q = kick<VISC>(d, C, c.irad, g, vx, vy, hdt, hdt, &Tu, &Tv);
             // cooling over dt/2; the predictor cools over mdt = dt/2 as well, so Q.p is also
             // the predicted pressure the dust's second stopping time reads (sweeps.cu:668-699)
-            if (d.cool) Q.p = p_cool(d, i, C.p, C.r, hdt);
+            if (!PLAIN && d.cool) Q.p = p_cool(d, i, C.p, C.r, hdt);
             const double Tp = Q.p;
             if (d.kill) {
                 // killwave (src/killwave/killwave.cu:48-100): relax towards init_C
@@ -749,7 +753,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 3)
                 }
             }
             if (!(Q.r > 0.0)) atomicOr(&sc->err, 1 << PG_ERR_NAN);
-            if (din) {  // dust corrector half-kick towards the predicted gas velocity (sweeps.cu:663-707)
+            if (!PLAIN && din) {  // dust corrector half-kick towards the predicted gas velocity (sweeps.cu:663-707)
                 const DCell D = dust_kick(d, C, Tu, Tv, Tp, load_dust(din, d.xarr, i, j), g.gx, g.gy, g.gz, c.irad,
                                           hdt, hdt);
                 emit_dust(d, dout, i, j, D);
@@ -758,7 +762,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 3)
                 vmax = fmax(vmax, signal_rate(d, Q, i, j));
             }
             emit_to(d, out, oj, i, j, Q);
-            if (d.ave) accumulate_average(d, i, j, Q, hdt);  // ... and after it
+            if (!PLAIN && d.ave) accumulate_average(d, i, j, Q, hdt);  // ... and after it
         }
     }
     block_max_to<32 * SW_WARPS>(&sc->vmax_bits, vmax);
@@ -1186,6 +1190,9 @@ static int kernel_occupancy(const void* kernel, int threads, size_t smem) {
 // the 2D isothermal instances of the sweeps and the advection apply
 static bool iso_2d(const DiskView& d) { return d.eos == 0 && d.ndim == 2; }
 
+// the instance of kick 2 without cooling, averages, dust and a second body applies
+static bool plain_kick(const DiskView& d) { return !d.cool && !d.ave && !d.dust && !d.twobd; }
+
 // Rows a warp of a pass takes one after the other: the tuned length, or the one of least
 // run_cost (pg_internal.h).  1024x3072, us a pass at 4 / 16 / 32 / 48 / 96 rows: radial
 // sweep 124 / 127 / 143 / 128 / 159, azimuthal 175 / 154 / 175 / 153 / 223 (2368 warps
@@ -1235,8 +1242,9 @@ void launch_kick1(const DiskView& d, const Cell* in, Cell* out, double* vis, cud
 void launch_kick2(const DiskView& d, const Cell* in, const double* vis, Cell* out, cudaStream_t s, const pg_dust* din,
                   pg_dust* dout, const Tune* t) {
     const int n = (int)cdiv(d.xres, KK_OUT);
-    if (d.visc && d.ndim == 2) march(t, -1, 4, k_kick2<true>, 0, d, n, 2.5, s, in, vis, d, out, din, dout);
-    else march(t, -1, 4, k_kick2<false>, 0, d, n, 1.0, s, in, vis, d, out, din, dout);
+    if (!(d.visc && d.ndim == 2)) march(t, -1, 4, k_kick2<false, false>, 0, d, n, 1.0, s, in, vis, d, out, din, dout);
+    else if (plain_kick(d)) march(t, -1, 4, k_kick2<true, true>, 0, d, n, 2.5, s, in, vis, d, out, din, dout);
+    else march(t, -1, 4, k_kick2<true, false>, 0, d, n, 2.5, s, in, vis, d, out, din, dout);
 }
 
 // CTAs per SM that fit for a pass (0 kick1, 1 sweep_x, 2 sweep_y, 3 advect, 4 kick2)
@@ -1248,7 +1256,9 @@ int pass_occupancy(const DiskView& d, int pass) {
         case 1: return kernel_occupancy(iso ? (const void*)k_sweep_x<true> : (const void*)k_sweep_x<false>, nt, RX_SMEM);
         case 2: return kernel_occupancy(iso ? (const void*)k_sweep_y<true> : (const void*)k_sweep_y<false>, nt, 0);
         case 3: return kernel_occupancy(iso ? (const void*)k_advect<true> : (const void*)k_advect<false>, nt, 0);
-        default: return kernel_occupancy(vis ? (const void*)k_kick2<true> : (const void*)k_kick2<false>, nt, 0);
+        default:
+            if (!vis) return kernel_occupancy((const void*)k_kick2<false, false>, nt, 0);
+            return kernel_occupancy(plain_kick(d) ? (const void*)k_kick2<true, true> : (const void*)k_kick2<true, false>, nt, 0);
     }
 }
 

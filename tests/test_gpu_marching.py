@@ -51,6 +51,27 @@ def test_disk_matches_oracle(size):
     assert all(e < 1e-13 for e in errs.values()), errs
 
 
+@pytest.mark.parametrize("size", [(30, 91), (62, 128)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_kick2_with_and_without_averages(size):
+    """A disk that averages takes the other instance of the second half-kick: the same cells to
+    the rounding bound above."""
+    p = P.reference_disk(*size).replace(planet_mass=0.0, kill_flag=0)
+    st = I.disk_state(p, seed=7)
+    out = []
+    for average in (False, True):
+        d = Disk(p)
+        d.set_state(T0, st)
+        if average:
+            d.set_average(1.0)
+        d.run(10)
+        d.check()
+        out.append(d.get_state())
+        d.close()
+    errs = {k: l1(out[1][k], out[0][k]) for k in ("r", "p")}
+    errs["momentum"] = momentum(out[1], out[0], "uv")
+    assert all(e < 1e-13 for e in errs.values()), errs
+
+
 @pytest.mark.parametrize("size", [(34, 97), (62, 300)], ids=lambda s: f"{s[0]}x{s[1]}")
 def test_run_lengths_agree_bitwise(size):
     """The ten run lengths and one CTA per SM (several runs a warp) of the FP64 passes, and
