@@ -679,7 +679,8 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
             for (int m = 0; m < 4; ++m) up[m] = nx[m];
             const double2 f = nf;
             fetch(jn + 1);
-            gup = row_gravity<PLAIN>(d, c, jn, 1, pl, star);
+            // without stress the last call finds no row; in 1D the planet's table has none to read either
+            if (VISC || jn <= jlast) gup = row_gravity<PLAIN>(d, c, jn, 1, pl, star);
             ++jn;
             if (!VISC) return;
             double u = up[2], v = up[3];
