@@ -577,17 +577,22 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
         const Emitter emit_to(d, c.i);
         double* o = cell_at(d, out, c.ic, j0);
         double q[4], up[4], nx[4];  // the middle row, the one above and the next in flight: r, p, v_r, v_phi
+        double w = 0.0, uw = 0.0, nw = 0.0;  // ... and in 1D v_z, zero in 2D
         Row3 lo{}, mid{}, hi{};
         int jl = VISC ? j0 - 1 : j0;             // the next row to load, and the last one
         const int jlast = VISC ? j1 : j1 - 1;
         auto fetch = [&]() {
-            if (jl <= jlast) load4(next, nx);
+            if (jl <= jlast) {
+                load4(next, nx);
+                if (!VISC && d.ndim == 1) nw = next[4];
+            }
             next += pitch;
             ++jl;
         };
         auto enter = [&]() {
 #pragma unroll
             for (int m = 0; m < 4; ++m) up[m] = nx[m];
+            uw = nw;
             fetch();
             if (VISC) hi = row3(up[2], up[3], up[0] * c.nu);
         };
@@ -601,6 +606,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
         for (int j = j0; j < j1; ++j) {
 #pragma unroll
             for (int m = 0; m < 4; ++m) q[m] = up[m];
+            w = uw;
             const Grav g = row_gravity(d, c, j, 0, pl, star);
             double vx = 0.0, vy = 0.0;
             if (VISC) {
@@ -621,7 +627,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
                 if (j < 2 * NPAD) s[(size_t)d.xarr * d.yres] = double2{vx, vy};
                 else if (j >= d.yres) *(s - (size_t)d.xarr * d.yres) = double2{vx, vy};
             }
-            const Cell C{q[0], q[1], q[2], q[3], 0.0};
+            const Cell C{q[0], q[1], q[2], q[3], w};
             Cell Q = kick<VISC>(d, C, c.irad, g, vx, vy, 0.0, hdt);
             if (d.cool) Q.p = p_cool(d, c.i, C.p, C.r, hdt);  // sweeps.cu:695-699
             emit_to(d, out, oj, c.i, j, Q);
@@ -664,10 +670,12 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
         const int jlast = VISC ? j1 : j1 - 1;
         double q[4], up[4], nx[4];  // the middle row, the one above, the next in flight (with its stress)
         double2 nf{0.0, 0.0};
+        double w = 0.0, uw = 0.0, nw = 0.0;  // v_z in 1D, zero in 2D
         auto fetch = [&](int j) {
             if (j <= jlast) {
                 load4(next, nx);
                 if (VISC) nf = *nvis;
+                else if (d.ndim == 1) nw = next[4];
             }
             next += pitch;
             nvis += d.xarr;
@@ -677,6 +685,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
         auto enter = [&]() {  // row jn into `up`, its prediction into `hi`
 #pragma unroll
             for (int m = 0; m < 4; ++m) up[m] = nx[m];
+            uw = nw;
             const double2 f = nf;
             fetch(jn + 1);
             // without stress the last call finds no row; in 1D the planet's table has none to read either
@@ -717,6 +726,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
         for (int j = j0; j < j1; ++j) {
 #pragma unroll
             for (int m = 0; m < 4; ++m) q[m] = up[m];
+            w = uw;
             g = gup;
             double vx = 0.0, vy = 0.0;
             if (VISC) {
@@ -731,7 +741,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
             o += pitch;
             if (!c.output) continue;
             const int i = c.i;
-            const Cell C{q[0], q[1], q[2], q[3], 0.0};
+            const Cell C{q[0], q[1], q[2], q[3], w};
             double Tu = C.u, Tv = C.v;
             Cell Q = kick<VISC>(d, C, c.irad, g, vx, vy, hdt, hdt, &Tu, &Tv);
             // cooling over dt/2; the predictor cools over mdt = dt/2 as well, so Q.p is also
@@ -750,6 +760,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
                         Q.p += f * (I[1] - Q.p);
                         Q.u += f * (I[2] - Q.u);
                         Q.v += f * (I[3] - Q.v);
+                        if (!VISC) Q.w += f * (I[4] - Q.w);
                     }
                 }
             }

@@ -42,3 +42,31 @@ def test_polar_ring_with_a_planet_matches_the_oracle(n, lft, rgh):
     # the radial velocity starts at zero: its rounding is that of the speeds it is made of
     errs["u"] = np.abs(g["u"] - ref["u"]).max() / np.abs(ref["v"]).max()
     assert all(e < 3e-10 for e in errs.values()), errs
+
+
+def test_drop_in_tube_carries_both_transverse_velocities():
+    """Cartesian v and w are transported by the same expressions and enter the energy through
+    v^2 + w^2 alone, so a tube with v = 3 s, w = 4 s that takes one launch per pass moves like
+    one with v = 5 s, w = 0 in the tube's own kernel.  40 steps at an ulp each, without growth
+    at CFL 0.5 (1e-13 of a field's size)."""
+    from penguin_b200.grid import ReferenceLoop
+
+    p = P.sod_tube(94)
+    rng = np.random.default_rng(7)
+    s = 0.1 * rng.uniform(-1, 1, (1, 94))
+    st = I.sod_state(p)
+    d = Disk(p)
+    d.set_state(0.0, dict(st, v=5.0 * s))
+    d.step_host(40)
+    ref = d.get_state()
+    d.close()
+    loop = ReferenceLoop(p, 0.0, dict(st, v=3.0 * s))
+    cells = loop._keep["C"].view(p.yarr, p.xarr, 5)
+    cells[0, 3:-3, 4] = loop.torch.from_numpy(4.0 * s[0]).cuda()
+    loop.torch.cuda.synchronize()
+    loop.step(40)
+    g = loop.interior()
+    loop.close()
+    want = dict(ref, v=0.6 * ref["v"], w=0.8 * ref["v"])
+    for k in "rpuvw":
+        assert np.abs(g[k] - want[k]).max() < 1e-13 * np.abs(want[k]).max(), k
