@@ -92,6 +92,7 @@ struct DiskView {
     // time average of the gas state over a save interval (ave_flag, src/output/output.cu:250-330)
     Cell* ave;            // null: off
     double ave_T;         // the save interval
+    int tube;             // 1D: CTAs of the largest cluster its device runs (pg_tube.cu), 0: none
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

@@ -620,6 +620,7 @@ static pg_status engine_setup(Engine& E, const double* dev_xa, const double* dev
     d.res = E.res;
     d.inc = E.inc;
     d.sc = E.sc;
+    d.tube = P.ndim == 1 ? tube_max_cluster() : 0;
     launch_init_tables(d, P, t, E.stream);
     PG_CUDA(cudaGetLastError());
     return PG_OK;

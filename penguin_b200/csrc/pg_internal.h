@@ -102,6 +102,7 @@ void launch_torque(const DiskView& d, const Cell* buf, double* part, int nblocks
 double compensated_sum(const double* a, int n);
 int kernels_per_step(const DiskView& d);
 // many steps of a 1D cartesian tube in one launch (pg_tube.cu)
+int tube_max_cluster();
 bool tube_applies(const DiskView& d);
 cudaError_t launch_tube(const DiskView& d, Cell* b0, Cell* b1, const Cell* in, int nsteps, double t, double dt,
                         cudaStream_t s);

@@ -263,33 +263,34 @@ static cudaError_t tube_launch(const DiskView& d, int nc, int warps, Cell* b0, C
     return cudaLaunchKernelEx(&cfg, k_tube, d, b0, b1, in, nsteps, t, dt);
 }
 
-// Largest cluster the device runs: 16 CTAs where it grants the non-portable size, else 8.
-static int tube_max_cluster(const DiskView& d) {
-    static int maxc = 0;
-    if (maxc == 0) {
+// CTAs of the largest cluster of full CTAs that the current device runs: 16 where it grants
+// the non-portable size, else 8, or 0 (no tube loop).  Asked when a tube is made, for its own
+// device: the attribute that allows 16 belongs to the device's context.
+int tube_max_cluster() {
+    const bool big = cudaFuncSetAttribute(k_tube, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    for (int nc = big ? TB_MAXCTAS : 8; nc >= 8; nc /= 2) {
         int got = 0;
-        const bool ok = cudaFuncSetAttribute(k_tube, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        tube_launch(d, 16, TB_MAXWARPS, nullptr, nullptr, nullptr, 0, 0.0, 0.0, nullptr, &got) == cudaSuccess &&
-                        got > 0;
-        if (!ok) cudaGetLastError();
-        maxc = ok ? 16 : 8;
+        if (tube_launch(DiskView{}, nc, TB_MAXWARPS, nullptr, nullptr, nullptr, 0, 0.0, 0.0, nullptr, &got) == cudaSuccess &&
+            got > 0)
+            return nc;
     }
-    return maxc;
+    cudaGetLastError();
+    return 0;
 }
 
 // A tube whose half-kicks are identities, of a size that one cluster holds: 7680 cells with
 // 16 CTAs take 4.9 us a step, 1024 cells 3.4; 7682 as separate launches 16.4.
 bool tube_applies(const DiskView& d) {
     int nc, warps;
-    return d.ndim == 1 && d.geomx == 0 && !d.kill && !d.cool && !d.ave && !d.dust && !d.twobd &&
-           tube_shape(d.xres, tube_max_cluster(d), &nc, &warps);
+    return d.ndim == 1 && d.geomx == 0 && !d.kill && !d.cool && !d.ave && !d.dust && !d.twobd && d.tube > 0 &&
+           tube_shape(d.xres, d.tube, &nc, &warps);
 }
 
 // nsteps of the device's clock, or with dt != 0 one step of the caller's t and dt
 cudaError_t launch_tube(const DiskView& d, Cell* b0, Cell* b1, const Cell* in, int nsteps, double t, double dt,
                         cudaStream_t s) {
     int nc, warps;
-    if (!tube_shape(d.xres, tube_max_cluster(d), &nc, &warps)) return cudaErrorInvalidConfiguration;
+    if (!tube_shape(d.xres, d.tube, &nc, &warps)) return cudaErrorInvalidConfiguration;
     return tube_launch(d, nc, warps, b0, b1, in, nsteps, t, dt, s, nullptr);
 }
 

@@ -91,3 +91,33 @@ def test_tube_loop_stops_at_its_end_time():
     d.check()
     d.close()
     h.close()
+
+
+def test_tubes_made_and_run_by_several_threads():
+    """Every tube asks its own device for the largest cluster when it is made: threads that make
+    and run tubes at the same time (16 CTAs each) get the states that one thread gets."""
+    import threading
+
+    from penguin_b200.disk import Disk
+
+    p = P.sod_tube(1024)
+    st = state(1024, 2, False)
+    out = [None] * 5
+
+    def work(k):
+        d = Disk(p)
+        d.set_state(0.0, st)
+        d.run(30)
+        d.check()
+        out[k] = d.get_state()
+        d.close()
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    work(4)
+    for g in out[:4]:
+        for k in ("r", "p", "u"):
+            assert np.array_equal(g[k], out[4][k]), k
