@@ -32,6 +32,15 @@ __device__ __forceinline__ T lesser(T a, T b) { return (b < a) ? b : a; }
 template <class T>
 __device__ __forceinline__ T larger(T a, T b) { return (b > a) ? b : a; }
 
+// a b + c in one rounding; of a derivative type, as it stands.  Which product of a sum the
+// compiler contracts may depend on the code around it: where two instances of a kernel have
+// to give the same bits, every product that is added is added by this.
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+template <class A, class B, class C>
+__device__ __forceinline__ auto mad(const A& a, const B& b, const C& c) {
+    return a * b + c;
+}
+
 // Reciprocal (of either sign) and reciprocal square root of a normal double to about an
 // ulp: the hardware's approximation (rcp/rsqrt.approx.ftz.f64, which reads and
 // returns the upper 32 bits of a double, so |e| < 2^-19) and one third-order step
@@ -272,33 +281,43 @@ __device__ __forceinline__ FluxT<T> hllc(int eos, int ie, double gam, const Half
 // (src/viscosity/viscosity.cu:9-22, 84-194, ndim 2).  Stencil order: n<3 row j,
 // 3..5 row j-1, 6..8 row j+1, columns i-1..i+1.  The grid spacings enter as
 // per-index reciprocals: X = {1/(r2-r0), 1/(r2-r1), 1/(r1-r0), 1/(0.5(r2-r0)), 1/r1},
-// Y = {1/(t2-t0), 1/(t2-t1), 1/(t1-t0), 1/(0.5(t2-t0))}.
+// Y = {1/(t2-t0), 1/(t2-t1), 1/(t1-t0), 1/(0.5(t2-t0))}.  Sums of products by mad: the
+// kicks' instances give the same bits.
 template <class T>
 __device__ __forceinline__ void viscous(const double* __restrict__ X, const double* __restrict__ Y, const T* u,
                                         const T* v, const T* nr, T& fx_out, T& fy_out) {
     const double i_r20 = X[0], i_r21 = X[1], i_r10 = X[2], i_hr20 = X[3], i_r1 = X[4];
     const double i_t20 = Y[0], i_t21 = Y[1], i_t10 = Y[2], i_ht20 = Y[3];
     const T dudx = (u[2] - u[0]) * i_r20;
-    const T d2udx2 = ((u[2] - u[1]) * i_r21 - (u[1] - u[0]) * i_r10) * i_hr20;
+    const T d2udx2 = mad(u[2] - u[1], i_r21, (u[0] - u[1]) * i_r10) * i_hr20;
     const T dndx = (nr[2] - nr[0]) * i_r20;
     const T dvdx = (v[2] - v[0]) * i_r20;
-    const T d2vdx2 = ((v[2] - v[1]) * i_r21 - (v[1] - v[0]) * i_r10) * i_hr20;
+    const T d2vdx2 = mad(v[2] - v[1], i_r21, (v[0] - v[1]) * i_r10) * i_hr20;
     const T dvdy = (v[7] - v[4]) * i_t20 * i_r1;
-    const T d2vdy2 = ((v[7] - v[1]) * i_t21 - (v[1] - v[4]) * i_t10) * i_ht20 * i_r1 * i_r1;
+    const T d2vdy2 = mad(v[7] - v[1], i_t21, (v[4] - v[1]) * i_t10) * i_ht20 * i_r1 * i_r1;
     const T d2vdxy = (v[8] - v[6] - v[5] + v[3]) * i_r20 * i_t20 * i_r1;
     const T dudy = (u[7] - u[4]) * i_t20 * i_r1;
-    const T d2udy2 = ((u[7] - u[1]) * i_t21 - (u[1] - u[4]) * i_t10) * i_ht20 * i_r1 * i_r1;
-    const T d2udxy = (u[8] - u[6] - u[5] + u[3]) * i_r20 * i_t20 * i_r1;
+    const T d2udxy = (u[8] - u[6] - u[5] + u[3]) * i_r20 * i_t20;  // times i_r1
+    const T d2udy2 = mad(u[7] - u[1], i_t21, (u[4] - u[1]) * i_t10) * i_ht20 * i_r1;  // times i_r1
     const T dndy = (nr[7] - nr[4]) * i_t20 * i_r1;
+    const T shear = mad(v[2] - v[0], i_r20, dudy);  // dudy + dvdx
 
     const T sxx = 2.0 * nr[1] * dudx;
-    T fx = 2.0 * dndx * dudx + 2.0 * nr[1] * d2udx2 + sxx * i_r1;
-    const T syy = 2.0 * nr[1] * (dvdy + u[1] * i_r1);
-    const T sxy = nr[1] * (dudy + dvdx - v[1] * i_r1);
-    T fy = 2.0 * dndy * dvdy + 2.0 * nr[1] * d2vdy2 + 2.0 * nr[1] * dudy * i_r1 + 2.0 * dndy * u[1] * i_r1;
-    fx += dndy * (dudy + dvdx) + nr[1] * (d2udy2 + d2vdxy) - dndy * v[1] * i_r1 - nr[1] * dvdy * i_r1 - syy * i_r1;
-    fy += dndx * (dudy + dvdx) + nr[1] * (d2udxy + d2vdx2) - dndx * v[1] * i_r1 - nr[1] * dvdx * i_r1 +
-          nr[1] * v[1] * i_r1 * i_r1 + 2.0 * sxy * i_r1;
+    T fx = mad(2.0 * dndx, dudx, mad(2.0 * nr[1], d2udx2, sxx * i_r1));
+    const T syy = 2.0 * nr[1] * mad(u[1], i_r1, dvdy);
+    const T sxy = nr[1] * mad(-v[1], i_r1, shear);
+    T fy = mad(2.0 * dndy, dvdy, mad(2.0 * nr[1], d2vdy2, mad(2.0 * nr[1] * dudy, i_r1, 2.0 * dndy * u[1] * i_r1)));
+    fx = mad(dndy, shear, fx);
+    fx = mad(nr[1], mad(d2udy2, i_r1, d2vdxy), fx);
+    fx = mad(-(dndy * v[1]), i_r1, fx);
+    fx = mad(-(nr[1] * dvdy), i_r1, fx);
+    fx = mad(-syy, i_r1, fx);
+    fy = mad(dndx, shear, fy);
+    fy = mad(nr[1], mad(d2udxy, i_r1, d2vdx2), fy);
+    fy = mad(-(dndx * v[1]), i_r1, fy);
+    fy = mad(-(nr[1] * dvdx), i_r1, fy);
+    fy = mad(nr[1] * v[1] * i_r1, i_r1, fy);
+    fy = mad(2.0 * sxy, i_r1, fy);
     fx_out = fx;
     fy_out = fy;
 }

@@ -64,10 +64,10 @@ __device__ __forceinline__ Grav gravity_at(const DiskView& d, double gstar, doub
         g.gz = -0.0;
         if (d.nplanet > 0) {
             const double plm = p.m, plx = p.x;
-            const double ir = rsq(rad * rad + plx * plx - 2.0 * plx * rad * cosfac + p.rs * p.rs);
-            const double rs_fac = ir * ir * ir;
-            g.gx += -plm * (rad - plx * cosfac) * rs_fac - plm * cosfac * iplx2;
-            g.gy += -plm * plx * sinfac * rs_fac + plm * sinfac * iplx2;
+            const double ir = rsq(mad(-2.0 * plx * rad, cosfac, mad(rad, rad, mad(plx, plx, p.rs * p.rs))));
+            const double pull = plm * (ir * ir * ir), ind = plm * iplx2;
+            g.gx = mad(-ind, cosfac, mad(-pull, mad(-plx, cosfac, rad), g.gx));
+            g.gy = mad(ind, sinfac, -(pull * plx * sinfac));
         }
     }
     return g;
@@ -125,29 +125,20 @@ __device__ __forceinline__ Cell kick(const DiskView& d, const Cell& C, double ix
     Cell T = C;
     const double ir = VISC ? inv(C.r) : 0.0;  // T.r == C.r throughout
     double fx = (d.geomx == 1) ? T.v * T.v * ix : 0.0;
-    double fy = 0.0;
-    const double fz = 0.0;
-    if (VISC) {
-        fx += vx * ir;
-        if (d.ndim > 1) fy += vy * ir;
-    }
+    const double fy = VISC ? vy * ir : 0.0, fz = 0.0;  // stress in 2D only
+    if (VISC) fx = mad(vx, ir, fx);
     if (mdt != 0.0) {
-        T.u = C.u + fx * mdt + g.gx * mdt;
-        T.v = C.v + fy * mdt + g.gy * mdt;
-        T.w = C.w + fz * mdt + g.gz * mdt;
+        T.u = mad(g.gx, mdt, mad(fx, mdt, C.u));
+        T.v = mad(g.gy, mdt, mad(fy, mdt, C.v));
         if (Tu) *Tu = T.u;  // the gas velocity the dust drag relaxes towards (sweeps.cu:679-687)
         if (Tv) *Tv = T.v;
         fx = (d.geomx == 1) ? T.v * T.v * ix : 0.0;
-        fy = 0.0;
-        if (VISC) {
-            fx += vx * ir;
-            if (d.ndim > 1) fy += vy * ir;
-        }
+        if (VISC) fx = mad(vx, ir, fx);
     }
     Cell o;
-    o.u = C.u + fx * dt + g.gx * dt;
-    o.v = C.v + fy * dt + g.gy * dt;
-    o.w = C.w + fz * dt + g.gz * dt;
+    o.u = mad(g.gx, dt, mad(fx, dt, C.u));
+    o.v = mad(g.gy, dt, mad(fy, dt, C.v));
+    o.w = mad(g.gz, dt, mad(fz, dt, C.w));
     o.r = C.r;
     o.p = C.p;
     return o;
@@ -174,8 +165,8 @@ __device__ __forceinline__ double signal_rate(const DiskView& d, const Cell& c, 
     if (dc) spd = fmax(fabs(dc->u), spd);
     double tmp = fmax(spd * d.idx_x[i], 0.0);
     if (d.ndim > 1) {
-        spd = fabs(c.v - rad_cyl * d.frame_omega - d.rot[i]) + cs;
-        if (dc) spd = fmax(fabs(dc->v - rad_cyl * d.frame_omega - d.rot[i]), spd);
+        spd = fabs(mad(-rad_cyl, d.frame_omega, c.v) - d.rot[i]) + cs;
+        if (dc) spd = fmax(fabs(mad(-rad_cyl, d.frame_omega, dc->v) - d.rot[i]), spd);
         tmp = fmax(spd * (d.idx_y[j] * ((d.geomy == 3) ? d.irad[i] : 1.0)), tmp);
     }
     return tmp;
@@ -594,7 +585,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
             for (int m = 0; m < 4; ++m) up[m] = nx[m];
             uw = nw;
             fetch();
-            if (VISC) hi = row3(up[2], up[3], up[0] * c.nu);
+            if (VISC) hi = row3(up[2], up[3], __dmul_rn(up[0], c.nu));
         };
         fetch();
         if (VISC) {
@@ -646,7 +637,9 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
 // corrector re-uses its gravity.
 // PLAIN: no cooling, averages, dust or second body, whose code holds registers also where it
 // does not run: 1024x3072 158 us without that instance, 149 with it at 3 CTAs per SM, 147 at 4
-// (96 bytes spilled).  Kick 1, 87 us at 4 CTAs per SM either way and 92 at 5, has none.
+// (96 bytes spilled).  Kick 1, 87 us at 4 CTAs per SM either way and 92 at 5, has none.  The
+// gas's sums of products are added by mad: both instances give the same bits, so a disk that
+// averages or carries dust moves like one that does not.
 template <bool VISC, bool PLAIN>
 __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
     k_kick2(const Cell* __restrict__ in, const double* __restrict__ vis, const DiskView d, Cell* __restrict__ out,
@@ -714,7 +707,7 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
                     v = b;
                 }
             }
-            hi = row3(u, v, up[0] * c.nu);
+            hi = row3(u, v, __dmul_rn(up[0], c.nu));
         };
         fetch(jn);
         enter();
@@ -756,11 +749,11 @@ __global__ void __launch_bounds__(32 * SW_WARPS, PLAIN ? 4 : 3)
                     const double tau = d.killx[4 * i + 2 * side + 1];
                     if (tau > 0.0) {
                         const double f = d.killx[4 * i + 2 * side] * (dt / tau);
-                        Q.r += f * (I[0] - Q.r);
-                        Q.p += f * (I[1] - Q.p);
-                        Q.u += f * (I[2] - Q.u);
-                        Q.v += f * (I[3] - Q.v);
-                        if (!VISC) Q.w += f * (I[4] - Q.w);
+                        Q.r = mad(f, I[0] - Q.r, Q.r);
+                        Q.p = mad(f, I[1] - Q.p, Q.p);
+                        Q.u = mad(f, I[2] - Q.u, Q.u);
+                        Q.v = mad(f, I[3] - Q.v, Q.v);
+                        if (!VISC) Q.w = mad(f, I[4] - Q.w, Q.w);
                     }
                 }
             }
