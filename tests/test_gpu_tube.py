@@ -121,3 +121,25 @@ def test_tubes_made_and_run_by_several_threads():
     for g in out[:4]:
         for k in ("r", "p", "u"):
             assert np.array_equal(g[k], out[4][k]), k
+
+
+@pytest.mark.parametrize("n,transverse", [(94, True), (1024, False)])
+def test_averages_leave_the_tube_as_it_is(n, transverse):
+    """A tube that averages takes one launch per pass: the same bits and the same clock."""
+    from penguin_b200.disk import Disk
+
+    p = P.sod_tube(n)
+    st = state(n, n, transverse)
+    out = []
+    for average in (False, True):
+        d = Disk(p)
+        d.set_state(0.0, st)
+        if average:
+            d.set_average(0.1)
+        d.run(200)
+        d.check()
+        out.append((d.get_state(), d.clock()))
+        d.close()
+    assert out[0][1] == out[1][1]
+    for k in ("r", "p", "u", "v"):
+        assert np.array_equal(out[0][0][k], out[1][0][k]), k
