@@ -407,6 +407,8 @@ pg_status pg_test_div_1p5(const double* x, long long n, double* out2);
 /* test support: the kernels' reciprocal and reciprocal square root of x[0..n) (positive
    normal doubles), interleaved in out2[2n]. */
 pg_status pg_test_inv_rsq(const double* x, long long n, double* out2);
+/* test support: the FP32 kernels' (a b)^-1/2 of n pairs of positive normal floats, ab[2n]. */
+pg_status pg_test_root32(const float* ab, long long n, float* out);
 /* test support: one step with host t and dt, the whole cell array (ghosts
    included) after each pass into out[5][zarr][yarr][xarr]: kick1, sweep_x,
    sweep_y, sweep_z, kick2 with the damping.  Blocking. */

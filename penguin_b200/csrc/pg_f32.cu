@@ -1329,6 +1329,12 @@ __global__ void k32_init_tables(const View32 w, float* tx, float* ty, double* cs
     }
 }
 
+// test support: the edge states' root of a product
+__global__ void k32_test_root(const float* ab, long long n, float* out) {
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+        out[k] = rsq32_product(ab[2 * k], ab[2 * k + 1]);
+}
+
 // ============================================================== launchers
 static inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) / b); }
 
@@ -1467,3 +1473,17 @@ void launch_init_tables32(const View32& w, float* tx, float* ty, double* cs64, c
 
 }  // namespace f32
 }  // namespace pg
+
+extern "C" pg_status pg_test_root32(const float* ab, long long n, float* out) {
+    if (!ab || !out || n <= 0) return PG_ERR_ARG;
+    float* d = nullptr;
+    if (cudaMalloc(&d, 3 * n * sizeof(float)) != cudaSuccess) return PG_ERR_CUDA;
+    cudaError_t e = cudaMemcpy(d, ab, 2 * n * sizeof(float), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        pg::f32::k32_test_root<<<592, 256>>>(d, n, d + 2 * n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * n, n * sizeof(float), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? PG_OK : PG_ERR_CUDA;
+}

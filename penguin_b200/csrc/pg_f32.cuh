@@ -121,8 +121,15 @@ __device__ __forceinline__ float rsq32(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-// of a product of two floored states, which may leave the normal range
-__device__ __forceinline__ float rsq32_floor(float x) { return rsq32(fmaxf(x, 1.0e-37f)); }
+// (a b)^-1/2 of two positive states: where the product leaves the normal range (floored
+// edges of a nearly empty cell), root by root, which rounds once more
+__device__ __forceinline__ float rsq32_product(float a, float b) {
+    const float x = a * b;
+    constexpr unsigned lo = 0x01000000u, hi = 0x7f000000u;  // 2^-125, 2^127
+    float y = rsq32(x);
+    if (__float_as_uint(x) - lo > hi - lo) y = rsq32(a) * rsq32(b);
+    return y;
+}
 
 // recon.cu:216-378 + PPM.cu:64-91 with the centre value subtracted: am2..ap2 are
 // the neighbours' differences from the centre.  Sizes and signs as in recon (pg_hydro.cuh).
@@ -205,7 +212,7 @@ __device__ __forceinline__ HS edge32(float gam, float sx, float cs0, float rc, f
         p0d = pmin - pc;
     }
     const float g = gam * p0;
-    const float s = rsq32_floor(g * r0);
+    const float s = rsq32_product(g, r0);
     q = frac32(fminf((g * s + m) * sx, 1.0f));
     const float eu = ave(q, U) - u0d, ep = ave(q, P) - p0d;
     const float u_ = (SIDE == 0 ? -eu : eu) * (r0 * s);
@@ -232,14 +239,14 @@ __device__ __forceinline__ FX hllc32(float gam, float rref, float pref, const HS
     const float Lr = rref + L.rd, Rr = rref + R.rd;
     const float Lp = pref + L.pd, Rp = pref + R.pd;
     const float gl = gam * Lp, gr = gam * Rp;
-    const float cl = gl * rsq32_floor(gl * Lr), cr = gr * rsq32_floor(gr * Rr);
+    const float cl = gl * rsq32_product(gl, Lr), cr = gr * rsq32_product(gr, Rr);
     const float ic = rcp32(cl + cr);
     const float pbd = 0.5f * (R.pd + L.pd);
     const float pb = pref + pbd;
     const float x = gam * (L.u - R.u) * ic;
     const float pmd = (1.0f + x > 1.0e-6f) ? pbd + pb * x : pb * 1.0e-6f - pref;
     // Roe's averages through the ratio of the roots of the densities
-    const float q = Rr * rsq32_floor(Lr * Rr), iq = rcp32(1.0f + q);
+    const float q = Rr * rsq32_product(Lr, Rr), iq = rcp32(1.0f + q);
     const float u_ = (L.u + q * R.u) * iq;
     const float du = R.u - L.u;
     const float c2 = (cl * cl + cr * cr * q) * iq + 0.5f * q * (iq * iq) * (du * du);

@@ -1,4 +1,4 @@
-"""The FP64 kernels' reciprocal and reciprocal square root (pg_hydro.cuh)."""
+"""The kernels' reciprocals and reciprocal square roots (pg_hydro.cuh, pg_f32.cuh)."""
 import ctypes
 
 import numpy as np
@@ -26,3 +26,18 @@ def test_inv_and_rsq_within_two_ulp(lo, hi):
     xl = x.astype(np.longdouble)
     for got, want in ((out[0::2], 1 / xl), (out[1::2], 1 / np.sqrt(xl))):
         assert np.abs((got.astype(np.longdouble) - want) / want).max() <= 2.0**-51
+
+
+@pytest.mark.parametrize("lo,hi", [(-4.0, 4.0), (-60.0, 60.0), (-100.0, -50.0), (50.0, 100.0)])
+def test_root_of_a_product_in_fp32(lo, hi):
+    """(a b)^-1/2 of factors 2^U(lo, hi), also where a b leaves the normal range: there two roots
+    good to 2^-22.9 and the rounding of their product, else one root of a rounded product."""
+    from penguin_b200._lib import check, lib
+
+    rng = np.random.default_rng(6)
+    ab = (2.0 ** rng.uniform(lo, hi, (200000, 2))).astype(np.float32)
+    out = np.empty(len(ab), dtype=np.float32)
+    fp = ctypes.POINTER(ctypes.c_float)
+    check(lib().pg_test_root32(ab.ctypes.data_as(fp), len(ab), out.ctypes.data_as(fp)))
+    want = 1.0 / np.sqrt(ab[:, 0].astype(np.float64) * ab[:, 1])
+    assert np.abs(out / want - 1.0).max() <= 2.0 * 2.0**-22.9 + 2.0**-24
