@@ -60,7 +60,10 @@ HostCopy::~HostCopy() {
 
 cudaError_t copy_planes_out(HostCopy& h, int device, const double* src, double* const* dst, int planes, size_t count,
                             cudaStream_t s) {
-    bool staged = count * planes >= COPY_DIRECT;
+    // a per-thread stream is another one in every thread; arrays that overlap are written in the planes' order
+    bool staged = count * planes >= COPY_DIRECT && s != cudaStreamPerThread;
+    for (int f = 0; f < planes; ++f)
+        for (int g = 0; g < f; ++g) staged = staged && !(dst[f] < dst[g] + count && dst[g] < dst[f] + count);
     for (int f = 0; f < planes && staged; ++f) {  // page-locked and managed arrays are copied to directly
         cudaPointerAttributes at{};
         staged = cudaPointerGetAttributes(&at, dst[f]) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;

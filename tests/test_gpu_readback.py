@@ -37,6 +37,38 @@ def test_get_state_returns_what_was_set(size):
     d.close()
 
 
+def test_get_state_of_a_disk_on_the_per_thread_stream():
+    """Every host thread has a per-thread stream of its own: a large read on that stream is not
+    split over threads, and follows the steps queued before it."""
+    p = P.reference_disk(512, 1024)
+    st = I.disk_state(p, seed=4)
+    out = []
+    for stream in (None, 2):  # 2: cudaStreamPerThread
+        d = Disk(p, stream=stream)
+        d.set_state(0.0, st)
+        d.get_state()
+        d.run(60)
+        out.append(d.get_state())
+        d.close()
+    for k in ("r", "p", "u", "v"):
+        assert np.array_equal(out[0][k], out[1][k]), k
+
+
+def test_get_state_into_one_array_leaves_the_last_plane():
+    """A caller who wants one field may hand one array for the others: the planes are written in
+    their order."""
+    p = P.reference_disk(512, 1024)
+    st = I.disk_state(p, seed=4)
+    d = Disk(p)
+    d.set_state(0.0, st)
+    d.run(3)
+    g = d.get_state()
+    v, rest = np.zeros_like(g["v"]), np.zeros_like(g["r"])
+    check(lib().pg_disk_get_state(d._h, _ptr(rest), _ptr(rest), _ptr(rest), _ptr(v), None))
+    d.close()
+    assert np.array_equal(rest, g["u"]) and np.array_equal(v, g["v"])
+
+
 def test_get_state_3d_returns_what_was_set():
     p = P.cartesian_box(66, 61, 63)
     st = I.box_state(p, seed=3)
