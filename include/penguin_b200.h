@@ -240,7 +240,9 @@ pg_status pg_disk_check(pg_disk* d);
    prints it divided by q^2/h^2).  2D polar disks with a planet; FP64 with
    compensated per-thread sums; syncs. */
 pg_status pg_disk_torque(pg_disk* d, double* torque);
-/* Launch count of the library's own kernels per step (for reporting). */
+/* Launches of the library's own kernels in a step (for reporting).  1 for a tube that
+   has its own loop (1D cartesian, up to 7680 cells, no damping, cooling or averages):
+   one launch per pg_disk_solve; pg_disk_run takes up to 2048 steps with one. */
 int pg_kernels_per_step(const pg_disk* d);
 /* Runs nsteps of the device-resident loop launching the kernels one by one with
    CUDA events between them on the disk's stream; ms[k] receives the average

@@ -1274,6 +1274,7 @@ void sweep_launch_shape(int* threads, int* minb) {
 }
 
 int kernels_per_step(const DiskView& d) {
+    if (tube_applies(d)) return 1;  // at most: the device loop's launch takes many steps
     int n = 1 /*clock and planet table*/ + 1 /*kick1*/ + 1 /*sweep x*/ + 1 /*kick2*/;
     if (d.ndim > 1) n += 1;
     if (d.ndim > 1 && d.orbadv) n += 1;

@@ -143,3 +143,13 @@ def test_averages_leave_the_tube_as_it_is(n, transverse):
     assert out[0][1] == out[1][1]
     for k in ("r", "p", "u", "v"):
         assert np.array_equal(out[0][0][k], out[1][0][k]), k
+
+
+@pytest.mark.parametrize("n,average,launches", [(1024, 0.0, 1), (7680, 0.0, 1), (7682, 0.0, 4), (1024, 0.1, 4)])
+def test_launches_of_a_step(n, average, launches):
+    from penguin_b200.disk import Disk
+
+    d = Disk(P.sod_tube(n))
+    d.set_average(average)
+    assert d.kernels_per_step == launches
+    d.close()
