@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(S3_THREADS, MB)
         const double cs2 = v.cs2[ic + d.xarr * k];
 #pragma unroll 1
         for (int j = j0; j < j1; j += S3_ROWS, ++n) {
-            if (!__all_sync(0xffffffffu, mbar_wait(&bar[n & 1], (uint32_t)((n >> 1) & 1), sc))) {
+            if (!warp_wait(&bar[n & 1], (uint32_t)((n >> 1) & 1), sc)) {
                 if (lane == 0 && j + S3_ROWS < j1) mbar_wait(&bar[(n + 1) & 1], (uint32_t)(((n + 1) >> 1) & 1), sc);
                 return;
             }

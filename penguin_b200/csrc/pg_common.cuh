@@ -129,7 +129,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 }
 // Bounded wait on a TMA completion: a tile lands in microseconds, so after 50 ms
 // the wait records PG_ERR_TIMEOUT, waits up to another 50 ms for the copy that
-// may still be in flight (the CTA must not leave with it pending) and returns
+// may still be in flight (the warp must not leave with it pending) and returns
 // false so the caller can exit.  A count of polls bounds both loops as well,
 // should the timer not advance.
 constexpr uint32_t MBAR_MAX_POLLS = 1u << 24;
@@ -253,18 +253,7 @@ __device__ __forceinline__ void block_max_to(unsigned long long* dst, double v) 
     }
 }
 
-// TMA pipeline of a persistent CTA with NS stages (NS - 1 tiles in flight while
-// one is computed): tile k computes from stage k % NS, barrier k % NS completes
-// phase (k / NS) & 1 when tile k has landed.
-template <int NS = 2>
-__device__ __forceinline__ void pipe_init(uint64_t* bar) {
-    if (threadIdx.x == 0) {
-        for (int n = 0; n < NS; ++n) mbar_init(&bar[n], 1);
-        fence_barrier_init();
-    }
-    __syncthreads();
-}
-// thread 0: one box into a stage (the stage's previous generic reads are ordered
+// one lane: one box into a stage (the stage's previous generic reads are ordered
 // before the async-proxy write by the fence)
 __device__ __forceinline__ void issue_box(double* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     tma_load_2d(dst, map, x, y, bar);
@@ -273,21 +262,9 @@ __device__ __forceinline__ void issue_begin(uint64_t* bar, uint32_t bytes) {
     fence_proxy_async();
     mbar_arrive_expect_tx(bar, bytes);
 }
-// every thread of the CTA gets the same answer, so a timed-out wait makes the
-// whole CTA leave together
-template <int NS = 2>
-__device__ __forceinline__ bool pipe_wait(uint64_t* bar, int k, Scalars* sc) {
-    const bool ok = mbar_wait(&bar[k % NS], (uint32_t)((k / NS) & 1), sc);
-    return __syncthreads_and(ok ? 1 : 0) != 0;
-}
-// after a timed-out wait: before the CTA leaves, wait (again bounded) for the
-// copies of tiles k+1 .. k+NS-1 that were issued (issued_ahead of them), so no
-// copy lands in released shared memory
-template <int NS = 2>
-__device__ __forceinline__ void pipe_drain(uint64_t* bar, int k, int issued_ahead, Scalars* sc) {
-    if (threadIdx.x == 0)
-        for (int m = 1; m <= issued_ahead && m < NS; ++m)
-            mbar_wait(&bar[(k + m) % NS], (uint32_t)(((k + m) / NS) & 1), sc);
+// A warp's wait for its own tile: false for all its lanes when it timed out, and the warp leaves
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, Scalars* sc) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, sc));
 }
 
 #ifdef __CUDACC__

@@ -209,10 +209,6 @@ __device__ __forceinline__ double* cell_at(const DiskView& d, Cell* out, int i, 
 // copy rate), so what counts is instructions: reciprocals and roots without their
 // IEEE tails (pg_hydro.cuh).
 
-// A warp's bounded wait for its own tile (mbar_wait: on a time-out the error word is set)
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, Scalars* sc) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, sc));
-}
 __device__ __forceinline__ double up1(double v) { return __shfl_up_sync(0xffffffffu, v, 1); }
 __device__ __forceinline__ double down1(double v) { return __shfl_down_sync(0xffffffffu, v, 1); }
 
@@ -1285,17 +1281,26 @@ int kernels_per_step(const DiskView& d) {
 }  // namespace pg
 
 namespace pg {
-// test support: the passes' bounded wait (pipe_wait) on a tile whose copy is
-// never issued: the stage's barrier expects `bytes` that nothing delivers, so
-// every thread gives up after the wait's limit, PG_ERR_TIMEOUT is recorded and
-// the CTA leaves together; nothing is in flight when it does.
+// test support: the radial sweeps' bounded wait on tiles whose copies are never issued: the
+// barriers of a warp's two stages expect `bytes` that nothing delivers, so the warp gives up
+// after the wait's limit, PG_ERR_TIMEOUT is recorded and it leaves as the sweeps' warps do,
+// after a wait for the other stage; nothing is in flight when it does.
 __global__ void k_test_bounded_wait(Scalars* sc, uint32_t bytes, int* left) {
-    __shared__ __align__(8) uint64_t bar[2];
-    pipe_init<2>(bar);
-    if (threadIdx.x == 0) issue_begin(&bar[0], bytes);
-    __syncthreads();
-    if (!pipe_wait<2>(bar, 0, sc)) {
-        pipe_drain<2>(bar, 0, 0, sc);
+    __shared__ __align__(8) uint64_t bars[2][2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t* bar = bars[warp];
+    if (lane == 0) {
+        mbar_init(&bar[0], 1);
+        mbar_init(&bar[1], 1);
+        fence_barrier_init();
+    }
+    __syncwarp();
+    if (lane == 0) {
+        issue_begin(&bar[0], bytes);
+        issue_begin(&bar[1], bytes);
+    }
+    if (!warp_wait(&bar[0], 0, sc)) {
+        if (lane == 0) mbar_wait(&bar[1], 0, sc);
         if (threadIdx.x == 0) *left = 1;
         return;
     }

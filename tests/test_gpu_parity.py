@@ -177,10 +177,10 @@ def test_error_word_reports_nan():
 
 
 def test_bounded_wait_gives_up_and_leaves_the_context_usable():
-    """A pass's wait on a tile copy that never lands (its barrier expects bytes
-    that no copy delivers) gives up after its limit instead of hanging: the
-    device error word reports PG_ERR_TIMEOUT, the CTA leaves through the
-    timed-out path, and the same context then steps a disk as before."""
+    """A radial sweep's wait on a tile copy that never lands (its barrier expects
+    bytes that no copy delivers) gives up after its limit instead of hanging: the
+    device error word reports PG_ERR_TIMEOUT, the warp waits for its other stage
+    and leaves, and the same context then steps a disk as before."""
     import ctypes
 
     from penguin_b200._lib import PG_ERR_TIMEOUT, check, lib
@@ -203,7 +203,7 @@ def test_bounded_wait_gives_up_and_leaves_the_context_usable():
     check(lib().pg_test_bounded_wait(ctypes.byref(err), ctypes.byref(left), ctypes.byref(ms)))
     assert err.value & (1 << PG_ERR_TIMEOUT), err.value
     assert left.value == 1
-    assert 45.0 <= ms.value < 2000.0, ms.value  # 50 ms, then up to 50 ms more
+    assert 45.0 <= ms.value < 2000.0, ms.value  # two stages: 50 ms, then up to 50 ms more, each
     after = five_steps()
     for k in _keys(p):
         assert np.array_equal(before[k], after[k]), k
