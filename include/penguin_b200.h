@@ -403,9 +403,9 @@ pg_status pg_disk3_read_snapshot(pg_disk3* d, const char* path, double* t_out);
    left through the timed-out path; ms: the kernel's duration (for each of a
    warp's two stages 50 ms, then up to 50 ms more for copies in flight). */
 pg_status pg_test_bounded_wait(int* err_bits, int* left, float* ms);
-/* test support: out2[2k] = the kernels' division-free x[k] / 1.5, out2[2k+1] =
-   the IEEE quotient, for n host values.  Uses the GPU. */
-pg_status pg_test_div_1p5(const double* x, long long n, double* out2);
+/* test support: the kernels' factors of a parabola's average over the fraction x[k] of
+   a cell: out2[2k] = x/2, out2[2k+1] = 1 - x/1.5. */
+pg_status pg_test_frac(const double* x, long long n, double* out2);
 /* test support: the kernels' reciprocal and reciprocal square root of x[0..n) (positive
    normal doubles), interleaved in out2[2n]. */
 pg_status pg_test_inv_rsq(const double* x, long long n, double* out2);

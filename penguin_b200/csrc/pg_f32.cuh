@@ -149,7 +149,6 @@ struct Frac32 {
     float h, g;  // x/2, 1 - x/1.5 for the swept fraction x (PPM.cu:95-113)
 };
 __device__ __forceinline__ Frac32 frac32(float x) { return {0.5f * x, 1.0f - x * (2.0f / 3.0f)}; }
-__device__ __forceinline__ float lim01f(float a) { return fminf(fmaxf(a, 0.0f), 1.0f); }
 __device__ __forceinline__ float aveL32(const Frac32& f, const Par32& p) {
     const float a6 = 3.0f * (p.sL - p.sR);
     return -p.sL + f.h * ((p.sR + p.sL) + f.g * a6);

@@ -99,17 +99,6 @@ struct FracT {
     T h, g;
 };
 using Frac = FracT<double>;
-// x / 1.5 correctly rounded without a division: with y = RN(1/1.5) = RN(2/3),
-// q = RN(x y) lies within an ulp of x / 1.5 and the remainder x - 1.5 q is
-// exact in one FMA, so RN(q + (x - 1.5 q) y) is the correctly rounded quotient
-// (Markstein, IBM J. Res. Dev. 34 (1990) 111-119); 2x/3 is never a midpoint of
-// two doubles.  Bit for bit the IEEE quotient x / 1.5.
-__device__ __forceinline__ double div_1p5(double x) {
-    constexpr double y = 2.0 / 3.0;
-    const double q = x * y;
-    const double r = fma(-q, 1.5, x);
-    return copysign(fma(r, y, q), x);  // the quotient of a positive divisor keeps x's sign (-0 / 1.5 = -0)
-}
 // of the swept fraction y of the cell at the edge (1 - x / 1.5 in one FMA: within
 // an ulp of 1 of the rounded quotient's)
 template <class T>

@@ -1307,12 +1307,12 @@ __global__ void k_test_bounded_wait(Scalars* sc, uint32_t bytes, int* left) {
     if (threadIdx.x == 0) *left = 2;  // the copy "landed": not expected
 }
 
-// test support: div_1p5 (pg_hydro.cuh) against the IEEE quotient x / 1.5
-__global__ void k_test_div_1p5(const double* x, long long n, double* out) {
+// test support: frac (pg_hydro.cuh)
+__global__ void k_test_frac(const double* x, long long n, double* out) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x) {
-        const double a = x[k];
-        out[2 * k] = div_1p5(a);
-        out[2 * k + 1] = __ddiv_rn(a, 1.5);
+        const Frac f = frac(x[k]);
+        out[2 * k] = f.h;
+        out[2 * k + 1] = f.g;
     }
 }
 // test support: inv and rsq (pg_hydro.cuh)
@@ -1374,8 +1374,8 @@ static pg_status test_pairs(void (*kernel)(const double*, long long, double*), c
     cudaFree(dout);
     return e == cudaSuccess ? PG_OK : PG_ERR_CUDA;
 }
-extern "C" pg_status pg_test_div_1p5(const double* x, long long n, double* out2) {
-    return test_pairs(pg::k_test_div_1p5, x, n, out2);
+extern "C" pg_status pg_test_frac(const double* x, long long n, double* out2) {
+    return test_pairs(pg::k_test_frac, x, n, out2);
 }
 extern "C" pg_status pg_test_inv_rsq(const double* x, long long n, double* out2) {
     return test_pairs(pg::k_test_inv_rsq, x, n, out2);
