@@ -167,9 +167,7 @@ __device__ __forceinline__ Cell increments(const DiskView& d, const Flux& a, dou
 
 // Radial sweep (sweeps.cu:263-335) of rows j of one plane k: 4 rows of 36 cells per TMA
 // copy, two copies in flight per warp; lane l holds cell 2 + 30 seg + l.  Compiled for MB
-// CTAs per SM: 3 (168 registers) when warps are few and each runs alone on its scheduler, 4
-// (128 registers, some spilled) when there are rows enough for all: 48x40x36 13.0 / 14.4 us,
-// 128x256x72 166 / 143 us at 3 / 4.
+// CTAs per SM, 3 (168 registers) or 4 (128, some spilled): create3 picks.
 template <int MB>
 __global__ void __launch_bounds__(S3_THREADS, MB)
     k3_sweep_x(const __grid_constant__ CUtensorMap tm, const View3 v, Cell* __restrict__ out, int nseg, int len,
@@ -689,7 +687,7 @@ struct Engine3 {
     bool pending = false;
     bool fresh = true;
     // of each sweep: CTAs, warps across the radius, rows of a run, runs per line, runs
-    bool dense = false;  // the radial sweep's instance
+    bool dense = false;  // the radial sweep's instance: 4 CTAs per SM, else 3
     unsigned grid_sweep[3] = {0, 0, 0};
     int across[3], len[3], chunks[3], items[3];
     unsigned grid_kick = 0;
@@ -976,11 +974,23 @@ static pg_status create3(const pg_params* P, int device, cudaStream_t stream, En
         return bad(fail3(PG_ERR_CUDA, "table kernel failed"));
     for (int b = 0; own && b < 2; ++b)
         if ((s = make_maps(*E, b)) != PG_OK) return bad(s);
-    // rows enough for eight a warp at 4 CTAs per SM
-    E->dense = (long long)((Q.xres + S3_OUT - 1) / S3_OUT) * Q.yres * Q.zres >= 8ll * 4 * S3_WARPS * 148;
+    // The radial sweep at 3 CTAs per SM is 1 to 10 % faster than at 4 with its spills (us:
+    // 48x40x36 13.2 / 14.6, 96x192x54 68 / 75, 192x384x108 409 / 429), unless its runs fill
+    // their last wave so badly that the other count's finer waves win (128x256x72 166 / 143,
+    // 96x96x96 69 / 64): by run_cost, with a wave's time proportional to its warps, those are
+    // the grids where 4 looks better by 3.5 % or more (0.957 and 0.962; 120x112x112, 0.948, loses 2.5 %).
+    double cost[2];
+    for (int k = 0; k < 2; ++k) {
+        const void* f = k == 0 ? (const void*)k3_sweep_x<3> : (const void*)k3_sweep_x<4>;
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
+        cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        const long long fit = S3_WARPS * (long long)occupancy_grid(f, S3_THREADS, S3_SMEM, 1ll << 40);
+        const long long lines = (long long)((Q.xres + S3_OUT - 1) / S3_OUT) * Q.zres;
+        const int len = run_length(lines, Q.yres, fit, 1.5);
+        cost[k] = (double)fit * run_cost(lines * ((Q.yres + len - 1) / len), fit, len + 1.5);
+    }
+    E->dense = cost[1] < 0.965 * cost[0];
     const void* sweep_x = E->dense ? (const void*)k3_sweep_x<4> : (const void*)k3_sweep_x<3>;
-    cudaFuncSetAttribute(sweep_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S3_SMEM);
-    cudaFuncSetAttribute(sweep_x, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     const int along[3] = {Q.yres, Q.yres, Q.zres};  // rows a run is cut from
     const int lines[3] = {Q.zres, Q.zres, Q.yres};
     for (int a = 0; a < 3; ++a) {

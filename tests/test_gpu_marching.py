@@ -129,7 +129,8 @@ def test_fp32_tracks_fp64(size, dust):
             assert np.abs(got[k] - ref[k]).sum() < 1e-4 * np.abs(ref[k] - start[k]).sum(), k
 
 
-@pytest.mark.parametrize("size", [(28, 9, 7), (30, 8, 12), (32, 13, 9), (34, 7, 8), (62, 6, 10)],
+# the last: the radial sweep's other instance (create3, pg_3d.cu)
+@pytest.mark.parametrize("size", [(28, 9, 7), (30, 8, 12), (32, 13, 9), (34, 7, 8), (62, 6, 10), (96, 96, 96)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_box_matches_oracle(size):
     """Uniform cartesian cells leave only rounding: the 40 passes of 8 steps round a cell to
