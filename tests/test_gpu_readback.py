@@ -11,6 +11,7 @@ from penguin_b200 import params as P
 from penguin_b200._lib import check, lib
 from penguin_b200.disk import Disk
 from penguin_b200.disk3 import Disk3
+from penguin_b200.ensemble import Ensemble
 
 pytestmark = pytest.mark.gpu
 
@@ -67,6 +68,34 @@ def test_get_state_into_one_array_leaves_the_last_plane():
     check(lib().pg_disk_get_state(d._h, _ptr(rest), _ptr(rest), _ptr(rest), _ptr(v), None))
     d.close()
     assert np.array_equal(rest, g["u"]) and np.array_equal(v, g["v"])
+
+
+# three planes of 8 MB and more
+@pytest.mark.parametrize("size", [(592, 591), (1030, 777)], ids=lambda s: f"{s[0]}x{s[1]}")
+def test_dust_and_ensemble_reads_return_what_was_set(size):
+    """FP64 dust as set; FP32 members to the residuals' rounding, 2^-24 of the deviation from the
+    initial disk (below 2 in all fields here)."""
+    p = P.dust_disk(*size)
+    st = I.disk_state(p, seed=3)
+    d = Disk(p)
+    d.set_state(0.0, st)
+    dust = d.get_dust()
+    rng = np.random.default_rng(1)
+    dust = {k: v * (1.0 + 1e-3 * rng.uniform(-1, 1, v.shape)) for k, v in dust.items()}
+    d.set_dust(dust)
+    g = d.get_dust()
+    d.close()
+    for k in ("r", "u", "v"):
+        assert np.array_equal(g[k], dust[k]), k
+    e = Ensemble([p, P.planet_disk(64, 96)])
+    e.set_state(0, 0.0, st)
+    e.set_dust(0, dust)
+    for _ in range(2):
+        g, q = e.get_state(0), e.get_dust(0)
+        for k in ("r", "u", "v"):
+            assert np.abs(g[k] - st[k]).max() < 2.0 * 2.0 ** -24, k
+            assert np.abs(q[k] - dust[k]).max() < 2.0 * 2.0 ** -24, k
+    e.close()
 
 
 def test_get_state_3d_returns_what_was_set():

@@ -70,7 +70,7 @@ def test_tube_loop_boundaries_and_equations_of_state(lft, rgh, eos, ie):
 
 def test_tube_loop_stops_at_its_end_time():
     """The step that crosses end_time is clipped, later launches do nothing, and the
-    next run starts from the step the clip replaced (more steps than one launch takes)."""
+    next run starts from the step the clip replaced."""
     from penguin_b200.disk import Disk
 
     p = P.sod_tube(1024)
@@ -86,8 +86,42 @@ def test_tube_loop_stops_at_its_end_time():
     a, b = d.get_state(), h.get_state()
     for k in ("r", "p", "u"):
         assert np.array_equal(a[k], b[k]), k
-    d.run(5000, end_time=0.6)
-    assert d.clock()[0] == pytest.approx(0.6, abs=1e-15) or d.clock()[2] == n + 5000
+    d.run(100000, end_time=0.3)
+    t, dt, m = d.clock()
+    assert t == pytest.approx(0.3, abs=1e-15) and m > n
+    d.check()
+    d.close()
+    h.close()
+
+
+@pytest.mark.parametrize("finite", [False, True])
+def test_tube_loop_longer_than_a_launch(finite):
+    """A launch takes up to 2048 steps and hands state, clock and signal rate to the next: 4100
+    steps (without an end time), or as many as an end time after some 2500 takes, against the same
+    steps launched one by one with the host's clock, bit for bit."""
+    from penguin_b200.disk import Disk
+
+    p = P.sod_tube(90)
+    st = state(90, 4, False)
+    end = 1.0e30
+    if finite:
+        h = Disk(p)
+        h.set_state(0.0, st)
+        h.step_host(2500)
+        end = h.t + 0.5 * h.dt
+        h.close()
+    d, h = Disk(p), Disk(p)
+    for x in (d, h):
+        x.set_state(0.0, st)
+    steps = 100000 if finite else 4100
+    d.run(steps, end_time=end)
+    nh = h.step_host(steps, end)
+    t, dt, n = d.clock()
+    assert n == nh and n > 2048 and (not finite or n < 4096)
+    assert t == h.t and dt == h.dt
+    a, b = d.get_state(), h.get_state()
+    for k in ("r", "p", "u"):
+        assert np.array_equal(a[k], b[k]), k
     d.check()
     d.close()
     h.close()
