@@ -13,8 +13,7 @@
 //                    (src/killwave/killwave.cu:17-103) and the CFL signal rate
 //                    (src/timestep/timestep.cu:18-97, ndim 3)
 //
-// plus the one-thread clock kernel and the per-row planet angle table of the 2D
-// form.  Lanes of a warp lie along the radius in every pass.  The radial sweep stages
+// plus the 2D form's one-block kernel of the clock and the per-row planet angles.  Lanes of a warp lie along the radius in every pass.  The radial sweep stages
 // rows with TMA and exchanges edge states and fluxes between lanes by shuffle; the
 // azimuthal and polar sweeps march along their direction with five cells of a column in
 // registers (the 2D form's work layout, pg_kernels.cu, and its building blocks,
@@ -256,9 +255,9 @@ __global__ void __launch_bounds__(S3_THREADS, MB)
 // Azimuthal (DIR 1, sweeps.cu:361-433) and polar (DIR 2, :458-554) sweeps: a lane marches
 // along its column with five cells in registers and the next in flight, like the 2D
 // azimuthal sweep.  Lines of a plane k (DIR 1) or of a row j (DIR 2).  128x256x72, us a
-// sweep, tiles -> runs: radial 250 -> 143, azimuthal 249 -> 132, polar 363 -> 146; FP64 issue
-// and latency bound all three.  At 2 / 3 / 4 CTAs per SM azimuthal 153 / 132 / 163, polar
-// 165 / 146 / 170.
+// sweep, tiles -> runs: radial 250 -> 143, azimuthal 249 -> 133, polar 363 -> 144; FP64 issue
+// and latency bound all three.  At 2 / 3 / 4 CTAs per SM azimuthal 150 / 133 / 164, polar
+// 165 / 144 / 167.
 template <int DIR>
 __global__ void __launch_bounds__(S3_THREADS, 3)
     k3_march(const Cell* __restrict__ in, const View3 v, Cell* __restrict__ out, int ncol, int len, int nchunk,

@@ -20,7 +20,7 @@ namespace pg {
 // or stay in registers from the row before (azimuthal passes), no barrier and no shared
 // memory.  Bound by FP64 issue and latency; with tiles of 32 x 4 cells whose phases met at
 // barriers the sweeps and the advection of gas and dust took 133 us at 384x1024, with these
-// 100.  Compiled for 4 CTAs per SM: at 5 the azimuthal sweep spills (38 -> 41 us with the
+// 103.  Compiled for 4 CTAs per SM: at 5 the azimuthal sweep spills (38 -> 41 us with the
 // gas's, the advection 28 -> 30).  The w velocity is identically zero (dust runs in 2D) and
 // stays as it is.
 constexpr int DS_WARPS = 4;  // warps per CTA, independent of one another

@@ -1644,7 +1644,7 @@ pg_status pg_recon_weights(const pg_params* P, int dir, double* w) {
 }
 
 pg_status pg_sweep_variant(int v, int* out6) {
-    if (v < 0 || v >= NSWEEP_VARIANTS || !out6) return fail(PG_ERR_ARG, "no such tile variant");
+    if (v < 0 || v >= NSWEEP_VARIANTS || !out6) return fail(PG_ERR_ARG, "no such variant");
     out6[0] = 32;                 // neighbouring radii of a warp
     out6[1] = SWEEP_LENGTHS[v];   // rows it takes (0: by the grid's size)
     out6[2] = SWEEP_LENGTHS[v];   // ... one after the other in each thread
@@ -1658,7 +1658,7 @@ pg_status pg_disk_set_tuning(pg_disk* dk, const int* choice) {
     Tune t;
     for (int k = 0; k < 3; ++k) {
         if (choice[k] < 0 || choice[k] >= NSWEEP_VARIANTS)
-            return fail(PG_ERR_ARG, "no such tile variant for this pass");
+            return fail(PG_ERR_ARG, "no such variant");
         t.v[k] = choice[k];
     }
     for (int k = 0; k < 5; ++k) {

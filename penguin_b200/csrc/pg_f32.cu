@@ -28,11 +28,11 @@ namespace f32 {
 // No shared memory and no barrier: tiles whose phases met at __syncthreads spent half
 // their instructions on table loads, tile addresses and the exchange, and waited on
 // barriers and L1 for most of the rest (55 % of issue slots at 1024x3072).  There, us a
-// pass, tiles -> runs: kick1 75 -> 53, sweep_x 148 -> 78, sweep_y 135 -> 70, advection
+// pass, tiles -> runs: kick1 75 -> 53, sweep_x 148 -> 82, sweep_y 135 -> 72, advection
 // 81 -> 39, kick2 140 -> 84; what bounds them is instruction issue.  All are compiled for 5
-// CTAs of 4 warps per SM; at 3 / 4 / 6 / 7 kick1 takes 80 / 85 / 67 / 74, sweep_x
-// 102 / 101 / 84 / 88, sweep_y 74 / 74 / 78 / 83, kick2 98 / 103 / 120 / 126, and the
-// advection at 4 / 6 / 7 39 / 43 / 43.
+// CTAs of 4 warps per SM; at 3 / 4 / 6 / 7 kick1 takes 78 / 78 / 66 / 73, sweep_x
+// 99 / 100 / 90 / 93, sweep_y 78 / 78 / 82 / 87, kick2 99 / 107 / 122 / 133, and the
+// advection 39 / 39 / 43 / 45.
 constexpr int MW = 4, MT = 32 * MW;  // warps of a CTA, independent of one another
 
 __device__ __forceinline__ float up1(float v) { return __shfl_up_sync(0xffffffffu, v, 1); }
@@ -1391,8 +1391,8 @@ int pass_occupancy32(int pass) {
 // Long runs waste little on the rows that only feed the stencils at their ends and on the
 // tables they load, short ones give the warps that hide latency: per kind the length with
 // the least run_cost (pg_internal.h) at 20 resident warps an SM.  1024x3072, us a pass at
-// 4 / 16 / 24 / 48 / 96 rows: radial sweep 92 / 90 / 90 / 90 / 128, azimuthal
-// 120 / 103 / 101 / 105 / 155, kick2 131 / 120 / 116 / 111 / 194.
+// 4 / 8 / 16 / 24 / 48 / 96 rows: radial sweep 82 / 78 / 77 / 85 / 80 / 115, azimuthal
+// 96 / 82 / 73 / 74 / 76 / 98, kick2 105 / 90 / 88 / 89 / 82 / 128; by the rule 82, 72, 84.
 // Variant 1 is half as long, for the autotuner to try.
 void build_runs32(const int* xres, const int* yres, int nd, std::vector<int4>* runs, Runs32* R) {
     runs->clear();

@@ -70,7 +70,7 @@ enum YSlot {
     Y_VISY = 8,  // 4 viscous-stencil reciprocals per j
     Y_NSLOT = 12
 };
-// Per-step planet table (k32_trig): rows [yn][6] = {sin, cos, 1-cos} of (phi - phi_p) for the
+// Per-step planet table (k32_time): rows [yn][6] = {sin, cos, 1-cos} of (phi - phi_p) for the
 // planet of the first half-kick, then of the planet at t+dt; columns [xn][2] = r - x_p for both;
 // then 8 scalars {m, x_p, rs^2, 1/x_p^2} x {first, second}.
 constexpr int TRIG_ROW = 6;

@@ -1,10 +1,18 @@
 // FP64 hydrodynamics building blocks of the Godunov sweep: 4th-order PPM
 // reconstruction, characteristic interface states, HLLC flux, conservative
-// update.  Expression order follows the reference line by line wherever it is
-// cited, so that results differ from it only at the rounding level; the one
-// deliberate change is that the 4th-order edge slopes use per-index linear
-// weights built once on the host instead of re-deriving 15 grid moments and 56
-// divisions per call.
+// update.  They compute what the cited lines of the reference compute and differ
+// from it at the rounding level, but not in its order: the 4th-order edge slopes
+// use per-index linear weights built once on the host instead of re-deriving 15
+// grid moments and 56 divisions per call, the slopes are limited by their sizes,
+// swept fractions come from the speeds, and quotients and roots are products of
+// inv and rsq (2 ulp).
+//
+// Range: a cell's density times its pressure and the densities of neighbours are
+// multiplied where the reference divides them, so the products have to be normal
+// doubles, 2^-1022 to 2^1024.  Every update floors density and pressure at 1e-10:
+// only a state the caller sets can leave that range, and gives a NaN that the error
+// word reports.  Roots taken factor by factor outside it, behind a test of the
+// product's exponent, cost 6.5 % of a step at 1024x3072 (532 -> 567 us).
 //
 // The functions are templates on the scalar type T: the sweeps instantiate
 // them with double, the adjoint kernels with dual numbers (pg_dual.cuh).
@@ -41,8 +49,8 @@ __device__ __forceinline__ auto mad(const A& a, const B& b, const C& c) {
     return a * b + c;
 }
 
-// Reciprocal (of either sign) and reciprocal square root of a normal double to about an
-// ulp: the hardware's approximation (rcp/rsqrt.approx.ftz.f64, which reads and
+// Reciprocal (of either sign) and reciprocal square root of a normal double within two
+// ulp (NaN at zero and infinity): the hardware's approximation (rcp/rsqrt.approx.ftz.f64, which reads and
 // returns the upper 32 bits of a double, so |e| < 2^-19) and one third-order step
 // of Newton's iteration (Householder, "The Numerical Treatment of a Single
 // Nonlinear Equation", 1970): with e = 1 - x y, y (1 + e + e^2) is off by e^3, and

@@ -33,11 +33,11 @@ namespace pg {
 // states and fluxes through shared memory spent 900-1000 instructions a cell, 350 of
 // them FP64, and a quarter of their time at the barriers; the sweeps spend 720-770 now.
 // What is left to bound them is FP64 issue and latency: the FP64 pipe is 57-60 % busy in
-// the sweeps, at a third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1 108 -> 88, sweep_x 298 -> 123,
-// sweep_y 328 -> 123, advection 154 -> 72, kick2 177 -> 147.
-// Each kernel is compiled for the CTAs per SM that were fastest there: sweep_x at 3 / 4 / 5
-// 123 / 129 / 151, sweep_y 123 / 139 / 246, advection at 4 / 5 / 6 72 / 72 / 115 (adiabatic
-// 512x1536: 26 / 32 / 43), kick1 at 3 / 4 / 5 106 / 88 / 104, kick2 at 2 / 3 / 4 201 / 160 / 182.
+// the sweeps, at a third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1
+// 108 -> 88, sweep_x 298 -> 124, sweep_y 328 -> 123, advection 154 -> 71, kick2 177 -> 142.
+// Each kernel is compiled for the CTAs per SM that were fastest there, at 2 / 3 / 4 / 5:
+// sweep_x 134 / 124 / 128 / 149, sweep_y 148 / 123 / 138 / 246, advection 76 / 76 / 71 / 72
+// (adiabatic 512x1536: 26.5 / 26.2 / 25.7 / 31.6), kick1 139 / 106 / 88 / 100.
 constexpr int SW_WARPS = 4;                       // warps per CTA, independent of one another
 constexpr int RX_OUT = 30;                        // radial sweep: outputs of a warp's 32 cells
 constexpr int RX_ROWS = RX_TILE_ROWS;             // rows per TMA copy
@@ -55,7 +55,7 @@ struct Grav {
 // Star + planet gravity in the 2D cylindrical frame (src/solver/force/forces.cu:41-58,
 // 182-327 with twobd_flag 0, pol = 0).  The star term is a per-radius table; the
 // planet's angle enters through the per-row sin/cos table of this step
-// (k_planet_trig) and 1/x_p^2 through the table's tail.
+// (planet_rows) and 1/x_p^2 through the table's tail.
 __device__ __forceinline__ Grav gravity_at(const DiskView& d, double gstar, double rad, double sinfac,
                                            double cosfac, double iplx2, const pg_body& p) {
     Grav g{0.0, 0.0, 0.0};
@@ -205,7 +205,7 @@ __device__ __forceinline__ double* cell_at(const DiskView& d, Cell* out, int i, 
 // ================================================================ sweeps
 // ISO: a 2D isothermal gas, which needs neither the energy flux nor the z-velocity
 // (identically zero in 2D): nothing is computed that the equation of state does not use.
-// The passes are bound by the latency and issue of their FP64 arithmetic (0.12 of the
+// The passes are bound by the latency and issue of their FP64 arithmetic (0.3 of the
 // copy rate), so what counts is instructions: reciprocals and roots without their
 // IEEE tails (pg_hydro.cuh).
 
@@ -632,8 +632,9 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
 // mdt = dt = dt/2) when it enters, with kick 1's stress and the bodies at t + dt; the
 // corrector re-uses its gravity.
 // PLAIN: no cooling, averages, dust or second body, whose code holds registers also where it
-// does not run: 1024x3072 158 us without that instance, 149 with it at 3 CTAs per SM, 147 at 4
-// (96 bytes spilled).  Kick 1, 87 us at 4 CTAs per SM either way and 92 at 5, has none.  The
+// does not run: 1024x3072 158 us with that code in, without it 191 / 150 / 142 / 183 at 2 / 3 /
+// 4 / 5 CTAs per SM (at 4 96 bytes are spilled); the general instance, averaging, 260 / 210 / 239
+// at 2 / 3 / 4.  Kick 1 has no such instance (87 us with and without that code).  The
 // gas's sums of products are added by mad: both instances give the same bits, so a disk that
 // averages or carries dust moves like one that does not.
 template <bool VISC, bool PLAIN>
@@ -1195,9 +1196,10 @@ static bool iso_2d(const DiskView& d) { return d.eos == 0 && d.ndim == 2; }
 static bool plain_kick(const DiskView& d) { return !d.cool && !d.ave && !d.dust && !d.twobd; }
 
 // Rows a warp of a pass takes one after the other: the tuned length, or the one of least
-// run_cost (pg_internal.h).  1024x3072, us a pass at 4 / 16 / 32 / 48 / 96 rows: radial
-// sweep 124 / 127 / 143 / 128 / 159, azimuthal 175 / 154 / 175 / 153 / 223 (2368 warps
-// fit: 48 rows are 2048 runs, 32 rows one and a third wave).
+// run_cost (pg_internal.h).  1024x3072, us a pass at 4 / 8 / 16 / 24 / 48 / 64 / 96 rows:
+// radial sweep 124 / 124 / 123 / 120 / 150 / 124 / 139, azimuthal 173 / 146 / 137 / 143 / 168 /
+// 137 / 171 (1776 warps fit: 48 rows are 2048 runs, a full wave and a sixth), advection 84 /
+// 82 / 78 / 77 / 74 / 90 / 124; with the rule's 64, 56 and 44 rows 124, 123 and 71.
 static int pass_length(const Tune* t, int k, const void* kernel, size_t smem, int lines, int rows, double extra) {
     const int len = (t && k >= 0) ? SWEEP_LENGTHS[t->v[k]] : 0;
     if (len > 0) return len;

@@ -2,12 +2,12 @@
 // cooling): many steps per launch, on one thread-block cluster.
 //
 // A tube's step is one sweep: without curvature, gravity and stress the half-kicks
-// add zeros.  As one launch per pass it takes 16 us whatever the size, launch gaps
+// add zeros.  As one launch per pass it takes 16 us up to 7682 cells, launch gaps
 // and the kernels' ramps, for work of under a microsecond.  Here every cell stays in
 // shared memory from step to step; a step costs the latency of one cell's
 // reconstruction, trace, HLLC flux and update plus one cluster barrier, which
-// publishes the edge cells and the signal rate.  Sod tube of 1024 cells to t = 0.2, us:
-// 24100 as launches, 3300 here.
+// publishes the edge cells and the signal rate: 3.7 us at 1024 cells, 3300 us for the
+// 897 steps of the Sod tube to t = 0.2.
 //
 // Layout: CTA k owns cells k m .. k m + m - 1 (m = 30 per warp) and holds three
 // more on either side, copies of its neighbours' cells or the tube's ghosts.  Lane l
@@ -279,7 +279,7 @@ int tube_max_cluster() {
 }
 
 // A tube whose half-kicks are identities, of a size that one cluster holds: 7680 cells with
-// 16 CTAs take 4.9 us a step, 1024 cells 3.4; 7682 as separate launches 16.4.
+// 16 CTAs take 4.9 us a step, 1024 cells 3.7; 7682 as separate launches 16.4.
 bool tube_applies(const DiskView& d) {
     int nc, warps;
     return d.ndim == 1 && d.geomx == 0 && !d.kill && !d.cool && !d.ave && !d.dust && !d.twobd && d.tube > 0 &&

@@ -1,7 +1,7 @@
-"""Grids whose sizes are not multiples of any tile: the last tile of every pass
-is partly outside the grid (TMA fills it, the kernels write only interior
-cells).  The CUDA path against the oracle on such grids, every tile variant
-against the default one bit for bit, the FP32-mixed form against FP64 and an
+"""Grids whose sizes are not multiples of any warp width or run length: the last
+warp of a row and the last run of a column are partly outside the grid (the kernels
+write only interior cells).  The CUDA path against the oracle on such grids, every run
+length against the default one bit for bit, the FP32-mixed form against FP64 and an
 ensemble of ragged members against their solo runs, and the 3D passes, whose
 boxes are ragged along all three axes here.  Needs a B200."""
 import numpy as np
@@ -10,7 +10,7 @@ import pytest
 from oracle.oracle import Oracle, Oracle3
 from penguin_b200 import initial as I
 from penguin_b200 import params as P
-from penguin_b200.disk import Disk, sweep_variant
+from penguin_b200.disk import Disk
 from penguin_b200.disk3 import Disk3
 from penguin_b200.ensemble import Ensemble
 
@@ -66,9 +66,8 @@ def test_ragged_disk_matches_oracle(size, full, bar):
 
 
 def test_ragged_disk_every_tile_variant_bitwise():
-    """Every tile variant the autotuner may choose (pencils per tile, pencil
-    length 16/32/64, cells per thread, TMA stages) gives the default variant's
-    result bit for bit when the tiles overhang the grid."""
+    """Every variant the autotuner may choose (the rows a warp takes) gives the default
+    one's result bit for bit when the last runs overhang the grid."""
     p = _disk(*RAGGED_2D[1])
     st = I.disk_state(p, seed=18)
     ref = Disk(p)
@@ -78,10 +77,9 @@ def test_ragged_disk_every_tile_variant_bitwise():
     a = ref.get_state()
     ref.close()
     for v in range(10):
-        vx = v if sweep_variant(v)["pencil_length"] + 6 <= 51 else 0  # radial boxes of at most 256 doubles
         forced = Disk(p)
         forced.set_state(T0, st)
-        forced.set_tuning(dict(zip(Disk.TUNING, (vx, v, v, 1, 1, 1, 1, 1))))
+        forced.set_tuning(dict(zip(Disk.TUNING, (v, v, v, 1, 1, 1, 1, 1))))
         forced.run(6)
         forced.sync()
         c = forced.get_state()
