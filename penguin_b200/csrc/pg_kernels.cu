@@ -65,9 +65,9 @@ __device__ __forceinline__ Grav gravity_at(const DiskView& d, double gstar, doub
         if (d.nplanet > 0) {
             const double plm = p.m, plx = p.x;
             const double ir = rsq(mad(-2.0 * plx * rad, cosfac, mad(rad, rad, mad(plx, plx, p.rs * p.rs))));
-            const double pull = plm * (ir * ir * ir), ind = plm * iplx2;
-            g.gx = mad(-ind, cosfac, mad(-pull, mad(-plx, cosfac, rad), g.gx));
-            g.gy = mad(ind, sinfac, -(pull * plx * sinfac));
+            const double rs_fac = ir * ir * ir;
+            g.gx = mad(-plm, mad(cosfac, iplx2, mad(-plx, cosfac, rad) * rs_fac), g.gx);
+            g.gy = plm * (sinfac * mad(-plx, rs_fac, iplx2));
         }
     }
     return g;
