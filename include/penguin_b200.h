@@ -162,7 +162,10 @@ pg_status pg_disk_destroy(pg_disk* d);
 pg_status pg_disk_dims(const pg_disk* d, int* xarr, int* yarr, int* npad);
 /* Restart injection from host arrays (yres x xres, x fastest), like load_grid
    (src/output/output.cu:182-248): ghosts take init_C, time is set to t.  v may
-   be NULL when ndim == 1.  Also initialises the planet at t (planet.cu:319). */
+   be NULL when ndim == 1.  Also initialises the planet at t (planet.cu:319).
+   The step multiplies a cell's density by its pressure and by its neighbours'
+   densities: the products have to be normal doubles (2^-1022 to 2^1024), or the
+   error word reports PG_ERR_NAN. */
 pg_status pg_disk_set_state(pg_disk* d, double t, const double* r, const double* p, const double* u,
                             const double* v);
 /* The newest state back to host arrays; t_out may be NULL. */
@@ -198,7 +201,9 @@ pg_status pg_disk_write_snapshot(pg_disk* d, const char* path, int average);
 pg_status pg_disk_read_snapshot(pg_disk* d, const char* path, double* t_out);
 /* ave_flag: the gas state averaged over a save interval by the trapezoid rule
    of main.cu:343-351, accumulated inside the step; interval <= 0: off.
-   reset = init_average after a save. */
+   reset = init_average after a save.  The state keeps its bits with and without
+   an average; a tube that averages takes one launch per pass (16 us a step)
+   instead of many steps per launch. */
 pg_status pg_disk_set_average(pg_disk* d, double interval);
 pg_status pg_disk_reset_average(pg_disk* d);
 pg_status pg_disk_get_average(pg_disk* d, double* r, double* p, double* u, double* v);
