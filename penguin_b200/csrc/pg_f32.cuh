@@ -122,7 +122,9 @@ __device__ __forceinline__ float rsq32(float x) {
     return y;
 }
 // (a b)^-1/2 of two positive states: where the product leaves the normal range (floored
-// edges of a nearly empty cell), root by root, which rounds once more
+// edges of a nearly empty cell), root by root.  That is off by 2^-21.8 at most (r.m.s.
+// 2^-24.0), the root of the product by 2^-22.4 (2^-24.4).  The test costs 1 % of the step at
+// 1024x3072 against a floor under the product, which gave such edges a wrong sound speed.
 __device__ __forceinline__ float rsq32_product(float a, float b) {
     const float x = a * b;
     constexpr unsigned lo = 0x01000000u, hi = 0x7f000000u;  // 2^-125, 2^127
