@@ -34,10 +34,10 @@ namespace pg {
 // them FP64, and a quarter of their time at the barriers; the sweeps spend 720-770 now.
 // What is left to bound them is FP64 issue and latency: the FP64 pipe is 57-60 % busy in
 // the sweeps, at a third of the copy rate.  1024x3072, us a pass, tiles -> runs: kick1
-// 108 -> 88, sweep_x 298 -> 124, sweep_y 328 -> 123, advection 154 -> 71, kick2 177 -> 142.
+// 108 -> 87, sweep_x 298 -> 124, sweep_y 328 -> 123, advection 154 -> 71, kick2 177 -> 140.
 // Each kernel is compiled for the CTAs per SM that were fastest there, at 2 / 3 / 4 / 5:
 // sweep_x 134 / 124 / 128 / 149, sweep_y 148 / 123 / 138 / 246, advection 76 / 76 / 71 / 72
-// (adiabatic 512x1536: 26.5 / 26.2 / 25.7 / 31.6), kick1 139 / 106 / 88 / 100.
+// (adiabatic 512x1536: 26.5 / 26.2 / 25.7 / 31.6), kick1 138 / 106 / 87 / 96.
 constexpr int SW_WARPS = 4;                       // warps per CTA, independent of one another
 constexpr int RX_OUT = 30;                        // radial sweep: outputs of a warp's 32 cells
 constexpr int RX_ROWS = RX_TILE_ROWS;             // rows per TMA copy
@@ -632,8 +632,8 @@ __global__ void __launch_bounds__(32 * SW_WARPS, 4)
 // mdt = dt = dt/2) when it enters, with kick 1's stress and the bodies at t + dt; the
 // corrector re-uses its gravity.
 // PLAIN: no cooling, averages, dust or second body, whose code holds registers also where it
-// does not run: 1024x3072 158 us with that code in, without it 191 / 150 / 142 / 183 at 2 / 3 /
-// 4 / 5 CTAs per SM (at 4 96 bytes are spilled); the general instance, averaging, 260 / 210 / 239
+// does not run: 1024x3072 158 us with that code in, without it 190 / 150 / 140 / 175 at 2 / 3 /
+// 4 / 5 CTAs per SM (at 4 92 bytes are spilled); the general instance, averaging, 260 / 209 / 244
 // at 2 / 3 / 4.  Kick 1 has no such instance (87 us with and without that code).  The
 // gas's sums of products are added by mad: both instances give the same bits, so a disk that
 // averages or carries dust moves like one that does not.
